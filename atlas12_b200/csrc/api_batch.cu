@@ -115,23 +115,23 @@ __global__ void __launch_bounds__(kRtSplitWarps * 32, 6) k_batch_rt_pre(const Rt
   if (!running(ctl, b)) return;
   rt_pre_body(args[b]);
 }
-__global__ void __launch_bounds__(kRtSolveThreads, kRtSolveMinBlocks) k_batch_rt_solve(const RtArgs* __restrict__ args,
+__global__ void __launch_bounds__(kScatterThreads, kScatterSolveMinBlocks) k_batch_rt_solve(const RtArgs* __restrict__ args,
                                                                                     const BatchCtl* ctl,
                                                                                     unsigned long long* work) {
   const int b = blockIdx.y;
   if (!running(ctl, b)) return;
   RtArgs a = args[b];
   a.work = work;
-  rt_solve_body(a);
+  scatter_solve_body<false>(rt_scatter_args(a));
 }
-__global__ void __launch_bounds__(kRtSolveThreads, kRtSeriesMinBlocks) k_batch_rt_series(const RtArgs* __restrict__ args,
+__global__ void __launch_bounds__(kScatterThreads, kScatterSeriesMinBlocks) k_batch_rt_series(const RtArgs* __restrict__ args,
                                                                                       const BatchCtl* ctl,
                                                                                       unsigned long long* work) {
   const int b = blockIdx.y;
   if (!running(ctl, b)) return;
   RtArgs a = args[b];
   a.work = work;
-  rt_series_body(a);
+  scatter_series_body<false>(rt_scatter_args(a));
 }
 __global__ void __launch_bounds__(kRtSplitWarps * 32, 4) k_batch_rt_post(const RtArgs* __restrict__ args,
                                                                         const BatchCtl* ctl) {
@@ -274,9 +274,9 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
       unsigned long long* work = work_counters(ctx, 3);
       {
         Timer t2(ctx, "batch_rt_solve");
-        k_batch_rt_series<<<dim3(sh.solve_blocks, nb), kRtSolveThreads, 0, s>>>(B->ra, B->d.ctl, work);
+        k_batch_rt_series<<<dim3(sh.solve_blocks, nb), kScatterThreads, 0, s>>>(B->ra, B->d.ctl, work);
         CKL(ctx);
-        k_batch_rt_solve<<<dim3(sh.solve_blocks, nb), kRtSolveThreads, rt_solve_smem_bytes(), s>>>(B->ra,
+        k_batch_rt_solve<<<dim3(sh.solve_blocks, nb), kScatterThreads, scatter_smem_bytes(), s>>>(B->ra,
                                                                                                  B->d.ctl, work);
         CKL(ctx);
       }
@@ -425,7 +425,7 @@ int atlasgpu_batch_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* dsc, int
     return fail(ctx, ATLASGPU_EINVAL, "batch_create: finish needs %zu B of shared memory", B->smem_fin);
   }
   CK(cudaFuncSetAttribute(k_batch_rt_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_pre_smem_bytes()));
-  CK(cudaFuncSetAttribute(k_batch_rt_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_solve_smem_bytes()));
+  CK(cudaFuncSetAttribute(k_batch_rt_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes()));
   CK(cudaFuncSetAttribute(k_batch_rt_post, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)rt_post_smem_bytes(B->nrhox)));
   CK(cudaFuncSetAttribute(k_batch_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B->smem_fin));

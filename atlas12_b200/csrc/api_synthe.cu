@@ -383,16 +383,29 @@ int atlasgpu_synthe_line_opacity(atlasgpu_ctx* ctx, const atlasgpu_lte_line* lin
 }
 
 // ---------------------------------------------------------------- spectrum
-static int spectrum_launch(atlasgpu_ctx* ctx, const SpecArgs& a) {
-  int nwarp = 4;
-  const size_t per = sizeof(SpecWS);
-  while (nwarp > 1 && sizeof(double) * kKwMax + nwarp * per > ctx->smem_optin) --nwarp;
-  const size_t smem = sizeof(double) * kKwMax + nwarp * per;
-  CK(cudaFuncSetAttribute(k_spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int blocks = std::min<int64_t>((a.length + nwarp - 1) / nwarp, (int64_t)ctx->nsm * 8);
+static int spectrum_launch(atlasgpu_ctx* ctx, SpecArgs a) {
+  const int chunk = std::min(a.length, kSpecChunk);
+  int r;
+  if ((r = bufT(ctx, "spec_rec", (size_t)2 * chunk * kSpecStride, &a.rec))) return r;
+  CK(cudaFuncSetAttribute(k_spec_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spec_smem_bytes()));
+  CK(cudaFuncSetAttribute(k_spec_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes()));
   Timer tm(ctx, "josh_spectrum");
-  k_spectrum<<<blocks, 32 * nwarp, smem, ctx->stream>>>(a);
-  CKL(ctx);
+  for (a.iw0 = 0; a.iw0 < a.length; a.iw0 += chunk) {
+    a.n = std::min(chunk, a.length - a.iw0);
+    const int pre = std::min((a.n + kSpecWarps - 1) / kSpecWarps, ctx->nsm * 8);
+    k_spec_pre<<<pre, kSpecWarps * 32, spec_smem_bytes(), ctx->stream>>>(a);
+    CKL(ctx);
+    // about four resident waves of pair groups, consecutive systems per group
+    const int groups = ctx->nsm * 8 * 4;
+    a.per = std::max(1, (2 * a.n + groups - 1) / groups);
+    const int blocks = ((2 * a.n + a.per - 1) / a.per + kScatterGroups - 1) / kScatterGroups;
+    k_spec_series<<<blocks, kScatterThreads, 0, ctx->stream>>>(a);
+    CKL(ctx);
+    k_spec_solve<<<blocks, kScatterThreads, scatter_smem_bytes(), ctx->stream>>>(a);
+    CKL(ctx);
+    k_spec_flux<<<(a.n + 255) / 256, 256, 0, ctx->stream>>>(a);
+    CKL(ctx);
+  }
   return 0;
 }
 
@@ -407,7 +420,7 @@ int atlasgpu_synthe_spectrum_dev(atlasgpu_ctx* ctx, const double* d_wledge, int 
     return fail(ctx, ATLASGPU_EINVAL, "synthe_spectrum: bad argument");
   cudaSetDevice(ctx->device);
   SpecArgs a{ctx->ops, d_wledge, d_contabs, d_contscat, d_rhox, d_hkt, nedge, stride, nrhox, length,
-             wbegin, ratio, d_opac, d_flux, d_cont};
+             wbegin, ratio, d_opac, d_flux, d_cont, nullptr, 0, 0, 1};
   return spectrum_launch(ctx, a);
 }
 

@@ -14,6 +14,7 @@
 #pragma once
 #include "common.cuh"
 #include "josh.cuh"
+#include "scatter.cuh"
 #include "surrogate.cuh"
 #include "voigt.cuh"
 
@@ -741,7 +742,7 @@ struct RtWS {
   JoshWS w;
   JoshWSFull f;
   double acont[kKwMax], sigmac[kKwMax], aline[kKwMax], stim[kKwMax];
-  double dab[kKwMax];           // SCONT while JOSH runs (when given), then d(abtot)/d(rhox)
+  double scont[kKwMax];         // SCONT (when given)
   alignas(16) double U[kNx * (kNx + 1)];  // pivot rows of the 51x51 factorisation (rows 16-byte aligned)
 };
 
@@ -757,15 +758,32 @@ constexpr int kRtMinBlocks = 3;
 constexpr int kRtGroups = 2;
 constexpr int kRtThreads = kRtGroups * RtG::N;
 
-// shared memory: RHOX and a zero vector (SIGMAL) for the CTA, then the groups' workspaces
-__host__ __device__ inline size_t rt_smem_bytes() { return 2 * sizeof(double) * kKwMax + kRtGroups * sizeof(RtWS); }
+// What a CTA's groups share: the grids with their reciprocal differences, and
+// HKT and HKT/T of every depth (the mode-2 sums' dB/dT factor).
+struct RtShared {
+  JoshGrid grid;
+  double hkt[kKwMax], hkt_t[kKwMax];
+};
+__device__ __forceinline__ void rt_shared_load(RtShared& R, const RtArgs& a) {
+  for (int j = threadIdx.x; j < a.nrhox; j += blockDim.x) {
+    const double h = a.hkt[j];
+    R.hkt[j] = h;
+    R.hkt_t[j] = h / a.t[j];
+  }
+  josh_grid_load(R.grid, *a.ops, a.rhox, a.nrhox);
+}
+
+// shared memory: the CTA's grids and a zero vector (SIGMAL), then the groups' workspaces
+__host__ __device__ inline size_t rt_smem_bytes() {
+  return sizeof(RtShared) + sizeof(double) * (kKwMax + (sizeof(RtShared) / 8) % 2) + kRtGroups * sizeof(RtWS);
+}
 
 // After JOSH: the negative floor (RUN_RT_PASS :3926-3937), HNU(1) for the
 // .flux record, and the TCORR / RADIAP / ROSS mode-2 terms of this frequency
 // added into the group's accumulators (threads over depths, C per thread).
 // add(q, c, j, v) adds term q of depth j (the thread's c-th depth) to its sum.
 template <class G, class WS, int C, class Add>
-static __device__ __forceinline__ void rt_accumulate(G& g, const RtArgs& a, WS& S, const double* rhox_s, int nu,
+static __device__ __forceinline__ void rt_accumulate(G& g, const RtArgs& a, WS& S, const RtShared& R, int nu,
                                                      double freq, double rcowt, Add&& add, double& pradk0) {
   const int nr = a.nrhox;
   // negative floor (RUN_RT_PASS :3926-3937)
@@ -780,8 +798,6 @@ static __device__ __forceinline__ void rt_accumulate(G& g, const RtArgs& a, WS& 
     g.sync();
   }
   if (g.r == 0) a.hsurf[nu - 1] = S.f.hnu[0];
-  // TCORR mode 2: d(abtot)/d(rhox)
-  g_deriv(g, rhox_s, S.w.abtot, S.dab, nr);
   // TERM2 per depth (E3 diagonal of Lambda); D(NRHOX) repeats D(NRHOX-1)
   for (int j = g.r; j < nr; j += G::N) {
     const int jd = j < nr - 1 ? j : nr - 2;
@@ -806,13 +822,14 @@ static __device__ __forceinline__ void rt_accumulate(G& g, const RtArgs& a, WS& 
     if (j >= nr) break;
     const double ab = S.w.abtot[j], al = S.w.alpha[j], h = S.f.hnu[j];
     const double rab = 1.0 / ab;
-    add(1, c, j, S.dab[j] * rab * h * rcowt);                // RDABH
+    // TCORR mode 2: d(abtot)/d(rhox)
+    const double dab = deriv_at(R.grid.rhox, S.w.abtot, nr, j, R.grid.rho());
+    add(1, c, j, dab * rab * h * rcowt);                     // RDABH
     add(0, c, j, ab * S.f.jmins[j] * rcowt);                 // RJMINS
     add(3, c, j, h * rcowt);                                 // FLXRAD
     const double diagj = (j > 0 ? S.w.t1[j - 1] : 0.0) + S.w.t1[j];
-    const double hk = a.hkt[j], tt = a.t[j];
     // dB/dT = BNU * freq * HKT / T / STIM (floored at 1e-30 for RDIAGJ, as the reference)
-    const double bft = S.f.bnu[j] * freq * hk / tt;
+    const double bft = S.f.bnu[j] * freq * R.hkt_t[j];
     const double dbdt = bft / fmax(S.stim[j], 1.0e-30);
     add(2, c, j, ab * (diagj - 1.0) / (1.0 - al * diagj) * (1.0 - al) * dbdt * rcowt);  // RDIAGJ
     add(4, c, j, S.f.jnu[j] * rcowt);                        // RADEN
@@ -845,14 +862,11 @@ static __device__ __forceinline__ void rt_write_partial(G& g, const RtArgs& a, i
 static __device__ __forceinline__ void rt_body(const RtArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int gid = threadIdx.x / RtG::N;
-  double* rhox_s = reinterpret_cast<double*>(smem_raw);
-  double* zero_s = rhox_s + kKwMax;
-  RtWS& S = reinterpret_cast<RtWS*>(smem_raw + 2 * sizeof(double) * kKwMax)[gid];
-  for (int j = threadIdx.x; j < a.nrhox; j += blockDim.x) {
-    rhox_s[j] = a.rhox[j];
-    zero_s[j] = 0.0;
-  }
-  __syncthreads();
+  RtShared& R = *reinterpret_cast<RtShared*>(smem_raw);
+  double* zero_s = reinterpret_cast<double*>(smem_raw + sizeof(RtShared));
+  RtWS& S = reinterpret_cast<RtWS*>(zero_s + kKwMax + (sizeof(RtShared) / 8) % 2)[gid];
+  for (int j = threadIdx.x; j < a.nrhox; j += blockDim.x) zero_s[j] = 0.0;
+  rt_shared_load(R, a);
   RtG g(threadIdx.x % RtG::N, 1 + gid, S.w.red);
   constexpr int C = (kKwMax + RtG::N - 1) / RtG::N;
   const JoshOps& ops = *a.ops;
@@ -872,22 +886,22 @@ static __device__ __forceinline__ void rt_body(const RtArgs& a) {
     const double rcowt = a.rcoset[nu - 1];
     const double f3 = powi(freq / 1.0e15, 3);
     for (int j = g.r; j < nr; j += RtG::N) {
-      const double ehvkt = exp(-freq * a.hkt[j]);
+      const double ehvkt = exp(-freq * R.hkt[j]);
       const double stim = 1.0 - ehvkt;
       const double bnu = kBnuPrefac * f3 * ehvkt / stim;
       S.stim[j] = stim;
       S.f.bnu[j] = bnu;
       S.acont[j] = a.acont[(size_t)(nu - 1) * a.kw + j];
       S.sigmac[j] = a.sigmac[(size_t)(nu - 1) * a.kw + j];
-      if (a.scont) S.dab[j] = a.scont[(size_t)(nu - 1) * a.kw + j];
+      if (a.scont) S.scont[j] = a.scont[(size_t)(nu - 1) * a.kw + j];
       S.aline[j] = 0.0 + a.xl[(size_t)j * a.xl_sj + (size_t)(nu - 1) * a.xl_snu] * stim;
     }
     g.sync();
-    const int sw = g_josh(g, ops, rhox_s, nr, S.acont, S.aline, S.sigmac, zero_s, a.scont ? S.dab : S.f.bnu,
-                          S.f.bnu, S.f.bnu, S.w, S.U, &S.f, nullptr);
+    const int sw = g_josh(g, R.grid, ops, nr, S.acont, S.aline, S.sigmac, zero_s, a.scont ? S.scont : S.f.bnu,
+                          S.f.bnu, S.f.bnu, S.w, S.U, S.f);
     if (a.sweeps && g.r == 0) a.sweeps[nu - 1] = sw;
     rt_accumulate<RtG, RtWS, C>(
-        g, a, S, rhox_s, nu, freq, rcowt, [&](int q, int c, int, double v) { acc[q][c] += v; }, pradk0);
+        g, a, S, R, nu, freq, rcowt, [&](int q, int c, int, double v) { acc[q][c] += v; }, pradk0);
     g.sync();
   }
   rt_write_partial(g, a, gw, acc, pradk0);
@@ -928,8 +942,8 @@ __host__ __device__ inline int rt_rec_stride(int kw) { return (kw + 3 * kNx + 2 
 struct RtDepth {
   double stim, bnu, abtot, alpha, snubar;
 };
-__device__ __forceinline__ RtDepth rt_depth(const RtArgs& a, int nu, double freq, double f3, int j) {
-  const double ehvkt = exp(-freq * a.hkt[j]);
+__device__ __forceinline__ RtDepth rt_depth(const RtArgs& a, const RtShared& R, int nu, double freq, double f3, int j) {
+  const double ehvkt = exp(-freq * R.hkt[j]);
   const double stim = 1.0 - ehvkt;
   const double bnu = kBnuPrefac * f3 * ehvkt / stim;
   const double ac = a.acont[(size_t)(nu - 1) * a.kw + j];
@@ -947,22 +961,11 @@ __device__ __forceinline__ RtDepth rt_depth(const RtArgs& a, int nu, double freq
 }
 
 constexpr int kRtSplitWarps = 4;      // warps per CTA of the pre and post stages
-constexpr int kRtSolveGroups = 2;     // pair groups per CTA of the solve stage
-constexpr int kRtSolveThreads = kRtSolveGroups * PairG::N;
-constexpr int kRtSolveMinBlocks = 4;  // 8 systems per SM (128 registers per thread)
 
 struct RtPreWS {
-  double abtot[kKwMax], alpha[kKwMax], snubar[kKwMax], taunu[kKwMax];
-  double t1[kKwMax], t2[kKwMax], t3[kKwMax];
+  double abtot[kKwMax], alpha[kKwMax], snubar[kKwMax], taunu[kKwMax], rd[kKwMax], r2[kKwMax];
   double xsbar[kNx], xalpha[kNx], xs[kNx];
-  int lidx[kKwMax + 4];
-};
-struct RtSolveWS {
-  double xs[kNx], xsbar[kNx], xalpha[kNx], piv[kNx];
-  double rowabs[kNx];  // row sums of |COEFJ| (the contraction bound's factors)
-  double red[8];
-  unsigned pk[4][3];
-  alignas(16) double U[kNx * (kNx + 1)];
+  int lidx[2];
 };
 // The post stage's workspace: one warp's vectors carved from shared memory
 // at a stride of kv >= NRHOX doubles (rt_post_kv), its 51-point vectors, the
@@ -973,22 +976,20 @@ struct RtPostFull {
   int& maxj;
 };
 struct RtPostVec {
-  double *abtot, *alpha, *snubar, *taunu, *t1, *t2, *t3, *xs, *xsbar, *xw;
-  int* lidx;
+  double *abtot, *alpha, *snubar, *taunu, *rd, *t1, *xs, *xsbar, *xw;
 };
 struct RtPostView {
   RtPostVec w;
   RtPostFull f;
-  double *stim, *dab, *acc;
+  double *stim, *acc;
 };
 __host__ __device__ inline int rt_post_kv(int nrhox) { return (nrhox + 1) & ~1; }
 __host__ __device__ inline size_t rt_post_warp_doubles(int kv) {
-  return (size_t)(12 + kAcc) * kv + 3 * kNx + 2 + (kv + 4 + 1) / 2 + 1;
+  return (size_t)(11 + kAcc) * kv + 3 * kNx + 2;
 }
-__host__ __device__ inline size_t rt_pre_smem_bytes() { return sizeof(double) * kKwMax + kRtSplitWarps * sizeof(RtPreWS); }
-__host__ __device__ inline size_t rt_solve_smem_bytes() { return kRtSolveGroups * sizeof(RtSolveWS); }
+__host__ __device__ inline size_t rt_pre_smem_bytes() { return sizeof(RtShared) + kRtSplitWarps * sizeof(RtPreWS); }
 __host__ __device__ inline size_t rt_post_smem_bytes(int nrhox) {
-  return sizeof(double) * (kKwMax + kRtSplitWarps * rt_post_warp_doubles(rt_post_kv(nrhox)));
+  return sizeof(RtShared) + sizeof(double) * kRtSplitWarps * rt_post_warp_doubles(rt_post_kv(nrhox));
 }
 
 __device__ __forceinline__ double* rt_rec(const RtArgs& a, int nu) {
@@ -997,13 +998,11 @@ __device__ __forceinline__ double* rt_rec(const RtArgs& a, int nu) {
 
 static __device__ __forceinline__ void rt_pre_body(const RtArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* rhox_s = reinterpret_cast<double*>(smem_raw);
+  RtShared& R = *reinterpret_cast<RtShared*>(smem_raw);
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  RtPreWS& S = reinterpret_cast<RtPreWS*>(smem_raw + sizeof(double) * kKwMax)[wid];
-  for (int j = threadIdx.x; j < a.nrhox; j += blockDim.x) rhox_s[j] = a.rhox[j];
-  __syncthreads();
+  RtPreWS& S = reinterpret_cast<RtPreWS*>(smem_raw + sizeof(RtShared))[wid];
+  rt_shared_load(R, a);
   WarpG g(lane);
-  const JoshOps& ops = *a.ops;
   const int nr = a.nrhox, kw = a.kw;
   const int w = blockIdx.x * kRtSplitWarps + wid;
   const int nu0 = a.nu_first + w * a.nu_per_pre;
@@ -1012,7 +1011,7 @@ static __device__ __forceinline__ void rt_pre_body(const RtArgs& a) {
     const double freq = kClightNms / a.waveset[nu - 1];
     const double f3 = powi(freq / 1.0e15, 3);
     for (int j = lane; j < nr; j += 32) {
-      const RtDepth d = rt_depth(a, nu, freq, f3, j);
+      const RtDepth d = rt_depth(a, R, nu, freq, f3, j);
       S.abtot[j] = d.abtot;
       S.alpha[j] = d.alpha;
       S.snubar[j] = d.snubar;
@@ -1021,186 +1020,56 @@ static __device__ __forceinline__ void rt_pre_body(const RtArgs& a) {
     bool mapped, solve;
     // (with IFSURF = 0 a mapped surface with MAXJ = 1 ends as an unmapped
     // one: the sweeps overwrite SNU at every depth, so XS is not needed)
-    const int maxj = g_josh_prepare(g, ops, rhox_s, nr, S, mapped, solve);
+    const int maxj = g_josh_prepare(g, R.grid, nr, S, mapped, solve);
     (void)mapped;
     double* rec = rt_rec(a, nu);
-    const RtRec R{kw};
+    const RtRec Q{kw};
     for (int j = lane; j < nr; j += 32) rec[j] = S.taunu[j];
     if (maxj != 1) {
       for (int l = lane; l < kNx; l += 32) {
-        rec[R.xalpha() + l] = S.xalpha[l];
-        rec[R.xsbar() + l] = S.xsbar[l];
-        if (!solve) rec[R.xs() + l] = S.xs[l];
+        rec[Q.xalpha() + l] = S.xalpha[l];
+        rec[Q.xsbar() + l] = S.xsbar[l];
+        if (!solve) rec[Q.xs() + l] = S.xs[l];
       }
     }
     if (lane == 0) {
-      rec[R.maxj()] = (double)maxj;
-      rec[R.solve()] = (solve && maxj != 1) ? 1.0 : 0.0;
+      rec[Q.maxj()] = (double)maxj;
+      rec[Q.solve()] = (solve && maxj != 1) ? 1.0 : 0.0;
     }
     g.sync();
   }
 }
 
-// The scattering system X = (1 - XALPHA) XSBAR + XALPHA (COEFJ X) is a
-// contraction with factor q = max_l XALPHA(l) sum_m |COEFJ(l,m)| (the
-// infinity norm of diag(XALPHA) COEFJ).  Where q <= kRtSeriesQ the solve
-// stage sums its Neumann series instead of eliminating: K steps of
-// X <- (1 - XALPHA) XSBAR + XALPHA (COEFJ X) from X = (1 - XALPHA) XSBAR
-// leave an error of at most q^(K+1) |X|, and K is taken so that
-// q^(K+1) <= 2^-60, far below the rounding of the elimination itself (the
-// two solutions agree to rounding).  A step is one matrix-vector product
-// with no sequential dependence between rows and one barrier, against the
-// elimination's 50 dependent pivot steps, so the series is cheaper up to
-// q ~ 0.5.  Systems with larger q (strongly scattering layers) are
-// eliminated as SOLVIT does.
-constexpr double kRtSeriesQ = 0.5;
-constexpr int kRtSeriesMaxSteps = 64;
-
-__device__ __forceinline__ int rt_series_steps(double q) {
-  if (!(q > 0.0)) return 1;
-  const int k = (int)ceil(-60.0 * 0.6931471805599453 / log(q)) - 1;
-  return k < 1 ? 1 : (k > kRtSeriesMaxSteps ? kRtSeriesMaxSteps : k);
-}
-
-static __device__ __forceinline__ void rt_solve_body(const RtArgs& a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int gid = threadIdx.x / PairG::N;
-  RtSolveWS& S = reinterpret_cast<RtSolveWS*>(smem_raw)[gid];
-  PairG g(threadIdx.x % PairG::N, 1 + gid, S.red);
-  const JoshOps& ops = *a.ops;
-  const int kw = a.kw;
-  const int grp = blockIdx.x * kRtSolveGroups + gid;
-  const int nu0 = a.nu_first + grp * a.nu_per_solve;
-  const int nu1 = min(nu0 + a.nu_per_solve - 1, a.nu_last > 0 ? a.nu_last : a.numnu);
-  for (int l = g.r; l < kNx; l += PairG::N) {
-    double r = 0.0;
-    for (int m = 0; m < kNx; ++m) r += fabs(ops.coefj[m * kNx + l]);
-    S.rowabs[l] = r;
-  }
-  g.sync();
-  unsigned long long nelim = 0, nseries = 0, nsteps = 0;
-  const RtRec R{kw};
-  for (int nu = nu0; nu <= nu1; ++nu) {
-    double* rec = rt_rec(a, nu);
-    if (rec[R.solve()] == 0.0) continue;  // the same word for the whole group
-    {
-      double qv = 0.0;
-      for (int l = g.r; l < kNx; l += PairG::N) {
-        const double xa = rec[R.xalpha() + l];
-        S.xalpha[l] = xa;
-        S.xsbar[l] = rec[R.xsbar() + l];
-        qv = fmax(qv, xa * S.rowabs[l]);
-      }
-      const double q = g.max(qv);  // (its barrier also publishes XALPHA, XSBAR)
-      if (q <= kRtSeriesQ) continue;  // summed by k_rt_series
-      solve_scatter(g, ops, S, S.U);
-      ++nelim;
-    }
-    for (int l = g.r; l < kNx; l += PairG::N) rec[R.xs() + l] = S.xs[l];
-    g.sync();
-  }
-  if (a.work && g.r == 0 && (nelim | nseries)) {
-    atomicAdd(a.work, nelim);
-    atomicAdd(a.work + 1, nseries);
-    atomicAdd(a.work + 2, nsteps);
-  }
-}
-
-// The Neumann series of the systems with q <= kRtSeriesQ, by their own
-// kernel (k_rt_series; k_rt_solve eliminates the rest): thread l of a pair
-// group keeps row l of COEFJ in registers for the whole launch (it is the
-// same for every frequency), so a step is 51 FMAs on registers and the
-// broadcast reads of X from shared memory, with no loads of COEFJ.  Sum k of
-// the four partial sums takes the terms m = k, k+4, ... in that order; q is
-// formed as in rt_solve_body, so the two kernels split the systems the same
-// way.  (The series inside k_rt_solve, reading COEFJ from L1 every step,
-// took 2.6k cycles per step at eight groups per SM.)
-constexpr int kRtSeriesMinBlocks = 3;
-struct RtSeriesWS {
-  alignas(16) double xa[kNx + 1];
-  alignas(16) double xb[kNx + 1];
-  double red[8];
-};
-
-static __device__ __forceinline__ void rt_series_body(const RtArgs& a) {
-  __shared__ RtSeriesWS s_ws[kRtSolveGroups];
-  const int gid = threadIdx.x / PairG::N;
-  RtSeriesWS& S = s_ws[gid];
-  PairG g(threadIdx.x % PairG::N, 1 + gid, S.red);
-  const JoshOps& ops = *a.ops;
-  const int kw = a.kw, l = g.r;
-  const bool own = l < kNx;
-  double c[kNx];
-  double rowabs = 0.0;
-#pragma unroll
-  for (int m = 0; m < kNx; ++m) c[m] = own ? ops.coefj[m * kNx + l] : 0.0;
-  for (int m = 0; m < kNx; ++m) rowabs += fabs(own ? ops.coefj[m * kNx + l] : 0.0);
-  const int grp = blockIdx.x * kRtSolveGroups + gid;
-  const int nu0 = a.nu_first + grp * a.nu_per_solve;
-  const int nu1 = min(nu0 + a.nu_per_solve - 1, a.nu_last > 0 ? a.nu_last : a.numnu);
-  unsigned long long nseries = 0, nsteps = 0;
-  const RtRec R{kw};
-  for (int nu = nu0; nu <= nu1; ++nu) {
-    double* rec = rt_rec(a, nu);
-    if (rec[R.solve()] == 0.0) continue;  // the same word for the whole group
-    const double al = own ? rec[R.xalpha() + l] : 0.0;
-    const double xb = own ? rec[R.xsbar() + l] : 0.0;
-    double qv = 0.0;
-    if (own) qv = fmax(qv, al * rowabs);
-    const double q = g.max(qv);
-    if (q > kRtSeriesQ) continue;  // eliminated by k_rt_solve
-    const int K = rt_series_steps(q);
-    const double b = own ? (1.0 - al) * xb : 0.0;
-    double* cur = S.xa;
-    double* nxt = S.xb;
-    if (own) cur[l] = b;
-    for (int k = 0; k < K; ++k) {
-      g.sync();
-      if (own) {
-        double s4[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int m = 0; m < kNx; ++m) s4[m & 3] = s4[m & 3] + c[m] * cur[m];
-        nxt[l] = b + al * ((s4[0] + s4[1]) + (s4[2] + s4[3]));
-      }
-      double* t = cur;
-      cur = nxt;
-      nxt = t;
-    }
-    g.sync();
-    if (own) rec[R.xs() + l] = cur[l];
-    ++nseries;
-    nsteps += K;
-  }
-  if (a.work && g.r == 0 && nseries) {
-    atomicAdd(a.work + 1, nseries);
-    atomicAdd(a.work + 2, nsteps);
-  }
+// the solve stage's view of the pass's records
+__device__ __forceinline__ ScatterArgs rt_scatter_args(const RtArgs& a) {
+  const RtRec Q{a.kw};
+  const int last = a.nu_last > 0 ? a.nu_last : a.numnu;
+  return ScatterArgs{a.ops, a.rec, a.rec_stride, Q.xalpha(), Q.xsbar(), Q.xs(), Q.solve(), last - a.nu_first + 1,
+                     a.nu_per_solve, a.work};
 }
 
 static __device__ __forceinline__ void rt_post_body(const RtArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* rhox_s = reinterpret_cast<double*>(smem_raw);
+  RtShared& R = *reinterpret_cast<RtShared*>(smem_raw);
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nr = a.nrhox, kw = a.kw, kv = rt_post_kv(nr);
-  double* p = rhox_s + kKwMax + (size_t)wid * rt_post_warp_doubles(kv);
+  double* p = reinterpret_cast<double*>(smem_raw + sizeof(RtShared)) + (size_t)wid * rt_post_warp_doubles(kv);
   auto take = [&](size_t n) {
     double* q = p;
     p += n;
     return q;
   };
-  double *abtot = take(kv), *alpha = take(kv), *snubar = take(kv), *taunu = take(kv), *t1 = take(kv);
+  // rd holds TAUNU's reciprocal differences for the sweeps, then the mode-2 sums' E3 terms
+  double *abtot = take(kv), *alpha = take(kv), *snubar = take(kv), *taunu = take(kv), *rd = take(kv);
   double *snu = take(kv), *hnu = take(kv), *jmins = take(kv), *jnu = take(kv), *bnu = take(kv);
-  double *stim = take(kv), *dab = take(kv), *acc = take((size_t)kAcc * kv);
+  double *stim = take(kv), *acc = take((size_t)kAcc * kv);
   double *xs = take(kNx), *xsbar = take(kNx), *xw = take(kNx);
   double* knu1 = take(1);
   int* maxj_s = reinterpret_cast<int*>(take(1));
-  int* lidx = reinterpret_cast<int*>(take((kv + 4 + 1) / 2));
-  // t2 and t3 serve JOSH only with IFSURF = 1, which this stage never runs
-  RtPostView S{RtPostVec{abtot, alpha, snubar, taunu, t1, t1, t1, xs, xsbar, xw, lidx},
-               RtPostFull{snu, hnu, jmins, jnu, bnu, *knu1, *maxj_s}, stim, dab, acc};
-  for (int j = threadIdx.x; j < nr; j += blockDim.x) rhox_s[j] = a.rhox[j];
+  RtPostView S{RtPostVec{abtot, alpha, snubar, taunu, rd, rd, xs, xsbar, xw},
+               RtPostFull{snu, hnu, jmins, jnu, bnu, *knu1, *maxj_s}, stim, acc};
   for (int e = lane; e < kAcc * kv; e += 32) acc[e] = 0.0;
-  __syncthreads();
+  rt_shared_load(R, a);
   WarpG g(lane);
   constexpr int C = (kKwMax + 31) / 32;
   const JoshOps& ops = *a.ops;
@@ -1213,10 +1082,10 @@ static __device__ __forceinline__ void rt_post_body(const RtArgs& a) {
     const double rcowt = a.rcoset[nu - 1];
     const double f3 = powi(freq / 1.0e15, 3);
     const double* rec = rt_rec(a, nu);
-    const RtRec R{kw};
-    const int maxj = (int)rec[R.maxj()];
+    const RtRec Q{kw};
+    const int maxj = (int)rec[Q.maxj()];
     for (int j = lane; j < nr; j += 32) {
-      const RtDepth d = rt_depth(a, nu, freq, f3, j);
+      const RtDepth d = rt_depth(a, R, nu, freq, f3, j);
       abtot[j] = d.abtot;
       alpha[j] = d.alpha;
       snubar[j] = d.snubar;
@@ -1225,12 +1094,16 @@ static __device__ __forceinline__ void rt_post_body(const RtArgs& a) {
       taunu[j] = rec[j];
     }
     if (maxj != 1)
-      for (int l = lane; l < kNx; l += 32) xs[l] = rec[R.xs() + l];
+      for (int l = lane; l < kNx; l += 32) xs[l] = rec[Q.xs() + l];
     g.sync();
-    const int sw = g_josh_finish(g, ops, nr, maxj, maxj != 1, S.w, &S.f, bnu, (double*)nullptr);
+    if (maxj != nr) {
+      for (int j = lane; j < nr - 1; j += 32) rd[j] = 1.0 / (taunu[j + 1] - taunu[j]);
+      g.sync();
+    }
+    const int sw = g_josh_finish(g, R.grid, ops, nr, maxj, maxj != 1, S.w, S.f, bnu);
     if (a.sweeps && lane == 0) a.sweeps[nu - 1] = sw;
     rt_accumulate<WarpG, RtPostView, C>(
-        g, a, S, rhox_s, nu, freq, rcowt, [&](int q, int, int j, double v) { acc[q * kv + j] += v; }, pradk0);
+        g, a, S, R, nu, freq, rcowt, [&](int q, int, int j, double v) { acc[q * kv + j] += v; }, pradk0);
     g.sync();
   }
   double* out = a.partial + (size_t)w * (kAcc * kw + 1);
@@ -1242,8 +1115,8 @@ static __device__ __forceinline__ void rt_post_body(const RtArgs& a) {
 }
 
 static __global__ void __launch_bounds__(kRtSplitWarps * 32, 6) k_rt_pre(RtArgs a) { rt_pre_body(a); }
-static __global__ void __launch_bounds__(kRtSolveThreads, kRtSolveMinBlocks) k_rt_solve(RtArgs a) { rt_solve_body(a); }
-static __global__ void __launch_bounds__(kRtSolveThreads, kRtSeriesMinBlocks) k_rt_series(RtArgs a) { rt_series_body(a); }
+static __global__ void __launch_bounds__(kScatterThreads, kScatterSolveMinBlocks) k_rt_solve(RtArgs a) { scatter_solve_body<false>(rt_scatter_args(a)); }
+static __global__ void __launch_bounds__(kScatterThreads, kScatterSeriesMinBlocks) k_rt_series(RtArgs a) { scatter_series_body<false>(rt_scatter_args(a)); }
 static __global__ void __launch_bounds__(kRtSplitWarps * 32, 4) k_rt_post(RtArgs a) { rt_post_body(a); }
 
 // Launch shape of the split pass over LEN frequencies with 1/NB of the GPU
@@ -1266,7 +1139,7 @@ inline RtSplitShape rt_split_shape(int len, int nsm, int nb, int waves) {
     return (int)(u < 1 ? 1 : u);
   };
   rt_split_fit(len, units(16), kRtSplitWarps, sh.pre_per, sh.pre_blocks);
-  rt_split_fit(len, units(8), kRtSolveGroups, sh.solve_per, sh.solve_blocks);
+  rt_split_fit(len, units(8), kScatterGroups, sh.solve_per, sh.solve_blocks);
   rt_split_fit(len, units(16), kRtSplitWarps, sh.post_per, sh.post_blocks);
   return sh;
 }
@@ -1281,7 +1154,7 @@ inline int rt_split_rows_max(int numnu, int nsm, int waves) {
 inline cudaError_t rt_split_attributes(int nrhox) {
   cudaError_t e = cudaFuncSetAttribute(k_rt_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_pre_smem_bytes());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_rt_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_solve_smem_bytes());
+    e = cudaFuncSetAttribute(k_rt_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_rt_post, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_post_smem_bytes(nrhox));
   return e;

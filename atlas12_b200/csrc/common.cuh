@@ -74,18 +74,19 @@ __device__ __forceinline__ double warp_max(double v) {
 __device__ __forceinline__ double expi1(double x) {
   const double ex = exp(-x);
   if (x > 4.0) {
+    const double r = 1.0 / x;  // the nested quotients of the approximation as polynomials in 1/x
     return (ex + ex * (-0.999999999998447 +
                        (-26.6271060431811 +
                         (-241.055827097015 +
-                         (-895.927957772937 + (-1298.85688746484 + (-545.374158883133 + -5.66575206533869 / x) / x) / x) /
-                             x) /
-                            x) /
-                           x) /
+                         (-895.927957772937 + (-1298.85688746484 + (-545.374158883133 - 5.66575206533869 * r) * r) * r) *
+                             r) *
+                            r) *
+                           r) /
                      (x + 28.6271060422192 +
                       (292.310039388533 +
-                       (1332.78537748257 + (2777.61949509163 + (2404.01713225909 + 631.657483280800 / x) / x) / x) / x) /
-                          x)) /
-           x;
+                       (1332.78537748257 + (2777.61949509163 + (2404.01713225909 + 631.657483280800 * r) * r) * r) * r) *
+                          r)) *
+           r;
   } else if (x > 1.0) {
     return ex *
            (0.430967839469389 +

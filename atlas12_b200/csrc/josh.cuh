@@ -7,18 +7,12 @@
 // reference formula for each output element (atlas12_modules.f90):
 //   PARCOE :5358-5434, INTEG :5293-5324, DERIV :5228-5266, MAP1 :5570-5692,
 //   SOLVIT :5739-5847, JOSH :18398-18776.
-// MAP1 is evaluated in parallel over output points: the sequential routine's
-// only cross-point state is the bracketing interval and the reuse of the
-// previous forward parabola as the next backward one, and both are recovered
-// per point from the bracket indices of the neighbouring outputs, so each
-// output gets the formula the sequential walk would have used.
-// Running sums whose order decides later branches (the INTEG cumulative sum)
-// are summed in the reference order by one thread.
+// Every output point of INTEG, DERIV and MAP1 is computed on its own, from the
+// interval it lies in (the Newton form below).
 //
-// The 51x51 scattering system: a warp group factors it in shared memory
-// (w_solvit); a pair group keeps one matrix row per thread in registers and
-// writes only the pivot rows to shared memory, which takes the row updates
-// off the shared-memory pipe.
+// The 51x51 scattering system: a pair group keeps one matrix row per thread
+// in registers and writes only the pivot rows to shared memory, which takes
+// the row updates off the shared-memory pipe.
 #pragma once
 #include "common.cuh"
 
@@ -78,11 +72,12 @@ using PairG = MultiG<2>;
 struct JoshWS {
   double xs[kNx], xsbar[kNx], xalpha[kNx], xw[kNx];
   double abtot[kKwMax], alpha[kKwMax], snubar[kKwMax], taunu[kKwMax];
-  double t1[kKwMax], t2[kKwMax], t3[kKwMax];  // scratch (PARCOE a,b,c / terms)
-  double red[8];                              // group reductions (multi-warp groups)
-  double piv[kNx];                            // pivots of the elimination without interchanges
-  int lidx[kKwMax + 4];                       // MAP1 bracket indices
-  unsigned pk[4][3];                          // pivot key exchange between a group's warps
+  double rd[kKwMax], r2[kKwMax];  // reciprocal differences of TAUNU (recip_range)
+  double t1[kKwMax];              // scratch (INTEG's terms)
+  double red[8];                  // group reductions (multi-warp groups)
+  double piv[kNx];                // pivots of the elimination without interchanges
+  int lidx[kKwMax + 4];           // MAP1 bracket indices
+  unsigned pk[4][3];              // pivot key exchange between a group's warps
 };
 
 // Full-solution extras for IFSURF = 0 (ATLAS)
@@ -94,322 +89,202 @@ struct JoshWSFull {
 
 __device__ __forceinline__ void wsync() { __syncwarp(0xffffffffu); }
 
-// ---------------------------------------------------------------- PARCOE/INTEG
-// Coefficients into (a, b, c); n >= 4 assumed (n = NRHOX >= 4 on the hot path).
-template <class G>
-__device__ inline void g_parcoe(G& g, const double* f, const double* x, double* a, double* b, double* c,
-                                int n) {
-  constexpr int C = (kKwMax + G::N - 1) / G::N;
-  // steps 1-3: endpoints linear, j = 1, 2 linear, interior parabolic
-  for (int j = g.r; j < n; j += G::N) {
-    double aj, bj, cj;
-    if (j == 0 || j == 1 || j == 2 || j == n - 1) {
-      const int i0 = (j == n - 1) ? n - 2 : j;
-      cj = 0.0;
-      bj = (f[i0 + 1] - f[i0]) / (x[i0 + 1] - x[i0]);
-      aj = f[j] - x[j] * bj;
-    } else {
-      const double d = (f[j] - f[j - 1]) / (x[j] - x[j - 1]);
-      cj = f[j + 1] / ((x[j + 1] - x[j]) * (x[j + 1] - x[j - 1])) -
-           f[j] / ((x[j] - x[j - 1]) * (x[j + 1] - x[j])) +
-           f[j - 1] / ((x[j] - x[j - 1]) * (x[j + 1] - x[j - 1]));
-      bj = d - (x[j] + x[j - 1]) * cj;
-      aj = f[j - 1] - x[j - 1] * d + x[j] * x[j - 1] * cj;
+// ---------------------------------------------------------------- interpolation
+// PARCOE, INTEG, DERIV and MAP1 in Newton form.  On the interval
+// [x(i), x(i+1)] both of the reference's parabolas (through i-1, i, i+1 and
+// through i, i+1, i+2) pass through its two end points, so any blend of them is
+//   f(i) + (v - x(i)) (slope(i) + (v - x(i+1)) q),
+// q the same blend of their second divided differences.  MAP1's reuse of the
+// previous forward parabola as the next backward one gives the same parabola,
+// so no state is carried from output to output.  A value costs one division
+// (the blend) where the reference's A, B, C form costs eleven, and with the
+// reciprocal differences of the grid given (recip_range, shared by every
+// function on the grid) none for the differences.  The A + (B + C v) v form loses
+// digits to cancellation where v is far from 0; this one does not.
+// (FP64 divisions bound the RT pass's prepare and finish stages: with the
+// reference's form they took 0.18 and 0.78 ms per 30,000 x 72 model-iteration.)
+
+// Reciprocal differences of a grid: rd(i) = 1/(x(i+1) - x(i)), i < n-1, and
+// r2(i) = 1/(x(i+1) - x(i-1)), 0 < i < n-1.  The caller synchronises.
+__device__ __forceinline__ void recip_range(int r, int step, const double* x, double* rd, double* r2, int n) {
+  for (int i = r; i < n - 1; i += step) {
+    rd[i] = 1.0 / (x[i + 1] - x[i]);
+    if (i > 0) r2[i] = 1.0 / (x[i + 1] - x[i - 1]);
+  }
+}
+
+// Reciprocals on the fly, for a grid that only one function is mapped on
+struct GridX {
+  const double* x;
+  __device__ __forceinline__ double rd(int i) const { return 1.0 / (x[i + 1] - x[i]); }
+  __device__ __forceinline__ double r2(int i) const { return 1.0 / (x[i + 1] - x[i - 1]); }
+};
+// ... or from recip_range's arrays
+struct GridP {
+  const double *rdp, *r2p;
+  __device__ __forceinline__ double rd(int i) const { return rdp[i]; }
+  __device__ __forceinline__ double r2(int i) const { return r2p[i]; }
+};
+
+// PARCOE's and MAP1's blend of the backward and forward second differences
+__device__ __forceinline__ double blend_curv(double cb, double cf) {
+  double wt = 0.0;
+  if (fabs(cf) != 0.0) wt = fabs(cf) / (fabs(cf) + fabs(cb));
+  return cf + wt * (cb - cf);
+}
+
+// fint = running parabolic integral of f over x, fint[0] = start (INTEG over
+// PARCOE's coefficients: linear on intervals 0..2 and the last, blended
+// parabolas between).  term: n doubles of scratch.  The running sum is formed
+// by the group's first warp, each lane a run of consecutive intervals, and a
+// scan of the lanes' sums (the one-thread sum was 71 dependent additions).
+template <class G, class R>
+__device__ inline void g_integ(G& g, const double* x, const double* f, double* fint, int n, double start,
+                               double* term, R gr) {
+  for (int i = g.r; i < n - 1; i += G::N) {
+    const double h = x[i + 1] - x[i];
+    double t = 0.5 * h * (f[i] + f[i + 1]);
+    if (i >= 3 && i <= n - 3) {
+      const double s = (f[i + 1] - f[i]) * gr.rd(i);
+      const double cb = (s - (f[i] - f[i - 1]) * gr.rd(i - 1)) * gr.r2(i);
+      const double cf = ((f[i + 2] - f[i + 1]) * gr.rd(i + 1) - s) * gr.r2(i + 1);
+      t -= blend_curv(cb, cf) * (h * h * h) * (1.0 / 6.0);
     }
-    a[j] = aj;
-    b[j] = bj;
-    c[j] = cj;
+    term[i] = t;
   }
   g.sync();
-  // step 4: blend each interval with its right neighbour's unsmoothed fit
-  double na[C], nb[C], nc[C];
-  int cnt = 0;
-  for (int j = g.r; j < n; j += G::N, ++cnt) {
-    na[cnt] = a[j];
-    nb[cnt] = b[j];
-    nc[cnt] = c[j];
-    if (j >= 1 && j <= n - 2 && c[j] != 0.0) {
-      const double wt = fabs(c[j + 1]) / (fabs(c[j + 1]) + fabs(c[j]));
-      na[cnt] = a[j + 1] + wt * (a[j] - a[j + 1]);
-      nb[cnt] = b[j + 1] + wt * (b[j] - b[j + 1]);
-      nc[cnt] = c[j + 1] + wt * (c[j] - c[j + 1]);
+  if (g.r < 32) {
+    const int per = (n - 1 + 31) >> 5, i0 = g.r * per, i1 = min(i0 + per, n - 1);
+    double own = 0.0;
+    for (int i = i0; i < i1; ++i) own += term[i];
+    double run = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, run, o);
+      if (g.r >= o) run += v;
     }
-  }
-  g.sync();
-  cnt = 0;
-  for (int j = g.r; j < n; j += G::N, ++cnt) {
-    a[j] = na[cnt];
-    b[j] = nb[cnt];
-    c[j] = nc[cnt];
-  }
-  g.sync();
-  // step 5: penultimate interval takes the endpoint linear fit
-  if (g.r == 0) {
-    a[n - 2] = a[n - 1];
-    b[n - 2] = b[n - 1];
-    c[n - 2] = c[n - 1];
+    run = __shfl_up_sync(0xffffffffu, run, 1);
+    run = g.r == 0 ? start : start + run;
+    if (g.r == 0) fint[0] = start;
+    for (int i = i0; i < i1; ++i) {
+      run += term[i];
+      fint[i + 1] = run;
+    }
   }
   g.sync();
 }
-
-// fint = running parabolic integral of f over x, fint[0] = start
 template <class G, class WS>
-__device__ inline void g_integ(G& g, const double* x, const double* f, double* fint, int n, double start,
-                               WS& ws) {
-  double *a = ws.t1, *b = ws.t2, *c = ws.t3;
-  g_parcoe(g, f, x, a, b, c, n);
-  for (int i = g.r; i < n - 1; i += G::N) {
-    const double xlo = x[i], xhi = x[i + 1];
-    const double term = (a[i] + b[i] * 0.5 * (xhi + xlo) +
-                         c[i] / 3.0 * ((xhi + xlo) * xhi + xlo * xlo)) *
-                        (xhi - xlo);
-    b[i] = term;
-  }
-  g.sync();
-  if (g.r == 0) {
-    double s = start;
-    fint[0] = s;
-    for (int i = 0; i < n - 1; ++i) {
-      s = s + b[i];
-      fint[i + 1] = s;
-    }
-  }
-  g.sync();
+__device__ inline void g_integ(G& g, const double* x, const double* f, double* fint, int n, double start, WS& ws) {
+  g_integ(g, x, f, fint, n, start, ws.t1, GridX{x});
 }
 
 // ---------------------------------------------------------------- DERIV
-template <class G>
-__device__ __noinline__ void g_deriv(G& g, const double* x, const double* f, double* dfdx, int n) {
+// DERIV at point j of the n points (x, f): the end points' slopes, and the
+// tangent of the mean of the two slopes' angles (in the reference's scaled
+// variables) between them.  tan of the mean from one quotient instead of the
+// reference's three.
+template <class R>
+__device__ __forceinline__ double deriv_at(const double* x, const double* f, int n, int j, R gr) {
+  if (j == 0) return (f[1] - f[0]) * gr.rd(0);
+  if (j == n - 1) return (f[n - 1] - f[n - 2]) * gr.rd(n - 2);
+  const double s = copysign(1.0, x[1] - x[0]);
+  const double top = fmax(fmax(fabs(f[j - 1]), fabs(f[j])), fabs(f[j + 1])), ax = fabs(x[j]);
+  const double rs = top == 0.0 ? 1.0 : ax / top;  // 1/SCALE, SCALE = top/|x| (1 where f is 0 around j)
+  const double dr = (f[j + 1] - f[j]) * gr.rd(j) * rs;
+  const double dl = (f[j] - f[j - 1]) * gr.rd(j - 1) * rs;
+  const double er = s * sqrt(1.0 + dr * dr) + 1.0, el = s * sqrt(1.0 + dl * dl) + 1.0;
+  return (dr * el + dl * er) / ((er * el - dr * dl) * rs);
+}
+
+// dfdx may alias f in callers
+template <class G, class R>
+__device__ __noinline__ void g_deriv_on(G g, const double* x, const double* f, double* dfdx, int n, R gr) {
   constexpr int C = (kKwMax + G::N - 1) / G::N;
-  const double s = fabs(x[1] - x[0]) / (x[1] - x[0]);
   double v[C];
-  int cnt = 0;
-  for (int j = g.r; j < n; j += G::N, ++cnt) {
-    if (j == 0) {
-      v[cnt] = (f[1] - f[0]) / (x[1] - x[0]);
-    } else if (j == n - 1) {
-      v[cnt] = (f[n - 1] - f[n - 2]) / (x[n - 1] - x[n - 2]);
-    } else {
-      double scale = fmax(fmax(fabs(f[j - 1]), fabs(f[j])), fabs(f[j + 1])) / fabs(x[j]);
-      if (scale == 0.0) scale = 1.0;
-      const double dr = (f[j + 1] - f[j]) / (x[j + 1] - x[j]) / scale;
-      const double dl = (f[j] - f[j - 1]) / (x[j] - x[j - 1]) / scale;
-      const double tr = dr / (s * sqrt(1.0 + dr * dr) + 1.0);
-      const double tl = dl / (s * sqrt(1.0 + dl * dl) + 1.0);
-      v[cnt] = (tr + tl) / (1.0 - tr * tl) * scale;
-    }
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int j = g.r + c * G::N;
+    if (j < n) v[c] = deriv_at(x, f, n, j, gr);
   }
-  g.sync();  // dfdx may alias f in callers
-  cnt = 0;
-  for (int j = g.r; j < n; j += G::N, ++cnt) dfdx[j] = v[cnt];
   g.sync();
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int j = g.r + c * G::N;
+    if (j < n) dfdx[j] = v[c];
+  }
+  g.sync();
+}
+template <class G>
+__device__ __forceinline__ void g_deriv(G& g, const double* x, const double* f, double* dfdx, int n) {
+  g_deriv_on(g, x, f, dfdx, n, GridX{x});
 }
 
 // ---------------------------------------------------------------- MAP1
-// backward parabola through (L-2, L-1, L) as MAP1 writes it (1-based L)
-__device__ __forceinline__ void map1_bac(const double* xo, const double* fo, int L, double& A,
-                                         double& B, double& C) {
-  const int l1 = L - 1, l2 = L - 2;
-#define XO(i) xo[(i)-1]
-#define FO(i) fo[(i)-1]
-  const double d = (FO(l1) - FO(l2)) / (XO(l1) - XO(l2));
-  C = FO(L) / ((XO(L) - XO(l1)) * (XO(L) - XO(l2))) +
-      (FO(l2) / (XO(L) - XO(l2)) - FO(l1) / (XO(L) - XO(l1))) / (XO(l1) - XO(l2));
-  B = d - (XO(l1) + XO(l2)) * C;
-  A = FO(l2) - XO(l2) * d + XO(l1) * XO(l2) * C;
+// MAP1's bracket of v: L = min{L >= 2 : XOLD(L) > v} (1-based), nold+1 past the end
+__device__ __forceinline__ int map1_bracket(const double* xo, int nold, double v) {
+  int lo = 2, hi = nold + 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (xo[mid - 1] > v) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
 }
-// forward parabola through (L-1, L, L+1)
-__device__ __forceinline__ void map1_for(const double* xo, const double* fo, int L, double& A,
-                                         double& B, double& C) {
-  const int l1 = L - 1;
-  const double d = (FO(L) - FO(l1)) / (XO(L) - XO(l1));
-  C = FO(L + 1) / ((XO(L + 1) - XO(L)) * (XO(L + 1) - XO(l1))) +
-      (FO(l1) / (XO(L + 1) - XO(l1)) - FO(L) / (XO(L + 1) - XO(L))) / (XO(L) - XO(l1));
-  B = d - (XO(L) + XO(l1)) * C;
-  A = FO(l1) - XO(l1) * d + XO(L) * XO(l1) * C;
-#undef XO
-#undef FO
-}
+
+// One output point of MAP1 with the differences its value needs, so that
+// several functions on the same old grid share them: linear in the first two
+// intervals and past the end, the backward parabola alone in the last
+// interval, the blend elsewhere.
+struct Map1At {
+  int i, mode;  // interval (0-based lower point); 0 linear, 1 backward, 2 blended
+  double v0, v1, rd0, rdm, rdp, r20, r2p;
+  template <class R>
+  __device__ __forceinline__ Map1At(const double* xo, int nold, int L, double v, R gr) {
+    i = (L > nold ? nold : L) - 2;
+    mode = (L <= 3 || L > nold) ? 0 : (L == nold ? 1 : 2);
+    v0 = v - xo[i];
+    v1 = v - xo[i + 1];
+    rd0 = gr.rd(i);
+    rdm = rdp = r20 = r2p = 0.0;
+    if (mode >= 1) {
+      rdm = gr.rd(i - 1);
+      r20 = gr.r2(i);
+    }
+    if (mode == 2) {
+      rdp = gr.rd(i + 1);
+      r2p = gr.r2(i + 1);
+    }
+  }
+  __device__ __forceinline__ double operator()(const double* fo) const {
+    const double f0 = fo[i], f1 = fo[i + 1];
+    const double s = (f1 - f0) * rd0;
+    if (mode == 0) return f1 + v1 * s;
+    double q = (s - (f0 - fo[i - 1]) * rdm) * r20;
+    if (mode == 2) q = blend_curv(q, ((fo[i + 2] - f1) * rdp - s) * r2p);
+    return f0 + v0 * (s + v1 * q);
+  }
+};
 
 // Returns MAP1 (index of the last old interval used).  xnew ascending.
 template <class G>
-__device__ __noinline__ int g_map1(G& g, const double* xo, const double* fo, int nold, const double* xn,
-                             double* fn, int nnew, int* lidx) {
-  // bracket: L_k = min{L >= 2 : XOLD(L) > XNEW(k)}, nold+1 when past the end
+__device__ __noinline__ int g_map1_on(G g, const double* xo, const double* fo, int nold, const double* xn,
+                                      double* fn, int nnew) {
   for (int k = g.r; k < nnew; k += G::N) {
     const double v = xn[k];
-    int lo = 2, hi = nold + 1;  // search in [2, nold+1)
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (xo[mid - 1] > v) hi = mid;
-      else lo = mid + 1;
-    }
-    lidx[k] = lo;
+    fn[k] = Map1At(xo, nold, map1_bracket(xo, nold, v), v, GridX{xo})(fo);
   }
+  const int L = map1_bracket(xo, nold, xn[nnew - 1]);
   g.sync();
-  for (int k = g.r; k < nnew; k += G::N) {
-    const int Lraw = lidx[k];
-    const bool past = Lraw > nold;
-    const double v = xn[k];
-    double A, B, C;
-    if (Lraw <= 3 || past) {
-      const int L = past ? nold : Lraw;
-      B = (fo[L - 1] - fo[L - 2]) / (xo[L - 1] - xo[L - 2]);
-      A = fo[L - 1] - xo[L - 1] * B;
-      fn[k] = A + B * v;  // a reused linear fit (C = 0) gives the same value
-      continue;
-    }
-    const int L = Lraw;
-    // first output point of this interval and the interval used before it
-    int k0 = k;
-    while (k0 > 0 && lidx[k0 - 1] == L) --k0;
-    int prevL = 0;
-    if (k0 > 0) prevL = lidx[k0 - 1] > nold ? nold : lidx[k0 - 1];
-    double ab, bb, cb;
-    if (L == prevL + 1 && L != 3 && L != 4) map1_for(xo, fo, L - 1, ab, bb, cb);
-    else map1_bac(xo, fo, L, ab, bb, cb);
-    if (L >= nold) {
-      A = ab;
-      B = bb;
-      C = cb;
-    } else {
-      double af, bf, cf;
-      map1_for(xo, fo, L, af, bf, cf);
-      double wt = 0.0;
-      if (fabs(cf) != 0.0) wt = fabs(cf) / (fabs(cf) + fabs(cb));
-      A = af + wt * (ab - af);
-      B = bf + wt * (bb - bf);
-      C = cf + wt * (cb - cf);
-    }
-    fn[k] = A + (B + C * v) * v;
-  }
-  g.sync();
-  const int Llast = lidx[nnew - 1];
-  const int ll = Llast > nold ? nold : Llast;
-  g.sync();
-  return ll - 1;
+  return (L > nold ? nold : L) - 1;
+}
+template <class G>
+__device__ __forceinline__ int g_map1(G& g, const double* xo, const double* fo, int nold, const double* xn,
+                                      double* fn, int nnew, int* /*lidx*/) {
+  return g_map1_on(g, xo, fo, nold, xn, fn, nnew);
 }
 
 // ---------------------------------------------------------------- SOLVIT
 constexpr double kPivotTol = 1.0e-30;
-
-// Gaussian elimination with partial pivoting on A (kNx x kNx, column-major,
-// ld kLd, shared memory), right-hand side / solution in b.  Reference pivot
-// rule: first maximum.  One warp.
-__device__ inline void w_solvit(double* __restrict__ A, double* __restrict__ b, int lane) {
-  constexpr int n = kNx;
-  int mypiv0 = 0, mypiv1 = 0;  // pivot of column i for i = lane, lane+32
-  for (int i = 0; i < n - 1; ++i) {
-    // (a) pivot search over rows i..n-1 of column i
-    double best = -1.0;
-    int bidx = n;
-    for (int k = i + lane; k < n; k += 32) {
-      const double v = fabs(A[i * kLd + k]);
-      if (v > best) {
-        best = v;
-        bidx = k;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-      if (ob > best || (ob == best && oi < bidx)) {
-        best = ob;
-        bidx = oi;
-      }
-    }
-    const int m = bidx;
-    if (lane == (i & 31)) {
-      if (i < 32) mypiv0 = m;
-      else mypiv1 = m;
-    }
-    // (b) swap rows i and m, columns i+1..n-1
-    if (m != i) {
-      for (int c = i + 1 + lane; c < n; c += 32) {
-        const double t = A[c * kLd + i];
-        A[c * kLd + i] = A[c * kLd + m];
-        A[c * kLd + m] = t;
-      }
-    }
-    wsync();
-    // (c) reciprocal pivot on the diagonal
-    double pv = A[i * kLd + m];
-    if (fabs(pv) < kPivotTol) pv = copysign(kPivotTol, pv);
-    const double pivot = 1.0 / pv;
-    const double aii = A[i * kLd + i];
-    wsync();
-    if (lane == 0) {
-      A[i * kLd + m] = aii;
-      A[i * kLd + i] = pivot;
-    }
-    wsync();
-    // (d) multipliers, (e) trailing update: lanes own rows i+1+lane, i+33+lane
-    const int r0 = i + 1 + lane, r1 = i + 33 + lane;
-    double l0 = 0.0, l1 = 0.0;
-    if (r0 < n) {
-      l0 = A[i * kLd + r0] * pivot;
-      A[i * kLd + r0] = l0;
-    }
-    if (r1 < n) {
-      l1 = A[i * kLd + r1] * pivot;
-      A[i * kLd + r1] = l1;
-    }
-    for (int j = i + 1; j < n; ++j) {
-      const double cj = A[j * kLd + i];
-      if (r0 < n) A[j * kLd + r0] = A[j * kLd + r0] - l0 * cj;
-      if (r1 < n) A[j * kLd + r1] = A[j * kLd + r1] - l1 * cj;
-    }
-    wsync();
-  }
-  if (lane == 0) {
-    double v = A[(n - 1) * kLd + n - 1];
-    if (fabs(v) < kPivotTol) v = copysign(kPivotTol, v);
-    A[(n - 1) * kLd + n - 1] = 1.0 / v;
-  }
-  wsync();
-  // forward substitution with the row interchanges
-  for (int i = 0; i < n - 1; ++i) {
-    const int m = __shfl_sync(0xffffffffu, i < 32 ? mypiv0 : mypiv1, i & 31);
-    if (m != i && lane == 0) {
-      const double t = b[m];
-      b[m] = b[i];
-      b[i] = t;
-    }
-    wsync();
-    const double c = b[i];
-    for (int k = i + 1 + lane; k < n; k += 32) b[k] = b[k] - A[i * kLd + k] * c;
-    wsync();
-  }
-  // back substitution
-  for (int j = n - 1; j >= 1; --j) {
-    double bj = 0.0;
-    if (lane == 0) {
-      bj = b[j] * A[j * kLd + j];
-      b[j] = bj;
-    }
-    bj = __shfl_sync(0xffffffffu, bj, 0);
-    for (int k = lane; k < j; k += 32) b[k] = b[k] - A[j * kLd + k] * bj;
-    wsync();
-  }
-  if (lane == 0) b[0] = b[0] * A[0];
-  wsync();
-}
-
-// (I - diag(XALPHA) COEFJ) XS = (1 - XALPHA) XSBAR by one warp: the matrix
-// AMAT(L,M) = -XALPHA(L)*COEFJ(L,M) (+1 on the diagonal) in shared memory A.
-__device__ inline void scatter_solve(WarpG& g, const JoshOps& ops, JoshWS& ws, double* A) {
-  for (int m = 0; m < kNx; ++m) {
-    for (int l = g.r; l < kNx; l += 32) {
-      double v = -ws.xalpha[l] * ops.coefj[m * kNx + l];
-      if (l == m) v = v + 1.0;
-      A[m * kLd + l] = v;
-    }
-  }
-  for (int l = g.r; l < kNx; l += 32) ws.xs[l] = (1.0 - ws.xalpha[l]) * ws.xsbar[l];
-  g.sync();
-  w_solvit(A, ws.xs, g.r);
-}
 
 // Pivot-row traffic in 16-byte words: the row owner stores [1/pivot, a[1..]]
 // and every pending row reads it back as double2 words (U rows are 16-byte
@@ -613,10 +488,6 @@ template <class WS>
 __device__ __forceinline__ void solve_scatter(PairG& g, const JoshOps& ops, WS& ws, double* U) {
   if (!scatter_solve_nopivot(g, ops, ws, U)) scatter_solve(g, ops, ws, U);
 }
-__device__ __forceinline__ void solve_scatter(WarpG& g, const JoshOps& ops, JoshWS& ws, double* A) {
-  scatter_solve(g, ops, ws, A);
-}
-
 // ---------------------------------------------------------------- JOSH
 // JOSH in three parts, so that a caller may run them in separate launches
 // (the ATLAS12 RT pass runs the 51x51 solve in its own kernel):
@@ -625,9 +496,9 @@ __device__ __forceinline__ void solve_scatter(WarpG& g, const JoshOps& ops, Josh
 //                   (atlas12_modules.f90:18491-18570); solve = max XALPHA > 0,
 //                   otherwise XS = XSBAR
 //   solve_scatter   (I - diag(XALPHA) COEFJ) XS = (1 - XALPHA) XSBAR
-//   g_josh_finish   XS floor, IFSURF = 1 surface flux or SNU = MAP1(XS),
-//                   the Eddington sweeps below MAXJ, J/H/K from the operators
-//                   mapped back onto the depths (:18571-18776)
+//   g_josh_finish   XS floor, SNU = MAP1(XS), J/H/K from the operators mapped
+//                   back onto the depths, the Eddington sweeps below MAXJ
+//                   (:18571-18776)
 // ws.abtot, ws.alpha and ws.snubar are formed by the caller (g_josh_fill).
 template <class G, class WS>
 __device__ inline void g_josh_fill(G& g, int nr, const double* acont, const double* aline, const double* sigmac,
@@ -641,41 +512,68 @@ __device__ inline void g_josh_fill(G& g, int nr, const double* acont, const doub
   g.sync();
 }
 
+// The grids every frequency of a launch shares, with their reciprocal
+// differences: RHOX and JOSH's 51-point tau grid.  One per CTA, in shared
+// memory; josh_grid_load by all its threads (it synchronises the CTA).
+struct JoshGrid {
+  double rhox[kKwMax], rrd[kKwMax], rr2[kKwMax];
+  double xtau[kNx], xrd[kNx], xr2[kNx];
+  __device__ __forceinline__ GridP rho() const { return GridP{rrd, rr2}; }
+  __device__ __forceinline__ GridP tau() const { return GridP{xrd, xr2}; }
+};
+__device__ __forceinline__ void josh_grid_load(JoshGrid& J, const JoshOps& ops, const double* rhox, int nr) {
+  for (int j = threadIdx.x; j < nr; j += blockDim.x) J.rhox[j] = rhox[j];
+  for (int l = threadIdx.x; l < kNx; l += blockDim.x) J.xtau[l] = ops.xtau[l];
+  recip_range(threadIdx.x, blockDim.x, rhox, J.rrd, J.rr2, nr);
+  recip_range(threadIdx.x, blockDim.x, ops.xtau, J.xrd, J.xr2, kNx);
+  __syncthreads();
+}
+
 // mapped: the surface is optically thin enough for the 51-point grid (MAP1
 // may still return MAXJ = 1 there, and IFSURF = 1 then takes H(1) from XS).
+// Leaves TAUNU's reciprocal differences in ws.rd and ws.r2.
 template <class G, class WS>
-__device__ inline int g_josh_prepare(G& g, const JoshOps& ops, const double* rhox, int nr, WS& ws, bool& mapped,
-                                     bool& solve) {
-  g_integ(g, rhox, ws.abtot, ws.taunu, nr, ws.abtot[0] * rhox[0], ws);
-  int maxj = 0;
+__device__ inline int g_josh_prepare(G& g, const JoshGrid& J, int nr, WS& ws, bool& mapped, bool& solve) {
+  g_integ(g, J.rhox, ws.abtot, ws.taunu, nr, ws.abtot[0] * J.rhox[0], ws.rd, J.rho());
+  recip_range(g.r, G::N, ws.taunu, ws.rd, ws.r2, nr);
+  g.sync();
   solve = false;
-  if (ws.taunu[0] > ops.xtau[kNx - 1]) maxj = 1;
-  mapped = maxj != 1;
-  if (mapped) {
-    maxj = g_map1(g, ws.taunu, ws.snubar, nr, ops.xtau, ws.xsbar, kNx, ws.lidx);
-    maxj = g_map1(g, ws.taunu, ws.alpha, nr, ops.xtau, ws.xalpha, kNx, ws.lidx);
-    const double tau1 = ws.taunu[0];
-    double amax = -1.0;
-    for (int l = g.r; l < kNx; l += G::N) {
-      double xa = fmax(ws.xalpha[l], 0.0);
-      double xb = fmax(ws.xsbar[l], 1.0e-38);
-      if (ops.xtau[l] < tau1) {
-        xb = fmax(ws.snubar[0], 1.0e-38);
-        xa = fmax(ws.alpha[0], 0.0);
-      }
-      ws.xalpha[l] = xa;
-      ws.xsbar[l] = xb;
-      amax = fmax(amax, xa);
+  const double tau1 = ws.taunu[0];
+  mapped = !(tau1 > J.xtau[kNx - 1]);
+  if (!mapped) return 1;
+  // SNUBAR and ALPHA onto the 51-point grid, one bracket and one set of
+  // differences for both; the surface values above the first depth's TAU
+  const GridP gr{ws.rd, ws.r2};
+  double amax = -1.0;
+  int last = 0;
+  for (int l = g.r; l < kNx; l += G::N) {
+    const double x = J.xtau[l];
+    last = map1_bracket(ws.taunu, nr, x);
+    double xa, xb;
+    if (x < tau1) {
+      xb = ws.snubar[0];
+      xa = ws.alpha[0];
+    } else {
+      const Map1At at(ws.taunu, nr, last, x, gr);
+      xb = at(ws.snubar);
+      xa = at(ws.alpha);
     }
-    amax = g.max(amax);
-    g.sync();
-    solve = amax > 0.0;
-    if (!solve) {
-      for (int l = g.r; l < kNx; l += G::N) ws.xs[l] = ws.xsbar[l];
-      g.sync();
-    }
+    xa = fmax(xa, 0.0);
+    xb = fmax(xb, 1.0e-38);
+    ws.xalpha[l] = xa;
+    ws.xsbar[l] = xb;
+    amax = fmax(amax, xa);
+    if (l == kNx - 1) ws.lidx[0] = last;
   }
-  return maxj;
+  amax = g.max(amax);
+  g.sync();
+  const int L = ws.lidx[0];
+  solve = amax > 0.0;
+  if (!solve) {
+    for (int l = g.r; l < kNx; l += G::N) ws.xs[l] = ws.xsbar[l];
+    g.sync();
+  }
+  return (L > nr ? nr : L) - 1;
 }
 
 // J - S and H on the 51-point grid from XS (COEFJ.XS - XS into xw, COEFH.XS
@@ -715,47 +613,50 @@ __device__ __forceinline__ void josh_operators(G& g, const JoshOps& ops, const d
   }
 }
 
-// ws.xs holds the solution (or XSBAR); ws.taunu, ws.alpha, ws.snubar as
-// g_josh_prepare left them.  full (JoshWSFull or a view with the same
-// members in shared memory) receives SNU, HNU, JMINS, JNU, KNU(1), MAXJ, or
-// is null for IFSURF = 1.  Returns the number of Eddington sweeps run.
-// kOpsGiven: the caller has floored XS and formed XW (J - S), XH (in
-// ws.xsbar) and KNU(1) with josh_operators already.
-template <bool kOpsGiven = false, class G, class WS, class FullT>
-__device__ inline int g_josh_finish(G& g, const JoshOps& ops, int nr, int maxj, bool mapped, WS& ws, FullT* full,
-                                    const double* bnu, double* hsurf) {
+// ws.xs holds the solution (or XSBAR); ws.taunu, ws.rd, ws.alpha, ws.snubar
+// as g_josh_prepare left them.  full (JoshWSFull or a view with the same
+// members in shared memory) receives SNU, HNU, JMINS, JNU, KNU(1), MAXJ.
+// hsurf_only (IFSURF = 1): only the surface flux HNU(1) is wanted; the caller
+// takes it from XS where the surface is mapped, so this is the unmapped case
+// (MAXJ = 1), and full needs only SNU, HNU and JMINS.  Returns the number of
+// Eddington sweeps run.
+template <bool hsurf_only = false, class G, class WS, class FullT>
+__device__ inline int g_josh_finish(G& g, const JoshGrid& J, const JoshOps& ops, int nr, int maxj, bool mapped, WS& ws,
+                                    FullT& F, const double* bnu) {
+  constexpr int C = (kKwMax + G::N - 1) / G::N;
+  double vj[C], vh[C];  // J - S and H of the thread's mapped depths
   if (mapped) {
-    if (!kOpsGiven) {
-      for (int l = g.r; l < kNx; l += G::N) ws.xs[l] = fmax(ws.xs[l], 1.0e-37);
+    for (int l = g.r; l < kNx; l += G::N) ws.xs[l] = fmax(ws.xs[l], 1.0e-37);
+    g.sync();
+    if (maxj != 1) {
+      josh_operators(g, ops, ws.xs, ws.xw, ws.xsbar, &F.knu1);  // XSBAR no longer needed: holds XH
       g.sync();
     }
-    if (full == nullptr) {
-      // IFSURF = 1: H(1) = sum CH_J * XS in the reference order
-      if (g.r == 0) {
-        double h = 0.0;
-        for (int m = 0; m < kNx; ++m) h = h + ops.ch[m] * ws.xs[m];
-        *hsurf = h;
+    // XS, J - S and H back onto the depths: one bracket for the three.  J and
+    // H go to memory after the sweeps, which use the same vectors below MAXJ.
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int j = g.r + c * G::N;
+      if (j >= maxj) break;
+      const double v = ws.taunu[j];
+      const Map1At at(J.xtau, kNx, map1_bracket(J.xtau, kNx, v), v, J.tau());
+      F.snu[j] = at(ws.xs);
+      if (maxj != 1) {
+        vj[c] = at(ws.xw);
+        vh[c] = at(ws.xsbar);
       }
-      g.sync();
-      return 0;
     }
-    g_map1(g, ops.xtau, ws.xs, kNx, ws.taunu, full->snu, maxj, ws.lidx);
+    g.sync();
   }
-  // JOSH with IFSURF = 1 and MAXJ = 1 falls through to the Eddington sweep
-  // IFSURF = 1 with an optically thick surface borrows the scratch vectors
-  // t1..t3 for SNU/HNU/JMINS (JNU is not needed beyond HNU(1)).
-  FullT* F = full;
   int sweeps = 0;
-  double* snu = F ? F->snu : ws.t1;
-  double* hnu = F ? F->hnu : ws.t2;
-  double* jmins = F ? F->jmins : ws.t3;
-  double* jnu = F ? F->jnu : nullptr;
+  double *snu = F.snu, *hnu = F.hnu, *jmins = F.jmins;
   if (maxj != nr) {
     const int maxj1 = (maxj == 1) ? 1 : maxj + 1;
     for (int j = maxj1 - 1 + g.r; j < nr; j += G::N) snu[j] = ws.snubar[j];
     g.sync();
     const int m = maxj - 1 > 1 ? maxj - 1 : 1;
     const int nm1 = nr - m + 1, nmj = nr - maxj + 1;
+    const GridP gm{ws.rd + m - 1, nullptr}, gj{ws.rd + maxj - 1, nullptr};
     for (int l = 1; l <= 50; ++l) {
       sweeps = l;
       // negative SNU -> reset to BNU
@@ -769,7 +670,7 @@ __device__ inline int g_josh_finish(G& g, const JoshOps& ops, int nr, int maxj, 
         }
         g.sync();
       }
-      g_deriv(g, ws.taunu + m - 1, snu + m - 1, hnu + m - 1, nm1);
+      g_deriv_on(g, ws.taunu + m - 1, snu + m - 1, hnu + m - 1, nm1, gm);
       bool hneg = false;
       for (int j = m - 1 + g.r; j < nr; j += G::N) hneg |= (hnu[j] <= 0.0);
       if (g.any(hneg)) {
@@ -779,16 +680,16 @@ __device__ inline int g_josh_finish(G& g, const JoshOps& ops, int nr, int maxj, 
           snu[j] = bnu[j];
         }
         g.sync();
-        g_deriv(g, ws.taunu + m - 1, snu + m - 1, hnu + m - 1, nm1);
+        g_deriv_on(g, ws.taunu + m - 1, snu + m - 1, hnu + m - 1, nm1, gm);
       }
       for (int j = m - 1 + g.r; j < nr; j += G::N) hnu[j] = hnu[j] / 3.0;
       g.sync();
-      g_deriv(g, ws.taunu + maxj - 1, hnu + maxj - 1, jmins + maxj - 1, nmj);
+      g_deriv_on(g, ws.taunu + maxj - 1, hnu + maxj - 1, jmins + maxj - 1, nmj, gj);
       double err = 0.0;
       for (int j = maxj1 - 1 + g.r; j < nr; j += G::N) {
         if (ifneg) jmins[j] = 0.0;
         const double jv = jmins[j] + snu[j];
-        if (jnu) jnu[j] = jv;
+        if (!hsurf_only) F.jnu[j] = jv;
         const double snew = (1.0 - ws.alpha[j]) * ws.snubar[j] + ws.alpha[j] * jv;
         err += fabs(snew - snu[j]) / snew;
         snu[j] = snew;
@@ -798,48 +699,39 @@ __device__ inline int g_josh_finish(G& g, const JoshOps& ops, int nr, int maxj, 
       if (err < 0.00001) break;
     }
   }
+  if (hsurf_only) return sweeps;
+  if (g.r == 0) F.maxj = maxj;
   if (maxj == 1) {
-    if (F) {
-      F->knu1 = jnu[0] / 3.0;
-      F->maxj = maxj;
-    } else if (g.r == 0) {
-      *hsurf = hnu[0];
-    }
+    if (g.r == 0) F.knu1 = F.jnu[0] / 3.0;
     g.sync();
     return sweeps;
   }
-  // (IFSURF = 1 never reaches here with MAXJ != 1: it returned above.)
-  if (!kOpsGiven) {
-    josh_operators(g, ops, ws.xs, ws.xw, ws.xsbar, &F->knu1);  // XSBAR no longer needed: holds XH
-    g.sync();
-  }
-  g_map1(g, ops.xtau, ws.xw, kNx, ws.taunu, F->jmins, maxj, ws.lidx);
-  g_map1(g, ops.xtau, ws.xsbar, kNx, ws.taunu, F->hnu, maxj, ws.lidx);
-  if (g.r == 0) F->maxj = maxj;
-  for (int j = g.r; j < maxj; j += G::N) {
-    F->snu[j] = fmax(F->snu[j], 1.0e-38);
-    F->jnu[j] = fmax(F->jmins[j] + F->snu[j], 1.0e-38);
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int j = g.r + c * G::N;
+    if (j >= maxj) break;
+    jmins[j] = vj[c];
+    hnu[j] = vh[c];
+    snu[j] = fmax(snu[j], 1.0e-38);
+    F.jnu[j] = fmax(vj[c] + snu[j], 1.0e-38);
   }
   g.sync();
   return sweeps;
 }
 
-// The whole of JOSH by one group.  Inputs in ws.*: abtot/alpha/snubar are
-// formed here from the opacity vectors.  rhox is shared by the CTA.
-// ifsurf = 1 returns H(1); ifsurf = 0 fills full (SNU, JNU, HNU, JMINS,
-// KNU(1), MAXJ) as the reference does.  A: shared-memory matrix for a warp
-// group, the U rows for a pair group.  Returns the number of Eddington
-// sweeps run (0 if none).
+// The whole of JOSH (IFSURF = 0) by a pair group.  ws.abtot/alpha/snubar are
+// formed here from the opacity vectors; the grids are shared by the CTA.
+// U: the pivot rows.  Returns the number of Eddington sweeps run.
 template <class G>
-__device__ inline int g_josh(G& g, const JoshOps& ops, const double* rhox, int nr, const double* acont,
+__device__ inline int g_josh(G& g, const JoshGrid& J, const JoshOps& ops, int nr, const double* acont,
                              const double* aline, const double* sigmac, const double* sigmal,
                              const double* scont, const double* sline, const double* bnu, JoshWS& ws,
-                             double* A, JoshWSFull* full, double* hsurf) {
+                             double* U, JoshWSFull& full) {
   g_josh_fill(g, nr, acont, aline, sigmac, sigmal, scont, sline, ws);
   bool mapped, solve;
-  const int maxj = g_josh_prepare(g, ops, rhox, nr, ws, mapped, solve);
-  if (solve) solve_scatter(g, ops, ws, A);
-  return g_josh_finish(g, ops, nr, maxj, mapped, ws, full, bnu, hsurf);
+  const int maxj = g_josh_prepare(g, J, nr, ws, mapped, solve);
+  if (solve) solve_scatter(g, ops, ws, U);
+  return g_josh_finish(g, J, ops, nr, maxj, mapped, ws, full, bnu);
 }
 
 }  // namespace atlasgpu
