@@ -149,7 +149,7 @@ int rt_launch(atlasgpu_ctx* ctx, RtArgs& a, double* d_sum, int* nwarps_out) {
   double *part, *rec;
   int r;
   if ((r = bufT(ctx, "rt_part", (size_t)nwl * (kAcc * a.kw + 1), &part))) return r;
-  if ((r = bufT(ctx, "rt_rec", (size_t)a.numnu * a.rec_stride, &rec))) return r;
+  if ((r = bufT(ctx, "rt_rec", rt_rec_doubles(a.numnu, a.kw), &rec))) return r;
   a.partial = part;
   a.rec = rec;
   CK(rt_split_attributes(a.nrhox));
@@ -157,7 +157,7 @@ int rt_launch(atlasgpu_ctx* ctx, RtArgs& a, double* d_sum, int* nwarps_out) {
     Timer tm(ctx, "atlas_rt");
     k_rt_pre<<<sh.pre_blocks, kRtSplitWarps * 32, rt_pre_smem_bytes(), ctx->stream>>>(a);
     CKL(ctx);
-    k_rt_series<<<sh.solve_blocks, kScatterThreads, 0, ctx->stream>>>(a);
+    k_rt_series<<<sh.series_blocks, kScatterThreads, 0, ctx->stream>>>(a);
     CKL(ctx);
     k_rt_solve<<<sh.solve_blocks, kScatterThreads, scatter_smem_bytes(), ctx->stream>>>(a);
     CKL(ctx);

@@ -49,7 +49,7 @@ struct BatchDev {
   const double* cgfmax;                        // [nspec] largest CGF per species (shared line list)
   double* tabcont;                             // [B][nwave+1][kw]
   double* partial;                             // [B][nwl][kAcc*kw+1]
-  double* rt_rec;                              // [B][numnu][rt_rec_stride(kw)] split RT pass records
+  double* rt_rec;                              // [B][rt_rec_doubles(numnu, kw)] split RT pass records
   double* sum;                                 // [B][kAcc*kw+1]
   double* hist;                                // [B][kHist]
   double* hsurf;                               // [B][numnu] HNU(1) of the last iteration
@@ -274,7 +274,7 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
       unsigned long long* work = work_counters(ctx, 3);
       {
         Timer t2(ctx, "batch_rt_solve");
-        k_batch_rt_series<<<dim3(sh.solve_blocks, nb), kScatterThreads, 0, s>>>(B->ra, B->d.ctl, work);
+        k_batch_rt_series<<<dim3(sh.series_blocks, nb), kScatterThreads, 0, s>>>(B->ra, B->d.ctl, work);
         CKL(ctx);
         k_batch_rt_solve<<<dim3(sh.solve_blocks, nb), kScatterThreads, scatter_smem_bytes(), s>>>(B->ra,
                                                                                                  B->d.ctl, work);
@@ -403,7 +403,7 @@ int atlasgpu_batch_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* dsc, int
       (r = balloc(ctx, &d.rho, (size_t)nb * kw)) || (r = balloc(ctx, &d.cc, (size_t)nb * kw)) ||
       (r = balloc(ctx, &d.acont, nb * nnk)) || (r = balloc(ctx, &d.sigmac, nb * nnk)) ||
       (r = balloc(ctx, &d.xl, nb * nnk)) || (r = balloc(ctx, &d.tabcont, (size_t)nb * (B->nwave + 1) * kw)) ||
-      (r = balloc(ctx, &d.sum, nb * stride)) || (r = balloc(ctx, &d.rt_rec, nb * (size_t)B->numnu * rt_rec_stride(kw))) ||
+      (r = balloc(ctx, &d.sum, nb * stride)) || (r = balloc(ctx, &d.rt_rec, nb * rt_rec_doubles(B->numnu, kw))) ||
       (r = balloc(ctx, &d.hist, (size_t)nb * kHist)) || (r = balloc(ctx, &d.hsurf, nb * (size_t)B->numnu)) ||
       (r = balloc(ctx, &B->waveset, B->numnu)) ||
       (r = balloc(ctx, &B->rcoset, B->numnu)) || (r = balloc(ctx, &B->cutwave, B->nwave)) ||
@@ -456,7 +456,7 @@ int atlasgpu_batch_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* dsc, int
     ra[b] = RtArgs{ctx->ops, B->numnu, B->nrhox, kw, B->waveset, B->rcoset, d.acont + on, d.sigmac + on, nullptr,
                    d.xl + on, ms[b].rhox, ms[b].t, d.hkt + o, 0.0, 1, 1, kw, nullptr,
                    d.hsurf + (size_t)b * B->numnu, nullptr};
-    ra[b].rec = d.rt_rec + (size_t)b * B->numnu * rt_rec_stride(kw);
+    ra[b].rec = d.rt_rec + (size_t)b * rt_rec_doubles(B->numnu, kw);
   }
   B->ra_host = ra;
   CK(cudaMemcpyAsync(d.ctl, ctl.data(), nb * sizeof(BatchCtl), cudaMemcpyHostToDevice, s));

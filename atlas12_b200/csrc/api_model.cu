@@ -38,7 +38,7 @@ struct atlasgpu_model {
   unsigned long long* cnt;
   int nwl;                 // partial-sum rows allocated
   RtSplitShape rt_sh;      // launch shape of the split RT pass over the shard
-  double* rt_rec;          // the split pass's per-frequency records [numnu][rt_rec_stride(kw)]
+  double* rt_rec;          // the split pass's per-frequency records [rt_rec_doubles(numnu, kw)]
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int graph_precision = -1;  // precision the captured graph was built with
@@ -173,7 +173,7 @@ int enqueue_begin(atlasgpu_ctx* ctx, atlasgpu_model* m, bool timed) {
     Timer tm(ctx, "atlas_rt");
     k_rt_pre<<<sh.pre_blocks, kRtSplitWarps * 32, rt_pre_smem_bytes(), s>>>(ra);
     CKL(ctx);
-    k_rt_series<<<sh.solve_blocks, kScatterThreads, 0, s>>>(ra);
+    k_rt_series<<<sh.series_blocks, kScatterThreads, 0, s>>>(ra);
     CKL(ctx);
     k_rt_solve<<<sh.solve_blocks, kScatterThreads, scatter_smem_bytes(), s>>>(ra);
     CKL(ctx);
@@ -338,7 +338,7 @@ int atlasgpu_model_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* d, atlas
   rt_shape(ctx, m);
   m->nwl = rt_split_rows_max(m->numnu, ctx->nsm, 4);
   if ((r = dalloc(ctx, &m->partial, (size_t)m->nwl * (kAcc * kw + 1))) ||
-      (r = dalloc(ctx, &m->rt_rec, (size_t)m->numnu * rt_rec_stride(kw)))) {
+      (r = dalloc(ctx, &m->rt_rec, rt_rec_doubles(m->numnu, kw)))) {
     atlasgpu_model_destroy(ctx, m);
     return r;
   }

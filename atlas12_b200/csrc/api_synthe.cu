@@ -139,6 +139,10 @@ int atlasgpu_set_operators(atlasgpu_ctx* ctx, const double* xtau8, const double*
   memcpy(h.ck, ck_j, sizeof h.ck);
   memcpy(h.coefj, coefj, sizeof h.coefj);
   memcpy(h.coefh, coefh, sizeof h.coefh);
+  for (int l = 0; l < kNx; ++l) {
+    h.rowabs[l] = 0.0;
+    for (int m = 0; m < kNx; ++m) h.rowabs[l] += fabs(coefj[m * kNx + l]);
+  }
   cudaSetDevice(ctx->device);
   CK(cudaMemcpyAsync(ctx->ops, &h, sizeof h, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -386,7 +390,7 @@ int atlasgpu_synthe_line_opacity(atlasgpu_ctx* ctx, const atlasgpu_lte_line* lin
 static int spectrum_launch(atlasgpu_ctx* ctx, SpecArgs a) {
   const int chunk = std::min(a.length, kSpecChunk);
   int r;
-  if ((r = bufT(ctx, "spec_rec", (size_t)2 * chunk * kSpecStride, &a.rec))) return r;
+  if ((r = bufT(ctx, "spec_rec", scatter_rec_doubles((size_t)2 * chunk, kSpecStride), &a.rec))) return r;
   CK(cudaFuncSetAttribute(k_spec_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spec_smem_bytes()));
   CK(cudaFuncSetAttribute(k_spec_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes()));
   Timer tm(ctx, "josh_spectrum");
@@ -395,13 +399,10 @@ static int spectrum_launch(atlasgpu_ctx* ctx, SpecArgs a) {
     const int pre = std::min((a.n + kSpecWarps - 1) / kSpecWarps, ctx->nsm * 8);
     k_spec_pre<<<pre, kSpecWarps * 32, spec_smem_bytes(), ctx->stream>>>(a);
     CKL(ctx);
-    // about four resident waves of pair groups, consecutive systems per group
-    const int groups = ctx->nsm * 8 * 4;
-    a.per = std::max(1, (2 * a.n + groups - 1) / groups);
-    const int blocks = ((2 * a.n + a.per - 1) / a.per + kScatterGroups - 1) / kScatterGroups;
-    k_spec_series<<<blocks, kScatterThreads, 0, ctx->stream>>>(a);
+    a.per_series = scatter_series_per(2 * a.n, ctx->nsm, 1);
+    k_spec_series<<<scatter_series_blocks(2 * a.n, a.per_series), kScatterThreads, 0, ctx->stream>>>(a);
     CKL(ctx);
-    k_spec_solve<<<blocks, kScatterThreads, scatter_smem_bytes(), ctx->stream>>>(a);
+    k_spec_solve<<<scatter_solve_blocks(2 * a.n, ctx->nsm), kScatterThreads, scatter_smem_bytes(), ctx->stream>>>(a);
     CKL(ctx);
     k_spec_flux<<<(a.n + 255) / 256, 256, 0, ctx->stream>>>(a);
     CKL(ctx);
@@ -420,7 +421,7 @@ int atlasgpu_synthe_spectrum_dev(atlasgpu_ctx* ctx, const double* d_wledge, int 
     return fail(ctx, ATLASGPU_EINVAL, "synthe_spectrum: bad argument");
   cudaSetDevice(ctx->device);
   SpecArgs a{ctx->ops, d_wledge, d_contabs, d_contscat, d_rhox, d_hkt, nedge, stride, nrhox, length,
-             wbegin, ratio, d_opac, d_flux, d_cont, nullptr, 0, 0, 1};
+             wbegin, ratio, d_opac, d_flux, d_cont, nullptr, 0, 0, kSeriesN};
   return spectrum_launch(ctx, a);
 }
 

@@ -732,7 +732,7 @@ struct RtArgs {
   // group (nu_per_warp is the post warps', one partial row per post warp)
   double* rec = nullptr;
   int rec_stride = 0;
-  int nu_per_pre = 1, nu_per_solve = 1;
+  int nu_per_pre = 1, nu_per_series = kSeriesN;
   // work counters of the solve stage (timed launches only, else null):
   // [0] systems eliminated, [1] systems summed as a series, [2] series steps
   unsigned long long* work = nullptr;
@@ -935,6 +935,8 @@ struct RtRec {
   __host__ __device__ int solve() const { return kw + 3 * kNx + 1; }
 };
 __host__ __device__ inline int rt_rec_stride(int kw) { return (kw + 3 * kNx + 2 + 1) & ~1; }
+// doubles of the record buffer of a pass over numnu frequencies
+__host__ __device__ inline size_t rt_rec_doubles(int numnu, int kw) { return scatter_rec_doubles(numnu, rt_rec_stride(kw)); }
 
 // STIM, BNU and JOSH's ABTOT, ALPHA, SNUBAR (SIGMAL = 0, SLINE = BNU) of one
 // depth at frequency NU, as the fused kernel forms them (RUN_RT_PASS
@@ -996,12 +998,15 @@ __device__ __forceinline__ double* rt_rec(const RtArgs& a, int nu) {
   return a.rec + (size_t)(nu - a.nu_first) * a.rec_stride;
 }
 
+__device__ __forceinline__ ScatterArgs rt_scatter_args(const RtArgs& a);
+
 static __device__ __forceinline__ void rt_pre_body(const RtArgs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RtShared& R = *reinterpret_cast<RtShared*>(smem_raw);
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   RtPreWS& S = reinterpret_cast<RtPreWS*>(smem_raw + sizeof(RtShared))[wid];
   rt_shared_load(R, a);
+  if (blockIdx.x == 0 && threadIdx.x == 0) scatter_reset(rt_scatter_args(a));
   WarpG g(lane);
   const int nr = a.nrhox, kw = a.kw;
   const int w = blockIdx.x * kRtSplitWarps + wid;
@@ -1044,8 +1049,10 @@ static __device__ __forceinline__ void rt_pre_body(const RtArgs& a) {
 __device__ __forceinline__ ScatterArgs rt_scatter_args(const RtArgs& a) {
   const RtRec Q{a.kw};
   const int last = a.nu_last > 0 ? a.nu_last : a.numnu;
-  return ScatterArgs{a.ops, a.rec, a.rec_stride, Q.xalpha(), Q.xsbar(), Q.xs(), Q.solve(), last - a.nu_first + 1,
-                     a.nu_per_solve, a.work};
+  ScatterArgs s{a.ops, a.rec, a.rec_stride, Q.xalpha(), Q.xsbar(), Q.xs(), Q.solve(), last - a.nu_first + 1,
+                a.nu_per_series, nullptr, nullptr, a.work};
+  scatter_lists(s, a.numnu);
+  return s;
 }
 
 static __device__ __forceinline__ void rt_post_body(const RtArgs& a) {
@@ -1123,7 +1130,8 @@ static __global__ void __launch_bounds__(kRtSplitWarps * 32, 4) k_rt_post(RtArgs
 // (NB slots of a batch share it): every stage gets about WAVES resident waves
 // of its units (warps or pair groups), frequencies contiguous per unit.
 struct RtSplitShape {
-  int pre_per = 1, pre_blocks = 1, solve_per = 1, solve_blocks = 1, post_per = 1, post_blocks = 1;
+  int pre_per = 1, pre_blocks = 1, post_per = 1, post_blocks = 1;
+  int series_per = kSeriesN, series_blocks = 1, solve_blocks = 1;
   int rows() const { return post_blocks * kRtSplitWarps; }
 };
 inline void rt_split_fit(int len, int units, int per_block, int& per, int& blocks) {
@@ -1139,7 +1147,9 @@ inline RtSplitShape rt_split_shape(int len, int nsm, int nb, int waves) {
     return (int)(u < 1 ? 1 : u);
   };
   rt_split_fit(len, units(16), kRtSplitWarps, sh.pre_per, sh.pre_blocks);
-  rt_split_fit(len, units(8), kScatterGroups, sh.solve_per, sh.solve_blocks);
+  sh.series_per = scatter_series_per(len, nsm, nb);
+  sh.series_blocks = scatter_series_blocks(len, sh.series_per);
+  sh.solve_blocks = scatter_solve_blocks(len, nsm);
   rt_split_fit(len, units(16), kRtSplitWarps, sh.post_per, sh.post_blocks);
   return sh;
 }
@@ -1161,7 +1171,7 @@ inline cudaError_t rt_split_attributes(int nrhox) {
 }
 inline void rt_split_args(RtArgs& a, const RtSplitShape& sh) {
   a.nu_per_pre = sh.pre_per;
-  a.nu_per_solve = sh.solve_per;
+  a.nu_per_series = sh.series_per;
   a.nu_per_warp = sh.post_per;
   a.rec_stride = rt_rec_stride(a.kw);
 }

@@ -33,6 +33,7 @@ struct JoshOps {
   double ck[kNx];
   double coefj[kNx * kNx];  // column-major
   double coefh[kNx * kNx];
+  double rowabs[kNx];  // row sums of |COEFJ| (the scattering systems' contraction bound)
 };
 
 // gfortran's REAL(8)**INTEGER (libgcc binary exponentiation), host and device

@@ -2,46 +2,65 @@
 //
 // The RT pass and the SYNTHE spectrum prepare one record per system (XALPHA,
 // XSBAR and a solve flag, `stride` doubles apart) and solve them here, in two
-// launches that split the systems by their contraction bound.  Both launches
-// read the same flags and form the bound the same way.
+// launches: scatter_series_body sums the Neumann series of every system
+// it settles, scatter_solve_body eliminates what is left as SOLVIT does.
 //
-// The system X = (1 - XALPHA) XSBAR + XALPHA (COEFJ X) is a
-// contraction with factor q = max_l XALPHA(l) sum_m |COEFJ(l,m)| (the
-// infinity norm of diag(XALPHA) COEFJ).  Where q <= kScatterSeriesQ
-// its Neumann series is summed instead of eliminating: K steps of
-// X <- (1 - XALPHA) XSBAR + XALPHA (COEFJ X) from X = (1 - XALPHA) XSBAR
-// leave an error of at most q^(K+1) |X|, and K is taken so that
-// q^(K+1) <= 2^-60, far below the rounding of the elimination itself (the
-// two solutions agree to rounding).  A step is one matrix-vector product
-// with no sequential dependence between rows and one barrier, against the
-// elimination's 50 dependent pivot steps, so the series is cheaper up to
-// q ~ 0.5.  Systems with larger q (strongly scattering layers) are
-// eliminated as SOLVIT does.
+// X = b + M X with b = (1 - XALPHA) XSBAR and M = diag(XALPHA) COEFJ is summed
+// as X = sum d_k, d_0 = b, d_(k+1) = M d_k.  A system is settled
+//   * by norm: q^(k+1) <= 2^-60 with q = max_l XALPHA(l) sum_m |COEFJ(l,m)| <= 1/2
+//     (the rest is at most q^(k+1) |X|), or
+//   * by its residual, which is the next increment: b + M X - X = d_(k+1), so the
+//     error is (I - M)^-1 d_(k+1), at most |d_(k+1)| / (1 - q); settled when
+//     d_(k+1) <= 2^-60 (1 - q) X in every row, q < 1.
+// Both bounds are in the infinity norm, and far below the elimination's rounding.
+// The norm bound counts the strongly scattering surface rows as if they fed
+// themselves; they feed on deeper ones with small XALPHA, and the spectral
+// radius of M is far smaller (0.04 where q = 0.49 in a solar spectrum at
+// 400 nm).  Measured, the 83,800 systems of a 35 nm spectrum: 1.32 ms one system
+// at a time from broadcast loads, 1.17 ms by matrix instructions with the norm
+// bound alone, 0.38 ms with both.
+// What 32 steps do not settle (spectral radius above ~0.27 at q > 1/2) is listed
+// and eliminated.  The list spreads those systems, which are neighbours in
+// frequency, over the GPU.  More steps hold the whole group of a slow system:
+// 64 and 192 steps, or a second round of up to 192 for the left-overs in groups
+// of their own, made the scattering stage of a 32-slot iteration 9.8, 15.7 and
+// 10.7 ms against 8.8 with 32.
 #pragma once
 #include "josh.cuh"
 
 namespace atlasgpu {
 
 // Records of n systems: system i at rec + i * stride, the 51-point vectors at
-// the offsets xalpha, xsbar, xs, the flag (1: solve) at solve; per: systems
-// of one group (consecutive).  work (timed launches only, else null):
-// [0] systems eliminated, [1] systems summed as a series, [2] series steps.
+// the offsets xalpha, xsbar, xs, the flag (1: solve) at solve; per_series:
+// (consecutive) systems of one group of the series.  left, *nleft: the systems
+// the series leaves over (zeroed by scatter_reset before it).  work (timed launches only, else
+// null): [0] systems eliminated, [1] systems summed as a series, [2] series steps.
 struct ScatterArgs {
   const JoshOps* ops;
   double* rec;
-  int stride, xalpha, xsbar, xs, solve, n, per;
+  int stride, xalpha, xsbar, xs, solve, n, per_series;
+  int* left;
+  unsigned* nleft;
   unsigned long long* work;
 };
+// doubles of a record buffer for cap systems, the list behind the records
+__host__ __device__ inline size_t scatter_rec_doubles(size_t cap, size_t stride) { return cap * stride + (cap + 1) / 2 + 1; }
+__host__ __device__ inline void scatter_lists(ScatterArgs& a, size_t cap) {
+  a.nleft = reinterpret_cast<unsigned*>(a.rec + cap * a.stride);
+  a.left = reinterpret_cast<int*>(a.nleft + 2);
+}
+// by one thread of the launch before the series
+__device__ __forceinline__ void scatter_reset(const ScatterArgs& a) { *a.nleft = 0; }
 
 constexpr int kScatterGroups = 2;  // pair groups per CTA
 constexpr int kScatterThreads = kScatterGroups * PairG::N;
 constexpr int kScatterSolveMinBlocks = 4;  // 8 systems per SM (128 registers per thread)
-constexpr double kScatterSeriesQ = 0.5;
-constexpr int kScatterMaxSteps = 64;
+constexpr double kScatterSeriesQ = 0.5;  // largest q that is settled by norm
+constexpr int kScatterMaxSteps = 64;     // ... within this many steps
+constexpr int kScatterTrySteps = 32;      // most steps where only the residual can tell
 
 struct ScatterWS {
   double xs[kNx], xsbar[kNx], xalpha[kNx], piv[kNx];
-  double rowabs[kNx];  // row sums of |COEFJ| (the contraction bound's factors)
   double red[8];
   unsigned pk[4][3];
   alignas(16) double U[kNx * (kNx + 1)];
@@ -73,26 +92,15 @@ static __device__ __forceinline__ void scatter_solve_body(const ScatterArgs& a) 
   ScatterWS& S = reinterpret_cast<ScatterWS*>(smem_raw)[gid];
   PairG g(threadIdx.x % PairG::N, 1 + gid, S.red);
   const JoshOps& ops = *a.ops;
-  const int i0 = (blockIdx.x * kScatterGroups + gid) * a.per, i1 = min(i0 + a.per, a.n);
-  for (int l = g.r; l < kNx; l += PairG::N) {
-    double r = 0.0;
-    for (int m = 0; m < kNx; ++m) r += fabs(ops.coefj[m * kNx + l]);
-    S.rowabs[l] = r;
-  }
-  g.sync();
+  const int n = (int)*a.nleft;
   unsigned long long nelim = 0;
-  for (int i = i0; i < i1; ++i) {
-    double* rec = a.rec + (size_t)i * a.stride;
-    if (rec[a.solve] != 1.0) continue;  // the same word for the whole group
-    double qv = 0.0;
+  for (int i = blockIdx.x * kScatterGroups + gid; i < n; i += gridDim.x * kScatterGroups) {
+    double* rec = a.rec + (size_t)a.left[i] * a.stride;
     for (int l = g.r; l < kNx; l += PairG::N) {
-      const double xa = rec[a.xalpha + l];
-      S.xalpha[l] = xa;
+      S.xalpha[l] = rec[a.xalpha + l];
       S.xsbar[l] = rec[a.xsbar + l];
-      qv = fmax(qv, xa * S.rowabs[l]);
     }
-    const double q = g.max(qv);  // (its barrier also publishes XALPHA, XSBAR)
-    if (q <= kScatterSeriesQ) continue;  // summed by scatter_series_body
+    g.sync();
     solve_scatter(g, ops, S, S.U);
     ++nelim;
     scatter_store<kSurf>(g, a, rec, g.r < kNx ? S.xs[g.r] : 0.0);
@@ -101,69 +109,203 @@ static __device__ __forceinline__ void scatter_solve_body(const ScatterArgs& a) 
   if (a.work && g.r == 0 && nelim) atomicAdd(a.work, nelim);
 }
 
-// The Neumann series of the systems with q <= kScatterSeriesQ: thread l of a
-// pair group keeps row l of COEFJ in registers for the whole launch (it is the
-// same for every system), so a step is 51 FMAs on registers and the
-// broadcast reads of X from shared memory, with no loads of COEFJ.  Sum k of
-// the four partial sums takes the terms m = k, k+4, ... in that order; q is
-// formed as in scatter_solve_body, so the two split the systems the same
-// way.  (The series inside the elimination's kernel, reading COEFJ from L1 every step,
-// took 2.6k cycles per step at eight groups per SM.)
+// The series, eight systems at a time by a pair of warps: a step is the product
+// of COEFJ (51 x 51, padded to 56 x 52) with the eight vectors (52 x 8), in FP64
+// matrix instructions (m8n8k4, which reach the FP64 pipe's 64 multiply-adds per
+// clock and SM from one warp per scheduler).  COEFJ's fragments stay in
+// registers for the whole launch, warp 0 of the pair holding rows 0..31 and
+// warp 1 rows 32..55; the vectors go through shared memory once per step
+// ([row][system]: fragment loads and result stores are both conflict-free).
+// Bounded by the FP64 pipe: 23.3k multiply-adds per step of eight systems.
+// A group runs the largest step count of its eight: further steps only add
+// ever smaller terms.
 constexpr int kScatterSeriesMinBlocks = 3;
+constexpr int kSeriesN = 8;                       // systems per group
+constexpr int kSeriesRows = 56, kSeriesK = 13;    // padded rows, 4-wide slices of the 52 columns
+constexpr int kSeriesTiles = 4;                   // 8-row tiles of warp 0 (warp 1 has three)
 struct ScatterSeriesWS {
-  alignas(16) double xa[kNx + 1];
-  alignas(16) double xb[kNx + 1];
-  double red[8];
+  alignas(16) double x[2][kSeriesRows][kSeriesN];
+  double part[3][2][kSeriesN];  // the two warps' parts of three reductions over rows (bound, settled, surface flux)
+  int done[2][2];               // by parity of the step: a warp's rows are settled
 };
+
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+// Launch shape of the series over n systems with 1/nb of the GPU: whole groups
+// of eight, about two resident waves of warp pairs (six per SM at 168 registers).
+inline int scatter_series_per(int n, int nsm, int nb) {
+  const int units = nsm * 2 * kScatterSeriesMinBlocks * kScatterGroups / (nb > 0 ? nb : 1);
+  const int batches = (n + kSeriesN - 1) / kSeriesN;
+  return kSeriesN * ((batches + (units > 0 ? units : 1) - 1) / (units > 0 ? units : 1));
+}
+inline int scatter_series_blocks(int n, int per) {
+  return ((n + per - 1) / per + kScatterGroups - 1) / kScatterGroups;
+}
+
+// CTAs of the elimination (they walk the list with a grid stride; one without work ends at once)
+inline int scatter_solve_blocks(int n, int nsm) {
+  const int need = (n + kScatterGroups - 1) / kScatterGroups, most = nsm * kScatterSolveMinBlocks;
+  return need < most ? need : most;
+}
 
 template <bool kSurf>
 static __device__ __forceinline__ void scatter_series_body(const ScatterArgs& a) {
   __shared__ ScatterSeriesWS s_ws[kScatterGroups];
+  const JoshOps& ops = *a.ops;
   const int gid = threadIdx.x / PairG::N;
   ScatterSeriesWS& S = s_ws[gid];
-  PairG g(threadIdx.x % PairG::N, 1 + gid, S.red);
-  const JoshOps& ops = *a.ops;
-  const int l = g.r;
-  const bool own = l < kNx;
-  double c[kNx];
-  double rowabs = 0.0;
+  PairG g(threadIdx.x % PairG::N, 1 + gid, nullptr);
+  const int lane = g.r & 31, warp = g.r >> 5;
+  const int tr = lane >> 2, tc = lane & 3;  // result fragment: row tr of a tile, systems 2 tc and 2 tc + 1
+  const int ntile = warp == 0 ? kSeriesTiles : kSeriesRows / 8 - kSeriesTiles;
+  const int row0 = warp * kSeriesTiles * 8 + tr;  // this lane's row of tile t: row0 + 8 t
+  double cf[kSeriesTiles][kSeriesK];
 #pragma unroll
-  for (int m = 0; m < kNx; ++m) c[m] = own ? ops.coefj[m * kNx + l] : 0.0;
-  for (int m = 0; m < kNx; ++m) rowabs += fabs(own ? ops.coefj[m * kNx + l] : 0.0);
-  const int i0 = (blockIdx.x * kScatterGroups + gid) * a.per, i1 = min(i0 + a.per, a.n);
+  for (int t = 0; t < kSeriesTiles; ++t) {
+    const int row = row0 + 8 * t;
+#pragma unroll
+    for (int k = 0; k < kSeriesK; ++k) {
+      const int m = 4 * k + tc;
+      cf[t][k] = (t < ntile && row < kNx && m < kNx) ? ops.coefj[m * kNx + row] : 0.0;
+    }
+  }
+  const int i0 = (blockIdx.x * kScatterGroups + gid) * a.per_series, i1 = min(i0 + a.per_series, a.n);
   unsigned long long nseries = 0, nsteps = 0;
-  for (int i = i0; i < i1; ++i) {
-    double* rec = a.rec + (size_t)i * a.stride;
-    if (rec[a.solve] != 1.0) continue;  // the same word for the whole group
-    const double al = own ? rec[a.xalpha + l] : 0.0;
-    const double xb = own ? rec[a.xsbar + l] : 0.0;
-    double qv = 0.0;
-    if (own) qv = fmax(qv, al * rowabs);
-    const double q = g.max(qv);
-    if (q > kScatterSeriesQ) continue;  // eliminated by scatter_solve_body
-    const int K = scatter_series_steps(q);
-    const double b = own ? (1.0 - al) * xb : 0.0;
-    double* cur = S.xa;
-    double* nxt = S.xb;
-    if (own) cur[l] = b;
-    for (int k = 0; k < K; ++k) {
-      g.sync();
-      if (own) {
-        double s4[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int ib = i0; ib < i1; ib += kSeriesN) {
+    // the lane's two systems: XALPHA and d_0 of its rows, 0 where there is nothing to sum
+    bool want[2];
+    double al[kSeriesTiles][2], x[kSeriesTiles][2], qv[2] = {0.0, 0.0};
 #pragma unroll
-        for (int m = 0; m < kNx; ++m) s4[m & 3] = s4[m & 3] + c[m] * cur[m];
-        nxt[l] = b + al * ((s4[0] + s4[1]) + (s4[2] + s4[3]));
+    for (int e = 0; e < 2; ++e) {
+      const int i = ib + 2 * tc + e;
+      const double* rec = a.rec + (size_t)i * a.stride;
+      want[e] = i < i1 && rec[a.solve] == 1.0;
+#pragma unroll
+      for (int t = 0; t < kSeriesTiles; ++t) {
+        const int row = row0 + 8 * t;
+        const bool on = want[e] && t < ntile && row < kNx;
+        al[t][e] = on ? rec[a.xalpha + row] : 0.0;
+        x[t][e] = on ? (1.0 - al[t][e]) * rec[a.xsbar + row] : 0.0;
+        if (on) qv[e] = fmax(qv[e], al[t][e] * ops.rowabs[row]);
       }
-      double* t = cur;
-      cur = nxt;
-      nxt = t;
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) qv[e] = fmax(qv[e], __shfl_xor_sync(0xffffffffu, qv[e], o));
+      if (tr == 0) S.part[0][warp][2 * tc + e] = qv[e];
     }
     g.sync();
-    scatter_store<kSurf>(g, a, rec, own ? cur[l] : 0.0);
-    ++nseries;
-    nsteps += K;
+    int cap[2], K = 0;  // steps after which the system is settled by norm; else given up
+    bool norm[2], had[2] = {want[0], want[1]};
+    double tol[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const double q = fmax(S.part[0][0][2 * tc + e], S.part[0][1][2 * tc + e]);
+      norm[e] = !(q > kScatterSeriesQ);
+      want[e] = want[e] && !(q >= 1.0);
+      tol[e] = 0x1p-60 * (1.0 - q);
+      cap[e] = !want[e] ? 0 : (norm[e] ? scatter_series_steps(q) : kScatterTrySteps);
+      K = max(K, cap[e]);
+#pragma unroll
+      for (int t = 0; t < kSeriesTiles; ++t)
+        if (!want[e]) al[t][e] = x[t][e] = 0.0;
+    }
+    K = __reduce_max_sync(0xffffffffu, K);  // the same for both warps
+#pragma unroll
+    for (int t = 0; t < kSeriesTiles; ++t)
+      if (t < ntile) *reinterpret_cast<double2*>(&S.x[0][row0 + 8 * t][2 * tc]) = make_double2(x[t][0], x[t][1]);
+    bool ok[2] = {true, true};  // this lane's rows are settled by the residual
+    int k = 0;
+    for (; k < K; ++k) {
+      g.sync();
+      if (k > 0 && S.done[k & 1][0] && S.done[k & 1][1]) break;
+      const double(*cur)[kSeriesN] = S.x[k & 1];
+      double y[kSeriesTiles][2];
+#pragma unroll
+      for (int t = 0; t < kSeriesTiles; ++t) y[t][0] = y[t][1] = 0.0;
+#pragma unroll
+      for (int kk = 0; kk < kSeriesK; ++kk) {
+        const double bf = cur[4 * kk + tc][tr];
+#pragma unroll
+        for (int t = 0; t < kSeriesTiles; ++t)
+          if (t < ntile) dmma(y[t][0], y[t][1], cf[t][kk], bf);
+      }
+      ok[0] = ok[1] = true;
+#pragma unroll
+      for (int t = 0; t < kSeriesTiles; ++t) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double dn = al[t][e] * y[t][e];
+          x[t][e] += dn;
+          ok[e] = ok[e] && fabs(dn) <= tol[e] * fabs(x[t][e]);
+          y[t][e] = dn;
+        }
+        if (t < ntile)
+          *reinterpret_cast<double2*>(&S.x[(k + 1) & 1][row0 + 8 * t][2 * tc]) = make_double2(y[t][0], y[t][1]);
+      }
+      const int done = __all_sync(0xffffffffu, (ok[0] || k + 1 >= cap[0]) && (ok[1] || k + 1 >= cap[1]));
+      if (lane == 0) S.done[(k + 1) & 1][warp] = done;
+    }
+    // settled: by norm within the steps run, or by the residual in every row
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const unsigned rows = 0x11111111u << tc;  // the lanes with this lane's systems
+      const bool all = (__ballot_sync(0xffffffffu, ok[e]) & rows) == rows;
+      if (tr == 0) S.part[1][warp][2 * tc + e] = all ? 1.0 : 0.0;
+    }
+    g.sync();
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      want[e] = want[e] && ((norm[e] && k >= cap[e]) ||
+                            (S.part[1][0][2 * tc + e] != 0.0 && S.part[1][1][2 * tc + e] != 0.0));
+    if (a.work && warp == 0 && tr == 0) {
+      nseries += (unsigned)want[0] + (unsigned)want[1];
+      nsteps += (unsigned long long)k * ((unsigned)want[0] + (unsigned)want[1]);
+    }
+    if (warp == 0 && tr == 0) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (had[e] && !want[e]) a.left[atomicAdd(a.nleft, 1u)] = ib + 2 * tc + e;
+    }
+    if (kSurf) {
+      double h[2] = {0.0, 0.0};
+#pragma unroll
+      for (int t = 0; t < kSeriesTiles; ++t) {
+        const int row = row0 + 8 * t;
+        if (t >= ntile || row >= kNx) continue;
+        const double ch = ops.ch[row];
+        h[0] += ch * fmax(x[t][0], 1.0e-37);
+        h[1] += ch * fmax(x[t][1], 1.0e-37);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) h[e] += __shfl_xor_sync(0xffffffffu, h[e], o);
+        if (tr == 0) S.part[2][warp][2 * tc + e] = h[e];
+      }
+      g.sync();
+      if (warp == 0 && tr == 0) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (want[e])
+            a.rec[(size_t)(ib + 2 * tc + e) * a.stride + a.xs] = S.part[2][0][2 * tc + e] + S.part[2][1][2 * tc + e];
+      }
+      g.sync();
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (want[e]) {
+          double* rec = a.rec + (size_t)(ib + 2 * tc + e) * a.stride + a.xs;
+#pragma unroll
+          for (int t = 0; t < kSeriesTiles; ++t)
+            if (t < ntile && row0 + 8 * t < kNx) rec[row0 + 8 * t] = x[t][e];
+        }
+      g.sync();
+    }
   }
-  if (a.work && g.r == 0 && nseries) {
+  if (a.work && nseries) {
     atomicAdd(a.work + 1, nseries);
     atomicAdd(a.work + 2, nsteps);
   }

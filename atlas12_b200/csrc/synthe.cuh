@@ -510,10 +510,13 @@ struct SpecArgs {
   double *flux, *cont;
   double* rec;        // [2 * chunk][kSpecStride]: wavelength i's continuum system at 2i, total at 2i+1
   int iw0, n;         // the round's wavelengths iw0 .. iw0 + n - 1
-  int per;            // systems per solve group
+  int per_series;     // systems per group of the series
 };
 __device__ __forceinline__ ScatterArgs spec_scatter_args(const SpecArgs& a) {
-  return ScatterArgs{a.ops, a.rec, kSpecStride, 0, kNx, kSpecXs, kSpecSolve, 2 * a.n, a.per, nullptr};
+  ScatterArgs s{a.ops, a.rec, kSpecStride, 0, kNx, kSpecXs, kSpecSolve, 2 * a.n, a.per_series, nullptr, nullptr,
+                nullptr};
+  scatter_lists(s, 2 * (size_t)a.n);
+  return s;
 }
 
 static __global__ void __launch_bounds__(kSpecWarps * 32, 4) k_spec_pre(SpecArgs a) {
@@ -524,6 +527,7 @@ static __global__ void __launch_bounds__(kSpecWarps * 32, 4) k_spec_pre(SpecArgs
   SpecWS& S = reinterpret_cast<SpecWS*>(smem_raw + sizeof(JoshGrid))[wid];
   const int nr = a.nrhox;
   josh_grid_load(J, *a.ops, a.rhox, nr);
+  if (blockIdx.x == 0 && threadIdx.x == 0) scatter_reset(spec_scatter_args(a));
   constexpr int C = (kKwMax + 31) / 32;
   for (int i = blockIdx.x * kSpecWarps + wid; i < a.n; i += gridDim.x * kSpecWarps) {
     const int iw = a.iw0 + i;
