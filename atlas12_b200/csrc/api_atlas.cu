@@ -270,7 +270,8 @@ int atlasgpu_atlas_linop(atlasgpu_ctx* ctx, const int32_t* linedata, int64_t n, 
                 d_cnt + 1};
     // exact fixed-point sums (fix_add): per-species CGF maxima, per-depth scales
     unsigned long long *d_fix, *d_cgf;
-    double *d_fs, *d_fu;
+    int* d_fs;
+    double* d_fu;
     if ((r = bufT(ctx, "al_fix", (size_t)kFixWords * kw * numnu, &d_fix)) || (r = bufT(ctx, "al_cgf", nspec, &d_cgf)) ||
         (r = bufT(ctx, "al_fs", kw, &d_fs)) || (r = bufT(ctx, "al_fu", kw, &d_fu)))
       return r;
@@ -379,8 +380,8 @@ int atlasgpu_atlas_xlinop(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* recs, int
                 (const double*)ctx->bufs["tab_h2"].first, (const float4*)ctx->bufs["tab_hf"].first, d_xl, nullptr,
                 nullptr, 1, 0, 2000, 0.5642, d_lc, d_em};
     Timer tm(ctx, "atlas_xlinop");
-    if (ctx->precision == ATLASGPU_PREC_MIXED) k_atlas_linop<true><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
-    else k_atlas_linop<false><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
+    if (ctx->precision == ATLASGPU_PREC_MIXED) k_xlinop_walk<true><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
+    else k_xlinop_walk<false><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
     CKL(ctx);
     if (pops) {
       double *d_xp, *d_rho;

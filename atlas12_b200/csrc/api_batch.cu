@@ -45,7 +45,8 @@ struct BatchDev {
   ContCoef* cc;                                // [B][kw]
   double *acont, *sigmac, *xl;                 // [B][numnu][kw]
   unsigned long long* xfix;                    // [B][numnu][3][kw] LINOP1's exact sums
-  double *fscale, *funscale;                   // [B][kw] their per-depth scale
+  int* fscale;                                 // [B][kw] the exponents k of their per-depth scales 2^k
+  double* funscale;                            // [B][kw] 2^-k
   const double* cgfmax;                        // [nspec] largest CGF per species (shared line list)
   double* tabcont;                             // [B][nwave+1][kw]
   double* partial;                             // [B][nwl][kAcc*kw+1]
@@ -99,13 +100,11 @@ __global__ void k_batch_kapp(BatchDev d) {
 // 2.27 ms per model-iteration.)
 // kDry: the counting pass of a timed iteration (the same walks, no adds)
 template <bool F32, bool kDry = false>
-__global__ void __launch_bounds__(256, kLinopMinBlocks) k_batch_linop(const LinopArgs* __restrict__ args, const BatchCtl* ctl,
-                                                                      unsigned long long* work) {
+__global__ void __launch_bounds__(256, kLinopMinBlocks) k_batch_linop(const __grid_constant__ LinopArgs a,
+                                                                      const BatchCtl* ctl) {
   const int b = blockIdx.y;
   if (!running(ctl, b)) return;
-  LinopArgs a = args[b];
-  a.work = work;
-  linop_body<F32, kDry>(a);
+  linop_body<F32, kDry>(a, b);
 }
 
 // the split RT pass (k_rt_pre / k_rt_solve / k_rt_post bodies) per running slot
@@ -192,7 +191,7 @@ struct atlasgpu_batch {
   double *ross = nullptr, *state = nullptr;
   int32_t *iwavetab = nullptr, *linedata = nullptr;
   AtlasLine* lines = nullptr;
-  LinopArgs* la = nullptr;
+  LinopArgs la{};  // slot 0's, with the slots' strides
   RtArgs* ra = nullptr;
   unsigned long long* cnt = nullptr;
   int grid_linop = 1, grid_kapp = 1;
@@ -228,6 +227,7 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
     CKL(ctx);
   }
   if (B->nlines > 0) {
+    LinopArgs la = B->la;
     if (ctx->timing) {
       // the atomics the exact sums issue, counted by a pass that walks the
       // same wings and adds nothing (the numerator of LINOP1's roofline; the
@@ -235,10 +235,11 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
       unsigned long long* dry;
       if (bufT(ctx, "linop_dry_cnt", 2, &dry) == 0 &&
           cudaMemsetAsync(dry, 0, 2 * sizeof(unsigned long long), s) == cudaSuccess) {
+        la.work = dry;
         if (ctx->precision == ATLASGPU_PREC_MIXED)
-          k_batch_linop<true, true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(B->la, B->d.ctl, dry);
+          k_batch_linop<true, true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
         else
-          k_batch_linop<false, true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(B->la, B->d.ctl, dry);
+          k_batch_linop<false, true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
         CKL(ctx);
         unsigned long long h[2] = {0, 0};
         CK(cudaMemcpyAsync(h, dry, sizeof h, cudaMemcpyDeviceToHost, s));
@@ -246,16 +247,16 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
         ctx->kwork["batch_linop_atomics"] = (double)h[1];
       }
     }
-    unsigned long long* work = work_counters(ctx, 1);
+    la.work = work_counters(ctx, 1);
     {
       Timer tm(ctx, "batch_linop");
       if (ctx->precision == ATLASGPU_PREC_MIXED)
-        k_batch_linop<true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(B->la, B->d.ctl, work);
+        k_batch_linop<true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
       else
-        k_batch_linop<false><<<dim3(B->grid_linop, nb), 256, 0, s>>>(B->la, B->d.ctl, work);
+        k_batch_linop<false><<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
       CKL(ctx);
     }
-    work_collect(ctx, work, {"batch_linop_points"});
+    work_collect(ctx, la.work, {"batch_linop_points"});
     {
       Timer tm(ctx, "batch_fixfin");
       k_batch_fixfin<<<dim3(B->grid_kapp, nb), 256, 0, s>>>(B->d);
@@ -358,7 +359,7 @@ int atlasgpu_batch_destroy(atlasgpu_ctx* ctx, atlasgpu_batch* B) {
   void* ps[] = {d.xfix, d.fscale, d.funscale, (void*)d.cgfmax,
                 d.ctl, d.ms, d.R, d.xnfdop, d.dopple, d.xne_eos, d.txnxn, d.hkt, d.hckt, d.rho, d.cc, d.acont,
                 d.sigmac, d.xl, d.tabcont, d.partial, d.rt_rec, d.sum, d.hist, d.hsurf, B->waveset, B->rcoset, B->cutwave, B->h0,
-                B->h1, B->h2, B->hf, B->ross, B->state, B->iwavetab, B->linedata, B->lines, B->la, B->ra, B->cnt};
+                B->h1, B->h2, B->hf, B->ross, B->state, B->iwavetab, B->linedata, B->lines, B->ra, B->cnt};
   for (void* p : ps)
     if (p) cudaFree(p);
   delete B;
@@ -411,7 +412,7 @@ int atlasgpu_batch_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* dsc, int
       (r = balloc(ctx, &B->h1, 2001)) || (r = balloc(ctx, &B->h2, 2001)) || (r = balloc(ctx, &B->hf, 2001)) ||
       (r = balloc(ctx, &B->ross, (size_t)nb * 3 * kRossMax)) || (r = balloc(ctx, &B->state, (size_t)nb * kNState * kw)) ||
       (r = balloc(ctx, &B->linedata, (size_t)B->nlines * 4)) || (r = balloc(ctx, &B->lines, (size_t)B->nlines)) ||
-      (r = balloc(ctx, &B->la, nb)) || (r = balloc(ctx, &B->ra, nb)) || (r = balloc(ctx, &B->cnt, 2)) ||
+      (r = balloc(ctx, &B->ra, nb)) || (r = balloc(ctx, &B->cnt, 2)) ||
       (r = balloc(ctx, &d.xfix, (size_t)kFixWords * nb * nnk)) || (r = balloc(ctx, &d.fscale, (size_t)nb * kw)) ||
       (r = balloc(ctx, &d.funscale, (size_t)nb * kw)) || (r = balloc(ctx, (double**)&d.cgfmax, (size_t)B->nspec))) {
     atlasgpu_batch_destroy(ctx, B);
@@ -434,7 +435,6 @@ int atlasgpu_batch_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* dsc, int
   std::vector<BatchCtl> ctl(nb);
   std::vector<ModelState> ms(nb);
   std::vector<RossStore> R(nb);
-  std::vector<LinopArgs> la(nb);
   std::vector<RtArgs> ra(nb);
   for (int b = 0; b < nb; ++b) {
     ctl[b] = BatchCtl{ATLASGPU_SLOT_IDLE, 0, 0, 0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0};
@@ -447,22 +447,24 @@ int atlasgpu_batch_create(atlasgpu_ctx* ctx, const atlasgpu_model_desc* dsc, int
     ms[b].maxerr = 0.0;
     double* rs = B->ross + (size_t)b * 3 * kRossMax;
     R[b] = RossStore{0, kRossMax, 0.0, 1.0, 0.0, 1.0, rs, rs + kRossMax, rs + 2 * kRossMax};
-    const size_t o = (size_t)b * kw, os = (size_t)b * nsk, on = (size_t)b * nnk;
-    la[b] = LinopArgs{B->lines, B->nlines, B->nrhox, kw, B->nspec, B->numnu, d.xnfdop + os, d.dopple + os,
-                      d.xne_eos + o, d.txnxn + o, d.hckt + o, d.tabcont + (size_t)b * (B->nwave + 1) * kw,
-                      B->waveset, B->h0, B->h1, B->h2, B->hf, d.xl + on, nullptr, B->cnt};
-    la[b].xfix = d.xfix + kFixWords * on;
-    la[b].fscale = d.fscale + o;
+    const size_t o = (size_t)b * kw, on = (size_t)b * nnk;
     ra[b] = RtArgs{ctx->ops, B->numnu, B->nrhox, kw, B->waveset, B->rcoset, d.acont + on, d.sigmac + on, nullptr,
                    d.xl + on, ms[b].rhox, ms[b].t, d.hkt + o, 0.0, 1, 1, kw, nullptr,
                    d.hsurf + (size_t)b * B->numnu, nullptr};
     ra[b].rec = d.rt_rec + (size_t)b * rt_rec_doubles(B->numnu, kw);
   }
   B->ra_host = ra;
+  B->la = LinopArgs{B->lines, B->nlines, B->nrhox, kw, B->nspec, B->numnu, d.xnfdop, d.dopple, d.xne_eos, d.txnxn,
+                    d.hckt, d.tabcont, B->waveset, B->h0, B->h1, B->h2, B->hf, d.xl, nullptr, B->cnt};
+  B->la.xfix = d.xfix;
+  B->la.fscale = d.fscale;
+  B->la.s_spec = nsk;
+  B->la.s_kw = kw;
+  B->la.s_tab = (size_t)(B->nwave + 1) * kw;
+  B->la.s_xl = nnk;
   CK(cudaMemcpyAsync(d.ctl, ctl.data(), nb * sizeof(BatchCtl), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d.ms, ms.data(), nb * sizeof(ModelState), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d.R, R.data(), nb * sizeof(RossStore), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(B->la, la.data(), nb * sizeof(LinopArgs), cudaMemcpyHostToDevice, s));
 
   CK(cudaMemsetAsync(B->state, 0, (size_t)nb * kNState * kw * sizeof(double), s));
   CK(cudaMemsetAsync(d.xnfdop, 0, nb * nsk * sizeof(double), s));

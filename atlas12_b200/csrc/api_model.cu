@@ -27,7 +27,8 @@ struct atlasgpu_model {
   AtlasLine* lines;
   double* xl;            // XLINES(J, NU): [numnu][kw]
   unsigned long long* xfix;  // LINOP1's exact fixed-point sums [numnu][3][kw]
-  double *fscale, *funscale;  // their per-depth scale [kw]
+  int* fscale;             // the exponents k of their per-depth scales 2^k [kw]
+  double* funscale;        // 2^-k [kw]
   unsigned long long* cgfmax;  // largest CGF per species [nspec] (FP64 bit patterns)
   double *partial, *sum, *hsurf;
   double *h0, *h1, *h2, *ross;  // ross: ROSSTAB points [3][kRossMax]
@@ -53,7 +54,7 @@ namespace {
 __global__ void k_model_eos(ModelState* ms, const int* iter_dev, int nrhox, int kw, double grav,
                             double vturb_cms, double mh, double* xnfdop, double* dopple, double* xne_eos,
                             double* txnxn, double* hkt, double* hckt, double* rho, ContCoef* cc, int nspec,
-                            const double* cgfmax, double* fscale, double* funscale) {
+                            const double* cgfmax, int* fscale, double* funscale) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nrhox) return;
   model_eos_depth(ms, *iter_dev + 1, j, kw, grav, vturb_cms, mh, xnfdop, dopple, xne_eos, txnxn, hkt, hckt, rho,

@@ -251,17 +251,64 @@ static __global__ void __launch_bounds__(256) k_xlinop_shore(XShoreArgs a) {
 // (J, NU) at ((NU-1)*3 + w)*kw + J-1): a warp's lanes at consecutive
 // depths add to consecutive words.
 constexpr int kFixWords = 3;
-constexpr double kFixTop = 0x1p-96, kFixMid = 0x1p-48;
 
-__device__ __forceinline__ void fix_add(unsigned long long* w, int wstride, double y) {
-  const double t2 = floor(y * kFixTop);
-  const double r2 = y - t2 * 0x1p96;  // exact: the bits of y below 2^96
-  const double t1 = floor(r2 * kFixMid);
-  const double r1 = r2 - t1 * 0x1p48;  // exact: the bits below 2^48
-  const double t0 = rint(r1);          // the one rounding, to the unit 2^-k
-  if (t2 > 0.0) atomicAdd(w + 2 * wstride, (unsigned long long)t2);
-  if (t1 > 0.0) atomicAdd(w + wstride, (unsigned long long)t1);
-  if (t0 > 0.0) atomicAdd(w, (unsigned long long)t0);
+// Adds value * 2^k (the words of one (J, NU) wstride apart).  The value's
+// mantissa is an integer at bit position p of the fixed-point number: one word
+// index, one shift and up to three pieces, in integer arithmetic (as floors and
+// conversions of FP64 values the split cost more than the profile itself).
+// Bits below the unit round to nearest, ties to even.  Returns the number of
+// words touched; kDry: adds nothing.
+template <bool kDry>
+__device__ __forceinline__ int fix_put(unsigned long long* w, int wstride, unsigned long long m, int p) {
+  constexpr unsigned long long m48 = (1ull << 48) - 1;
+  if (p < 0) {  // below the unit: the one rounding
+    const int r = -p;
+    if (r > 54) return 0;
+    const unsigned long long q = m >> r, rest = m & ((1ull << r) - 1), half = 1ull << (r - 1);
+    m = q + (unsigned long long)(rest > half || (rest == half && (q & 1ull)));
+    p = 0;
+  }
+  // nothing reaches past the third word: the values are below 2^140 (and a value
+  // that is not finite, in a model that has left the physical range, is dropped)
+  if (p >= 96) {
+    if (p >= 96 + __clzll((long long)m)) return 0;
+    if (!kDry) atomicAdd(w + 2 * wstride, m << (p - 96));
+    return 1;
+  }
+  const int k = p >= 48 ? 1 : 0, sh = p - 48 * k;
+  const unsigned long long lo = (m << sh) & m48, rest = m >> (48 - sh);
+  const unsigned long long mid = k ? rest : rest & m48, hi = k ? 0ull : rest >> 48;
+  w += k * wstride;
+  if (!kDry) {
+    if (lo) atomicAdd(w, lo);
+    if (mid) atomicAdd(w + wstride, mid);
+    if (hi) atomicAdd(w + 2 * wstride, hi);
+  }
+  return (lo != 0) + (mid != 0) + (hi != 0);
+}
+template <bool kDry>
+__device__ __forceinline__ int fix_add(unsigned long long* w, int wstride, double v, int k) {
+  constexpr unsigned long long m48 = (1ull << 48) - 1;
+  const long long b = __double_as_longlong(v);
+  const int e = (int)(b >> 52), p = e - 1075 + k;
+  // a normal value whose pieces lie in the words of bit 0..143; the rest is rare
+  if (e < 1 || p < 0 || p >= 92) {
+    if (b <= 0 || (e == 0 && k < 1000)) return 0;  // zero (values are never negative) or far below the unit
+    const unsigned long long f = (unsigned long long)b & ((1ull << 52) - 1);
+    return fix_put<kDry>(w, wstride, e ? f | (1ull << 52) : f, (e ? e : 1) - 1075 + k);
+  }
+  const unsigned long long m = ((unsigned long long)b & ((1ull << 52) - 1)) | (1ull << 52);
+  const bool up = p >= 48;
+  const int sh = up ? p - 48 : p;
+  const unsigned long long lo = (m << sh) & m48, rest = m >> (48 - sh);
+  const unsigned long long mid = rest & m48;
+  w += up ? wstride : 0;
+  if (!kDry) {
+    if (lo) atomicAdd(w, lo);
+    if (mid) atomicAdd(w + wstride, mid);
+    if (rest >> 48) atomicAdd(w + 2 * wstride, rest >> 48);  // (p < 48 only: above, MID has at most 48 bits)
+  }
+  return (lo != 0) + (mid != 0) + ((rest >> 48) != 0);
 }
 
 // The exact integer x2 2^96 + x1 2^48 + x0, rounded to nearest FP64, times unscale (a power of 2)
@@ -311,22 +358,22 @@ __host__ __device__ inline double fix_to_double(unsigned long long x0, unsigned 
   return ldexp(d, e) * unscale;
 }
 
-// The scale 2^k of depth j: every value added there is at most
+// The exponent k of depth j's scale 2^k, and 2^-k: every value added there is at most
 // CGF(line) * XNFDOP(J, NELION) (the Boltzmann factor and the profile are at
 // most 1; 8x margin), so the largest value maps below 2^140 and a bin's
 // words stay below 2^64.  cgfmax: the largest CGF of each species' lines.
 __device__ inline void fix_scale_depth(const double* xnfdop, int nspec, int kw, int j, const double* cgfmax,
-                                       double* scale, double* unscale) {
+                                       int* scale, double* unscale) {
   double bound = 0.0;
   for (int s = 0; s < nspec; ++s) bound = fmax(bound, cgfmax[s] * xnfdop[(size_t)s * kw + j]);
   if (!(bound > 0.0) || !(bound < 1e300)) {
-    scale[j] = 1.0;
+    scale[j] = 0;
     unscale[j] = 1.0;
     return;
   }
   int e;
   frexp(bound, &e);  // bound < 2^e
-  scale[j] = ldexp(1.0, 137 - e);
+  scale[j] = 137 - e;
   unscale[j] = ldexp(1.0, e - 137);
 }
 
@@ -358,30 +405,15 @@ struct LinopArgs {
   const double* emerge = nullptr;
   // work counter (timed launches only, else null): wing points added into XLINES
   unsigned long long* work = nullptr;
-  // exact fixed-point XLINES (see fix_add): words [numnu][3][kw] and the
-  // per-depth scale; null: FP64 atomics into xl (XLINOP adds to a caller's XLINES)
+  // LINOP1: exact fixed-point XLINES (see fix_add), words [numnu][3][kw] and the
+  // per-depth exponents of their scale (XLINOP adds FP64 atomics into a caller's XLINES)
   unsigned long long* xfix = nullptr;
-  const double* fscale = nullptr;
+  const int* fscale = nullptr;
+  // a batch's slots: the per-model arrays above are slot 0's, slot b's lie b
+  // strides further (the arguments stay in the constant bank; copied per slot
+  // they went through local memory)
+  size_t s_spec = 0, s_kw = 0, s_tab = 0, s_xl = 0;  // [nspec][kw], [kw], TABCONT, [numnu][kw]
 };
-
-// Adds one wing value into XLINES(J, IW).  kDry: adds nothing and returns
-// the number of atomics the add would issue (the counting pass of a timed
-// measurement; the walk is the same), else returns 0.
-template <bool kDry>
-__device__ __forceinline__ int linop_add(const LinopArgs& a, int J, int iw, double cv) {
-  if (kDry) {
-    if (!a.xfix) return 1;
-    const double y = cv * a.fscale[J - 1];
-    const double t2 = floor(y * kFixTop);
-    const double r2 = y - t2 * 0x1p96;
-    const double t1 = floor(r2 * kFixMid);
-    const double t0 = rint(r2 - t1 * 0x1p48);
-    return (t2 > 0.0) + (t1 > 0.0) + (t0 > 0.0);
-  }
-  if (a.xfix) fix_add(a.xfix + ((size_t)(iw - 1) * kFixWords) * a.kw + (J - 1), a.kw, cv * a.fscale[J - 1]);
-  else atomicAdd(a.xl + (size_t)(iw - 1) * a.kw + (J - 1), cv);
-  return 0;
-}
 
 // LINOP1's profile value at one wing point, V = (distance in nm) * RDOP with
 // RDOP = 1 / (DOPPLE * WLVAC) taken once per (line, depth): tabulated H(v, a)
@@ -391,144 +423,195 @@ __device__ __forceinline__ int linop_add(const LinopArgs& a, int J, int iw, doub
 // from FP32 copies of the tables (hf = H0, H1, H2); V, the table index and
 // the regime tests stay FP64, so every point uses the table entry the FP64
 // walk uses.
-static __device__ __noinline__ double linop_full_voigt(const LinopArgs& a, double vv, double adamp) {
-  return voigt_kurucz(vv, adamp, a.h0, a.h1, a.h2);
+static __device__ __noinline__ double linop_near_voigt(const double* h0, const double* h1, const double* h2, double vv,
+                                                       double adamp) {
+  return voigt_kurucz(vv, adamp, h0, h1, h2);
+}
+__device__ __forceinline__ double linop_full_voigt(const LinopArgs& a, double vv, double adamp) {
+  if (adamp <= 1.4 && adamp + vv <= 3.2) return linop_near_voigt(a.h0, a.h1, a.h2, vv, adamp);
+  return voigt_far(vv, adamp);
 }
 
-template <bool F32>
-__device__ __forceinline__ double linop_cv(const LinopArgs& a, double center, double adamp, double dl, double rdop) {
-  const double vv = dl * rdop;
-  if (adamp > 0.20) return center * linop_full_voigt(a, vv, adamp);
+// one (line, depth) walk's constants
+struct LinopPair {
+  double center, adamp, rdop, tc;
+  float cf, la, tlo, thi;  // F32: CENTER, LORENTZ * ADAMP; TABCONT less and more 2e-5
+  int kexp;
+};
+
+__device__ __forceinline__ double linop_cv64(const LinopArgs& a, const LinopPair& w, double vv) {
+  if (w.adamp > 0.20) return w.center * linop_full_voigt(a, vv, w.adamp);
   // written as !(vv <= 10): a V that is not a number (a non-finite model
   // structure) takes the Lorentz branch and never reaches the table index
-  if (!(vv <= 10.0)) {
-    if (F32) return (double)((float)center * ((float)(a.lorentz * adamp) * __frcp_rn((float)(vv * vv))));
-    return center * a.lorentz * adamp / (vv * vv);
-  }
+  if (!(vv <= 10.0)) return w.center * a.lorentz * w.adamp / (vv * vv);
   const int iv = (int)(vv * 200.0 + 1.5);
-  if (F32) {
-    const float4 h = a.hf[iv - 1];
-    const float af = (float)adamp;
-    return (double)((float)center * fmaf(fmaf(h.z, af, h.y), af, h.x));
-  }
-  return center * ((a.h2[iv - 1] * adamp + a.h1[iv - 1]) * adamp + a.h0[iv - 1]);
+  return w.center * ((a.h2[iv - 1] * w.adamp + a.h1[iv - 1]) * w.adamp + a.h0[iv - 1]);
 }
 
-// The wing walk stops at the first point whose value is below TABCONT.  In
-// FP32 a value within 1e-5 of the threshold is re-evaluated in FP64 for the
-// decision, so both precisions stop at the same point.
+// The value of one wing point (vv >= 0) of a lane that is walking (act), and
+// whether it is below TABCONT, which ends the walk.  The decision is the FP64
+// value's in both precisions: an FP32 value within 2e-5 of the threshold is
+// evaluated again.
 template <bool F32>
-__device__ __forceinline__ bool linop_below(const LinopArgs& a, double cv, double tc, double center, double adamp,
-                                            double dl, double rdop) {
-  if (F32 && fabs(cv - tc) <= 1.0e-5 * tc) return linop_cv<false>(a, center, adamp, dl, rdop) < tc;
-  return cv < tc;
+__device__ __forceinline__ double linop_value(const LinopArgs& a, const LinopPair& w, double vv, bool act,
+                                              bool& below) {
+  if (!F32) {
+    const double cv = act ? linop_cv64(a, w, vv) : 0.0;
+    below = cv < w.tc;
+    return cv;
+  }
+  // the Lorentz wing for every lane, then the few that need the table or the full profile
+  float f = w.cf * (w.la * __frcp_rn((float)(vv * vv)));
+  if (act && vv <= 10.0 && !(w.adamp > 0.20)) {
+    const float4 h = a.hf[(int)(vv * 200.0 + 1.5) - 1];
+    const float af = (float)w.adamp;
+    f = w.cf * fmaf(fmaf(h.z, af, h.y), af, h.x);
+  }
+  double cv = (double)f;
+  below = f < w.tlo;
+  bool sure = below || f > w.thi;
+  if (act && w.adamp > 0.20) {
+    cv = w.center * linop_full_voigt(a, vv, w.adamp);
+    below = cv < w.tc;
+    sure = true;
+  }
+  if (act && !sure) below = linop_cv64(a, w, vv) < w.tc;
+  return cv;
 }
 
-// The rest of one (line, depth) walk after a lane gave up on it, by the
-// whole warp (lanes over wing points), add-then-test as in the reference:
-// red points rnext..iwmax unless rdone, blue offsets bnext..100 unless bdone.
-template <bool F32, bool kDry>
-static __device__ __noinline__ unsigned linop_finish_warp(const LinopArgs& a, int J, double center, double adamp,
-                                                          double rdop, double wlvac, int nu, double tc, int rnext,
-                                                          bool rdone, int bnext, bool bdone, double wcon, int lane,
-                                                          unsigned long long& atoms) {
-  unsigned added = 0;  // points this lane added
-  const int iwmax = min(nu + a.max_wing, a.numnu);
-  const int nuh = a.nu_hi > 0 ? a.nu_hi : a.numnu;
-  if (!rdone) {
-    for (int base = rnext; base <= iwmax; base += 32) {
-      const int iw = base + lane;
-      const bool valid = iw <= iwmax;
-      double cv = 0.0;
-      bool below = false;
-      if (valid) {
-        const double dl = a.waveset[iw - 1] - wlvac;
-        cv = linop_cv<F32>(a, center, adamp, dl, rdop);
-        below = linop_below<F32>(a, cv, tc, center, adamp, dl, rdop);
-      }
-      const unsigned stop = __ballot_sync(0xffffffffu, valid && below);
-      const int last = stop ? base + __ffs(stop) - 1 : iwmax;
-      if (valid && iw <= last && iw >= a.nu_lo && iw <= nuh) {
-        atoms += linop_add<kDry>(a, J, iw, cv);
-        ++added;
-      }
-      if (stop) break;
-    }
+// The rest of one XLINOP (record, depth) walk on one side by the whole warp
+// (lanes over wing points), each point added, then tested: points iw0, iw0 + dir,
+// ..., np of them.
+template <bool F32>
+static __device__ __noinline__ void linop_finish_warp(const LinopArgs& a, const LinopPair w, int J, double wlvac,
+                                                      int iw0, int dir, int np, double wcon, int lane) {
+  for (int s0 = 0; s0 < np; s0 += 32) {
+    const int s = s0 + lane, iw = iw0 + dir * s;
+    // a blue wing ends before the continuum edge
+    const bool valid = s < np && !(dir < 0 && a.waveset[iw - 1] < wcon);
+    bool below = false;
+    const double vv = valid ? fabs(a.waveset[iw - 1] - wlvac) * w.rdop : 0.0;
+    const double cv = linop_value<F32>(a, w, vv, valid, below);
+    const unsigned stop = __ballot_sync(0xffffffffu, valid && below);
+    const unsigned inval = __ballot_sync(0xffffffffu, !valid);
+    const int last = stop ? s0 + __ffs(stop) - 1 : np;
+    if (valid && s <= last) atomicAdd(a.xl + (size_t)(iw - 1) * a.kw + (J - 1), cv);
+    if (stop || inval) break;
   }
-  if (!bdone) {
-    for (int i0 = bnext; i0 <= a.max_wing; i0 += 32) {
-      const int i = i0 + lane;
-      const int iw = nu - i;
-      // the walk ends before the grid start and (XLINOP) before the continuum edge
-      const bool valid = i <= a.max_wing && iw >= 1 && !(a.waveset[iw - 1] < wcon);
-      double cv = 0.0;
-      bool below = false;
-      if (valid) {
-        const double dl = wlvac - a.waveset[iw - 1];
-        cv = linop_cv<F32>(a, center, adamp, dl, rdop);
-        below = linop_below<F32>(a, cv, tc, center, adamp, dl, rdop);
-      }
-      const unsigned stop = __ballot_sync(0xffffffffu, valid && below);
-      const unsigned inval = __ballot_sync(0xffffffffu, !valid);
-      const int ilast = stop ? i0 + __ffs(stop) - 1 : a.max_wing;
-      if (valid && i <= ilast && iw >= a.nu_lo && iw <= nuh) {
-        atoms += linop_add<kDry>(a, J, iw, cv);
-        ++added;
-      }
-      if (stop || inval) break;
-    }
-  }
-  return added;
 }
 
-// Warp per line, lane per depth.  Most (line, depth) wing walks stop after a
-// few points (the C2 grid is ~50 Doppler widths per step), so each lane
-// walks its own depth's red and blue wings for up to kLinopLanePts points,
-// and the walks still going are finished by the whole warp.  Lanes of a
-// warp touch XLINES(J, IW) at consecutive J: one coalesced atomic per step.
+// Warp per line, lane per depth.  The lanes of a warp walk both wings of the
+// line together, one frequency per wing and step: the frequency is the same for
+// all lanes (one broadcast load of WAVESET, coalesced adds to XLINES at
+// consecutive J), and a lane drops out of a wing at its own last point.  Two
+// thirds of the walks end after one point per side, and neighbouring depths
+// walk about as far (41-62 % of the lanes of a step are active on models of
+// 4000-7500 K).  Bounded by instruction issue.  The former loop of 16 steps,
+// with the fixed-point split in FP64 and every longer walk finished by the whole
+// warp with lanes over points, took 2.31 ms per model-iteration of the 32-slot
+// batch of 500,000 lines and 30,000 frequencies (1.5e9 warp instructions); now
+// 1.19 ms (one model of 500,000 lines, FP64: 3.41 to 1.91 ms).  Tried and not
+// kept: padding WAVESET instead of testing its ends, an FP32-only loop for rounds
+// without a full VOIGT, a 24-bit split for FP32 values (1.20 ms together, the
+// larger loop costs in instruction fetch what it saves), the table test peeled
+// into a loop of its own (1.51 ms), 48 or 80 registers (1.32, 1.32 ms).
+// XLINOP's wings reach 2000 points: when at most kLinopFew lanes are left after
+// kLinopLanePts steps, the warp finishes them one at a time, lanes over points.
+// (LINOP1 with that from step 16 on: 2.12 ms with at most 4 lanes left, 2.31 with
+// 8, against 1.72 without at the time; its adds do not coalesce.)
 // A warp takes kLinopChunk consecutive lines at a time, so the warps of a
 // CTA work on neighbouring lines (the lines are in wavelength order) and
 // share the WAVESET window and the XLINES lines they touch in cache.
-// Measured on the 500,000-line, 30,000-frequency pass (solar / cool model):
-// 4 points per lane and one line per warp 4.45 / 5.49 ms; 16 points, chunks
-// of 8 lines and four CTAs per SM (64 registers) 3.74 / 4.80 ms.  In the
-// 32-slot batch of one model (per model-iteration, solar / cool giant): 16
-// points 2.42 / 3.39 ms, 32 points 2.36 / 3.39, 64 points 2.31 / 3.39; but on
-// the bench's mixed 32-model batch 64 points took 2.37 ms against 2.27 for 16.
-constexpr int kLinopLanePts = 16;
-constexpr int kLinopChunk = 8;
+constexpr int kLinopLanePts = 128;
+constexpr int kLinopFew = 4;
+constexpr int kLinopChunk = 4;
 constexpr int kLinopMinBlocks = 4;
 
-// One stored line by one warp (lanes over depths): the coarse and fine
-// depth gates and the red and blue wing walks of LINOP1 (:18236-18370).
-// walked / points count the walked (line, depth) pairs and the wing points
-// this lane added.
-template <bool F32, bool kDry = false>
-static __device__ __forceinline__ void linop_line(const LinopArgs& a, int64_t il, int lane, unsigned long long& walked,
-                                                  unsigned long long& points, unsigned long long& atoms) {
+// The wings of the walking lanes: nu, nu+1, ... (nr points at most) and nu-1,
+// nu-2, ... (nb at most).  kX: XLINOP's walk (the continuum edge, long wings).
+template <bool F32, bool kDry, bool kX>
+static __device__ __forceinline__ void linop_wings(const LinopArgs& a, int slot, const LinopPair& w, int J,
+                                                   double wlvac, int nu, int nr, int nb, bool walk, double wcon,
+                                                   int lane, unsigned& points, unsigned& atoms) {
   const int nuh = a.nu_hi > 0 ? a.nu_hi : a.numnu;
-  const AtlasLine L = a.lines[il];
-  if (L.nelion == 0 || L.nu + a.max_wing < a.nu_lo || L.nu - a.max_wing > nuh) return;
-  const double cx = a.lcontx ? a.lcontx[il] : 0.0;
-  const double* xdn = a.xnfdop + (size_t)(L.nelion - 1) * a.kw;
-  const double* dpn = a.dopple + (size_t)(L.nelion - 1) * a.kw;
-  const double* tcv = a.tabcont + (size_t)(L.nucont - 1) * a.kw;
-  // coarse gates: depths 8, 16, ... (lane k -> depth 8(k+1)); bit k = IFJ at depth 8(k+1)
-  int pass = 0;
-  {
-    const int J = 8 * (lane + 1);
-    if (J <= a.nrhox) {
-      double c = L.cgf * xdn[J - 1];
-      if (c >= tcv[J - 1]) {
-        c = c * exp(-L.elo * a.hckt[J - 1]);
-        pass = c >= tcv[J - 1];
+  bool red = walk, blue = walk && nb > 0;
+  const double* ws = a.waveset + nu - 1;  // ws[s] red, ws[-1 - s] blue
+  double wr = ws[0], wb = nb > 0 ? ws[-1] : 0.0;
+  const size_t o = (size_t)slot * a.s_xl + (size_t)(nu - 1) * a.kw + (J - 1);
+  double* xl = a.xl + o;
+  unsigned long long* xf = a.xfix + kFixWords * ((size_t)slot * a.s_xl + (size_t)(nu - 1) * a.kw) + (J - 1);
+#pragma unroll 1
+  for (int s = 0;;) {
+    if (kX) blue = blue && !(wb < wcon);  // the continuum edge
+    const double vr = (wr - wlvac) * w.rdop, vb = (wlvac - wb) * w.rdop;
+    // the next grid wavelengths, one step ahead
+    if (s + 1 < nr) wr = ws[s + 1];
+    if (s + 1 < nb) wb = ws[-2 - s];
+    bool rend, bend;
+    const double cr = linop_value<F32>(a, w, vr, red, rend), cb = linop_value<F32>(a, w, vb, blue, bend);
+    const int off = s * a.kw;
+    if (red && nu + s >= a.nu_lo && nu + s <= nuh) {
+      ++points;
+      if (kX) {
+        atomicAdd(xl + off, cr);
+      } else {
+        const int n = fix_add<kDry>(xf + kFixWords * off, a.kw, cr, w.kexp);
+        if (kDry) atoms += n;
       }
     }
+    if (blue && nu - 1 - s >= a.nu_lo && nu - 1 - s <= nuh) {
+      ++points;
+      if (kX) {
+        atomicAdd(xl - off - a.kw, cb);
+      } else {
+        const int n = fix_add<kDry>(xf - kFixWords * (off + a.kw), a.kw, cb, w.kexp);
+        if (kDry) atoms += n;
+      }
+    }
+    ++s;
+    red = red && !rend && s < nr;
+    blue = blue && !bend && s < nb;
+    const unsigned left = __ballot_sync(0xffffffffu, red || blue);
+    if (!left) return;
+    if (kX && s >= kLinopLanePts && __popc(left) <= kLinopFew) {
+      for (unsigned l = left; l; l &= l - 1) {
+        const int src = __ffs(l) - 1;
+        LinopPair q;
+        q.center = __shfl_sync(0xffffffffu, w.center, src);
+        q.adamp = __shfl_sync(0xffffffffu, w.adamp, src);
+        q.rdop = __shfl_sync(0xffffffffu, w.rdop, src);
+        q.tc = __shfl_sync(0xffffffffu, w.tc, src);
+        if (F32) {
+          q.cf = __shfl_sync(0xffffffffu, w.cf, src);
+          q.la = __shfl_sync(0xffffffffu, w.la, src);
+          q.tlo = __shfl_sync(0xffffffffu, w.tlo, src);
+          q.thi = __shfl_sync(0xffffffffu, w.thi, src);
+        }
+        const int Jq = __shfl_sync(0xffffffffu, J, src);
+        const double wq = __shfl_sync(0xffffffffu, wcon, src);
+        const bool rq = __shfl_sync(0xffffffffu, (int)red, src) != 0, bq = __shfl_sync(0xffffffffu, (int)blue, src) != 0;
+        if (rq) linop_finish_warp<F32>(a, q, Jq, wlvac, nu + s, 1, nr - s, wq, lane);
+        if (bq) linop_finish_warp<F32>(a, q, Jq, wlvac, nu - 1 - s, -1, nb - s, wq, lane);
+      }
+      return;
+    }
   }
-  const unsigned ifj = __ballot_sync(0xffffffffu, pass);
-  if (ifj == 0) return;
-  if (lane == 0 && a.used) atomicAdd(a.used, 1ull);
-  const int iwmax = min(L.nu + a.max_wing, a.numnu);
+}
+
+// The walks of one stored line by one warp (lanes over depths): the fine depth
+// gates and the red and blue wing walks of LINOP1 (:18236-18370); ifj: bit k
+// set where the coarse depth 8(k+1) passed.  walked / points count the walked
+// (line, depth) pairs and the wing points this lane added.
+template <bool F32, bool kDry, bool kX>
+static __device__ __forceinline__ void linop_line(const LinopArgs& a, int slot, int64_t il, unsigned ifj, int lane,
+                                                  unsigned& walked, unsigned& points, unsigned& atoms) {
+  const AtlasLine L = a.lines[il];
+  const double cx = kX ? a.lcontx[il] : 0.0;
+  const size_t os = (size_t)slot * a.s_spec + (size_t)(L.nelion - 1) * a.kw, ok = (size_t)slot * a.s_kw;
+  const double* xdn = a.xnfdop + os;
+  const double* dpn = a.dopple + os;
+  const double* tcv = a.tabcont + (size_t)slot * a.s_tab + (size_t)(L.nucont - 1) * a.kw;
+  const double* hckt = a.hckt + ok;
   for (int J0 = 1; J0 <= a.nrhox; J0 += 32) {
     // a round of 32 depths can walk only where its coarse blocks, or the
     // block just above its first, passed: skip it before any load if none did
@@ -539,100 +622,52 @@ static __device__ __forceinline__ void linop_line(const LinopArgs& a, int64_t il
     }
     const int J = J0 + lane;
     bool walk = false;
-    double center = 0.0, tc = 0.0;
+    LinopPair w;
+    w.center = 0.0;
+    w.tc = 0.0;
     const int K = 8 * ((J + 7) / 8);  // the coarse depth closing J's block
     if (J <= a.nrhox && K <= a.nrhox) {
       const int k = K / 8 - 1;
       const bool cur = (ifj >> k) & 1u;
-      tc = tcv[J - 1];
+      w.tc = tcv[J - 1];
       if (J == K) {
         walk = cur;
-        if (walk) center = L.cgf * xdn[J - 1] * exp(-L.elo * a.hckt[J - 1]);
+        if (walk) w.center = L.cgf * xdn[J - 1] * exp(-L.elo * hckt[J - 1]);
       } else if (cur || (k > 0 && ((ifj >> (k - 1)) & 1u))) {
         // fine depth K-7..K-1 of a block next to a passing coarse depth
-        center = L.cgf * xdn[J - 1];
-        if (center >= tc) {
-          center = center * exp(-L.elo * a.hckt[J - 1]);
-          walk = center >= tc;
+        w.center = L.cgf * xdn[J - 1];
+        if (w.center >= w.tc) {
+          w.center = w.center * exp(-L.elo * hckt[J - 1]);
+          walk = w.center >= w.tc;
         }
       }
     }
-    if (!__any_sync(0xffffffffu, walk)) continue;
     // XLINOP: no walk at a depth whose continuum edge lies redward of the line
     double wcon = 0.0;
-    if (walk && cx > 0.0) {
+    if (kX && walk && cx > 0.0) {
       wcon = 1.0e7 / (cx - a.emerge[J - 1]);
       if (L.wlvac < wcon) walk = false;
     }
-    double adamp = 0.0, rdop = 1.0;
+    if (!__any_sync(0xffffffffu, walk)) continue;
+    w.adamp = 0.0;
+    w.rdop = 1.0;
+    w.kexp = 0;
     if (walk) {
-      adamp = (L.gr + L.gs * a.xne[J - 1] + L.gw * a.txnxn[J - 1]) / dpn[J - 1];
-      rdop = 1.0 / (dpn[J - 1] * L.wlvac);
+      w.adamp = (L.gr + L.gs * a.xne[ok + J - 1] + L.gw * a.txnxn[ok + J - 1]) / dpn[J - 1];
+      w.rdop = 1.0 / (dpn[J - 1] * L.wlvac);
+      if (!kX) w.kexp = a.fscale[ok + J - 1];
       ++walked;
     }
-    bool rdone = !walk, bdone = !walk;
-    int rnext = L.nu, bnext = 1;
-    // each walk's next grid wavelength is loaded one point ahead, so the load
-    // is in flight while the current point is evaluated (the last load of a
-    // walk goes unused; every index stays inside WAVESET)
-    double wr = walk ? a.waveset[rnext - 1] : 0.0;
-    double wb = (walk && L.nu >= 2) ? a.waveset[L.nu - 2] : 0.0;
-#pragma unroll 1
-    for (int s = 0; s < kLinopLanePts && __any_sync(0xffffffffu, !rdone || !bdone); ++s) {
-      if (!rdone) {
-        const int iw = rnext;
-        const double wr_next = iw < a.numnu ? a.waveset[iw] : 0.0;
-        const double dl = wr - L.wlvac;
-        const double cv = linop_cv<F32>(a, center, adamp, dl, rdop);
-        if (iw >= a.nu_lo && iw <= nuh) {
-          atoms += linop_add<kDry>(a, J, iw, cv);
-          ++points;
-        }
-        if (linop_below<F32>(a, cv, tc, center, adamp, dl, rdop) || iw >= iwmax) {
-          rdone = true;
-        } else {
-          rnext = iw + 1;
-          wr = wr_next;
-        }
-      }
-      if (!bdone) {
-        const int iw = L.nu - bnext;
-        if (iw < 1 || wb < wcon) {
-          bdone = true;
-        } else {
-          const double wb_next = iw >= 2 ? a.waveset[iw - 2] : 0.0;
-          const double dl = L.wlvac - wb;
-          const double cv = linop_cv<F32>(a, center, adamp, dl, rdop);
-          if (iw >= a.nu_lo && iw <= nuh) {
-            atoms += linop_add<kDry>(a, J, iw, cv);
-            ++points;
-          }
-          if (linop_below<F32>(a, cv, tc, center, adamp, dl, rdop) || bnext >= a.max_wing) {
-            bdone = true;
-          } else {
-            bnext = bnext + 1;
-            wb = wb_next;
-          }
-        }
-      }
+    if (F32) {
+      w.cf = (float)w.center;
+      w.la = (float)(a.lorentz * w.adamp);
+      // thresholds of the FP32 tests; a TABCONT outside FP32's comfortable range leaves every test to FP64
+      const bool fits = w.tc > 1.0e-30 && w.tc < 1.0e30;
+      w.tlo = fits ? (float)(w.tc * (1.0 - 2.0e-5)) : -1.0f;
+      w.thi = fits ? (float)(w.tc * (1.0 + 2.0e-5)) : __int_as_float(0x7f800000);
     }
-    // walks still going: the warp finishes them one at a time
-    unsigned ov = __ballot_sync(0xffffffffu, !rdone || !bdone);
-    while (ov) {
-      const int src = __ffs(ov) - 1;
-      ov &= ov - 1;
-      const int Js = __shfl_sync(0xffffffffu, J, src);
-      const double cs = __shfl_sync(0xffffffffu, center, src);
-      const double as = __shfl_sync(0xffffffffu, adamp, src);
-      const double ds = __shfl_sync(0xffffffffu, rdop, src);
-      const double ts = __shfl_sync(0xffffffffu, tc, src);
-      const int rn = __shfl_sync(0xffffffffu, rnext, src);
-      const int bn = __shfl_sync(0xffffffffu, bnext, src);
-      const bool rd = __shfl_sync(0xffffffffu, (int)rdone, src) != 0;
-      const bool bd = __shfl_sync(0xffffffffu, (int)bdone, src) != 0;
-      const double wc = __shfl_sync(0xffffffffu, wcon, src);
-      points += linop_finish_warp<F32, kDry>(a, Js, cs, as, ds, L.wlvac, L.nu, ts, rn, rd, bn, bd, wc, lane, atoms);
-    }
+    const int nr = min(a.max_wing, a.numnu - L.nu) + 1, nb = min(a.max_wing, L.nu - 1);
+    linop_wings<F32, kDry, kX>(a, slot, w, J, L.wlvac, L.nu, nr, nb, walk, wcon, lane, points, atoms);
   }
 }
 
@@ -654,20 +689,49 @@ __device__ __forceinline__ void linop_counts(const LinopArgs& a, int lane, unsig
 
 // kDry: the counting pass (walks, counts the wing points and the atomics the
 // adds would issue, adds nothing)
-template <bool F32, bool kDry = false>
-static __device__ __forceinline__ void linop_body(const LinopArgs& a) {
+template <bool F32, bool kDry = false, bool kX = false>
+static __device__ __forceinline__ void linop_body(const LinopArgs& a, int slot) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long walked = 0, points = 0, atoms = 0;
-  for (int64_t il0 = w0 * kLinopChunk; il0 < a.n; il0 += nw * kLinopChunk)
-    for (int64_t il = il0; il < il0 + kLinopChunk && il < a.n; ++il)
-      linop_line<F32, kDry>(a, il, lane, walked, points, atoms);
+  unsigned walked = 0, points = 0, atoms = 0;
+  const int nuh = a.nu_hi > 0 ? a.nu_hi : a.numnu;
+  // coarse gates: depths 8, 16, ... of several lines at a time (lane g * ng + k:
+  // line g of the round at depth 8(k+1)); bit k of a line = IFJ at depth 8(k+1)
+  const int ng = min(a.nrhox >> 3, 32), per = 32 / ng;
+  const int lg = lane / ng, J = 8 * (lane - lg * ng + 1);
+  for (int64_t il0 = w0 * kLinopChunk; il0 < a.n; il0 += nw * kLinopChunk) {
+    const int64_t il1 = il0 + kLinopChunk < a.n ? il0 + kLinopChunk : a.n;
+    for (int64_t ib = il0; ib < il1; ib += per) {
+      bool pass = false;
+      if (lg < per && ib + lg < il1) {
+        const AtlasLine& L = a.lines[ib + lg];
+        const int nel = L.nelion, nu = L.nu;
+        if (nel != 0 && nu + a.max_wing >= a.nu_lo && nu - a.max_wing <= nuh) {
+          const double tc = a.tabcont[(size_t)slot * a.s_tab + (size_t)(L.nucont - 1) * a.kw + J - 1];
+          double c = L.cgf * a.xnfdop[(size_t)slot * a.s_spec + (size_t)(nel - 1) * a.kw + J - 1];
+          if (c >= tc) {
+            c = c * exp(-L.elo * a.hckt[(size_t)slot * a.s_kw + J - 1]);
+            pass = c >= tc;
+          }
+        }
+      }
+      const unsigned gates = __ballot_sync(0xffffffffu, pass);
+      for (int g = 0; g < per; ++g) {
+        const unsigned ifj = (gates >> (g * ng)) & (0xffffffffu >> (32 - ng));
+        if (ifj == 0) continue;
+        if (lane == 0 && a.used) atomicAdd(a.used, 1ull);
+        linop_line<F32, kDry, kX>(a, slot, ib + g, ifj, lane, walked, points, atoms);
+      }
+    }
+  }
   linop_counts(a, lane, walked, points, atoms);
 }
 
 template <bool F32>
-static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_atlas_linop(LinopArgs a) { linop_body<F32>(a); }
+static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_atlas_linop(const __grid_constant__ LinopArgs a) { linop_body<F32>(a, 0); }
+template <bool F32>
+static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_xlinop_walk(const __grid_constant__ LinopArgs a) { linop_body<F32, false, true>(a, 0); }
 
 // XLINES(J, NU) from the fixed-point words, which are cleared for the next
 // accumulation (grid-stride over NU, threads over depths J < nrhox)
@@ -703,7 +767,7 @@ static __global__ void k_cgf_max(const AtlasLine* __restrict__ lines, int64_t n,
 
 // the per-depth scales of a model (threads over depths)
 static __global__ void k_fix_scale(const double* xnfdop, int nspec, int kw, int nrhox, const double* cgfmax,
-                                   double* scale, double* unscale) {
+                                   int* scale, double* unscale) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < nrhox) fix_scale_depth(xnfdop, nspec, kw, j, cgfmax, scale, unscale);
 }

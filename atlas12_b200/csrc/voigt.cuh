@@ -58,6 +58,17 @@ __device__ __forceinline__ double voigt_weideman(double v, double a) {
   return term1 + term2;
 }
 
+// VOIGT's third regime (a > 1.4 or a + v > 3.2), the quotients by U taken as
+// products with its reciprocal
+__device__ __forceinline__ double voigt_far(double v, double a) {
+  const double aa = a * a, vv = v * v;
+  const double ru = 1.0 / ((aa + vv) * 1.4142);
+  const double r = a * 0.79788 * ru;
+  if (!(a <= 100.0)) return r;
+  const double aau = aa * ru, vvu = vv * ru;
+  return ((((aau - 10.0 * vvu) * aau * 3.0 + 15.0 * vvu * vvu) + 3.0 * vv - aa) * (ru * ru) + 1.0) * r;
+}
+
 // VOIGT(V, A) with 1-based table index IV = INT(V*200 + 1.5)
 __device__ __forceinline__ double voigt_kurucz(double v, double a, const double* __restrict__ h0,
                                                const double* __restrict__ h1,
@@ -66,7 +77,8 @@ __device__ __forceinline__ double voigt_kurucz(double v, double a, const double*
   if (a < 0.2) {
     if (v <= 10.0) return (h2[iv - 1] * a + h1[iv - 1]) * a + h0[iv - 1];
     return 0.5642 * a / (v * v);
-  } else if (a <= 1.4 && a + v <= 3.2) {
+  }
+  if (a <= 1.4 && a + v <= 3.2) {
     const double vv = v * v;
     const double H0 = h0[iv - 1], H1 = h1[iv - 1], H2 = h2[iv - 1];
     const double hh1 = H1 + H0 * 1.12838;
@@ -75,16 +87,8 @@ __device__ __forceinline__ double voigt_kurucz(double v, double a, const double*
     const double hh4 = (3.0 * hh3 - hh1) * 0.37613 + H0 * 0.66667 * vv * vv;
     return ((((hh4 * a + hh3) * a + hh2) * a + hh1) * a + H0) *
            (((-.122727278 * a + .532770573) * a - .96284325) * a + .979895032);
-  } else {
-    const double aa = a * a, vv = v * v;
-    const double u = (aa + vv) * 1.4142;
-    double r = a * 0.79788 / u;
-    if (a <= 100.0) {
-      const double aau = aa / u, vvu = vv / u, uu = u * u;
-      r = ((((aau - 10.0 * vvu) * aau * 3.0 + 15.0 * vvu * vvu) + 3.0 * vv - aa) / uu + 1.0) * r;
-    }
-    return r;
   }
+  return voigt_far(v, a);
 }
 
 }  // namespace atlasgpu
