@@ -295,6 +295,13 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
       (r = bufT(ctx, "lo_fill", (size_t)nj * ntiles, &fillptr)) || (r = bufT(ctx, "lo_tot", nj, &tot)) ||
       (r = bufT(ctx, "lo_base", nj, &base)))
     return r;
+  double* inv2;
+  const bool fresh = ctx->bufs.find("lo_inv2") == ctx->bufs.end();
+  if ((r = bufT(ctx, "lo_inv2", kFarInv, &inv2))) return r;
+  if (fresh) {
+    k_far_inverse<<<kFarInv / 256, 256, 0, ctx->stream>>>(inv2);
+    CKL(ctx);
+  }
   std::vector<int64_t> htot(nj), hbase(nj);
   unsigned long long* work = work_counters(ctx, 4);
   // the families run once per depth batch: their times add up over the call
@@ -306,12 +313,19 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
     CK(cudaMemsetAsync(tdiff, 0, (size_t)nb * (ntiles + 1) * sizeof(int), ctx->stream));
     if (n > 0) {
       CoreArgs a{d_lines, n, length, nrhox, nspec, maxprof, j0, nb, resolu, d_cont, d_xnfdop,
-                 d_dopple, d_xne, d_txnxn, d_hckt, acc, far, nfar, tdiff, ntiles, work};
+                 d_dopple, d_xne, d_txnxn, d_hckt, acc, far, nfar, work};
       Timer tm(ctx, "synthe_core", true);
       const int64_t groups = n * nb;
-      k_core<<<grid_for(ctx, groups, 256, 4), 256, 0, ctx->stream>>>(a);
+      k_core<<<grid_for(ctx, groups, 32 * kCoreWarps, 4), 32 * kCoreWarps, 0, ctx->stream>>>(a);
       CKL(ctx);
     }
+    // list kernels: blocks of kFarBlock far-wing records, at most about four waves over the depths
+    const dim3 gfar((unsigned)std::max<int64_t>(1, std::min<int64_t>((nn + kFarBlock - 1) / kFarBlock,
+                                                                     ctx->nsm * 32 / std::max(1, nb) + 1)), nb);
+    const bool fsm = ntiles < kFarTilesMax;
+    k_far_count<<<gfar, 256, fsm ? (ntiles + 1) * sizeof(int) : 0, ctx->stream>>>(far, nfar, nn, length, ntiles,
+                                                                                  tdiff);
+    CKL(ctx);
     k_far_scan<<<nb, 32, 0, ctx->stream>>>(tdiff, ntiles, off, fillptr, tot);
     CKL(ctx);
     CK(cudaMemcpyAsync(htot.data(), tot, nb * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
@@ -326,19 +340,19 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
     CK(cudaMemcpyAsync(base, hbase.data(), nb * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     {
       Timer tm(ctx, "synthe_farfill", true);
-      dim3 g(std::max(1, std::min(ctx->nsm * 4 / std::max(1, nb) + 1, 1024)), nb);
-      k_far_fill<<<g, 256, 0, ctx->stream>>>(far, nfar, nn, length, base, fillptr, ntiles, csr);
+      const size_t fsmem = fsm ? ntiles * (sizeof(int64_t) + sizeof(int)) : 0;
+      CK(cudaFuncSetAttribute(k_far_fill, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(kFarTilesMax * (sizeof(int64_t) + sizeof(int)))));
+      k_far_fill<<<gfar, 256, fsmem, ctx->stream>>>(far, nfar, nn, length, base, fillptr, ntiles, csr);
       CKL(ctx);
     }
     {
       Timer tm(ctx, "synthe_farwing", true);
       dim3 g(ntiles * kSubs, nb);
-      if (ctx->precision == ATLASGPU_PREC_MIXED)
-        k_farwing<true><<<g, 32, 0, ctx->stream>>>(far, nn, off, base, csr, ntiles, length, j0, acc, d_opac,
-                                                            work);
+      if (run < (int64_t)kFarLong * ntiles * nb)
+        k_farwing<4><<<g, 128, 0, ctx->stream>>>(far, nn, off, base, csr, ntiles, length, j0, inv2, acc, d_opac, work);
       else
-        k_farwing<false><<<g, 32, 0, ctx->stream>>>(far, nn, off, base, csr, ntiles, length, j0, acc, d_opac,
-                                                             work);
+        k_farwing<1><<<g, 32, 0, ctx->stream>>>(far, nn, off, base, csr, ntiles, length, j0, inv2, acc, d_opac, work);
       CKL(ctx);
     }
   }

@@ -88,8 +88,6 @@ struct CoreArgs {
   double* acc;           // [nrhox][length] core accumulator
   FarLine* far;          // [nj][n]
   unsigned int* nfar;    // [nj]
-  int* tdiff;            // [nj][ntiles+1]
-  int ntiles;
   // work counters (timed launches only, else null): [0] Voigt evaluations,
   // [1] far-wing bin updates the gather will make
   unsigned long long* work = nullptr;
@@ -100,139 +98,181 @@ struct CoreArgs {
 // s = 1, 2, ... until the first value below kapmin (scattered too, as the
 // reference's loop does) or s = n10dop.  The evaluation is the only
 // expensive step, and all lanes with a pair run it together whatever the
-// lengths of their walks, so the warp keeps every lane supplied: it gates
-// the pairs 32 at a time (a chunk of its grid-stride sequence, one pair per
-// lane), a pair that passes both kapmin gates stays with its lane as a
-// pending candidate, and a lane whose walk has ended takes the next pending
-// candidate of the warp (k-th idle lane, k-th candidate, by shuffles).
+// lengths of their walks, so the warp keeps its lanes supplied: it gates the
+// pairs 32 at a time (a chunk of its grid-stride sequence, one pair per lane;
+// the next chunk's line records are already in flight), pairs that pass both
+// kapmin gates go into the warp's queue in shared memory, and when at least
+// kCoreRefill lanes are idle each takes the next queued pair.  (Handing the
+// candidates from lane to lane by shuffles as soon as one lane was idle took
+// as many instructions as the evaluation itself.)
 // With MAXPROF < n10dop the reference scatters only min(n10dop, maxstep)
 // core points when no point falls below kapmin; that limit is known only
 // after the walk, so such pairs walk once to decide (phase 1) and once to
 // scatter (phase 2).
 // A walk that reaches n10dop without a point below kapmin records its far
-// wing x_wing/n^2 (n10dop < n <= maxstep) for k_farwing.
-static __global__ void __launch_bounds__(256, 4) k_core(CoreArgs a) {
+// wing x_wing/n^2 (n10dop < n <= maxstep) for k_farwing, through a buffer of the
+// warp: the depth's list is extended 32 records at a time.  (One counter update
+// per record bounded the whole kernel: all warps work on the same depth, and
+// updates of one address with a returned value pass at one per ~4 clocks;
+// 18.3 ms for 1M lines x 72 depths against 13.4.)
+constexpr int kCoreWarps = 8;
+constexpr int kCoreQueue = 64;   // fewer than 32 left over when a chunk adds up to 32
+constexpr int kCoreRefill = 8;
+struct CoreQueue {
+  double k0[kCoreQueue], km[kCoreQueue], ad[kCoreQueue], dv[kCoreQueue];
+  int nb[kCoreQueue], n10[kCoreQueue], jj[kCoreQueue];
+  FarLine far[kCoreQueue];  // far-wing records not yet in their lists, pad = depth
+};
+
+// The first n (<= 32) far-wing records of a warp's buffer into their depths'
+// lists, one counter update per depth (nearly always one depth); the rest moves up.
+static __device__ __forceinline__ void core_flush(const CoreArgs& a, CoreQueue& Q, int lane, int n, int count) {
   constexpr unsigned FULL = 0xffffffffu;
+  __syncwarp();
+  FarLine f = Q.far[lane];
+  const int jj = f.pad;
+  unsigned todo = __ballot_sync(FULL, lane < n);
+  while (todo) {
+    const int lead = __ffs(todo) - 1;
+    const int jl = __shfl_sync(FULL, jj, lead);
+    const bool in = lane < n && jj == jl;
+    const unsigned mine = __ballot_sync(FULL, in);
+    unsigned base = 0;
+    if (lane == lead) base = atomicAdd(a.nfar + jl, (unsigned)__popc(mine));
+    base = __shfl_sync(FULL, base, lead);
+    if (in) {
+      f.pad = 0;
+      a.far[(size_t)jj * a.n + base + __popc(mine & ((1u << lane) - 1u))] = f;
+    }
+    todo &= ~mine;
+  }
+  FarLine m = f;
+  if (n + lane < count) m = Q.far[n + lane];
+  __syncwarp();
+  if (n + lane < count) Q.far[lane] = m;
+  __syncwarp();
+}
+
+static __global__ void __launch_bounds__(32 * kCoreWarps, 4) k_core(const __grid_constant__ CoreArgs a) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ CoreQueue s_q[kCoreWarps];
+  CoreQueue& Q = s_q[threadIdx.x >> 5];
   const int64_t npairs = a.n * a.nj;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  int64_t chunk = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;  // next chunk of 32 pairs
+  int64_t pair = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 32 + lane;  // the lane's pair of the next chunk
   unsigned long long nev = 0, nfw = 0;  // counted only when a.work is set
+  // the next chunk's pair of this lane: its depth and line record, loaded one chunk ahead
+  int g_j = 0;
+  atlasgpu_lte_line g_line;
+  g_line.nelion = 0;
+  auto fetch = [&]() {
+    g_line.nelion = 0;
+    if (pair < npairs) {
+      g_j = (int)(pair / a.n);
+      g_line = a.lines[pair - (int64_t)g_j * a.n];
+    }
+  };
+  fetch();
+  int head = 0, count = 0;  // the queue, the same in every lane
+  int nbuf = 0;             // buffered far-wing records
   // the lane's walk
   bool act = false;
   int phase = 0, s = 0, lim = 0, nb = 0, n10 = 0, jj = 0;
   double kappa0 = 0.0, adamp = 0.0, dv = 0.0, kapmin = 0.0;
-  double* accj = nullptr;
-  // the lane's pending candidate
-  bool pend = false;
-  int c_nb = 0, c_n10 = 0, c_jj = 0;
-  double c_k0 = 0.0, c_km = 0.0, c_ad = 0.0, c_dv = 0.0;
   while (true) {
-    // refill the idle lanes: pending candidates first, new chunks when none is left
-    while (true) {
-      const unsigned idle = __ballot_sync(FULL, !act);
-      if (!idle) break;
-      const unsigned pm = __ballot_sync(FULL, pend);
-      if (!pm) {
-        if (chunk * 32 >= npairs) break;
-        const int64_t pp = chunk * 32 + lane;
-        chunk += nw;
-        if (pp < npairs) {
-          const int jp = (int)(pp / a.n);
-          const int64_t il = pp - (int64_t)jp * a.n;
-          const int j = a.j0 + jp;
-          const atlasgpu_lte_line L = a.lines[il];
-          const int nel = L.nelion - 1;
-          if (nel >= 0 && nel < a.nspec) {  // invalid species: no opacity
-            const int ic = L.nbuff < 1 ? 1 : (L.nbuff > a.length ? a.length : L.nbuff);
-            const double xd = a.xnfdop[(size_t)j * a.nspec + nel];
-            const double dp = a.dopple[(size_t)j * a.nspec + nel];
-            double k0 = (double)L.cgf * xd;
-            const double km = (double)a.cont[(size_t)j * a.length + ic - 1] * kLineCutoff;
-            if (k0 >= km) {
-              k0 = k0 * exp(-(double)L.elo * a.hckt[j]);
-              if (k0 >= km) {
-                pend = true;
-                c_k0 = k0;
-                c_km = km;
-                c_ad = ((double)L.gamrf + (double)L.gamsf * a.xne[j] + (double)L.gamwf * a.txnxn[j]) / dp;
-                c_n10 = (int)(10.0 * dp * a.resolu);
-                c_dv = 1.0 / dp / a.resolu;
-                c_nb = L.nbuff;
-                c_jj = jp;
-              }
-            }
+    const unsigned idle = __ballot_sync(FULL, !act);
+    const int nidle = __popc(idle);
+    if (nidle >= kCoreRefill) {
+      // gate chunks until every idle lane can be served
+      while (count < nidle && pair - lane < npairs) {
+        const atlasgpu_lte_line L = g_line;
+        const int jp = g_j, j = a.j0 + jp;
+        pair += nw * 32;
+        fetch();
+        bool pass = false;
+        const int nel = L.nelion - 1;
+        double k0 = 0.0, km = 0.0, dp = 1.0;
+        if (nel >= 0 && nel < a.nspec) {  // invalid species: no opacity
+          const int ic = L.nbuff < 1 ? 1 : (L.nbuff > a.length ? a.length : L.nbuff);
+          const double xd = a.xnfdop[(size_t)j * a.nspec + nel];
+          dp = a.dopple[(size_t)j * a.nspec + nel];
+          k0 = (double)L.cgf * xd;
+          km = (double)a.cont[(size_t)j * a.length + ic - 1] * kLineCutoff;
+          if (k0 >= km) {
+            k0 = k0 * exp(-(double)L.elo * a.hckt[j]);
+            pass = k0 >= km;
           }
         }
-        continue;
+        const unsigned pm = __ballot_sync(FULL, pass);
+        if (pass) {
+          const int e = (head + count + __popc(pm & lt)) & (kCoreQueue - 1);
+          Q.k0[e] = k0;
+          Q.km[e] = km;
+          Q.ad[e] = ((double)L.gamrf + (double)L.gamsf * a.xne[j] + (double)L.gamwf * a.txnxn[j]) / dp;
+          Q.dv[e] = 1.0 / dp / a.resolu;
+          Q.nb[e] = L.nbuff;
+          Q.n10[e] = (int)(10.0 * dp * a.resolu);
+          Q.jj[e] = jp;
+        }
+        count += __popc(pm);
+        __syncwarp();
       }
-      // the k-th idle lane takes the k-th pending candidate
-      const int npend = __popc(pm), nidle = __popc(idle);
-      const int rank = __popc(idle & lt);
-      const bool take = !act && rank < npend;
-      int src = lane;
-      if (take) {
-        unsigned m = pm;
-        for (int q = 0; q < rank; ++q) m &= m - 1u;
-        src = __ffs(m) - 1;
-      }
-      const double t_k0 = __shfl_sync(FULL, c_k0, src), t_km = __shfl_sync(FULL, c_km, src);
-      const double t_ad = __shfl_sync(FULL, c_ad, src), t_dv = __shfl_sync(FULL, c_dv, src);
-      const int t_n10 = __shfl_sync(FULL, c_n10, src), t_nb = __shfl_sync(FULL, c_nb, src);
-      const int t_jj = __shfl_sync(FULL, c_jj, src);
-      if (pend && __popc(pm & lt) < nidle) pend = false;  // this candidate was taken
-      if (take) {
+      const int rank = __popc(idle & lt), served = min(nidle, count);
+      if (!act && rank < served) {
+        const int e = (head + rank) & (kCoreQueue - 1);
         act = true;
-        kappa0 = t_k0;
-        kapmin = t_km;
-        adamp = t_ad;
-        dv = t_dv;
-        n10 = t_n10;
-        nb = t_nb;
-        jj = t_jj;
-        accj = a.acc + (size_t)(a.j0 + jj) * a.length;
+        kappa0 = Q.k0[e];
+        kapmin = Q.km[e];
+        adamp = Q.ad[e];
+        dv = Q.dv[e];
+        nb = Q.nb[e];
+        n10 = Q.n10[e];
+        jj = Q.jj[e];
         s = 0;
         phase = a.maxprof < n10 ? 1 : 0;
       }
+      head = (head + served) & (kCoreQueue - 1);
+      count -= served;
+      __syncwarp();
+      if (nidle == 32 && served == 0) break;
     }
-    if (!__any_sync(FULL, act)) break;
-    if (!act) continue;
-    const double pv = kappa0 * voigt_weideman((double)s * dv, adamp);
-    ++nev;
     bool far = false;
-    if (s == 0) {
-      // the line centre, then the core walk (none when n10dop < 1)
-      if (nb >= 1 && nb <= a.length) atomicAdd(accj + nb - 1, pv);
-      s = 1;
-      act = n10 >= 1;
-    } else if (phase == 1) {
-      // deciding walk: the scatter limit, then the walk again from s = 1
-      const bool below = pv < kapmin;
-      if (below || s == n10) {
-        lim = below ? s : a.maxprof;
-        phase = 2;
+    double pv = 0.0;
+    if (act) {
+      pv = kappa0 * voigt_weideman((double)s * dv, adamp);
+      ++nev;
+      double* accj = a.acc + (size_t)(a.j0 + jj) * a.length;
+      if (s == 0) {
+        // the line centre, then the core walk (none when n10dop < 1)
+        if (nb >= 1 && nb <= a.length) atomicAdd(accj + nb - 1, pv);
         s = 1;
+        act = n10 >= 1;
+      } else if (phase == 1) {
+        // deciding walk: the scatter limit, then the walk again from s = 1
+        const bool below = pv < kapmin;
+        if (below || s == n10) {
+          lim = below ? s : a.maxprof;
+          phase = 2;
+          s = 1;
+        } else {
+          ++s;
+        }
       } else {
-        ++s;
-      }
-    } else {
-      const int r = nb + s, b = nb - s;
-      if (r >= 1 && r <= a.length) atomicAdd(accj + r - 1, pv);
-      if (b >= 1 && b <= a.length) atomicAdd(accj + b - 1, pv);
-      if (phase == 2) {
-        act = s < lim;
-        ++s;
-      } else if (pv < kapmin) {
-        act = false;
-      } else if (s == n10) {
-        act = false;
-        far = true;
-      } else {
-        ++s;
+        const int r = nb + s, b = nb - s;
+        if (r >= 1 && r <= a.length) atomicAdd(accj + r - 1, pv);
+        if (b >= 1 && b <= a.length) atomicAdd(accj + b - 1, pv);
+        if (phase == 2) {
+          act = s < lim;
+        } else {
+          act = !(pv < kapmin) && s != n10;
+          far = !(pv < kapmin) && s == n10;
+        }
+        s += far ? 0 : 1;
       }
     }
-    if (far) {
+    if (__any_sync(FULL, far)) {
       // far wing: x_wing/n**2 for n10dop < n <= maxstep
       const double xw = pv * ((double)n10 * (double)n10);
       // INT(SQRT(x_wing/kapmin))+1 capped at MAXPROF; saturate before the
@@ -240,25 +280,29 @@ static __global__ void __launch_bounds__(256, 4) k_core(CoreArgs a) {
       const double q = sqrt(xw / kapmin);
       const int maxstep = q >= (double)a.maxprof ? a.maxprof : min((int)q + 1, a.maxprof);
       const int lo = max(nb - maxstep, 1), hi = min(nb + maxstep, a.length);
-      if (maxstep > n10 && lo <= hi) {
-        const unsigned slot = atomicAdd(a.nfar + jj, 1u);
+      const bool put = far && maxstep > n10 && lo <= hi;
+      const unsigned pm = __ballot_sync(FULL, put);
+      if (put) {
         FarLine f;
         f.c = nb;
         f.n10 = n10;
         f.m = maxstep;
-        f.pad = 0;
+        f.pad = jj;
         f.x = xw;
-        a.far[(size_t)jj * a.n + slot] = f;
-        int* td = a.tdiff + (size_t)jj * (a.ntiles + 1);
-        atomicAdd(td + (lo - 1) / kTile, 1);
-        atomicAdd(td + (hi - 1) / kTile + 1, -1);
+        Q.far[nbuf + __popc(pm & lt)] = f;
         // bins n10 < |i - nb| <= maxstep inside the grid
         const int r0 = max(nb + n10 + 1, 1), r1 = min(nb + maxstep, a.length);
         const int b0 = max(nb - maxstep, 1), b1 = min(nb - n10 - 1, a.length);
         nfw += (unsigned long long)(r1 >= r0 ? r1 - r0 + 1 : 0) + (unsigned long long)(b1 >= b0 ? b1 - b0 + 1 : 0);
       }
+      nbuf += __popc(pm);
+      if (nbuf >= 32) {
+        core_flush(a, Q, lane, 32, nbuf);
+        nbuf -= 32;
+      }
     }
   }
+  if (nbuf) core_flush(a, Q, lane, nbuf, nbuf);
   if (a.work) {
     for (int o = 16; o > 0; o >>= 1) {
       nev += __shfl_xor_sync(0xffffffffu, nev, o);
@@ -292,32 +336,96 @@ static __global__ void k_far_scan(int* __restrict__ tdiff, int ntiles, int64_t* 
   total[jj] = run;
 }
 
-static __global__ void k_far_fill(const FarLine* __restrict__ far, const unsigned* __restrict__ nfar,
-                           int64_t nlines, int length, const int64_t* __restrict__ base,
-                           int64_t* __restrict__ fillptr, int ntiles, int* __restrict__ csr) {
+// The far-wing lists' counts and entries.  A block takes kFarBlock consecutive
+// far-wing records of one depth (blockIdx.y) at a time and keeps the tile
+// counters in shared memory (nsm of them; grids with more tiles use the global
+// ones): a line touches every tile within its wing, and all lines of a depth
+// touching the same few global counters bounded the fill (4.3 ms for 1M lines x
+// 72 depths against 0.45 for count and fill).
+constexpr int kFarBlock = 1024;
+constexpr int kFarTilesMax = 8192;
+
+__device__ __forceinline__ int2 far_tiles(const FarLine& f, int length) {
+  return make_int2((max(f.c - f.m, 1) - 1) / kTile, (min(f.c + f.m, length) - 1) / kTile);
+}
+
+// tile counts of every depth as differences (tdiff zeroed before)
+static __global__ void __launch_bounds__(256) k_far_count(const FarLine* __restrict__ far,
+                                                          const unsigned* __restrict__ nfar, int64_t nlines,
+                                                          int length, int ntiles, int* __restrict__ tdiff) {
+  extern __shared__ int s_cnt[];
   const int jj = blockIdx.y;
   const unsigned nf = nfar[jj];
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (unsigned s = warp; s < nf; s += nwarps) {
-    const FarLine f = far[(size_t)jj * nlines + s];
-    const int lo = max(f.c - f.m, 1), hi = min(f.c + f.m, length);
-    const int t0 = (lo - 1) / kTile, t1 = (hi - 1) / kTile;
-    for (int t = t0 + lane; t <= t1; t += 32) {
-      const int64_t pos = atomicAdd((unsigned long long*)(fillptr + (size_t)jj * ntiles + t), 1ull);
-      csr[base[jj] + pos] = (int)s;
+  int* td = tdiff + (size_t)jj * (ntiles + 1);
+  if (blockIdx.x * kFarBlock >= nf) return;
+  const bool sm = ntiles < kFarTilesMax;
+  int* cnt = sm ? s_cnt : td;
+  if (sm)
+    for (int t = threadIdx.x; t <= ntiles; t += blockDim.x) s_cnt[t] = 0;
+  __syncthreads();
+  for (unsigned s0 = blockIdx.x * kFarBlock; s0 < nf; s0 += gridDim.x * kFarBlock)
+    for (unsigned s = s0 + threadIdx.x; s < min(s0 + kFarBlock, nf); s += blockDim.x) {
+      const int2 t = far_tiles(far[(size_t)jj * nlines + s], length);
+      atomicAdd(cnt + t.x, 1);
+      atomicAdd(cnt + t.y + 1, -1);
     }
+  __syncthreads();
+  if (sm)
+    for (int t = threadIdx.x; t <= ntiles; t += blockDim.x)
+      if (s_cnt[t]) atomicAdd(td + t, s_cnt[t]);
+}
+
+static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restrict__ far,
+                                                         const unsigned* __restrict__ nfar, int64_t nlines,
+                                                         int length, const int64_t* __restrict__ base,
+                                                         int64_t* __restrict__ fillptr, int ntiles,
+                                                         int* __restrict__ csr) {
+  extern __shared__ __align__(8) unsigned char s_raw[];
+  int64_t* s_pos = reinterpret_cast<int64_t*>(s_raw);  // [ntiles] where the block's next entry of a tile goes
+  int* s_cnt = reinterpret_cast<int*>(s_pos + ntiles);  // [ntiles] entries of this round
+  const int jj = blockIdx.y;
+  const unsigned nf = nfar[jj];
+  const FarLine* fj = far + (size_t)jj * nlines;
+  unsigned long long* fp = reinterpret_cast<unsigned long long*>(fillptr) + (size_t)jj * ntiles;
+  const bool sm = ntiles < kFarTilesMax;
+  for (unsigned s0 = blockIdx.x * kFarBlock; s0 < nf; s0 += gridDim.x * kFarBlock) {
+    const unsigned s1 = min(s0 + kFarBlock, nf);
+    if (sm) {
+      for (int t = threadIdx.x; t < ntiles; t += blockDim.x) s_cnt[t] = 0;
+      __syncthreads();
+      for (unsigned s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
+        const int2 t = far_tiles(fj[s], length);
+        for (int q = t.x; q <= t.y; ++q) atomicAdd(s_cnt + q, 1);
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
+        if (s_cnt[t]) {
+          s_pos[t] = base[jj] + (int64_t)atomicAdd(fp + t, (unsigned long long)s_cnt[t]);
+          s_cnt[t] = 0;
+        }
+      __syncthreads();
+    }
+    for (unsigned s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
+      const int2 t = far_tiles(fj[s], length);
+      for (int q = t.x; q <= t.y; ++q) {
+        const int64_t pos = sm ? s_pos[q] + atomicAdd(s_cnt + q, 1) : base[jj] + (int64_t)atomicAdd(fp + q, 1ull);
+        csr[pos] = (int)s;
+      }
+    }
+    __syncthreads();
   }
 }
 
 // far-wing gather + core accumulator -> REAL(4) opacity; zeroes acc for reuse.
 //
-// One warp (one CTA) takes one sub-tile of kSub bins at one depth, lane l
-// the bins lane + 32k; it walks the CSR list of the kTile-bin tile the
-// sub-tile belongs to, 32 lines at a time (one line record per lane, the
-// next group's records already in flight), and classifies each line
-// against the sub-tile:
+// One CTA of kFarWarps warps takes one sub-tile of kSub bins at one depth, lane l
+// of each warp the bins lane + 32k; its warps walk the CSR list of the kTile-bin
+// tile the sub-tile belongs to in turn, 32 lines at a time (one line record per
+// lane, the next group's records already in flight), and classify each line
+// against the sub-tile.  Four warps where the lists are short (fewer than
+// kFarLong entries on average), so that small grids fill the GPU (0.5 nm, 500
+// lines: 45 against 22 us); one where they are long and the sums of four warps
+// only cost (1M lines: 8.2 against 8.8 ms).
 //   * distant: the whole sub-tile lies inside one far wing of the line
 //     (n10 < |i - c| <= m for every bin i) and the sub-tile centre is at
 //     least kFarSep bins from c.  The line's terms x/(i - c)^2 are then the
@@ -326,30 +434,44 @@ static __global__ void k_far_fill(const FarLine* __restrict__ far, const unsigne
 //     |h v / D| < 1/4, and the lane adds the first kFarTerms coefficients
 //     (relative truncation below 1e-8);
 //   * otherwise, if any of its bins is in the line's far wing, the line is
-//     broadcast to the warp (shuffles) and every bin takes x/n^2 itself,
-//     the lines in list order.
-// At the end the warp adds its lanes' coefficients and each bin evaluates
+//     broadcast to the warp (shuffles) and every bin takes x * (1/n^2) itself,
+//     the lines in list order.  n is a whole number, so 1/n^2 comes from a
+//     table (kFarInv entries in FP64, 32 consecutive ones per load) instead of
+//     a reciprocal per bin (FP32 in mixed precision, a division in FP64).
+// Bounded by instruction issue, two thirds of it the direct lines (4 of a group
+// of 32): 1M lines x 72 depths over 41,940 bins 9.1 -> 8.2 ms, 20,000 lines over
+// 12,346 bins 0.33 -> 0.29 ms.
+// At the end the lanes' and warps' coefficients are added and each bin evaluates
 // the polynomial.  Most of the C3 far-wing terms come from strong lines
 // thousands of bins away, so the direct work drops to a few per cent of
-// the terms.  Warps share nothing, so a sub-tile next to strong line
-// centres (long direct list) holds up no other sub-tile.
+// the terms.
 constexpr int kSub = 128;       // bins per sub-tile (one warp)
 constexpr int kSubs = kTile / kSub;
 constexpr int kFarSep = 256;    // minimum |centre - c| for an expansion
-constexpr int kFarTerms = 16;   // Taylor terms
+constexpr int kFarLong = 4096;  // entries
+constexpr int kFarTerms = 16;   // Taylor terms; half of them where every line of a group is
+constexpr int kFarSep8 = 1024;  // this far away (|h v / D| < 1/16, truncation below 3e-9)
+constexpr int kFarInv = 65536;  // 1/n^2, n < kFarInv (512 KB)
 
-template <bool kMixed>
-static __global__ void __launch_bounds__(32) k_farwing(const FarLine* __restrict__ far, int64_t nlines,
+static __global__ void k_far_inverse(double* __restrict__ inv2) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < kFarInv) inv2[n] = n ? 1.0 / ((double)n * (double)n) : 0.0;
+}
+
+template <int kFarWarps>
+static __global__ void __launch_bounds__(32 * kFarWarps) k_farwing(const FarLine* __restrict__ far, int64_t nlines,
                                                  const int64_t* __restrict__ off,
                                                  const int64_t* __restrict__ base,
                                                  const int* __restrict__ csr, int ntiles, int length,
-                                                 int j0, double* __restrict__ acc,
+                                                 int j0, const double* __restrict__ inv2,
+                                                 double* __restrict__ acc,
                                                  float* __restrict__ opac,
                                                  unsigned long long* __restrict__ work) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kPer = kSub / 32;
   const int jj = blockIdx.y, t = blockIdx.x / kSubs, j = j0 + jj;
-  const int lane = threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ double s_b[kFarWarps][kFarTerms], s_sum[kFarWarps][kSub];
   const int lo = t * kTile + (blockIdx.x % kSubs) * kSub + 1;  // first bin of the sub-tile (1-based)
   if (lo > length) return;
   const int hi = min(lo + kSub - 1, length);                   // last bin inside the grid
@@ -363,107 +485,101 @@ static __global__ void __launch_bounds__(32) k_farwing(const FarLine* __restrict
   for (int k = 0; k < kFarTerms; ++k) b[k] = 0.0;
   unsigned nexp = 0, ndir = 0;
   const int64_t* o = off + (size_t)jj * (ntiles + 1);
-  const int64_t e0 = base[jj] + o[t], e1 = base[jj] + o[t + 1];
+  const int* list = csr + base[jj] + o[t];
+  const int ne = (int)(o[t + 1] - o[t]);
   const FarLine* fj = far + (size_t)jj * nlines;
-  const FarLine none{0, 0, 0, 0, 0.0};
+  const FarLine none{0, 0x7fffffff, 0, 0, 0.0};  // no bin of any sub-tile in its far wing
   // two-stage prefetch: the record of the next group, the index of the one after
-  int idx = e0 + lane < e1 ? csr[e0 + lane] : -1;
+  constexpr int kStep = 32 * kFarWarps;
+  int e = 32 * warp + lane;
+  int idx = e < ne ? list[e] : -1;
   FarLine f = idx >= 0 ? fj[idx] : none;
-  idx = e0 + 32 + lane < e1 ? csr[e0 + 32 + lane] : -1;
-  for (int64_t c0 = e0; c0 < e1; c0 += 32) {
+  idx = e + kStep < ne ? list[e + kStep] : -1;
+  for (int g0 = 32 * warp; g0 < ne; g0 += kStep, e += kStep) {
     const FarLine fn = idx >= 0 ? fj[idx] : none;
-    idx = c0 + 64 + lane < e1 ? csr[c0 + 64 + lane] : -1;
-    bool direct = false;
-    if (c0 + lane < e1) {
-      int dmin, dmax;
-      bool outside = true;
-      if (f.c < lo) {
-        dmin = lo - f.c;
-        dmax = hi - f.c;
-      } else if (f.c > hi) {
-        dmin = f.c - hi;
-        dmax = f.c - lo;
-      } else {
-        outside = false;
-        dmin = 0;
-        dmax = max(f.c - lo, hi - f.c);
-      }
-      const double D = centre - (double)f.c;
-      if (outside && dmin > f.n10 && dmax <= f.m && fabs(D) >= (double)kFarSep) {
-        // 1/D from the single-precision reciprocal and one Newton-Raphson
-        // step (relative error ~1e-14, far below the truncation)
-        const double r0 = (double)__frcp_rn((float)D);
-        const double r = fma(r0, fma(-D, r0, 1.0), r0);
-        const double g = -0.5 * kSub * r, g2 = g * g, g4 = g2 * g2;
-        // powers p*g^k in four independent chains (k mod 4)
-        double p0 = f.x * r * r, p1 = p0 * g, p2 = p0 * g2, p3 = p1 * g2;
+    idx = e + 2 * kStep < ne ? list[e + 2 * kStep] : -1;
+    // distances of the nearest and the farthest bin; 0 if the centre lies inside
+    const int dl = lo - f.c, dr = f.c - hi;
+    const int dmin = max(max(dl, dr), 0), dmax = max(f.c - lo, hi - f.c);
+    const double D = centre - (double)f.c;
+    const bool distant = dmin > f.n10 && dmax <= f.m && fabs(D) >= (double)kFarSep;
+    const bool direct = !distant && dmax > f.n10 && dmin <= f.m;
+    if (__any_sync(FULL, distant)) {
+      // 1/D from the single-precision reciprocal and one Newton-Raphson
+      // step (relative error ~1e-14, far below the truncation)
+      const double Ds = distant ? D : 1.0e9, x = distant ? f.x : 0.0;
+      const double r0 = (double)__frcp_rn((float)Ds);
+      const double r = fma(r0, fma(-Ds, r0, 1.0), r0);
+      const double g = -0.5 * kSub * r, g2 = g * g, g4 = g2 * g2;
+      // powers p*g^k in four independent chains (k mod 4)
+      double p0 = x * r * r, p1 = p0 * g, p2 = p0 * g2, p3 = p1 * g2;
+      const bool all = __any_sync(FULL, distant && fabs(D) < (double)kFarSep8);
 #pragma unroll
-        for (int k = 0; k < kFarTerms; k += 4) {
-          b[k] = fma((double)(k + 1), p0, b[k]);
-          b[k + 1] = fma((double)(k + 2), p1, b[k + 1]);
-          b[k + 2] = fma((double)(k + 3), p2, b[k + 2]);
-          b[k + 3] = fma((double)(k + 4), p3, b[k + 3]);
-          p0 *= g4;
-          p1 *= g4;
-          p2 *= g4;
-          p3 *= g4;
-        }
-        ++nexp;
-      } else {
-        direct = dmax > f.n10 && dmin <= f.m;
+      for (int k = 0; k < kFarTerms; k += 4) {
+        if (k == 8 && !all) break;
+        b[k] = fma((double)(k + 1), p0, b[k]);
+        b[k + 1] = fma((double)(k + 2), p1, b[k + 1]);
+        b[k + 2] = fma((double)(k + 3), p2, b[k + 2]);
+        b[k + 3] = fma((double)(k + 4), p3, b[k + 3]);
+        p0 *= g4;
+        p1 *= g4;
+        p2 *= g4;
+        p3 *= g4;
       }
+      nexp += distant;
     }
     // the direct lines of this group, in list order, broadcast to every bin
     unsigned bal = __ballot_sync(FULL, direct);
     ndir += __popc(bal);
+    const int span = f.m - f.n10;
     while (bal) {
       const int src = __ffs(bal) - 1;
       bal &= bal - 1u;
-      const int c = __shfl_sync(FULL, f.c, src);
-      const int n10 = __shfl_sync(FULL, f.n10, src);
-      const int m = __shfl_sync(FULL, f.m, src);
+      const int di = i0 - __shfl_sync(FULL, f.c, src);
+      const int n1 = __shfl_sync(FULL, f.n10, src) + 1;
+      const unsigned sp = (unsigned)__shfl_sync(FULL, span, src);
       const double x = __shfl_sync(FULL, f.x, src);
-      if (kMixed) {
-        const float xf = (float)x;
-        const float fb = (float)(i0 - c);  // exact: |i - c| < 2^24
+      double v[kPer];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          const int d = abs(i0 + 32 * k - c);
-          if (d > n10 && d <= m) {
-            const float df = fb + (float)(32 * k);
-            sum[k] += (double)(xf * __frcp_rn(df * df));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          const int d = abs(i0 + 32 * k - c);
-          if (d > n10 && d <= m) {
-            const double dd = (double)d;
-            sum[k] += x / (dd * dd);
-          }
-        }
+      for (int k = 0; k < kPer; ++k) {
+        const int d = abs(di + 32 * k);
+        v[k] = 0.0;
+        if ((unsigned)(d - n1) < sp) v[k] = d < kFarInv ? inv2[d] : 1.0 / ((double)d * (double)d);
       }
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) sum[k] = fma(x, v[k], sum[k]);
     }
     f = fn;
   }
-  // the warp's expansion: lane sums, then the polynomial at each bin
+  // the expansion: lane sums, then the warps' sums in order, then the polynomial at each bin
 #pragma unroll
-  for (int k = 0; k < kFarTerms; ++k)
+  for (int k = 0; k < kFarTerms; ++k) {
     for (int sh = 16; sh > 0; sh >>= 1) b[k] += __shfl_xor_sync(FULL, b[k], sh);
+    if (lane == k) s_b[warp][k] = b[k];
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) s_sum[warp][lane + 32 * k] = sum[k];
+  __syncthreads();
+  double c[kFarTerms];
+#pragma unroll
+  for (int q = 0; q < kFarTerms; ++q) {
+    c[q] = s_b[0][q];
+#pragma unroll
+    for (int w = 1; w < kFarWarps; ++w) c[q] += s_b[w][q];
+  }
   double* accj = acc + (size_t)j * length;
-  float* oj = opac + (size_t)j * length;
+  for (int n = threadIdx.x; n < kSub; n += 32 * kFarWarps) {
+    const int i = lo + n;
+    if (i > length) break;
+    double near = s_sum[0][n];
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int i = i0 + 32 * k;
-    if (i <= length) {
-      const double v = ((double)i - centre) * (2.0 / kSub);
-      double pv = b[kFarTerms - 1];
+    for (int w = 1; w < kFarWarps; ++w) near += s_sum[w][n];
+    const double v = ((double)i - centre) * (2.0 / kSub);
+    double pv = c[kFarTerms - 1];
 #pragma unroll
-      for (int q = kFarTerms - 2; q >= 0; --q) pv = fma(pv, v, b[q]);
-      oj[i - 1] = (float)(accj[i - 1] + (sum[k] + pv));
-      accj[i - 1] = 0.0;
-    }
+    for (int q = kFarTerms - 2; q >= 0; --q) pv = fma(pv, v, c[q]);
+    opac[(size_t)j * length + i - 1] = (float)(accj[i - 1] + (near + pv));
+    accj[i - 1] = 0.0;
   }
   if (work) {
     for (int sh = 16; sh > 0; sh >>= 1) nexp += __shfl_xor_sync(FULL, nexp, sh);
