@@ -279,7 +279,7 @@ int atlasgpu_atlas_linop(atlasgpu_ctx* ctx, const int32_t* linedata, int64_t n, 
     CK(cudaMemsetAsync(d_cgf, 0, (size_t)nspec * sizeof(unsigned long long), s));
     k_cgf_max<<<grid_for(ctx, n, 256, 8), 256, 0, s>>>(d_lines, n, nspec, d_cgf);
     CKL(ctx);
-    k_fix_scale<<<1, 128, 0, s>>>(d_xd, nspec, kw, nrhox, (const double*)d_cgf, d_fs, d_fu);
+    k_fix_scale<<<(nrhox + 3) / 4, 128, 0, s>>>(d_xd, nspec, kw, nrhox, (const double*)d_cgf, d_fs, d_fu);
     CKL(ctx);
     a.xfix = d_fix;
     a.fscale = d_fs;

@@ -61,13 +61,14 @@ struct BatchDev {
 __device__ __forceinline__ bool running(const BatchCtl* ctl, int b) { return ctl[b].status == ATLASGPU_SLOT_RUNNING; }
 
 __global__ void k_batch_eos(BatchDev d) {
-  const int b = blockIdx.x, j = threadIdx.x;
+  const int b = blockIdx.y, j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (!running(d.ctl, b) || j >= d.nrhox) return;
   const BatchCtl c = d.ctl[b];
   const size_t o = (size_t)b * d.kw, os = (size_t)b * d.nspec * d.kw;
-  model_eos_depth(d.ms + b, c.iter + 1, j, d.kw, c.grav, c.vturb_cms, c.mh, d.xnfdop + os, d.dopple + os,
+  model_eos_depth(lane, d.ms + b, c.iter + 1, j, d.kw, c.grav, c.vturb_cms, c.mh, d.xnfdop + os, d.dopple + os,
                   d.xne_eos + o, d.txnxn + o, d.hkt + o, d.hckt + o, d.rho + o, d.cc + o);
-  fix_scale_depth(d.xnfdop + os, d.nspec, d.kw, j, d.cgfmax, d.fscale + o, d.funscale + o);
+  __syncwarp();
+  fix_scale_depth(lane, d.xnfdop + os, d.nspec, d.kw, j, d.cgfmax, d.fscale + o, d.funscale + o);
 }
 
 // XLINES of every running slot from its fixed-point sums
@@ -213,7 +214,7 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
   const int nb = B->nslots;
   {
     Timer tm(ctx, "batch_eos");
-    k_batch_eos<<<nb, 128, 0, s>>>(B->d);
+    k_batch_eos<<<dim3((B->nrhox + 3) / 4, nb), 128, 0, s>>>(B->d);
     CKL(ctx);
   }
   {

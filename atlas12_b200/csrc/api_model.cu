@@ -55,11 +55,12 @@ __global__ void k_model_eos(ModelState* ms, const int* iter_dev, int nrhox, int 
                             double vturb_cms, double mh, double* xnfdop, double* dopple, double* xne_eos,
                             double* txnxn, double* hkt, double* hckt, double* rho, ContCoef* cc, int nspec,
                             const double* cgfmax, int* fscale, double* funscale) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (j >= nrhox) return;
-  model_eos_depth(ms, *iter_dev + 1, j, kw, grav, vturb_cms, mh, xnfdop, dopple, xne_eos, txnxn, hkt, hckt, rho,
+  model_eos_depth(lane, ms, *iter_dev + 1, j, kw, grav, vturb_cms, mh, xnfdop, dopple, xne_eos, txnxn, hkt, hckt, rho,
                   cc);
-  fix_scale_depth(xnfdop, nspec, kw, j, cgfmax, fscale, funscale);
+  __syncwarp();
+  fix_scale_depth(lane, xnfdop, nspec, kw, j, cgfmax, fscale, funscale);
 }
 
 // KAPCONT (atlas12_modules.f90:19072-19138) on the surrogate continuum
@@ -93,10 +94,12 @@ __global__ void k_surrogate_eval(int nrhox, const double* t, const double* p, do
                                  double* kabs, double* sigma, double* xne, double* rho) {
   const int j = blockIdx.x;
   if (j >= nrhox) return;
-  if (threadIdx.x == 0) {
-    const EosOut e = surrogate_depth(t[j], p[j], vturb_cms, 0.0, j, nrhox, xnfdop, dopple, cc + j);
-    xne[j] = e.xne;
-    rho[j] = e.rho;
+  if (threadIdx.x < 32) {
+    const EosOut e = surrogate_depth(threadIdx.x, t[j], p[j], vturb_cms, 0.0, j, nrhox, xnfdop, dopple, cc + j);
+    if (threadIdx.x == 0) {
+      xne[j] = e.xne;
+      rho[j] = e.rho;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nw; i += blockDim.x) {
@@ -125,7 +128,7 @@ int enqueue_begin(atlasgpu_ctx* ctx, atlasgpu_model* m, bool timed) {
   ctx->timing = was && timed;
   {
     Timer tm(ctx, "model_eos");
-    k_model_eos<<<1, 128, 0, s>>>(m->ms, m->iter_dev, m->nrhox, m->kw, m->grav, m->vturb * 1.0e5, m->mh,
+    k_model_eos<<<(m->nrhox + 3) / 4, 128, 0, s>>>(m->ms, m->iter_dev, m->nrhox, m->kw, m->grav, m->vturb * 1.0e5, m->mh,
                                   m->xnfdop,
                                   m->dopple, m->xne_eos, m->txnxn, m->hkt, m->hckt, m->rho, m->cc, m->nspec,
                                   (const double*)m->cgfmax, m->fscale, m->funscale);

@@ -362,10 +362,13 @@ __host__ __device__ inline double fix_to_double(unsigned long long x0, unsigned 
 // CGF(line) * XNFDOP(J, NELION) (the Boltzmann factor and the profile are at
 // most 1; 8x margin), so the largest value maps below 2^140 and a bin's
 // words stay below 2^64.  cgfmax: the largest CGF of each species' lines.
-__device__ inline void fix_scale_depth(const double* xnfdop, int nspec, int kw, int j, const double* cgfmax,
+// One warp per depth, lanes over species.
+__device__ inline void fix_scale_depth(int lane, const double* xnfdop, int nspec, int kw, int j, const double* cgfmax,
                                        int* scale, double* unscale) {
   double bound = 0.0;
-  for (int s = 0; s < nspec; ++s) bound = fmax(bound, cgfmax[s] * xnfdop[(size_t)s * kw + j]);
+  for (int s = lane; s < nspec; s += 32) bound = fmax(bound, cgfmax[s] * xnfdop[(size_t)s * kw + j]);
+  bound = warp_max(bound);
+  if (lane != 0) return;
   if (!(bound > 0.0) || !(bound < 1e300)) {
     scale[j] = 0;
     unscale[j] = 1.0;
@@ -765,11 +768,11 @@ static __global__ void k_cgf_max(const AtlasLine* __restrict__ lines, int64_t n,
   }
 }
 
-// the per-depth scales of a model (threads over depths)
+// the per-depth scales of a model (warp per depth)
 static __global__ void k_fix_scale(const double* xnfdop, int nspec, int kw, int nrhox, const double* cgfmax,
                                    int* scale, double* unscale) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nrhox) fix_scale_depth(xnfdop, nspec, kw, j, cgfmax, scale, unscale);
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (j < nrhox) fix_scale_depth(threadIdx.x & 31, xnfdop, nspec, kw, j, cgfmax, scale, unscale);
 }
 
 // ---------------------------------------------------------------- RT pass

@@ -14,8 +14,8 @@ constexpr int kNState = 17;        // ModelState vectors
 constexpr int kRossMax = 80 * 60;  // ROSSTAB_MAXTAB = kw*60 with the reference's kw = 80
 
 // hydrostatics (iteration > 1), surrogate EOS / populations, Planck factors
-// at depth j (0-based) of iteration `iter` (1-based)
-__device__ inline void model_eos_depth(ModelState* ms, int iter, int j, int kw, double grav, double vturb_cms,
+// at depth j (0-based) of iteration `iter` (1-based), by one warp
+__device__ inline void model_eos_depth(int lane, ModelState* ms, int iter, int j, int kw, double grav, double vturb_cms,
                                        double mh, double* xnfdop, double* dopple, double* xne_eos, double* txnxn,
                                        double* hkt, double* hckt, double* rho, ContCoef* cc) {
   const double t = ms->t[j];
@@ -24,11 +24,11 @@ __device__ inline void model_eos_depth(ModelState* ms, int iter, int j, int kw, 
     // P = GRAV*RHOX - PRAD - PTURB - PCON (atlas12c.f90:513-519), PCON = 0
     p = grav * ms->rhox[j] - ms->prad[j] - ms->pturb[j] - 0.0;
     if (p <= 0.0) p = fmax(grav * ms->rhox[j] * 1.0e-4, 1.0e-10);
-    ms->p[j] = p;
+    __syncwarp();
+    if (lane == 0) ms->p[j] = p;
   }
-  ContCoef c;
-  const EosOut e = surrogate_depth(t, p, vturb_cms, mh, j, kw, xnfdop, dopple, &c);
-  cc[j] = c;
+  const EosOut e = surrogate_depth(lane, t, p, vturb_cms, mh, j, kw, xnfdop, dopple, cc + j);
+  if (lane != 0) return;
   xne_eos[j] = e.xne;
   ms->xne[j] = e.xne;
   rho[j] = e.rho;

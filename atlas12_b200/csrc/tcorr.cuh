@@ -19,69 +19,7 @@ namespace atlasgpu {
 constexpr double kSigmaSB = 5.670374419e-5;
 constexpr int kAcc8 = 8;  // mode-2 sums per depth (RJMINS ... ABROSS), then PRADK0
 
-// ---- serial numerics (one thread) -------------------------------------
-__device__ inline void s_parcoe(const double* f, const double* x, double* a, double* b, double* c,
-                                int n) {
-  c[0] = 0.0;
-  b[0] = (f[1] - f[0]) / (x[1] - x[0]);
-  a[0] = f[0] - x[0] * b[0];
-  c[n - 1] = 0.0;
-  b[n - 1] = (f[n - 1] - f[n - 2]) / (x[n - 1] - x[n - 2]);
-  a[n - 1] = f[n - 1] - x[n - 1] * b[n - 1];
-  for (int j = 1; j <= n - 2; ++j) {
-    if (j <= 2) {
-      c[j] = 0.0;
-      b[j] = (f[j + 1] - f[j]) / (x[j + 1] - x[j]);
-      a[j] = f[j] - x[j] * b[j];
-    } else {
-      const double d = (f[j] - f[j - 1]) / (x[j] - x[j - 1]);
-      c[j] = f[j + 1] / ((x[j + 1] - x[j]) * (x[j + 1] - x[j - 1])) -
-             f[j] / ((x[j] - x[j - 1]) * (x[j + 1] - x[j])) +
-             f[j - 1] / ((x[j] - x[j - 1]) * (x[j + 1] - x[j - 1]));
-      b[j] = d - (x[j] + x[j - 1]) * c[j];
-      a[j] = f[j - 1] - x[j - 1] * d + x[j] * x[j - 1] * c[j];
-    }
-  }
-  for (int j = 1; j <= n - 2; ++j) {
-    if (c[j] != 0.0) {
-      const double wt = fabs(c[j + 1]) / (fabs(c[j + 1]) + fabs(c[j]));
-      a[j] = a[j + 1] + wt * (a[j] - a[j + 1]);
-      b[j] = b[j + 1] + wt * (b[j] - b[j + 1]);
-      c[j] = c[j + 1] + wt * (c[j] - c[j + 1]);
-    }
-  }
-  a[n - 2] = a[n - 1];
-  b[n - 2] = b[n - 1];
-  c[n - 2] = c[n - 1];
-}
-
-__device__ inline void s_integ(const double* x, const double* f, double* fint, int n, double start,
-                               double* wa, double* wb, double* wc) {
-  s_parcoe(f, x, wa, wb, wc, n);
-  fint[0] = start;
-  for (int i = 0; i < n - 1; ++i) {
-    const double xlo = x[i], xhi = x[i + 1];
-    fint[i + 1] = fint[i] + (wa[i] + wb[i] * 0.5 * (xhi + xlo) +
-                             wc[i] / 3.0 * ((xhi + xlo) * xhi + xlo * xlo)) * (xhi - xlo);
-  }
-}
-
-__device__ inline void s_deriv(const double* x, const double* f, double* d, int n) {
-  d[0] = (f[1] - f[0]) / (x[1] - x[0]);
-  d[n - 1] = (f[n - 1] - f[n - 2]) / (x[n - 1] - x[n - 2]);
-  if (n == 2) return;
-  const double s = fabs(x[1] - x[0]) / (x[1] - x[0]);
-  for (int j = 1; j <= n - 2; ++j) {
-    double scale = fmax(fmax(fabs(f[j - 1]), fabs(f[j])), fabs(f[j + 1])) / fabs(x[j]);
-    if (scale == 0.0) scale = 1.0;
-    const double dr = (f[j + 1] - f[j]) / (x[j + 1] - x[j]) / scale;
-    const double dl = (f[j] - f[j - 1]) / (x[j] - x[j - 1]) / scale;
-    const double tr = dr / (s * sqrt(1.0 + dr * dr) + 1.0);
-    const double tl = dl / (s * sqrt(1.0 + dl * dl) + 1.0);
-    d[j] = (tr + tl) / (1.0 - tr * tl) * scale;
-  }
-}
-
+// ---- serial numerics -----------------------------------------------------
 // MAP1 as a sequential walk (1-based L as in the reference)
 __host__ __device__ inline int s_map1(const double* xo, const double* fo, int nold, const double* xn,
                              double* fn, int nnew) {
@@ -209,17 +147,16 @@ __device__ __forceinline__ void group_bar(int id) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(kFinGroup) : "memory");
 }
 
-// lexicographic (r2, index) minimum: the sequential scan keeps the first minimum
+// lexicographic (r2, index) minimum over a warp (the sequential scan keeps the
+// first minimum): r2 >= 0, so its bits order as its values
 __device__ __forceinline__ void wmin2(double& r, int& i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double orr = __shfl_xor_sync(0xffffffffu, r, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (orr < r || (orr == r && oi < i)) {
-      r = orr;
-      i = oi;
-    }
-  }
+  constexpr unsigned FULL = 0xffffffffu;
+  const unsigned long long b = (unsigned long long)__double_as_longlong(r);
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
+  const unsigned mh = __reduce_min_sync(FULL, hi);
+  const unsigned ml = __reduce_min_sync(FULL, hi == mh ? lo : 0xffffffffu);
+  i = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)i : 0xffffffffu);
+  r = __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
 }
 
 // ROSSTAB(T, P, V) lookup (atlas12_modules.f90:5937-6228): nearest stored point
@@ -230,73 +167,141 @@ struct RossView {
   int n;
   double zerot, slopet, zerop, slopep;
   const double *t, *p, *k;
+  double rslopep;  // 1 / SLOPEP
 };
 
-// tl = (log10 T - zerot) / slopet, hoisted by the caller (T is fixed per depth)
-__device__ inline double b_rosstab(const RossView& R, double tl, double pres, int gtid, FinFold& fold,
-                                   int& parity, int bar) {
-  const double pl = (log10(pres) - R.zerop) / R.slopep;
-  double r[4] = {1e30, 1e30, 1e30, 1e30};  // PP, PM, MP, MM
-  int id[4] = {1 << 30, 1 << 30, 1 << 30, 1 << 30};
-  for (int i = gtid; i < R.n; i += kFinGroup) {
-    const double dt = R.t[i] - tl, dp = R.p[i] - pl;
-    const double r2 = dt * dt + dp * dp;
-    const int q = (dt >= 0.0) ? (dp >= 0.0 ? 0 : 1) : (dp >= 0.0 ? 2 : 3);
-    if (r2 < r[q]) {
-      r[q] = r2;
-      id[q] = i + 1;
+// A depth's view of the table for one warp: T is fixed per depth, so each lane
+// keeps its points' offsets in log T for all of the depth's lookups.  Used while
+// the table has at most kFinLane points a lane (the first iterations); the scan
+// of a larger one is split over the group's warps.
+constexpr int kFinLane = 8;
+struct RossDepth {
+  double dt[kFinLane], p[kFinLane];
+};
+
+// nearest points of the four quadrants over the table's points c * 32 + lane
+__device__ __forceinline__ void ross_scan(const RossView& R, const RossDepth& D, double pl, int lane, double (&r)[4],
+                                          int (&id)[4]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    r[q] = 1e30;
+    id[q] = 1 << 30;
+  }
+#pragma unroll
+  for (int c = 0; c < kFinLane; ++c) {
+    if (c * 32 >= R.n) break;
+    const int i = c * 32 + lane;
+    if (i < R.n) {
+      const double dt = D.dt[c], dp = D.p[c] - pl;
+      const double r2 = dt * dt + dp * dp;
+      const int q = (dt >= 0.0) ? (dp >= 0.0 ? 0 : 1) : (dp >= 0.0 ? 2 : 3);
+#pragma unroll
+      for (int z = 0; z < 4; ++z)
+        if (z == q && r2 < r[z]) {
+          r[z] = r2;
+          id[z] = i + 1;
+        }
     }
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) wmin2(r[q], id[q]);
-  const int w = gtid >> 5;
-  if ((gtid & 31) == 0) {
+}
+
+// tl = (log10 T - zerot) / slopet, hoisted by the caller (T is fixed per depth).
+// kOne: one warp (D given), else the whole group.  TTAUP is one chain of such
+// lookups (about 20 per depth until its pressure has converged), each of them a
+// chain of an EXP, a LOG10, the scan, three quotients deep, an EXP10 and a
+// quotient: its latency is the finish.  Minima by warp-wide integer minima
+// instead of shuffles, the fold of the warps' minima in parallel, the quotients
+// with a common denominator as one, and one warp instead of eight while the
+// table is short: 2.0 -> 1.0 ms per iteration (first iterations).
+template <bool kOne>
+__device__ inline double b_rosstab(const RossView& R, const RossDepth& D, double tl, double pres, int gtid,
+                                   FinFold& fold, int& parity, int bar, double& rinv) {
+  const double pl = (log10(pres) - R.zerop) * R.rslopep;
+  double r[4];  // PP, PM, MP, MM
+  int id[4];
+  const int lane = gtid & 31;
+  if (kOne) {
+    ross_scan(R, D, pl, lane, r, id);
+  } else {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      fold.r[parity][w][q] = r[q];
-      fold.i[parity][w][q] = id[q];
+      r[q] = 1e30;
+      id[q] = 1 << 30;
     }
-  }
-  group_bar(bar);
+    for (int i = gtid; i < R.n; i += kFinGroup) {
+      const double dt = R.t[i] - tl, dp = R.p[i] - pl;
+      const double r2 = dt * dt + dp * dp;
+      const int q = (dt >= 0.0) ? (dp >= 0.0 ? 0 : 1) : (dp >= 0.0 ? 2 : 3);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    double rr = fold.r[parity][0][q];
-    int ii = fold.i[parity][0][q];
-    for (int v = 1; v < kFinGroupWarps; ++v) {
-      const double orr = fold.r[parity][v][q];
-      const int oi = fold.i[parity][v][q];
+      for (int z = 0; z < 4; ++z)
+        if (z == q && r2 < r[z]) {
+          r[z] = r2;
+          id[z] = i + 1;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) wmin2(r[q], id[q]);
+    const int w = gtid >> 5;
+    if (lane < 4) {
+      fold.r[parity][w][lane] = lane == 0 ? r[0] : lane == 1 ? r[1] : lane == 2 ? r[2] : r[3];
+      fold.i[parity][w][lane] = lane == 0 ? id[0] : lane == 1 ? id[1] : lane == 2 ? id[2] : id[3];
+    }
+    group_bar(bar);
+    // lane 4 w + q takes warp w's minimum of quadrant q
+    static_assert(kFinGroupWarps == 8, "one lane per (warp, quadrant)");
+    double rr = fold.r[parity][lane >> 2][lane & 3];
+    int ii = fold.i[parity][lane >> 2][lane & 3];
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      const double orr = __shfl_xor_sync(0xffffffffu, rr, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, ii, o);
       if (orr < rr || (orr == rr && oi < ii)) {
         rr = orr;
         ii = oi;
       }
     }
-    r[q] = rr;
-    id[q] = ii == (1 << 30) ? 0 : ii;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      r[q] = __shfl_sync(0xffffffffu, rr, q);
+      id[q] = __shfl_sync(0xffffffffu, ii, q);
+    }
+    parity ^= 1;
   }
-  parity ^= 1;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (id[q] == (1 << 30)) id[q] = 0;
   double res;
   if (id[0] && id[1] && id[2] && id[3]) {
     const double Tpp = R.t[id[0] - 1], Ppp = R.p[id[0] - 1], Rpp = R.k[id[0] - 1];
     const double Tpm = R.t[id[1] - 1], Ppm = R.p[id[1] - 1], Rpm = R.k[id[1] - 1];
     const double Tmp = R.t[id[2] - 1], Pmp = R.p[id[2] - 1], Rmp = R.k[id[2] - 1];
     const double Tmm = R.t[id[3] - 1], Pmm = R.p[id[3] - 1], Rmm = R.k[id[3] - 1];
-    const double rhi = ((tl - Tmp) * Rpp + (Tpp - tl) * Rmp) / (Tpp - Tmp);
-    const double phi = ((tl - Tmp) * Ppp + (Tpp - tl) * Pmp) / (Tpp - Tmp);
-    const double rlo = ((tl - Tmm) * Rpm + (Tpm - tl) * Rmm) / (Tpm - Tmm);
-    const double plo = ((tl - Tmm) * Ppm + (Tpm - tl) * Pmm) / (Tpm - Tmm);
-    res = ((pl - plo) * rhi + (phi - pl) * rlo) / (phi - plo);
+    // RHI, PHI on the high-pressure side and RLO, PLO on the low one, and the blend
+    // of the two, over one common denominator
+    const double hh = Tpp - Tmp, hl = Tpm - Tmm;
+    const double rh = (tl - Tmp) * Rpp + (Tpp - tl) * Rmp, ph = (tl - Tmp) * Ppp + (Tpp - tl) * Pmp;
+    const double rl = (tl - Tmm) * Rpm + (Tpm - tl) * Rmm, pm = (tl - Tmm) * Ppm + (Tpm - tl) * Pmm;
+    res = ((pl * hl - pm) * rh + (ph - pl * hh) * rl) / (ph * hl - pm * hh);
   } else {
     double d[4], rwt = 0.0, num = 0.0;
-    for (int q = 0; q < 4; ++q) d[q] = sqrt(r[q]) + 1.0e-5;
-    for (int q = 0; q < 4; ++q) rwt += 1.0 / d[q];
-    for (int q = 0; q < 4; ++q) num += R.k[(id[q] > 1 ? id[q] : 1) - 1] / d[q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) d[q] = 1.0 / (sqrt(r[q]) + 1.0e-5);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) rwt += d[q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) num += R.k[(id[q] > 1 ? id[q] : 1) - 1] * d[q];
     res = num / rwt;
   }
+  rinv = exp10(-res);  // (beside the value, off the chain of a quotient)
   return exp10(res);
 }
 
 // TTAUP (atlas12_modules.f90:6303-6523; radiative: P_turb = 0) by one group.
 // Values are carried in registers; thread 0 of the group stores the outputs.
+// kOne: called by the group's first warp alone.
+template <bool kOne>
 __device__ inline void b_ttaup(const RossView& R, double g, const double* tin, const double* tau,
                                double* abstd, double* ptotal, double* pout, const double* prad, int n,
                                int gtid, FinFold& fold, int bar) {
@@ -313,6 +318,17 @@ __device__ inline void b_ttaup(const RossView& R, double g, const double* tin, c
     const int j = J - 1;
     const double tj = tin[j], tauj = tau[j], pradj = prad[j];
     const double tlj = (log10(tj) - R.zerot) / R.slopet;
+    RossDepth D;
+    if (kOne) {
+#pragma unroll
+      for (int c = 0; c < kFinLane; ++c) {
+        const int i = max(min(c * 32 + gtid, R.n - 1), 0);
+        D.dt[c] = R.t[i] - tlj;
+        D.p[c] = R.p[i];
+      }
+    }
+    const double gtau = g * tauj * dlgtau;
+    double rab = 0.0;  // 1 / abj
     double ptj = 0.0, poj = 0.0, abj = 0.0;
     if (J == 1) plog = log(g / ab0 * tau[0]);
     else if (J <= 4) plog = plog1 + dplog1;
@@ -327,18 +343,18 @@ __device__ inline void b_ttaup(const RossView& R, double g, const double* tin, c
         poj = ptj * 1.0e-4;
         if (poj <= 0.0) poj = 1.0e-10;
       }
-      abj = b_rosstab(R, tlj, poj, gtid, fold, parity, bar);
+      abj = b_rosstab<kOne>(R, D, tlj, poj, gtid, fold, parity, bar, rab);
       if (J == 1) ab0 = abj;
-      dplog = g / abj * tauj / ptj * dlgtau;
+      dplog = gtau / ptj * rab;
       dplog = fmax(0.0, fmin(10.0, dplog));
       N = N + 1;
       if (N == 1) continue;
       double pnew;
       if (J == 1) pnew = log(g / ab0 * tau[0]);
-      else if (J <= 4) pnew = (plog + 2.0 * plog1 + dplog + dplog1) / 3.0;
+      else if (J <= 4) pnew = (plog + 2.0 * plog1 + dplog + dplog1) * (1.0 / 3.0);
       else
         pnew = (126.0 * plog1 - 14.0 * plog3 + 9.0 * plog4 + 42.0 * dplog + 108.0 * dplog1 -
-                54.0 * dplog2 + 24.0 * dplog3) / 121.0;
+                54.0 * dplog2 + 24.0 * dplog3) * (1.0 / 121.0);
       perr = err;
       err = fabs(pnew - plog);
       if (err < best_err) {
@@ -367,9 +383,9 @@ __device__ inline void b_ttaup(const RossView& R, double g, const double* tin, c
       ptj = exp(plog);
       poj = ptj + (prad0 - pradj);
       if (poj <= 0.0) poj = fmax(ptj * 1.0e-4, 1.0e-10);
-      abj = b_rosstab(R, tlj, poj, gtid, fold, parity, bar);
+      abj = b_rosstab<kOne>(R, D, tlj, poj, gtid, fold, parity, bar, rab);
       if (J == 1) ab0 = abj;
-      dplog = g / abj * tauj / ptj * dlgtau;
+      dplog = gtau / ptj * rab;
       dplog = fmax(0.0, fmin(10.0, dplog));
     }
     if (J == 1 && (ab0 / ab1init > 2.0 || ab1init / ab0 > 2.0)) {
@@ -378,7 +394,7 @@ __device__ inline void b_ttaup(const RossView& R, double g, const double* tin, c
       ptj = exp(plog);
       poj = ptj;
       if (poj > 0.0) {
-        ab0 = b_rosstab(R, (log10(tin[0]) - R.zerot) / R.slopet, poj, gtid, fold, parity, bar);
+        ab0 = b_rosstab<kOne>(R, D, tlj, poj, gtid, fold, parity, bar, rab);
         abj = ab0;
         plog = log(g / ab0 * tau[0]);
         ptj = exp(plog);
@@ -579,10 +595,16 @@ __device__ inline double b_atlas_finish(ModelState* gms, double* gacc, int kw, i
   }
   __syncthreads();
   {
-    const RossView RV{s_n[1], s_scal[0], s_scal[1], s_scal[2], s_scal[3], rt, rp, rk};
+    const RossView RV{s_n[1], s_scal[0], s_scal[1], s_scal[2], s_scal[3], rt, rp, rk, 1.0 / s_scal[3]};
     const int grp = tid / kFinGroup, gtid = tid % kFinGroup;
-    if (grp == 0) b_ttaup(RV, grav, tnew1, taustd, ab1, pt1, p1, prdnew, n, gtid, fold[0], 1);
-    else if (grp == 1) b_ttaup(RV, grav, tnew2, taustd, ab2, pt2, p2, prdnew, n, gtid, fold[1], 2);
+    const double* tn = grp == 0 ? tnew1 : tnew2;
+    double *ab = grp == 0 ? ab1 : ab2, *pt = grp == 0 ? pt1 : pt2, *po = grp == 0 ? p1 : p2;
+    if (grp < 2) {
+      if (RV.n > 32 * kFinLane)
+        b_ttaup<false>(RV, grav, tn, taustd, ab, pt, po, prdnew, n, gtid, fold[grp], 1 + grp);
+      else if (gtid < 32)
+        b_ttaup<true>(RV, grav, tn, taustd, ab, pt, po, prdnew, n, gtid, fold[grp], 1 + grp);
+    }
   }
   __syncthreads();
   if (tid < 32) {
