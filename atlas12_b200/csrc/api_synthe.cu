@@ -481,8 +481,8 @@ int merged_bins(double wl, int nlast, int nelion, double xne, double wbegin, dou
 // hydrogen_line_profile at that depth)
 static int synthe_hydrogen_launch(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* recs, int64_t n, int length, int nrhox,
                                   double wbegin, double ratio, double wlend, double dopratio, const float* continuum,
-                                  const double* xnfdop, const float* d_cont, const double* d_xd, const double* d_dp,
-                                  int nspec, const double* xne, const double* d_xne, const double* hckt,
+                                  const double* xnfdop, const double* d_wave, const float* d_cont, const double* d_xd,
+                                  const double* d_dp, int nspec, const double* xne, const double* d_xne, const double* hckt,
                                   const double* d_hc, const atlasgpu_synthe_hydrogen* hyd, double* d_acc) {
   static const double conth[15] = {109678.764, 27419.659, 12186.462, 6854.871, 4387.113, 3046.604, 2238.320, 1713.713,
                                    1354.044,   1096.776,  906.426,   761.650,  648.980,  559.579,  487.456};
@@ -603,13 +603,12 @@ static int synthe_hydrogen_launch(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* r
   const double* hv[5] = {hyd->t, hyd->xnfph1, hyd->xnfph2, hyd->xnfhe1, hyd->xnfh2};
   for (int q = 0; q < 5; ++q)
     CK(cudaMemcpyAsync(d_hv + (size_t)q * nrhox, hv[q], nrhox * sizeof(double), cudaMemcpyHostToDevice, s));
-  ShArgs a{d_hr, d_pair, nh, nrhox, length, nspec, wbegin, ratio, wlend, d_cont, d_xd, d_dp, d_xne, d_hc,
+  ShArgs a{d_hr, d_pair, nh, nrhox, length, nspec, wbegin, ratio, wlend, d_wave, d_cont, d_xd, d_dp, d_xne, d_hc,
            d_hv, d_hv + nrhox, d_hv + 2 * nrhox, d_hv + 3 * nrhox, d_hv + 4 * nrhox,
            (const atlasgpu_hydrogen_tables*)ctx->bufs["sh_tab"].first,
            (const StehleDev*)ctx->bufs["sh_stehle"].first, d_acc};
-  const int64_t nwarps = nh * nrhox;
-  const int blocks = grid_for(ctx, nwarps * 32, 32 * kShWarps, 32);
-  k_synthe_hydrogen<<<blocks, 32 * kShWarps, 0, s>>>(a);
+  const int blocks = grid_for(ctx, nh * nrhox * kShThreads, kShThreads, 32);
+  k_synthe_hydrogen<<<blocks, kShThreads, 0, s>>>(a);
   CKL(ctx);
   CK(cudaStreamSynchronize(s));  // the host vectors go out of scope
   return 0;
@@ -761,8 +760,16 @@ int atlasgpu_synthe_nlte_opacity(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* re
   CK(cudaMemcpyAsync(d_cx, contx, 26 * 17 * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemsetAsync(d_acc, 0, nm * sizeof(double), s));
   if (n > 0) {
-    NlteArgs a{d_rec, n, length, nrhox, nspec, wbegin, ratio, wlend, 1.0 + velshift_kms / 299792.458, d_cont, d_xd,
-               d_dp, d_xne, d_tx, d_hc, d_em, d_cx, d_acc};
+    double* d_wave;
+    NlteRest* d_rest;
+    int* d_nrest;
+    const int64_t restcap = std::min<int64_t>(2 * n * nrhox, kNlteRestMax);
+    if ((r = bufT(ctx, "sn_wave", (size_t)2 * length, &d_wave)) || (r = bufT(ctx, "sn_rest", (size_t)restcap, &d_rest)) ||
+        (r = bufT(ctx, "sn_nrest", 2, &d_nrest)))
+      return r;
+    CK(cudaMemsetAsync(d_nrest, 0, 2 * sizeof(int), s));
+    NlteArgs a{d_rec, n, length, nrhox, nspec, wbegin, ratio, wlend, 1.0 + velshift_kms / 299792.458, d_wave,
+               d_wave + length, d_cont, d_xd, d_dp, d_xne, d_tx, d_hc, d_em, d_cx, d_acc, d_rest, d_nrest, (int)restcap};
     if (xnfpel) {
       double* d_xp;
       if ((r = bufT(ctx, "sn_xp", nd, &d_xp))) return r;
@@ -795,10 +802,15 @@ int atlasgpu_synthe_nlte_opacity(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* re
       }
     }
     Timer tm(ctx, "synthe_nlte");
+    k_grid_wave<<<(length + 255) / 256, 256, 0, s>>>(wbegin, ratio, length, d_wave, d_wave + length);
+    CKL(ctx);
     k_synthe_nlte<<<grid_for(ctx, n * nrhox * 32, 256, 16), 256, 0, s>>>(a);
     CKL(ctx);
+    k_synthe_nlte_rest<<<grid_for(ctx, restcap * 32 * kNlteWarps, 32 * kNlteWarps, 4), 32 * kNlteWarps, 0, s>>>(a);
+    CKL(ctx);
     if (hyd && (r = synthe_hydrogen_launch(ctx, recs, n, length, nrhox, wbegin, ratio, wlend, a.dopratio, continuum,
-                                           xnfdop, d_cont, d_xd, d_dp, nspec, xne, d_xne, hckt, d_hc, hyd, d_acc)))
+                                           xnfdop, d_wave, d_cont, d_xd, d_dp, nspec, xne, d_xne, hckt, d_hc, hyd,
+                                           d_acc)))
       return r;
     k_add_f64_to_f32<<<grid_for(ctx, (int64_t)nm, 256, 8), 256, 0, s>>>(d_acc, d_op, (int64_t)nm);
     CKL(ctx);

@@ -58,6 +58,32 @@ __host__ __device__ inline double powi(double x, int m) {
   return m < 0 ? 1.0 / y : y;
 }
 
+// The smallest thread index of a block of kWarps warps with each of two
+// predicates (32 * kWarps: none).  Two slots in turn, so one barrier a call; par
+// is the caller's, 0 before its first call.
+template <int kWarps>
+struct BlockVote {
+  int w[2][2][kWarps];
+};
+template <int kWarps>
+__device__ __forceinline__ void block_vote(BlockVote<kWarps>& v, int& par, bool p0, bool p1, int tid, int& f0,
+                                           int& f1) {
+  const unsigned b0 = __ballot_sync(0xffffffffu, p0), b1 = __ballot_sync(0xffffffffu, p1);
+  const int w = tid >> 5;
+  if ((tid & 31) == 0) {
+    v.w[par][0][w] = b0 ? w * 32 + __ffs(b0) - 1 : 32 * kWarps;
+    v.w[par][1][w] = b1 ? w * 32 + __ffs(b1) - 1 : 32 * kWarps;
+  }
+  __syncthreads();
+  f0 = f1 = 32 * kWarps;
+#pragma unroll
+  for (int k = 0; k < kWarps; ++k) {
+    f0 = min(f0, v.w[par][0][k]);
+    f1 = min(f1, v.w[par][1][k]);
+  }
+  par ^= 1;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -735,22 +735,42 @@ static __global__ void k_spec_flux(SpecArgs a) {
 
 // ---------------------------------------------------------------- NLTE list
 // compute_line_opacity's normal-metal branch (TYPE 0, 3 and the He I
-// fallthrough TYPE <= -3; synthe_module.f90:3400-3458), FP64.  One warp per
-// (record, depth); lanes take 32 consecutive grid points of a wing, the
-// first lane below the cutoff ends the wing (red: tested before the add,
-// blue: after it).  Points blueward of WCON are skipped, WCON..WTAIL tapers.
-// Grid wavelengths are wbegin * ratio**(i-1) per point (the reference walks
-// them by repeated multiplication; the two agree to ~1e-11 relative).
+// fallthrough TYPE <= -3; synthe_module.f90:3400-3458), its autoionizing (Shore)
+// lines (:3609-3650) and merged-continuum edges (:3652-3696), FP64.  The wings
+// of a (record, depth) are walked over consecutive grid points, one per lane;
+// the first lane below the cutoff ends a wing (metals, red: tested before the
+// add; everywhere else after it).  Points blueward of WCON are skipped,
+// WCON..WTAIL tapers.  Grid wavelengths are wbegin * ratio**(i-1) (the reference
+// walks them by repeated multiplication; the two agree to ~1e-11 relative).
+//
+// Most wings end within a few steps of 32 points, a Shore line's or an edge's
+// run over the window (15,000 points for 12 nm at 390 nm), and those few chains
+// of 470 latency-bound steps were the kernel.  So a warp walks a wing for
+// kNlteSolo steps and then lists what is left; a block per listed wing walks on,
+// 256 points a step (k_synthe_nlte_rest).  With the wavelengths from a table
+// (a power per point before) and one division a Shore point for five: 300
+// records, 72 depths, 12 nm: 818 -> 290 us.
+struct NlteRest {
+  int64_t pair;  // record * nrhox + depth
+  int pos, red;  // next grid point (1-based) and direction
+};
+constexpr int kNlteSolo = 8;                // steps of a warp before a wing is listed
+constexpr int kNlteWarps = 8;               // warps per listed wing
+constexpr int64_t kNlteRestMax = 1 << 18;   // a full list: the warp walks its wing to the end
 struct NlteArgs {
   const atlasgpu_nlte_line* rec;
   int64_t n;
   int length, nrhox, nspec;
   double wbegin, ratio, wlend, dopratio;
+  const double *wave, *freq;        // [length] grid wavelengths and frequencies (k_grid_wave)
   const float* cont;                // [nrhox][length]
   const double *xnfdop, *dopple;    // [nrhox][nspec]
   const double *xne, *txnxn, *hckt, *emerge;  // [nrhox]
   const double* contx;              // CONTX(26,17) column-major
   double* acc;                      // [nrhox][length]
+  NlteRest* rest;                   // [restcap]
+  int* nrest;                       // items listed, items taken
+  int restcap;
   const double* xnfpel = nullptr;   // [nrhox][nspec] XNFPEL = populations / RHO; null: Shore lines skipped
   // merged-continuum edges (TYPE >= 4): per record its ordinal m (-1: none)
   // and per (m, depth) the grid indices NBUFF1, NBUFF2, NBUFF3 and a flag
@@ -759,156 +779,201 @@ struct NlteArgs {
   const int4* mbins = nullptr;
 };
 
-// compute_line_opacity's autoionizing (Shore) lines, synthe_module.f90:3609-3650:
-// KAPPA0 = GAMMAW*GF*XNFPEL with the two continuum gates around the Boltzmann
-// factor, then the Fano profile KAPPA0*(GAMMAS*EPSIL + GAMMAW)/(EPSIL**2+1)/GAMMAW,
-// EPSIL = 2*(FREQ - FRELIN)/GAMMAR, red wing from nbuff to the grid end and blue
-// wing to its start, each point added and then tested against
-// continuum(i)*LINE_CUTOFF.  One warp per (record, depth), 32 points per step.
-static __device__ __forceinline__ void synthe_shore_pair(const NlteArgs& a, const atlasgpu_nlte_line& r, int j,
-                                                         int lane) {
-  const int nel = r.nelion - 1;
-  const float* cont = a.cont + (size_t)j * a.length;
-  double* acc = a.acc + (size_t)j * a.length;
-  const double wl = r.wlvac * a.dopratio;
-  const int nbuff = r.nbuff;
-  const double gr = (double)r.gammar, gs = (double)r.gammas, gw = (double)r.gammaw;
-  double kappa0 = gw * (double)r.gf * a.xnfpel[(size_t)j * a.nspec + nel];
-  const int ic = nbuff < 1 ? 1 : (nbuff > a.length ? a.length : nbuff);
-  const double kapmin = (double)cont[ic - 1] * kLineCutoff;
-  if (kappa0 < kapmin) return;
-  kappa0 = kappa0 * exp(-(double)r.elo * a.hckt[j]);
-  if (kappa0 < kapmin) return;
-  const double frelin = kClightNms / wl;
-  auto kappa_at = [&](int ib) {
-    const double freq = kClightNms / (a.wbegin * powi(a.ratio, ib - 1));
-    const double eps = 2.0 * (freq - frelin) / gr;
-    return kappa0 * (gs * eps + gw) / (eps * eps + 1.0) / gw;
-  };
-  if (wl <= a.wlend) {
-    const int minred = nbuff > 1 ? nbuff : 1;
-    for (int base = minred; base <= a.length; base += 32) {
-      const int ib = base + lane;
-      const bool in = ib <= a.length;
-      const double k = in ? kappa_at(ib) : 0.0;
-      const unsigned sb = __ballot_sync(0xffffffffu, in && k < (double)cont[ib - 1] * kLineCutoff);
-      const int first = sb ? __ffs(sb) - 1 : 32;
-      if (in && lane <= first) atomicAdd(acc + ib - 1, k);
-      if (sb) break;
-    }
-    if (nbuff == 1 || wl < a.wbegin) return;
-  }
-  const int ib0 = a.length + 1 < nbuff ? a.length + 1 : nbuff;
-  const int maxblue = ib0 - 1;
-  for (int i0 = 1; i0 <= maxblue; i0 += 32) {
-    const int i = i0 + lane;
-    const int ib = ib0 - i;
-    const bool in = i <= maxblue;
-    const double k = in ? kappa_at(ib) : 0.0;
-    const unsigned sb = __ballot_sync(0xffffffffu, in && k < (double)cont[ib - 1] * kLineCutoff);
-    const int first = sb ? __ffs(sb) - 1 : 32;
-    if (in && lane <= first) atomicAdd(acc + ib - 1, k);
-    if (sb) break;
-  }
+static __global__ void k_grid_wave(double wbegin, double ratio, int length, double* __restrict__ wave,
+                                   double* __restrict__ freq) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= length) return;
+  const double w = wbegin * powi(ratio, i);
+  wave[i] = w;
+  freq[i] = kClightNms / w;
 }
 
-static __global__ void __launch_bounds__(256) k_synthe_nlte(NlteArgs a) {
+// one (record, depth): what its points need, and where its wings start
+struct NlteWalk {
+  int kind;  // 0 metal, 1 Shore, 2 merged-continuum edge
+  double k0, wl, wcon, wtail, rtaper, adamp, rdopwl;  // metal (k0, wl: all)
+  double frelin, gr2, gs, gw;                         // Shore: GAMMAS, GAMMAW, 2 / GAMMAR
+  int flat, last;                                     // edge: flat to here, zero at
+  int red, redend, blue;                              // first points (0: no such wing), last red point
+};
+
+__device__ __forceinline__ bool nlte_setup(const NlteArgs& a, int64_t p, NlteWalk& w) {
+  const int64_t il = p / a.nrhox;
+  const int j = (int)(p - il * a.nrhox);
+  const atlasgpu_nlte_line r = a.rec[il];
+  const int t = r.itype;
+  w.red = w.blue = 0;
+  w.redend = a.length;
+  if (t >= 4) {
+    // flat to NBUFF2, then tapering to zero at NBUFF3
+    if (!a.mbins) return false;
+    const int m = a.mord[il];
+    if (m < 0) return false;
+    const int4 b = a.mbins[(size_t)m * a.nrhox + j];
+    if (!b.w) return false;
+    w.kind = 2;
+    w.k0 = (double)r.gf * a.xnfpel[(size_t)j * a.nspec + r.nelion - 1] * exp(-(double)r.elo * a.hckt[j]);
+    w.rtaper = 1.0 / (double)(b.z - b.y);
+    w.flat = b.y;
+    w.last = b.z;
+    w.red = b.x;
+    w.redend = b.z < a.length ? b.z : a.length;
+    return true;
+  }
+  const bool shore = t == 1 && a.xnfpel;
+  if (!(shore || t == 0 || t == 3 || t <= -3) || r.nelion < 1 || r.nelion > a.nspec) return false;
+  const float* cont = a.cont + (size_t)j * a.length;
+  const int nbuff = r.nbuff, nel = r.nelion - 1;
+  const int ic = nbuff < 1 ? 1 : (nbuff > a.length ? a.length : nbuff);
+  const double kapmin = (double)cont[ic - 1] * kLineCutoff;
+  w.wl = r.wlvac * a.dopratio;
+  if (shore) {
+    // KAPPA0 = GAMMAW*GF*XNFPEL with the two continuum gates around the Boltzmann
+    // factor, then the Fano profile KAPPA0*(GAMMAS*EPSIL + GAMMAW)/(EPSIL**2+1)/GAMMAW,
+    // EPSIL = 2*(FREQ - FRELIN)/GAMMAR
+    w.kind = 1;
+    w.gs = (double)r.gammas;
+    w.gw = (double)r.gammaw;
+    w.gr2 = 2.0 / (double)r.gammar;
+    double kappa0 = w.gw * (double)r.gf * a.xnfpel[(size_t)j * a.nspec + nel];
+    if (kappa0 < kapmin) return false;
+    kappa0 = kappa0 * exp(-(double)r.elo * a.hckt[j]);
+    if (kappa0 < kapmin) return false;
+    w.k0 = kappa0 / w.gw;
+    w.frelin = kClightNms / w.wl;
+  } else {
+    const double xd = a.xnfdop[(size_t)j * a.nspec + nel], dp = a.dopple[(size_t)j * a.nspec + nel];
+    double kappa0 = (double)r.gf * xd;
+    if (kappa0 < kapmin) return false;
+    kappa0 = kappa0 * exp(-(double)r.elo * a.hckt[j]);
+    if (kappa0 < kapmin) return false;
+    w.kind = 0;
+    w.k0 = kappa0;
+    w.wcon = w.wtail = 0.0;
+    if (r.ncon > 0) {
+      const double cx = a.contx[(size_t)(r.nelionx - 1) * 26 + (r.ncon - 1)];
+      w.wcon = 1.0e7 / (cx - a.emerge[j]) * a.dopratio;
+      w.wtail = 1.0e7 / (cx - a.emerge[j] - 500.0) * a.dopratio;
+    }
+    w.rtaper = 1.0 / (w.wtail - w.wcon);
+    w.adamp = ((double)r.gammar + (double)r.gammas * a.xne[j] + (double)r.gammaw * a.txnxn[j]) / dp;
+    w.rdopwl = 1.0 / (dp * w.wl);
+  }
+  bool blue = true;
+  if (w.wl <= a.wlend) {
+    w.red = nbuff > 1 ? nbuff : 1;
+    blue = !((shore ? nbuff : w.red) == 1 || w.wl < a.wbegin);
+  }
+  if (blue) w.blue = (a.length + 1 < nbuff ? a.length + 1 : nbuff) - 1;
+  return true;
+}
+
+// walks one wing from point pos on, 32 (kBlock: 32 kNlteWarps) points a step;
+// returns where it stands after maxsteps steps, 0 when the wing has ended
+template <bool kBlock>
+__device__ __forceinline__ int nlte_walk(const NlteArgs& a, const NlteWalk& w, int j, bool red, int pos, int maxsteps,
+                                         int t, BlockVote<kNlteWarps>* vote, int& par) {
+  constexpr int W = kBlock ? 32 * kNlteWarps : 32;
+  const float* cont = a.cont + (size_t)j * a.length;
+  double* acc = a.acc + (size_t)j * a.length;
+  const bool before = w.kind == 0 && red;  // tested before the add
+  for (int steps = 0; red ? pos <= w.redend : pos >= 1; pos += red ? W : -W) {
+    if (steps++ == maxsteps) return pos;
+    const int ib = red ? pos + t : pos - t;
+    bool use = red ? ib <= w.redend : ib >= 1, stop = false;
+    double kappa = 0.0;
+    if (use) {
+      if (w.kind == 0) {
+        const double wave = a.wave[ib - 1];
+        use = wave >= w.wcon;
+        if (use) {
+          kappa = w.k0 * voigt_weideman(fabs(wave - w.wl) * w.rdopwl, w.adamp);
+          if (wave < w.wtail) kappa = kappa * ((wave - w.wcon) * w.rtaper);
+          stop = kappa < (double)cont[ib - 1] * kLineCutoff;
+        }
+      } else if (w.kind == 1) {
+        const double eps = w.gr2 * (a.freq[ib - 1] - w.frelin);
+        kappa = w.k0 * (w.gs * eps + w.gw) / (eps * eps + 1.0);
+        stop = kappa < (double)cont[ib - 1] * kLineCutoff;
+      } else {
+        kappa = ib > w.flat ? w.k0 * ((double)(w.last - ib) * w.rtaper) : w.k0;
+      }
+    }
+    int first, none;
+    if (kBlock) {
+      block_vote(*vote, par, stop, false, t, first, none);
+    } else {
+      const unsigned sb = __ballot_sync(0xffffffffu, stop);
+      first = sb ? __ffs(sb) - 1 : 32;
+    }
+    if (use && (before ? t < first : t <= first)) atomicAdd(acc + ib - 1, kappa);
+    if (first < W) return 0;
+  }
+  return 0;
+}
+
+static __global__ void __launch_bounds__(256) k_synthe_nlte(const __grid_constant__ NlteArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t npair = a.n * a.nrhox;
+  int par = 0;
   for (int64_t p = w0; p < npair; p += nw) {
-    const int64_t il = p / a.nrhox;
+    NlteWalk w;
+    if (!nlte_setup(a, p, w)) continue;
     const int j = (int)(p % a.nrhox);
-    const atlasgpu_nlte_line r = a.rec[il];
-    const int t = r.itype;
-    if (t == 1 && a.xnfpel && r.nelion >= 1 && r.nelion <= a.nspec) {
-      synthe_shore_pair(a, r, j, lane);
-      continue;
-    }
-    if (t >= 4) {
-      // merged-continuum edge (synthe_module.f90:3652-3696): flat to NBUFF2,
-      // then tapering to zero at NBUFF3
-      if (!a.mbins) continue;
-      const int m = a.mord[il];
-      if (m < 0) continue;
-      const int4 b = a.mbins[(size_t)m * a.nrhox + j];
-      if (!b.w) continue;
-      const double kappa = (double)r.gf * a.xnfpel[(size_t)j * a.nspec + r.nelion - 1] *
-                           exp(-(double)r.elo * a.hckt[j]);
-      const double dn = (double)(b.z - b.y);
-      const int hi = b.z < a.length ? b.z : a.length;
-      double* acc = a.acc + (size_t)j * a.length;
-      for (int ib = b.x + lane; ib <= hi; ib += 32) {
-        const double tail = ib > b.y ? (double)(b.z - ib) / dn : 1.0;
-        atomicAdd(acc + ib - 1, kappa * tail);
+#pragma unroll 1
+    for (int dir = 0; dir < 2; ++dir) {
+      const bool red = dir == 0;
+      int pos = red ? w.red : w.blue;
+      if (pos < 1) continue;
+      pos = nlte_walk<false>(a, w, j, red, pos, kNlteSolo, lane, nullptr, par);
+      if (pos < 1) continue;
+      int slot = 0;
+      if (lane == 0) slot = atomicAdd(a.nrest, 1);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (slot < a.restcap) {
+        if (lane == 0) a.rest[slot] = NlteRest{p, pos, red};
+      } else {
+        nlte_walk<false>(a, w, j, red, pos, 0x7fffffff, lane, nullptr, par);
       }
-      continue;
     }
-    if (!(t == 0 || t == 3 || t <= -3) || r.nelion < 1 || r.nelion > a.nspec) continue;
-    const float* cont = a.cont + (size_t)j * a.length;
-    double* acc = a.acc + (size_t)j * a.length;
-    const double wl = r.wlvac * a.dopratio;
-    const int nbuff = r.nbuff;
-    const int nel = r.nelion - 1;
-    const double xd = a.xnfdop[(size_t)j * a.nspec + nel], dp = a.dopple[(size_t)j * a.nspec + nel];
-    double kappa0 = (double)r.gf * xd;
-    const int ic = nbuff < 1 ? 1 : (nbuff > a.length ? a.length : nbuff);
-    const double kapmin = (double)cont[ic - 1] * kLineCutoff;
-    if (kappa0 < kapmin) continue;
-    kappa0 = kappa0 * exp(-(double)r.elo * a.hckt[j]);
-    if (kappa0 < kapmin) continue;
-    double wcon = 0.0, wtail = 0.0;
-    if (r.ncon > 0) {
-      const double cx = a.contx[(size_t)(r.nelionx - 1) * 26 + (r.ncon - 1)];
-      wcon = 1.0e7 / (cx - a.emerge[j]) * a.dopratio;
-      wtail = 1.0e7 / (cx - a.emerge[j] - 500.0) * a.dopratio;
-    }
-    const double adamp = ((double)r.gammar + (double)r.gammas * a.xne[j] + (double)r.gammaw * a.txnxn[j]) / dp;
-    const double dopwl = dp * wl;
-    if (wl <= a.wlend) {
-      const int minred = nbuff > 1 ? nbuff : 1;
-      for (int base = minred; base <= a.length; base += 32) {
-        const int ib = base + lane;
-        bool use = false, stop = false;
-        double kappa = 0.0;
-        if (ib <= a.length) {
-          const double wave = a.wbegin * powi(a.ratio, ib - 1);
-          if (wave >= wcon) {
-            use = true;
-            kappa = kappa0 * voigt_weideman(fabs(wave - wl) / dopwl, adamp);
-            if (wave < wtail) kappa = kappa * ((wave - wcon) / (wtail - wcon));
-            stop = kappa < (double)cont[ib - 1] * kLineCutoff;
-          }
-        }
-        const unsigned sb = __ballot_sync(0xffffffffu, stop);
-        const int first = sb ? __ffs(sb) - 1 : 32;
-        if (use && lane < first) atomicAdd(acc + ib - 1, kappa);
-        if (sb) break;
+  }
+}
+
+// (items are taken from the list in turn: their lengths differ by factors of ten)
+static __global__ void __launch_bounds__(32 * kNlteWarps, 3) k_synthe_nlte_rest(const __grid_constant__ NlteArgs a) {
+  __shared__ BlockVote<kNlteWarps> vote;
+  __shared__ NlteWalk walk;
+  __shared__ NlteRest item;
+  __shared__ int s_i;
+  const int n = min(a.nrest[0], a.restcap);
+  int par = 0;
+  for (;;) {
+    if (threadIdx.x < 32) {
+      int i = 0;
+      if (threadIdx.x == 0) i = atomicAdd(a.nrest + 1, 1);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      NlteWalk w;
+      NlteRest q{0, 0, 0};
+      if (i < n) {
+        q = a.rest[i];
+        nlte_setup(a, q.pair, w);
       }
-      if (minred == 1 || wl < a.wbegin) continue;
-    }
-    const int ib0 = a.length + 1 < nbuff ? a.length + 1 : nbuff;
-    const int maxblue = ib0 - 1;
-    for (int i0 = 1; i0 <= maxblue; i0 += 32) {
-      const int i = i0 + lane;
-      const int ib = ib0 - i;
-      bool use = false, stop = false;
-      double kappa = 0.0;
-      if (i <= maxblue) {
-        const double wave = a.wbegin * powi(a.ratio, ib - 1);
-        if (wave >= wcon) {
-          use = true;
-          kappa = kappa0 * voigt_weideman(fabs(wave - wl) / dopwl, adamp);
-          if (wave < wtail) kappa = kappa * ((wave - wcon) / (wtail - wcon));
-          stop = kappa < (double)cont[ib - 1] * kLineCutoff;
+      if (threadIdx.x == 0) {
+        s_i = i;
+        if (i < n) {
+          walk = w;
+          item = q;
         }
       }
-      const unsigned sb = __ballot_sync(0xffffffffu, stop);
-      const int first = sb ? __ffs(sb) - 1 : 32;
-      if (use && lane <= first) atomicAdd(acc + ib - 1, kappa);
-      if (sb) break;
     }
+    __syncthreads();
+    if (s_i >= n) break;
+    const NlteWalk w = walk;
+    const NlteRest q = item;
+    nlte_walk<true>(a, w, (int)(q.pair % a.nrhox), q.red != 0, q.pos, 0x7fffffff, threadIdx.x, &vote, par);
+    __syncthreads();
   }
 }
 
