@@ -75,6 +75,8 @@ SIGNATURES = {
     "atlasgpu_synthe_continuum": (_I, [_P, _P, _I, _P, _I, _I, _D, _D, _I, _P]),
     "atlasgpu_synthe_line_opacity": (_I, [_P, _P, _I64, _I, _I, _D, _P, _P, _P, _I, _P, _P, _P, _I, _P]),
     "atlasgpu_synthe_line_opacity_dev": (_I, [_P, _P, _I64, _I, _I, _D, _P, _P, _P, _I, _P, _P, _P, _I, _P]),
+    "atlasgpu_synthe_window": (_I, [_P, _P, _I, _P, _P, _P, _I, _I, _I, _P, _I64, _D, _P, _P, _I, _P, _P, _P, _I, _P, _P,
+                                    _D, _D, _I, _P, _P, _P]),
     "atlasgpu_synthe_spectrum": (_I, [_P, _P, _I, _P, _P, _I, _I, _P, _P, _D, _D, _I, _P, _P, _P]),
     "atlasgpu_synthe_spectrum_dev": (_I, [_P, _P, _I, _P, _P, _I, _I, _P, _P, _D, _D, _I, _P, _P, _P]),
     "atlasgpu_atlas_set_voigt_tables": (_I, [_P, _P, _P, _P, _I]),

@@ -252,13 +252,13 @@ int atlasgpu_atlas_linop(atlasgpu_ctx* ctx, const int32_t* linedata, int64_t n, 
       (r = bufT(ctx, "al_cnt", 2, &d_cnt)) || (r = ensure_tablog(ctx, &tl)))
     return r;
   if (n > 0) CK(cudaMemcpyAsync(d_ld, linedata, n * 4 * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(d_tc, tabcont, (size_t)(nwave + 1) * kw * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_iw, iwavetab, (nwave + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_xd, xnfdop, nd * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_dp, dopple, nd * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_xne, xne, nrhox * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_tx, txnxn, nrhox * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_hc, hckt, nrhox * sizeof(double), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(d_tc, tabcont, (size_t)(nwave + 1) * kw * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d_ws, waveset, numnu * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemsetAsync(d_xl, 0, (size_t)kw * numnu * sizeof(double), s));
   CK(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), s));
@@ -295,7 +295,7 @@ int atlasgpu_atlas_linop(atlasgpu_ctx* ctx, const int32_t* linedata, int64_t n, 
     }
     work_collect(ctx, a.work, {"atlas_linop_points"});
   }
-  CK(cudaMemcpyAsync(xlines_out, d_xl, (size_t)kw * numnu * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if ((r = host_out(ctx, {{xlines_out, d_xl, (size_t)kw * numnu * sizeof(double)}}))) return r;
   unsigned long long cnt[2];
   CK(cudaMemcpyAsync(cnt, d_cnt, sizeof cnt, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -405,7 +405,7 @@ int atlasgpu_atlas_xlinop(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* recs, int
       }
     }
   }
-  CK(cudaMemcpyAsync(xlines_inout, d_xl, (size_t)kw * numnu * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if ((r = host_out(ctx, {{xlines_inout, d_xl, (size_t)kw * numnu * sizeof(double)}}))) return r;
   CK(cudaStreamSynchronize(s));
   return 0;
 }

@@ -328,10 +328,11 @@ int kapp_run(atlasgpu_ctx* ctx, const char* name, int numnu, const double* waves
       k_kapp_nu<false, false><<<blocks, kKappWarps * 32, 0, s>>>(a);
     CKL(ctx);
   }
-  CK(cudaMemcpyAsync(acont, a.acont, nt * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(sigmac, a.sigmac, nt * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(scont, a.scont, nt * sizeof(double), cudaMemcpyDeviceToHost, s));
-  if (parts) CK(cudaMemcpyAsync(parts, d_parts, (size_t)nparts * nt * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if ((r = host_out(ctx, {{acont, a.acont, nt * sizeof(double)},
+                          {sigmac, a.sigmac, nt * sizeof(double)},
+                          {scont, a.scont, nt * sizeof(double)},
+                          {parts, d_parts, parts ? (size_t)nparts * nt * sizeof(double) : 0}})))
+    return r;
   CK(cudaStreamSynchronize(s));
   return 0;
 }
@@ -441,8 +442,8 @@ int atlasgpu_atlas_hlinop(atlasgpu_ctx* ctx, int numnu, const double* waveset, i
     k_hlinop<<<blocks, kKappWarps * 32, 0, s>>>(a);
     CKL(ctx);
   }
-  CK(cudaMemcpyAsync(ahline, a.ahline, nt * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(shline, a.shline, nt * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if ((r = host_out(ctx, {{ahline, a.ahline, nt * sizeof(double)}, {shline, a.shline, nt * sizeof(double)}})))
+    return r;
   CK(cudaStreamSynchronize(s));
   return 0;
 }

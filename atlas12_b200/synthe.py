@@ -133,6 +133,25 @@ class Synthe:
                       ptr(np.ascontiguousarray(contx, np.float64)), hy, ptr(out))
         return out
 
+    def _window(self, case, grid, lines):
+        """continuum, line_opacity and spectrum of one window in one call, the matrices
+        staying on the device: (opacity, flux, continuum flux)."""
+        atm = case["atm"]
+        we, ca, sa, ss, xd, dp, xne, tx, hc, rx, hk = [
+            np.ascontiguousarray(v, np.float64) for v in (case["wledge"], case["continall"], case["contabs"],
+                                                          case["contscat"], atm["xnfdop"], atm["dopple"], atm["xne"],
+                                                          atm["txnxn"], atm["hckt"], atm["rhox"], atm["hkt"])]
+        nrhox, nspec = xd.shape
+        if not ca.shape[0] == sa.shape[0] == nrhox or ss.shape != sa.shape:
+            return None  # tables of other depth counts than the populations: the calls one by one
+        op = np.zeros((nrhox, grid["length"]), np.float32)
+        flux, cflux = np.zeros(grid["length"]), np.zeros(grid["length"])
+        self.ctx.call("atlasgpu_synthe_window", ptr(we), we.size, ptr(ca), ptr(sa), ptr(ss), ca.shape[1], sa.shape[1],
+                      nrhox, ptr(lines), lines.size, float(case["resolu"]), ptr(xd), ptr(dp), nspec, ptr(xne), ptr(tx),
+                      ptr(hc), MAXPROF, ptr(rx), ptr(hk), grid["wbegin"], grid["ratio"], grid["length"], ptr(op),
+                      ptr(flux), ptr(cflux))
+        return op, flux, cflux
+
     def run(self, case):
         """PROGRAM SYNTHE on a prepared case dict (see synthetic.synthe_case):
         returns (wavelength_angstrom, flux, continuum_flux, opacity_matrix).
@@ -145,16 +164,21 @@ class Synthe:
         nb = self.bin_lines(L["wlvac"], grid)
         lines = make_lte_lines(nb, L["cgf"], L["nelion"], L["elo"], L["gamrf"], L["gamsf"], L["gamwf"])
         atm = case["atm"]
-        cont = self.continuum(case["wledge"], case["continall"], grid)
-        op = self.line_opacity(lines, grid, case["resolu"], cont, atm["xnfdop"], atm["dopple"], atm["xne"],
-                               atm["txnxn"], atm["hckt"])
-        if case.get("nlte") is not None and len(case["nlte"]):
-            # unit-19 lines (compute_line_opacity, called per depth before the LTE loop at synthe.f90:554)
-            op = self.nlte_opacity(case["nlte"], grid, case["wlend"], cont, atm["xnfdop"], atm["dopple"], atm["xne"],
-                                   atm["txnxn"], atm["hckt"], case["contx"], op, xnfpel=case.get("xnfpel"),
-                                   hydrogen=case.get("hydrogen"))
-        flux, cflux = self.spectrum(case["wledge"], case["contabs"], case["contscat"], atm["rhox"], atm["hkt"],
-                                    grid, op)
+        nlte = case.get("nlte") is not None and len(case["nlte"])
+        one = None if nlte else self._window(case, grid, lines)
+        if one is not None:
+            op, flux, cflux = one
+        else:
+            cont = self.continuum(case["wledge"], case["continall"], grid)
+            op = self.line_opacity(lines, grid, case["resolu"], cont, atm["xnfdop"], atm["dopple"], atm["xne"],
+                                   atm["txnxn"], atm["hckt"])
+            if nlte:
+                # unit-19 lines (compute_line_opacity, called per depth before the LTE loop at synthe.f90:554)
+                op = self.nlte_opacity(case["nlte"], grid, case["wlend"], cont, atm["xnfdop"], atm["dopple"],
+                                       atm["xne"], atm["txnxn"], atm["hckt"], case["contx"], op,
+                                       xnfpel=case.get("xnfpel"), hydrogen=case.get("hydrogen"))
+            flux, cflux = self.spectrum(case["wledge"], case["contabs"], case["contscat"], atm["rhox"], atm["hkt"],
+                                        grid, op)
         wave = grid["wbegin"] * grid["ratio"] ** np.arange(grid["length"]) * 10.0
         return wave, flux, cflux, op
 

@@ -243,6 +243,16 @@ int atlasgpu_synthe_spectrum_dev(atlasgpu_ctx *ctx, const double *d_wledge, int 
                                  const double *d_hkt, double wbegin, double ratio, int length,
                                  const float *d_opacity, double *d_flux, double *d_cont);
 
+/* The three of a window in one call: continuum, LTE line opacity and spectrum,
+ * as atlasgpu_synthe_continuum, _line_opacity and _spectrum in a row (their
+ * arguments, checks and results), the matrices staying on the device. */
+int atlasgpu_synthe_window(atlasgpu_ctx *ctx, const double *wledge, int nedge, const double *continall,
+                           const double *contabs, const double *contscat, int continall_stride,
+                           int ncont_stride, int nrhox, const atlasgpu_lte_line *lines, int64_t n,
+                           double resolu, const double *xnfdop, const double *dopple, int nspec,
+                           const double *xne, const double *txnxn, const double *hckt, int maxprof,
+                           const double *rhox, const double *hkt, double wbegin, double ratio, int length,
+                           float *opacity_out, double *flux, double *cont);
 
 /* ---- ATLAS12 ---------------------------------------------------------- */
 /* TABVOIGT (atlas12_modules.f90:19796-19851) on the host: H0 = exp(-v^2),
