@@ -7,8 +7,19 @@
 //
 // Layers: h1 = tanh(W1 x + b1), h2 = tanh(W2 h1 + b2), y = W3 h2 + b3,
 // W_l stored [out][in] row-major.  Loss: mean over samples and outputs of
-// (y - target)^2.  Every sum runs in a fixed order (tile by tile, then a
-// fixed-order reduction of per-block partials), so results repeat exactly.
+// (y - target)^2.  Every sum runs in a fixed order (chunk by chunk, then folds of
+// K groups and of per-block partials in fixed orders), so results repeat exactly.
+//
+// A training batch is 64 samples: each of the eight products is 4 MFLOP, and
+// the time is latency and launches.  With 32x32 tiles, one 32-deep chunk in
+// flight and 16 blocks a product took 14 us; 16x16 tiles (64 to 256 blocks), K
+// split over four groups of a block and the next chunk's loads in flight
+// before a chunk is multiplied take 6 us.  The bias gradients are row sums of tiles that
+// the weight gradients load anyway, the loss and its gradient are the last
+// layer's epilogue, and a layer's two backward products share a launch: 13
+// launches a step became 6.  From nsm tiles of 64x64 on the product is bound by
+// arithmetic and takes those (4x4 per thread).  Loss and gradient plus a forward
+// pass of 64 samples: kernels 176 -> 52 us; 4,000 samples 1860 -> 457 us.
 #include <cmath>
 #include <vector>
 
@@ -24,90 +35,178 @@ struct atlasgpu_mlp {
   // activations / gradients for up to cap samples
   int cap = 0;
   float *x, *t, *h1, *h2, *y, *d1, *d2, *dy, *lpart;
+  float* loss;       // [1]
+  unsigned* ticket;  // [1] blocks of the last layer that are done (0 between launches)
 };
 
 namespace {
 
-constexpr int kT = 32;  // tile edge
+// One product C[m][n] = sum_k A(m,k) B(k,n) with A(m,k) = A[m*sam + k*sak],
+// B(k,n) = B[k*sbk + n*sbn] (one stride of each is 1), and what its epilogue does.
+struct Prod {
+  int M, N, K;
+  const float* A;
+  int sam, sak;
+  const float* B;
+  int sbk, sbn;
+  float* C;           // [M][N]
+  const float* bias;  // + bias[n], or null
+  int act;            // then tanh
+  const float* pact;  // result * (1 - pact(m,n)^2): tanh derivative of a layer output [M][N], or null
+  float* rowsum;      // [M] sum_k A(m,k), or null
+  // the last layer's loss: dy = 2 (y - t) / (M N) and sum of (y - t)^2 / (M N), or null
+  const float* t;
+  float *dy, *part, *loss;
+  unsigned* ticket;
+};
+struct Prods {
+  Prod p[2];
+  int tiles0;  // blocks of p[0]; the rest are p[1]'s
+};
 
-// C[m][n] (+)= sum_k A(m,k) B(k,n) with A(m,k) = A[m*sam + k*sak],
-// B(k,n) = B[k*sbk + n*sbn]; epilogue: + bias[n], then tanh when act.
-// mode 0: C = result; 1: C = result * (1 - Pact(m,n)^2) (tanh derivative
-// of the layer output Pact, row-major [m][n]).
-__global__ void k_gemm(int M, int N, int K, const float* __restrict__ A, int sam, int sak,
-                       const float* __restrict__ B, int sbk, int sbn, const float* __restrict__ bias, int act,
-                       int mode, const float* __restrict__ pact, float* __restrict__ C) {
-  __shared__ float As[kT][kT + 1], Bs[kT][kT + 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  const int m0 = blockIdx.y * kT, n0 = blockIdx.x * kT;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < K; k0 += kT) {
-    for (int r = ty; r < kT; r += 8) {
-      const int mm = m0 + r, kk = k0 + tx;
-      As[r][tx] = (mm < M && kk < K) ? A[(size_t)mm * sam + (size_t)kk * sak] : 0.f;
-      const int kb = k0 + r, nn = n0 + tx;
-      Bs[r][tx] = (kb < K && nn < N) ? B[(size_t)kb * sbk + (size_t)nn * sbn] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ty + 8 * q;
-      float s = acc[q];
-#pragma unroll 8
-      for (int kk = 0; kk < kT; ++kk) s = fmaf(As[r][kk], Bs[kk][tx], s);
-      acc[q] = s;
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int mm = m0 + ty + 8 * q, nn = n0 + tx;
-    if (mm < M && nn < N) {
-      float v = acc[q];
-      if (bias) v += bias[nn];
-      if (act) v = tanhf(v);
-      if (mode == 1) {
-        const float p = pact[(size_t)mm * N + nn];
-        v = v * (1.f - p * p);
-      }
-      C[(size_t)mm * N + nn] = v;
-    }
-  }
-}
+constexpr int kMlpThreads = 256;
 
-// column sums: out[n] = sum_m A[m][n] (bias gradients), fixed order in m
-__global__ void k_colsum(int M, int N, const float* __restrict__ A, float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.f;
-  for (int m = 0; m < M; ++m) s += A[(size_t)m * N + n];
-  out[n] = s;
-}
-
-// dy = 2 (y - t) / (n * nout); per-block partial sums of (y - t)^2
-__global__ void k_mse(int64_t total, float scale, const float* __restrict__ y, const float* __restrict__ t,
-                      float* __restrict__ dy, float* __restrict__ part) {
-  __shared__ float sh[256];
-  float s = 0.f;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const float d = y[e] - t[e];
-    if (dy) dy[e] = 2.f * d * scale;
-    s += d * d;
-  }
-  sh[threadIdx.x] = s;
+__device__ __forceinline__ float block_sum(float v, float* sh) {
+  sh[threadIdx.x] = v;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
+  for (int o = kMlpThreads / 2; o > 0; o >>= 1) {
     if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+  const float r = sh[0];
+  __syncthreads();
+  return r;
 }
 
-__global__ void k_sum_parts(int n, const float* __restrict__ part, float scale, float* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s * scale;
+// BM x BN tiles, chunks of BK, TM x TN outputs a thread, KG groups of the block
+// taking every KG-th chunk; the next chunk's loads are issued before a chunk is
+// multiplied
+template <int BM, int BN, int BK, int TM, int TN, int KG>
+__global__ void __launch_bounds__(kMlpThreads) k_prod(const __grid_constant__ Prods ps) {
+  constexpr int GT = kMlpThreads / KG;  // threads of a group
+  static_assert((BM / TM) * (BN / TN) == GT && KG * BM * BN >= kMlpThreads, "tile shape");
+  constexpr int LA = BM * BK / GT, LB = BN * BK / GT;
+  __shared__ float As[KG][BK][BM + 1], Bs[KG][BK][BN + 1];
+  __shared__ float red[KG > 1 ? KG * BM * BN : kMlpThreads];
+  const bool second = (int)blockIdx.x >= ps.tiles0;
+  const Prod& p = ps.p[second];
+  const int tile = blockIdx.x - (second ? ps.tiles0 : 0), ntn = (p.N + BN - 1) / BN;
+  const int m0 = tile / ntn * BM, n0 = tile % ntn * BN;
+  const int g = threadIdx.x / GT, t = threadIdx.x % GT;
+  const int tx = t % (BN / TN), ty = t / (BN / TN);
+  float ra[LA], rb[LB], acc[TM][TN] = {}, rs[TM] = {};
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+      const int e = q * GT + t;
+      const int k = p.sak == 1 ? e % BK : e / BM, m = p.sak == 1 ? e / BK : e % BM;
+      ra[q] = (m0 + m < p.M && k0 + k < p.K) ? p.A[(size_t)(m0 + m) * p.sam + (size_t)(k0 + k) * p.sak] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+      const int e = q * GT + t;
+      const int k = p.sbk == 1 ? e % BK : e / BN, n = p.sbk == 1 ? e / BK : e % BN;
+      rb[q] = (n0 + n < p.N && k0 + k < p.K) ? p.B[(size_t)(k0 + k) * p.sbk + (size_t)(n0 + n) * p.sbn] : 0.f;
+    }
+  };
+  const bool rows = p.rowsum && n0 == 0 && tx == 0;
+  fetch(g * BK);
+  for (int c = 0; c * KG * BK < p.K; ++c) {
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+      const int e = q * GT + t;
+      As[g][p.sak == 1 ? e % BK : e / BM][p.sak == 1 ? e / BK : e % BM] = ra[q];
+    }
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+      const int e = q * GT + t;
+      Bs[g][p.sbk == 1 ? e % BK : e / BN][p.sbk == 1 ? e / BK : e % BN] = rb[q];
+    }
+    __syncthreads();
+    if ((c + 1) * KG * BK < p.K) fetch(((c + 1) * KG + g) * BK);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      float a[TM], b[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = As[g][k][ty * TM + i];
+#pragma unroll
+      for (int i = 0; i < TN; ++i) b[i] = Bs[g][k][tx * TN + i];
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int l = 0; l < TN; ++l) acc[i][l] = fmaf(a[i], b[l], acc[i][l]);
+      if (rows)
+#pragma unroll
+        for (int i = 0; i < TM; ++i) rs[i] += a[i];
+    }
+    __syncthreads();
+  }
+  const float scale = 1.f / ((float)p.M * (float)p.N);
+  float lsum = 0.f;
+  auto finish = [&](int m, int n, float v) {
+    if (m >= p.M || n >= p.N) return;
+    const size_t e = (size_t)m * p.N + n;
+    if (p.bias) v += p.bias[n];
+    if (p.act) v = tanhf(v);
+    if (p.pact) v = v * (1.f - p.pact[e] * p.pact[e]);
+    p.C[e] = v;
+    if (p.dy) {
+      const float d = v - p.t[e];
+      p.dy[e] = 2.f * d * scale;
+      lsum += d * d;
+    }
+  };
+  if (KG > 1) {
+    __shared__ float rrow[KG][BM];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int l = 0; l < TN; ++l) red[(g * BM + ty * TM + i) * BN + tx * TN + l] = acc[i][l];
+    if (rows)
+#pragma unroll
+      for (int i = 0; i < TM; ++i) rrow[g][ty * TM + i] = rs[i];
+    __syncthreads();
+    for (int e = threadIdx.x; e < BM * BN; e += kMlpThreads) {
+      float v = red[e];
+#pragma unroll
+      for (int q = 1; q < KG; ++q) v += red[q * BM * BN + e];
+      finish(m0 + e / BN, n0 + e % BN, v);
+    }
+    if (p.rowsum && n0 == 0 && threadIdx.x < BM && m0 + threadIdx.x < p.M) {
+      float v = rrow[0][threadIdx.x];
+#pragma unroll
+      for (int q = 1; q < KG; ++q) v += rrow[q][threadIdx.x];
+      p.rowsum[m0 + threadIdx.x] = v;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int l = 0; l < TN; ++l) finish(m0 + ty * TM + i, n0 + tx * TN + l, acc[i][l]);
+    if (rows)
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+        if (m0 + ty * TM + i < p.M) p.rowsum[m0 + ty * TM + i] = rs[i];
+  }
+  if (!p.dy) return;
+  // the loss: per-block partials, summed in a fixed order by the last block
+  __syncthreads();
+  lsum = block_sum(lsum, red);
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    p.part[tile] = lsum;
+    __threadfence();
+    last = atomicAdd(p.ticket, 1u) == (unsigned)ps.tiles0 - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  float v = 0.f;
+  for (int i = threadIdx.x; i < ps.tiles0; i += kMlpThreads) v += __ldcg(p.part + i);
+  v = block_sum(v, red);
+  if (threadIdx.x == 0) {
+    *p.loss = v * scale;
+    *p.ticket = 0;
   }
 }
 
@@ -147,68 +246,98 @@ Off offsets(const atlasgpu_mlp* p) {
   return o;
 }
 
-int gemm(atlasgpu_ctx* ctx, int M, int N, int K, const float* A, int sam, int sak, const float* B, int sbk, int sbn,
-         const float* bias, int act, int mode, const float* pact, float* C) {
-  dim3 grid((N + kT - 1) / kT, (M + kT - 1) / kT), block(kT, 8);
-  k_gemm<<<grid, block, 0, ctx->stream>>>(M, N, K, A, sam, sak, B, sbk, sbn, bias, act, mode, pact, C);
+constexpr int kSmallTile = 16, kLargeTile = 64;
+int tiles(const Prod& p, int edge) { return ((p.M + edge - 1) / edge) * ((p.N + edge - 1) / edge); }
+
+// one or two independent products: together in small tiles, each by itself in
+// large ones where those fill the chip
+int products(atlasgpu_ctx* ctx, const Prod& a, const Prod* b) {
+  const bool la = tiles(a, kLargeTile) >= ctx->nsm, lb = b && tiles(*b, kLargeTile) >= ctx->nsm;
+  if (b && (la || lb)) {
+    const int r = products(ctx, a, nullptr);
+    return r ? r : products(ctx, *b, nullptr);
+  }
+  Prods ps{{a, b ? *b : a}, tiles(a, la ? kLargeTile : kSmallTile)};
+  const int blocks = ps.tiles0 + (b ? tiles(*b, kSmallTile) : 0);
+  if (la) k_prod<kLargeTile, kLargeTile, 16, 4, 4, 1><<<blocks, kMlpThreads, 0, ctx->stream>>>(ps);
+  else k_prod<kSmallTile, kSmallTile, 32, 2, 2, 4><<<blocks, kMlpThreads, 0, ctx->stream>>>(ps);
   CKL(ctx);
   return 0;
 }
 
 int ensure_cap(atlasgpu_ctx* ctx, atlasgpu_mlp* p, int n) {
   if (n <= p->cap) return 0;
-  float** bufs[] = {&p->x, &p->t, &p->h1, &p->h2, &p->y, &p->d1, &p->d2, &p->dy};
-  for (float** b : bufs)
+  float** bufs[] = {&p->x, &p->t, &p->h1, &p->h2, &p->y, &p->d1, &p->d2, &p->dy, &p->lpart};
+  p->cap = 0;
+  for (float** b : bufs) {
     if (*b) cudaFree(*b);
-  const int widths[] = {p->nin, p->nout, p->nh1, p->nh2, p->nout, p->nh1, p->nh2, p->nout};
-  for (int i = 0; i < 8; ++i)
-    if (cudaMalloc(bufs[i], sizeof(float) * (size_t)n * widths[i]) != cudaSuccess)
+    *b = nullptr;
+  }
+  Prod last{};
+  last.M = n;
+  last.N = p->nout;
+  const size_t counts[] = {(size_t)n * p->nin, (size_t)n * p->nout, (size_t)n * p->nh1, (size_t)n * p->nh2,
+                           (size_t)n * p->nout, (size_t)n * p->nh1, (size_t)n * p->nh2, (size_t)n * p->nout,
+                           (size_t)tiles(last, kSmallTile)};
+  for (int i = 0; i < 9; ++i)
+    if (cudaMalloc(bufs[i], sizeof(float) * counts[i]) != cudaSuccess) {
+      cudaGetLastError();
       return fail(ctx, ATLASGPU_ENOMEM, "mlp: activations for %d samples", n);
+    }
   p->cap = n;
   return 0;
 }
 
-// forward over n samples already in p->x
-int forward(atlasgpu_ctx* ctx, atlasgpu_mlp* p, int n) {
-  const Off o = offsets(p);
-  int r;
-  if ((r = gemm(ctx, n, p->nh1, p->nin, p->x, p->nin, 1, p->w + o.w1, 1, p->nin, p->w + o.b1, 1, 0, nullptr, p->h1)))
-    return r;
-  if ((r = gemm(ctx, n, p->nh2, p->nh1, p->h1, p->nh1, 1, p->w + o.w2, 1, p->nh1, p->w + o.b2, 1, 0, nullptr, p->h2)))
-    return r;
-  return gemm(ctx, n, p->nout, p->nh2, p->h2, p->nh2, 1, p->w + o.w3, 1, p->nh2, p->w + o.b3, 0, 0, nullptr, p->y);
+// y = act(x W^T + b) of one layer
+Prod layer(int n, int nin, int nout, const float* x, const float* w, const float* b, int act, float* y) {
+  Prod p{};
+  p.M = n, p.N = nout, p.K = nin;
+  p.A = x, p.sam = nin, p.sak = 1;
+  p.B = w, p.sbk = 1, p.sbn = nin;
+  p.bias = b, p.act = act, p.C = y;
+  return p;
+}
+// dW = d^T h and db = column sums of d
+Prod grad_w(int n, int nin, int nout, const float* d, const float* h, float* gw, float* gb) {
+  Prod p{};
+  p.M = nout, p.N = nin, p.K = n;
+  p.A = d, p.sam = 1, p.sak = nout;
+  p.B = h, p.sbk = nin, p.sbn = 1;
+  p.C = gw, p.rowsum = gb;
+  return p;
+}
+// d of the layer below: (d W) (1 - h^2)
+Prod grad_x(int n, int nin, int nout, const float* d, const float* w, const float* h, float* dx) {
+  Prod p{};
+  p.M = n, p.N = nin, p.K = nout;
+  p.A = d, p.sam = nout, p.sak = 1;
+  p.B = w, p.sbk = nin, p.sbn = 1;
+  p.pact = h, p.C = dx;
+  return p;
 }
 
-// loss and gradient (p->g) over n samples in p->x, p->t; loss to *d_loss (device)
-int backward(atlasgpu_ctx* ctx, atlasgpu_mlp* p, int n, float* d_loss) {
+// forward over n samples already in p->x; with d_loss also the loss over p->t and its gradient in p->dy
+int forward(atlasgpu_ctx* ctx, atlasgpu_mlp* p, int n, float* d_loss = nullptr) {
   const Off o = offsets(p);
   int r;
-  const int64_t total = (int64_t)n * p->nout;
-  const int nb = 64;
-  k_mse<<<nb, 256, 0, ctx->stream>>>(total, 1.f / (float)total, p->y, p->t, p->dy, p->lpart);
-  CKL(ctx);
-  k_sum_parts<<<1, 32, 0, ctx->stream>>>(nb, p->lpart, 1.f / (float)total, d_loss);
-  CKL(ctx);
-  // layer 3: dW3 = dy^T h2, db3 = colsum dy, d2 = (dy W3) * (1 - h2^2)
-  if ((r = gemm(ctx, p->nout, p->nh2, n, p->dy, 1, p->nout, p->h2, p->nh2, 1, nullptr, 0, 0, nullptr, p->g + o.w3)))
+  if ((r = products(ctx, layer(n, p->nin, p->nh1, p->x, p->w + o.w1, p->w + o.b1, 1, p->h1), nullptr)) ||
+      (r = products(ctx, layer(n, p->nh1, p->nh2, p->h1, p->w + o.w2, p->w + o.b2, 1, p->h2), nullptr)))
     return r;
-  k_colsum<<<(p->nout + 127) / 128, 128, 0, ctx->stream>>>(n, p->nout, p->dy, p->g + o.b3);
-  CKL(ctx);
-  if ((r = gemm(ctx, n, p->nh2, p->nout, p->dy, p->nout, 1, p->w + o.w3, p->nh2, 1, nullptr, 0, 1, p->h2, p->d2)))
+  Prod last = layer(n, p->nh2, p->nout, p->h2, p->w + o.w3, p->w + o.b3, 0, p->y);
+  if (d_loss) last.t = p->t, last.dy = p->dy, last.part = p->lpart, last.loss = d_loss, last.ticket = p->ticket;
+  return products(ctx, last, nullptr);
+}
+
+// gradient (p->g) from p->dy and the activations of forward
+int backward(atlasgpu_ctx* ctx, atlasgpu_mlp* p, int n) {
+  const Off o = offsets(p);
+  int r;
+  const Prod x2 = grad_x(n, p->nh2, p->nout, p->dy, p->w + o.w3, p->h2, p->d2);
+  const Prod x1 = grad_x(n, p->nh1, p->nh2, p->d2, p->w + o.w2, p->h1, p->d1);
+  if ((r = products(ctx, grad_w(n, p->nh2, p->nout, p->dy, p->h2, p->g + o.w3, p->g + o.b3), &x2)) ||
+      (r = products(ctx, grad_w(n, p->nh1, p->nh2, p->d2, p->h1, p->g + o.w2, p->g + o.b2), &x1)))
     return r;
-  // layer 2
-  if ((r = gemm(ctx, p->nh2, p->nh1, n, p->d2, 1, p->nh2, p->h1, p->nh1, 1, nullptr, 0, 0, nullptr, p->g + o.w2)))
-    return r;
-  k_colsum<<<(p->nh2 + 127) / 128, 128, 0, ctx->stream>>>(n, p->nh2, p->d2, p->g + o.b2);
-  CKL(ctx);
-  if ((r = gemm(ctx, n, p->nh1, p->nh2, p->d2, p->nh2, 1, p->w + o.w2, p->nh1, 1, nullptr, 0, 1, p->h1, p->d1)))
-    return r;
-  // layer 1
-  if ((r = gemm(ctx, p->nh1, p->nin, n, p->d1, 1, p->nh1, p->x, p->nin, 1, nullptr, 0, 0, nullptr, p->g + o.w1)))
-    return r;
-  k_colsum<<<(p->nh1 + 127) / 128, 128, 0, ctx->stream>>>(n, p->nh1, p->d1, p->g + o.b1);
-  CKL(ctx);
-  return 0;
+  return products(ctx, grad_w(n, p->nin, p->nh1, p->d1, p->x, p->g + o.w1, p->g + o.b1), nullptr);
 }
 
 // splitmix64 for the initial weights (deterministic per seed)
@@ -242,7 +371,11 @@ int atlasgpu_mlp_create(atlasgpu_ctx* ctx, int nin, int nh1, int nh2, int nout, 
       delete p;
       return fail(ctx, ATLASGPU_ENOMEM, "mlp_create");
     }
-  CK(cudaMalloc(&p->lpart, sizeof(float) * 65));  // 64 block partials + the loss
+  if (cudaMalloc(&p->loss, sizeof(float)) != cudaSuccess || cudaMalloc(&p->ticket, sizeof(unsigned)) != cudaSuccess) {
+    delete p;
+    return fail(ctx, ATLASGPU_ENOMEM, "mlp_create");
+  }
+  CK(cudaMemset(p->ticket, 0, sizeof(unsigned)));
   // Glorot-uniform weights, zero biases
   std::vector<float> h(p->nparam, 0.f);
   uint64_t s = seed;
@@ -269,9 +402,10 @@ int atlasgpu_mlp_destroy(atlasgpu_ctx* ctx, atlasgpu_mlp* p) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
   }
-  float* bufs[] = {p->w, p->g, p->m, p->v, p->x, p->t, p->h1, p->h2, p->y, p->d1, p->d2, p->dy, p->lpart};
+  float* bufs[] = {p->w, p->g, p->m, p->v, p->x, p->t, p->h1, p->h2, p->y, p->d1, p->d2, p->dy, p->lpart, p->loss};
   for (float* b : bufs)
     if (b) cudaFree(b);
+  if (p->ticket) cudaFree(p->ticket);
   delete p;
   return 0;
 }
@@ -317,11 +451,10 @@ int atlasgpu_mlp_loss_grad(atlasgpu_ctx* ctx, atlasgpu_mlp* p, const float* x, c
   if ((r = ensure_cap(ctx, p, n))) return r;
   CK(cudaMemcpyAsync(p->x, x, sizeof(float) * (size_t)n * p->nin, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(p->t, t, sizeof(float) * (size_t)n * p->nout, cudaMemcpyHostToDevice, ctx->stream));
-  if ((r = forward(ctx, p, n))) return r;
-  if ((r = backward(ctx, p, n, p->lpart + 64))) return r;
+  if ((r = forward(ctx, p, n, p->loss)) || (r = backward(ctx, p, n))) return r;
   if (grad) CK(cudaMemcpyAsync(grad, p->g, sizeof(float) * p->nparam, cudaMemcpyDeviceToHost, ctx->stream));
   float l = 0.f;
-  CK(cudaMemcpyAsync(&l, p->lpart + 64, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(&l, p->loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (loss) *loss = l;
   return 0;
@@ -359,7 +492,7 @@ int atlasgpu_mlp_train(atlasgpu_ctx* ctx, atlasgpu_mlp* p, const float* x, const
       k_gather<<<grid_for(ctx, (int64_t)batch * p->nin, 256, 4), 256, 0, st>>>(batch, p->nin, didx + b0, dx, p->x);
       k_gather<<<grid_for(ctx, (int64_t)batch * p->nout, 256, 4), 256, 0, st>>>(batch, p->nout, didx + b0, dt, p->t);
       CKL(ctx);
-      if ((r = forward(ctx, p, batch)) || (r = backward(ctx, p, batch, dloss + ep))) break;
+      if ((r = forward(ctx, p, batch, dloss + ep)) || (r = backward(ctx, p, batch))) break;
       p->step += 1;
       const float c1 = 1.f - powf(b1, (float)p->step), c2 = 1.f - powf(b2, (float)p->step);
       k_adam<<<grid_for(ctx, p->nparam, 256, 4), 256, 0, st>>>(p->nparam, p->w, p->g, p->m, p->v, lr, b1, b2, eps,

@@ -47,3 +47,29 @@ def test_training_lowers_loss(gpu_ctx):
     assert np.all(np.isfinite(hist))
     assert l1 < 0.1 * l0, (l0, l1)
     m.close()
+
+
+@pytest.mark.parametrize("shape", [(4, 256, 256, 216), (3, 17, 33, 1)])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 64, 129, 2369])
+def test_tile_edges(gpu_ctx, shape, n):
+    """Sample counts and layer widths around the tile edges, up to where 64x64
+    tiles fill the chip.  Sums of at most 2,369 FP32 terms in chunks: relative
+    error of a few 1e-6 in norm through three layers, 2e-5 allowed; and the
+    same bits when run again."""
+    from atlas12_b200.warmstart import MLP
+    import mlp_ref
+    m = MLP(gpu_ctx, shape=shape, seed=3)
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, (n, shape[0])).astype(np.float32)
+    t = rng.normal(size=(n, shape[3])).astype(np.float32)
+    p = m.params().astype(np.float64)
+    lr, gr = mlp_ref.loss_grad(p, x.astype(np.float64), t.astype(np.float64), shape)
+    yr = mlp_ref.forward(p, x.astype(np.float64), shape)[2]
+    loss, g = m.loss_grad(x, t)
+    y = m.forward(x)
+    assert abs(loss - lr) <= 2e-5 * lr
+    assert np.linalg.norm(y - yr) <= 2e-5 * np.linalg.norm(yr)
+    assert np.linalg.norm(g - gr) <= 2e-5 * np.linalg.norm(gr)
+    loss2, g2 = m.loss_grad(x, t)
+    assert loss2 == loss and np.array_equal(g, g2)
+    m.close()
