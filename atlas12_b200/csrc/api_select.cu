@@ -43,8 +43,6 @@ double ratiolg_lines() { return log(1.0 + 1.0 / 2000000.0); }
 
 size_t rec_bytes(int kind) { return kind == kSelTio ? 32 : kind == kSelH2o ? 8 : 16; }
 
-size_t sel_smem(int kind) { return std::max<size_t>(rec_bytes(kind), 16) * (kSelTile + kSelThreads); }
-
 // pass A (tile maxima of UB), the scan of NU at each tile's entry, pass B
 template <int K>
 int launch_select(atlasgpu_ctx* ctx, const SelArgs& a, int ntiles) {
@@ -55,9 +53,7 @@ int launch_select(atlasgpu_ctx* ctx, const SelArgs& a, int ntiles) {
   CKL(ctx);
   k_sel_scan<true><<<1, 1024, 0, ctx->stream>>>(d_tub, ntiles, a.nu0, const_cast<long long*>(a.tile_nu));
   CKL(ctx);
-  const size_t smem = sel_smem(K);
-  CK(cudaFuncSetAttribute(k_selectlines<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_selectlines<K><<<ntiles, kSelThreads, smem, ctx->stream>>>(a);
+  k_selectlines<K><<<ntiles, kSelThreads, 0, ctx->stream>>>(a);
   CKL(ctx);
   return 0;
 }
@@ -140,16 +136,14 @@ int select_chunk(atlasgpu_ctx* ctx, int kind, const void* d_recs, int64_t n, atl
   int *d_tub, *d_cnt;
   long long *d_nu, *d_off;
   int4* d_scr;
-  unsigned long long* d_err;
-  unsigned* d_nfix;
+  SelCtl* d_ctl;
   SelFix* d_fix;
   if ((r = bufT(ctx, "sel_tub", ntiles, &d_tub)) || (r = bufT(ctx, "sel_tcnt", ntiles, &d_cnt)) ||
       (r = bufT(ctx, "sel_tnu", ntiles + 1, &d_nu)) || (r = bufT(ctx, "sel_toff", ntiles + 1, &d_off)) ||
-      (r = bufT(ctx, "sel_scratch", (size_t)ntiles * kSelTile, &d_scr)) || (r = bufT(ctx, "sel_err", 1, &d_err)) ||
-      (r = bufT(ctx, "sel_nfix", 1, &d_nfix)) || (r = bufT(ctx, "sel_fix", kFixCap, &d_fix)))
+      (r = bufT(ctx, "sel_scratch", (size_t)ntiles * kSelTile, &d_scr)) || (r = bufT(ctx, "sel_ctl", 1, &d_ctl)) ||
+      (r = bufT(ctx, "sel_fix", kFixCap, &d_fix)))
     return r;
-  CK(cudaMemsetAsync(d_err, 0xff, sizeof(unsigned long long), ctx->stream));
-  CK(cudaMemsetAsync(d_nfix, 0, sizeof(unsigned), ctx->stream));
+  CK(cudaMemsetAsync(d_ctl, 0, sizeof(SelCtl), ctx->stream));
 
   SelArgs a{};
   a.recs = d_recs;
@@ -159,16 +153,23 @@ int select_chunk(atlasgpu_ctx* ctx, int kind, const void* d_recs, int64_t n, atl
   a.freq0 = st->freq;
   int *d_iwt, *d_mol;
   double *d_freq, *d_xmax, *d_tablog;
+  float *d_xlog, *d_lfreq;
   short* d_igr;
   if ((r = bufT(ctx, "sel_iwt", nwave + 1, &d_iwt)) || (r = bufT(ctx, "sel_freq", nwave, &d_freq)) ||
       (r = bufT(ctx, "sel_igr", nwave, &d_igr)) || (r = bufT(ctx, "sel_mol", kSelMolN + 9, &d_mol)) ||
-      (r = bufT(ctx, "sel_xmax", (size_t)(nwave + 1) * ctx->sel_nspec, &d_xmax)) || (r = ensure_tablog(ctx, &d_tablog)))
+      (r = bufT(ctx, "sel_xmax", (size_t)(nwave + 1) * ctx->sel_nspec, &d_xmax)) ||
+      (r = bufT(ctx, "sel_xlog", (size_t)(nwave + 1) * ctx->sel_nspec, &d_xlog)) ||
+      (r = bufT(ctx, "sel_lfreq", nwave, &d_lfreq)) || (r = ensure_tablog(ctx, &d_tablog)))
     return r;
   a.iwt = d_iwt;
   a.nwave = nwave;
   a.freqtab = d_freq;
   a.igrtab = d_igr;
   a.xmax = d_xmax;
+  a.xlog = d_xlog;
+  a.lfreq = d_lfreq;
+  a.lfreq0 = (float)(log2(kCenPrefac) - log2(st->freq));
+  a.hlog = (float)(ctx->sel_hckt_last / log(2.0));
   a.nspec = ctx->sel_nspec;
   a.tablog = d_tablog;
   a.hckt_last = ctx->sel_hckt_last;
@@ -184,33 +185,27 @@ int select_chunk(atlasgpu_ctx* ctx, int kind, const void* d_recs, int64_t n, atl
   a.tile_count = d_cnt;
   a.scratch = d_scr;
   a.fix = d_fix;
-  a.nfix = d_nfix;
   a.fixcap = kFixCap;
-  a.err = d_err;
+  a.ctl = d_ctl;
   {
     Timer tk(ctx, "k_selectlines");
     if ((r = dispatch(ctx, kind, a, ntiles))) return r;
     k_sel_scan<false><<<1, 1024, 0, ctx->stream>>>(d_cnt, ntiles, 0, d_off);
     CKL(ctx);
-    k_sel_move<<<std::min(ntiles, ctx->nsm * 8), 256, 0, ctx->stream>>>(d_scr, d_cnt, d_off, ntiles, d_out, cap);
+    k_sel_move<<<std::min(ntiles, ctx->nsm * 8), 256, 0, ctx->stream>>>(d_scr, d_cnt, d_off, d_nu, ntiles, d_out, cap,
+                                                                        d_fix, kFixCap, d_ctl);
     CKL(ctx);
   }
-  k_sel_fixpos<<<(kFixCap + 255) / 256, 256, 0, ctx->stream>>>(d_fix, d_nfix, kFixCap, d_off);
-  CKL(ctx);
 
-  long long last[2];
-  unsigned long long err;
-  unsigned nfix;
-  CK(cudaMemcpyAsync(&last[0], d_nu + ntiles, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(&last[1], d_off + ntiles, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(&err, d_err, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(&nfix, d_nfix, sizeof nfix, cudaMemcpyDeviceToHost, ctx->stream));
+  SelCtl ctl;
+  CK(cudaMemcpyAsync(&ctl, d_ctl, sizeof ctl, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (err != ~0ull)
-    return fail(ctx, ATLASGPU_EINVAL, "selectlines: record %lld: %s", (long long)(err >> 8) + (long long)rec0,
-                err_text((int)(err & 0xff)));
-  const int nu = (int)last[0];
-  int64_t total = (int64_t)last[1];
+  if (ctl.err)
+    return fail(ctx, ATLASGPU_EINVAL, "selectlines: record %lld: %s", (long long)(~ctl.err >> 8) + (long long)rec0,
+                err_text((int)(~ctl.err & 0xff)));
+  const int nu = (int)ctl.nu;
+  const unsigned nfix = ctl.nfix;
+  int64_t total = (int64_t)ctl.total;
   if (total > cap)
     return fail(ctx, ATLASGPU_EINVAL, "selectlines: LINEDATA overflow (record set beyond cap %lld)", (long long)cap);
   if (nfix > kFixCap) return fail(ctx, ATLASGPU_EINVAL, "selectlines: %u records near a rounding boundary", nfix);
@@ -314,25 +309,30 @@ int atlasgpu_atlas_select_tables(atlasgpu_ctx* ctx, int nrhox, int kw, const dou
   cudaSetDevice(ctx->device);
   ctx->sel_ready = false;
   double *d_xn, *d_tc, *d_xmax, *d_freq, *d_tl;
+  float *d_xlog, *d_lfreq;
   int *d_iwt, *d_mol;
   short* d_igr;
   int r;
   if ((r = bufT(ctx, "sel_xnfdop", (size_t)nspec * kw, &d_xn)) ||
       (r = bufT(ctx, "sel_tabcont", (size_t)(nwave + 1) * kw, &d_tc)) ||
       (r = bufT(ctx, "sel_xmax", (size_t)(nwave + 1) * nspec, &d_xmax)) || (r = bufT(ctx, "sel_iwt", nwave + 1, &d_iwt)) ||
+      (r = bufT(ctx, "sel_xlog", (size_t)(nwave + 1) * nspec, &d_xlog)) ||
+      (r = bufT(ctx, "sel_lfreq", nwave, &d_lfreq)) ||
       (r = bufT(ctx, "sel_freq", nwave, &d_freq)) || (r = bufT(ctx, "sel_igr", nwave, &d_igr)) ||
       (r = bufT(ctx, "sel_mol", kSelMolN + 9, &d_mol)) || (r = ensure_tablog(ctx, &d_tl)))
     return r;
   CK(cudaMemcpyAsync(d_xn, xnfdop, (size_t)nspec * kw * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(d_tc, tabcont, (size_t)(nwave + 1) * kw * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   k_sel_xnfdopmax<<<grid_for(ctx, (int64_t)(nwave + 1) * nspec, 256, 8), 256, 0, ctx->stream>>>(nrhox, kw, d_xn, nspec,
-                                                                                                 d_tc, nwave, d_xmax);
+                                                                                                 d_tc, nwave, d_xmax, d_xlog);
   CKL(ctx);
   // FREQ and H2O's IGR after the advance past bin k (:19614, :19668-19673)
   std::vector<double> freq(nwave);
   std::vector<int16_t> igr(nwave);
+  std::vector<float> lfreq(nwave);
   for (int k = 0; k < nwave; ++k) {
     freq[k] = kClightNms / wavetab[k];
+    lfreq[k] = (float)(log2(kCenPrefac) - log2(freq[k]));
     volatile double f2 = freq[k] * freq[k];
     volatile double g = 2.474e-22 * f2;
     volatile double gammar = g * (double)0.001f;  // 0.001 is a default REAL literal there
@@ -345,6 +345,7 @@ int atlasgpu_atlas_select_tables(atlasgpu_ctx* ctx, int nrhox, int kw, const dou
   std::copy(kH2oIsocorr, kH2oIsocorr + 4, mol.begin() + kSelMolN + 5);
   CK(cudaMemcpyAsync(d_iwt, iwavetab, (nwave + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(d_freq, freq.data(), nwave * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(d_lfreq, lfreq.data(), nwave * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(d_igr, igr.data(), nwave * sizeof(short), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(d_mol, mol.data(), mol.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));

@@ -5,9 +5,9 @@
 //
 //  * the NU advance (DO WHILE (IWL >= IWAVETAB(NU)) ...) is a running
 //    maximum: after a record, NU = max(NU at entry, UB(max IWL so far)) with
-//    UB(x) = the first bin whose IWAVETAB exceeds x.  k_sel_tile_ub takes
-//    each tile's maximum UB and k_sel_scan the exclusive maximum over tiles,
-//    so a tile knows NU at its entry;
+//    UB(x) = the first bin whose IWAVETAB exceeds x, which grows with x:
+//    k_sel_tile_ub takes UB of each tile's largest IWL and k_sel_scan the
+//    exclusive maximum over tiles, so a tile knows NU at its entry;
 //  * k_selectlines filters each tile at its records' NU and writes the
 //    selected LINEDATA compacted at the tile's own place in a scratch array,
 //    with the tile's count; k_sel_scan sums the counts and k_sel_move puts
@@ -21,8 +21,17 @@
 // host, which decides with the C library: the TiO IWL before the passes (an
 // override table), the Boltzmann test and the IELO / IGR fields after them
 // (a fix list with output positions).
+//
+// Most records are far below the cut.  The exact tests need up to three FP64
+// table gathers, a division and an exponential each, and those bounded the
+// filter (107 us for 8M LINEREC records, whose one reading takes 20), so
+// k_selectlines first forms log2 of CENRATIO * exp(-E/kT) in FP32 from the
+// record's fields, drops what lies kSelQuick below the cut (the estimate is
+// within 0.03, see sel_quick_reject) and takes the rest, gathered into full
+// warps, through the exact tests.  8M records, 15 % selected: filter 107 ->
+// 73 us, tile maxima 38 -> 25 us (one binary search a tile, eight loads in
+// flight, instead of a search a record), the call 246 -> 165 us.
 #pragma once
-#include <type_traits>
 
 #include "common.cuh"
 
@@ -31,9 +40,9 @@ namespace atlasgpu {
 constexpr int kSelThreads = 256;
 constexpr int kSelItems = 8;
 constexpr int kSelTile = kSelThreads * kSelItems;  // records per tile
-constexpr int kSelGroup = 2;                       // records whose table loads are issued together
 constexpr int kSelMaxWave = 1024;                  // IWAVETAB entries held in shared memory
 constexpr double kSelKeepBand = 1.0e-12;  // |CENRATIO*exp(...) - 1| left to the host
+constexpr float kSelQuick = 0.05f;        // log2 below the cut from which the FP32 estimate decides
 constexpr double kSelIntBand = 1.0e-6;    // distance of an INT() argument from an integer left to the host
 
 enum SelKind { kSelLowPred = 1, kSelLowObs = 2, kSelHi = 3, kSelDiatomic = 4, kSelTio = 5, kSelH2o = 6, kSelH3plus = 7 };
@@ -60,6 +69,13 @@ struct alignas(8) SelH2o {
   short ielo, igflog;
 };
 
+// what one chunk's passes report: errors as the complement, so that zero is none
+struct SelCtl {
+  unsigned long long err;  // max over ~(record << 8 | code)
+  long long nu, total;     // NU at the end, records selected
+  unsigned int nfix, pad;
+};
+
 struct SelArgs {
   const void* recs;
   long long n;
@@ -70,6 +86,10 @@ struct SelArgs {
   const double* freqtab;  // [nwave]: CLIGHT_NMS / WAVETAB(k) at k-1 (FREQ after advancing past bin k)
   const short* igrtab;    // [nwave]: H2O's IGR after advancing past bin k
   const double* xmax;     // XNFDOPMAX [nwave+1][nspec]
+  const float* xlog;      // log2 of it
+  const float* lfreq;     // [nwave]: log2(CEN_PREFAC / FREQ) after advancing past bin k; at entry
+  float lfreq0;
+  float hlog;             // HCKT_LAST / ln 2
   int nspec;
   const double* tablog;   // TABLOG for every INTEGER(2), index I + 32768
   double hckt_last, cen_prefac, ratiolg;
@@ -83,9 +103,8 @@ struct SelArgs {
   int* tile_count;      // [ntiles] selected records per tile
   int4* scratch;        // [ntiles * kSelTile] each tile's LINEDATA, compacted at the tile's start
   SelFix* fix;
-  unsigned int* nfix;
   unsigned int fixcap;
-  unsigned long long* err;  // min over (record << 8 | code)
+  SelCtl* ctl;
 };
 
 __device__ __forceinline__ int sel_fint(double x) {
@@ -125,7 +144,8 @@ __global__ void __launch_bounds__(256) k_sel_tio_border(const SelMol2* __restric
 
 // XNFDOPMAX(NELION, NU) = max_J XNFDOP(J, NELION) / TABCONT(J, NU) (:19248-19256)
 __global__ void __launch_bounds__(256) k_sel_xnfdopmax(int nrhox, int kw, const double* __restrict__ xnfdop, int nspec,
-                                                       const double* __restrict__ tabcont, int nwave, double* xmax) {
+                                                       const double* __restrict__ tabcont, int nwave, double* xmax,
+                                                       float* __restrict__ xlog) {
   const long long total = (long long)(nwave + 1) * nspec;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total; k += (long long)gridDim.x * blockDim.x) {
     const int nu = (int)(k / nspec), e = (int)(k % nspec);
@@ -135,6 +155,7 @@ __global__ void __launch_bounds__(256) k_sel_xnfdopmax(int nrhox, int kw, const 
       if (r > m) m = r;
     }
     xmax[k] = m;
+    xlog[k] = (float)log2(m);
   }
 }
 
@@ -150,11 +171,6 @@ template <>
 struct SelRecType<kSelH2o> {
   using T = SelH2o;
 };
-
-// padded slot of the k-th record of a tile: each thread's kSelItems
-// consecutive records are followed by one spare, so the blocked reads of a
-// warp fall in different banks
-__device__ __forceinline__ int sel_slot(int k) { return k + k / kSelItems; }
 
 // UB(x): the first 1-based bin k with IWAVETAB(k) > x, over the shared copy
 __device__ __forceinline__ int sel_ub(const int* s_iwt, int nwave, int x, int hint) {
@@ -176,8 +192,8 @@ __device__ __forceinline__ int4 sel_pack(int iwl, short ielion, short ielo, shor
   return make_int4(iwl, w(ielion, ielo), w(igflog, igr), w(igs, igw));
 }
 
-__device__ __forceinline__ void sel_error(unsigned long long* err, long long rec, int code) {
-  atomicMin(err, ((unsigned long long)rec << 8) | (unsigned)code);
+__device__ __forceinline__ void sel_error(SelCtl* ctl, long long rec, int code) {
+  atomicMax(&ctl->err, ~(((unsigned long long)rec << 8) | (unsigned)code));
 }
 
 // Per-record pass 1: the IWL taking part in the NU advance (or none).
@@ -199,7 +215,7 @@ __device__ __forceinline__ bool sel_advance_iwl(const typename SelRecType<KIND>:
       if (lo < a.novr && a.ovr_idx[lo] == gi)
         *iwl = a.ovr_iwl[lo];
       else
-        sel_error(a.err, gi, kSelErrOverride);
+        sel_error(a.ctl, gi, kSelErrOverride);
     }
     return true;
   } else if constexpr (KIND == kSelH2o) {
@@ -225,31 +241,33 @@ struct SelOps {
   short igflog;  // IGFLOG after the database's correction
 };
 
+// A record's XNFDOPMAX row, IGFLOG after the database's correction and (LINEREC
+// kinds) IELO; bad: kSelErrMolcode for an unknown diatomic MOLCODE.
 template <int KIND>
-__device__ __forceinline__ void sel_gather(const typename SelRecType<KIND>::T& r, const SelArgs& a, int nu,
-                                           const int* s_molcor, SelOps& o) {
-  o.freq = nu > a.nu0 ? a.freqtab[nu - 2] : a.freq0;
-  o.tel = 0.0;
-  o.bad = 0;
+__device__ __forceinline__ void sel_species(const typename SelRecType<KIND>::T& r, const SelArgs& a,
+                                            const int* s_molcor, int& nelion, short& igflog, short& ielo, int& bad) {
+  bad = 0;
+  ielo = 0;
   if constexpr (KIND == kSelTio) {
     const int iso = min(max(r.iso - 45, 1), 5);  // records outside 46-50 are dropped before any test
     const int kgflog = sel_fint(round(__dmul_rn((double)r.gflog, 1000.0))) + 16384;
     const int g = kgflog + a.tio_isocorr[iso - 1];
-    o.igflog = sel_i16(g > 1 ? g : 1);
-    o.nelion = 895;
+    igflog = sel_i16(g > 1 ? g : 1);
+    nelion = 895;
   } else if constexpr (KIND == kSelH2o) {
     const int iso = (r.ielo > 0 && r.igflog > 0) ? 1 : r.ielo > 0 ? 2 : r.igflog > 0 ? 3 : 4;
     const int g = abs((int)r.igflog) + a.h2o_isocorr[iso - 1];
-    o.igflog = sel_i16(g > 1 ? g : 1);
-    o.nelion = 940;
+    igflog = sel_i16(g > 1 ? g : 1);
+    nelion = 940;
   } else {
-    const short ielion = (short)(r.y & 0xffff), ielo = (short)((unsigned)r.y >> 16);
-    short igflog = (short)(r.z & 0xffff);
+    const short ielion = (short)(r.y & 0xffff);
+    ielo = (short)((unsigned)r.y >> 16);
+    igflog = (short)(r.z & 0xffff);
     if constexpr (KIND == kSelDiatomic) {
       const int c = (int)ielion - kSelMolLo;
       const int cor = (c >= 0 && c < kSelMolN) ? s_molcor[c] : kSelMolUnknown;
       if (cor == kSelMolUnknown) {
-        o.bad = kSelErrMolcode;
+        bad = kSelErrMolcode;
       } else {
         const int g = (int)igflog + cor;
         igflog = sel_i16(g > 1 ? g : 1);
@@ -258,13 +276,51 @@ __device__ __forceinline__ void sel_gather(const typename SelRecType<KIND>::T& r
       const int g = (int)igflog - 1272;
       igflog = sel_i16(g > 1 ? g : 1);
     }
-    o.igflog = igflog;
-    o.nelion = KIND == kSelH3plus ? 895 : abs((int)ielion / 10);
-    o.tel = a.tablog[ielo + 32768];
+    nelion = KIND == kSelH3plus ? 895 : abs((int)ielion / 10);
   }
+}
+
+template <int KIND>
+__device__ __forceinline__ void sel_gather(const typename SelRecType<KIND>::T& r, const SelArgs& a, int nu,
+                                           const int* s_molcor, SelOps& o) {
+  short ielo;
+  sel_species<KIND>(r, a, s_molcor, o.nelion, o.igflog, ielo, o.bad);
+  o.freq = nu > a.nu0 ? a.freqtab[nu - 2] : a.freq0;
+  o.tel = (KIND == kSelTio || KIND == kSelH2o) ? 0.0 : a.tablog[ielo + 32768];
   const bool row = nu >= 1 && o.nelion >= 1 && o.nelion <= a.nspec;
   o.xm = row ? a.xmax[(size_t)(nu - 1) * a.nspec + (o.nelion - 1)] : 0.0;
   o.tgf = a.tablog[o.igflog + 32768];
+}
+
+// True where sel_decide returns 0 without an error: log2 of CENRATIO * exp(-E/kT)
+// estimated in FP32 is kSelQuick below 0.  With l = log2(CEN_PREFAC / FREQ) +
+// log2 XNFDOPMAX + log2 TABLOG(IGFLOG), the terms below 2^10: three roundings of
+// 2^-14; E of LINEREC records as 2^x, |x| < 164, to 2e-5 relative, and E/kT counts
+// only up to about l, so it is off by 0.02 at most.  Terms near the overflow of
+// the exact product (whose infinity passes its tests) are left to those; what is
+// not a number, not in the tables or an error compares false and stays.
+template <int KIND>
+__device__ __forceinline__ bool sel_quick_reject(const typename SelRecType<KIND>::T& r, const SelArgs& a, int nu,
+                                                 const int* s_molcor) {
+  if constexpr (KIND == kSelTio)
+    if (r.code != 822 || r.iso - 45 < 1 || r.iso - 45 > 5 || (double)r.wl <= 0.0) return true;
+  constexpr float kDex = 3.3219281e-3f;  // log2 of the tables' step, 10**0.001
+  int nelion, bad;
+  short igflog, ielo;
+  sel_species<KIND>(r, a, s_molcor, nelion, igflog, ielo, bad);
+  if (bad || nu < 1 || nelion < 1 || nelion > a.nspec) return false;
+  const float x = a.xlog[(size_t)(nu - 1) * a.nspec + (nelion - 1)] + (float)((int)igflog - 16384) * kDex;
+  const float l = (nu > a.nu0 ? a.lfreq[nu - 2] : a.lfreq0) + x;
+  float e;
+  if constexpr (KIND == kSelTio) {
+    const float a1 = fabsf(r.e1), a2 = fabsf(r.e2);
+    e = a2 < a1 ? a2 : a1;
+  } else if constexpr (KIND == kSelH2o) {
+    e = (float)abs((int)r.ielo);
+  } else {
+    e = exp2f((float)((int)ielo - 16384) * kDex);
+  }
+  return x < 900.0f && l < 900.0f && (l < -kSelQuick || l - e * a.hlog < -kSelQuick);
 }
 
 // Per-record pass 2: the filter at bin nu with the gathered operands.
@@ -286,7 +342,7 @@ __device__ __forceinline__ int sel_decide(const typename SelRecType<KIND>::T& r,
     const double w = (double)r.wl;
     sel_advance_iwl<KIND>(r, a, gi, &iwl);
     if (o.nelion > a.nspec) {
-      sel_error(a.err, gi, kSelErrNelion);
+      sel_error(a.ctl, gi, kSelErrNelion);
       return 0;
     }
     if (o.xm == 0.0) return 0;
@@ -321,7 +377,7 @@ __device__ __forceinline__ int sel_decide(const typename SelRecType<KIND>::T& r,
     e = (double)abs((int)r.ielo);
     igr = nu > a.nu0 ? a.igrtab[nu - 2] : (short)a.igr0;
     if (o.nelion > a.nspec) {
-      sel_error(a.err, gi, kSelErrNelion);
+      sel_error(a.ctl, gi, kSelErrNelion);
       return 0;
     }
     if (o.xm == 0.0) return 0;
@@ -353,11 +409,11 @@ __device__ __forceinline__ int sel_decide(const typename SelRecType<KIND>::T& r,
       igw = 9384;
     }
     if (o.bad) {
-      sel_error(a.err, gi, o.bad);
+      sel_error(a.ctl, gi, o.bad);
       return 0;
     }
     if (o.nelion < 1 || o.nelion > a.nspec) {
-      if (KIND != kSelLowPred) sel_error(a.err, gi, kSelErrNelion);
+      if (KIND != kSelLowPred) sel_error(a.ctl, gi, kSelErrNelion);
       return 0;
     }
     if (KIND == kSelLowPred || KIND == kSelLowObs) {
@@ -379,41 +435,6 @@ __device__ __forceinline__ int sel_decide(const typename SelRecType<KIND>::T& r,
   }
 }
 
-template <int T>
-__device__ __forceinline__ int block_scan_excl(int v, int* s_warp, int* total, bool use_max) {
-  // exclusive scan over the block (sum, or max with identity 0); T threads
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x = use_max ? (y > x ? y : x) : x + y;
-  }
-  if (lane == 31) s_warp[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    int w = lane < T / 32 ? s_warp[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w = use_max ? (y > w ? y : w) : w + y;
-    }
-    if (lane < T / 32) s_warp[lane] = w;  // inclusive over warps
-  }
-  __syncthreads();
-  const int before = wid > 0 ? s_warp[wid - 1] : 0;
-  const int xin = __shfl_up_sync(0xffffffffu, x, 1);
-  int excl = lane > 0 ? (use_max ? (before > xin ? before : xin) : before + xin) : before;
-  *total = s_warp[T / 32 - 1];
-  __syncthreads();
-  return excl;
-}
-
-// shared-memory slot of one record: at least 16 bytes, so a selected
-// record's LINEDATA can be staged where the record was
-template <class R>
-using SelSlotT = typename std::conditional<(sizeof(R) < sizeof(int4)), int4, R>::type;
-
 template <int KIND>
 __device__ __forceinline__ void sel_push_fixes(const SelArgs& a, const typename SelRecType<KIND>::T& r, long long gi,
                                                long long pos, int nu, unsigned keep, unsigned fx,
@@ -431,7 +452,7 @@ __device__ __forceinline__ void sel_push_fixes(const SelArgs& a, const typename 
     f.arg = 0;
     f.a = c;
     f.b = y;
-    const unsigned s = atomicAdd(a.nfix, 1u);
+    const unsigned s = atomicAdd(&a.ctl->nfix, 1u);
     if (s < a.fixcap) a.fix[s] = f;
   }
   if constexpr (KIND == kSelTio || KIND == kSelH2o) {
@@ -446,7 +467,7 @@ __device__ __forceinline__ void sel_push_fixes(const SelArgs& a, const typename 
         f.a = (double)abs((int)r.ielo);
       }
       f.b = 0.0;
-      const unsigned s = atomicAdd(a.nfix, 1u);
+      const unsigned s = atomicAdd(&a.ctl->nfix, 1u);
       if (s < a.fixcap) a.fix[s] = f;
     }
     if constexpr (KIND == kSelTio) {
@@ -455,44 +476,55 @@ __device__ __forceinline__ void sel_push_fixes(const SelArgs& a, const typename 
         f.arg = r.gr;
         f.a = (double)r.wl;
         f.b = 0.0;
-        const unsigned s = atomicAdd(a.nfix, 1u);
+        const unsigned s = atomicAdd(&a.ctl->nfix, 1u);
         if (s < a.fixcap) a.fix[s] = f;
       }
     }
   }
 }
 
-// Pass A: the largest UB of each tile's records (the NU a tile leaves
-// behind, before the carry from earlier tiles).  Record k of the tile is
-// read by thread k % 256: the maximum does not depend on the order.
+// Pass A: UB of each tile's largest IWL (the NU a tile leaves behind, before
+// the carry from earlier tiles).  Record k of the tile is read by thread
+// k % 256: the maximum does not depend on the order.  Bound by the reading.
 template <int KIND>
 __global__ void __launch_bounds__(kSelThreads) k_sel_tile_ub(SelArgs a, int* __restrict__ tile_ub) {
   using R = typename SelRecType<KIND>::T;
-  __shared__ int s_iwt[kSelMaxWave];
-  __shared__ int s_warp[kSelThreads / 32];
+  __shared__ int s_warp[kSelThreads / 32], s_any[kSelThreads / 32];
   const int t = threadIdx.x, tile = blockIdx.x;
-  for (int k = t; k <= a.nwave; k += kSelThreads) s_iwt[k] = a.iwt[k];
-  __syncthreads();
   const long long base = (long long)tile * kSelTile;
   const int cnt = (int)min((long long)kSelTile, a.n - base);
   const R* g = reinterpret_cast<const R*>(a.recs) + base;
-  int m = 0;
-#pragma unroll 4
-  for (int k = t; k < cnt; k += kSelThreads) {
+  int m = -2147483647 - 1, any = 0;
+  auto take = [&](const R& r, int k) {
     int iwl;
-    if (sel_advance_iwl<KIND>(g[k], a, base + k, &iwl)) {
-      const int u = min(sel_ub(s_iwt, a.nwave, iwl, 0), a.nwave + 1);
-      m = u > m ? u : m;
+    if (sel_advance_iwl<KIND>(r, a, base + k, &iwl)) {
+      m = max(m, iwl);
+      any = 1;
     }
-  }
+  };
+  if (cnt == kSelTile) {
+    R v[kSelItems];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((t & 31) == 0) s_warp[t >> 5] = m;
+    for (int i = 0; i < kSelItems; ++i) v[i] = g[i * kSelThreads + t];
+#pragma unroll
+    for (int i = 0; i < kSelItems; ++i) take(v[i], i * kSelThreads + t);
+  } else {
+    for (int k = t; k < cnt; k += kSelThreads) take(g[k], k);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  any = __any_sync(0xffffffffu, any);
+  if ((t & 31) == 0) {
+    s_warp[t >> 5] = m;
+    s_any[t >> 5] = any;
+  }
   __syncthreads();
   if (t == 0) {
-    int r = 0;
-    for (int w = 0; w < kSelThreads / 32; ++w) r = max(r, s_warp[w]);
-    tile_ub[tile] = r;
+    int x = s_warp[0], some = s_any[0];
+    for (int w = 1; w < kSelThreads / 32; ++w) {
+      x = max(x, s_warp[w]);
+      some |= s_any[w];
+    }
+    tile_ub[tile] = some ? min(sel_ub(a.iwt, a.nwave, x, 0), a.nwave + 1) : 0;
   }
 }
 
@@ -544,119 +576,154 @@ __global__ void __launch_bounds__(1024) k_sel_scan(const int* __restrict__ in, i
   if (t == 0) out[n] = s_carry;
 }
 
-// Pass B: the filter.  One tile of kSelTile records per CTA, staged
-// coalesced in shared memory; thread t takes records 8t..8t+7.  NU at the
-// tile's entry comes from the scan of pass A.  The selected records'
-// LINEDATA goes to the tile's place in the scratch array, compacted in file
-// order, with the host's cases listed at their scratch positions.
+// Pass B: the filter.  One tile of kSelTile records per CTA; a warp takes 256
+// records in file order, 32 neighbours at a time, through the NU advance and
+// the FP32 estimate.  NU at the tile's entry comes from the scan of pass A.  The
+// records left, in file order, are then taken one a thread through the exact
+// tests, and the selected ones' LINEDATA goes to the tile's place in the scratch
+// array, compacted in file order, with the host's cases listed at their scratch
+// positions.  Latency bound: the records stay in registers (a tile staged in
+// shared memory, eight neighbours a thread, held it to four CTAs an SM and took
+// 94 us where this takes 73).
 template <int KIND>
-__global__ void __launch_bounds__(kSelThreads, 4) k_selectlines(SelArgs a) {
+__global__ void __launch_bounds__(kSelThreads, KIND == kSelTio ? 4 : 5)
+    k_selectlines(const __grid_constant__ SelArgs a) {
   using R = typename SelRecType<KIND>::T;
-  using Slot = SelSlotT<R>;
-  extern __shared__ __align__(16) unsigned char sel_smem[];
-  Slot* s_slot = reinterpret_cast<Slot*>(sel_smem);  // padded tile
+  constexpr bool kKeep = sizeof(R) <= 16;  // (TiO's are read again, from L1)
+  constexpr int kWarps = kSelThreads / 32;
+  constexpr unsigned FULL = 0xffffffffu;
   __shared__ int s_iwt[kSelMaxWave];
+  __shared__ int s_left[kSelTile];  // record | NU << 11, in file order
   __shared__ int s_molcor[KIND == kSelDiatomic ? kSelMolN : 1];
-  __shared__ int s_warp[kSelThreads / 32];
-  auto rec = [&](int k) -> const R& { return *reinterpret_cast<const R*>(&s_slot[sel_slot(k)]); };
+  __shared__ int s_nu[kWarps], s_cnt[2][kWarps], s_n[kWarps];
+  static_assert(kSelTile <= 2048, "a record's index takes 11 bits");
 
-  const int t = threadIdx.x, tile = blockIdx.x;
-  for (int k = t; k <= a.nwave; k += kSelThreads) s_iwt[k] = a.iwt[k];
-  if constexpr (KIND == kSelDiatomic)
-    for (int k = t; k < kSelMolN; k += kSelThreads) s_molcor[k] = a.molcor[k];
+  const int t = threadIdx.x, tile = blockIdx.x, lane = t & 31, wid = t >> 5;
   const long long base = (long long)tile * kSelTile;
   const int cnt = (int)min((long long)kSelTile, a.n - base);
   const R* g = reinterpret_cast<const R*>(a.recs) + base;
-  for (int k = t; k < cnt; k += kSelThreads) *reinterpret_cast<R*>(&s_slot[sel_slot(k)]) = g[k];
-  const int tile_nu = (int)a.tile_nu[tile];
+  const int k0 = wid * 32 * kSelItems + lane;  // record of row i: k0 + 32 i
+  R v[kKeep ? kSelItems : 1];
+  if constexpr (kKeep)
+#pragma unroll
+    for (int i = 0; i < kSelItems; ++i)
+      if (k0 + 32 * i < cnt) v[i] = g[k0 + 32 * i];
+  auto rec = [&](int i) -> R {
+    if constexpr (kKeep) return v[i];
+    else return g[k0 + 32 * i];
+  };
+  for (int k = t; k <= a.nwave; k += kSelThreads) s_iwt[k] = a.iwt[k];
+  if constexpr (KIND == kSelDiatomic)
+    for (int k = t; k < kSelMolN; k += kSelThreads) s_molcor[k] = a.molcor[k];
+  int pre = (int)a.tile_nu[tile];
   __syncthreads();
 
   // UB of each record's IWL, running maximum in file order
   int run = 0, hint = 0;
-  int ubs[kSelItems];
+  int nus[kSelItems];
 #pragma unroll
   for (int i = 0; i < kSelItems; ++i) {
-    const int k = t * kSelItems + i;
-    ubs[i] = 0;
+    const int k = k0 + 32 * i;
+    int u = 0;
     if (k < cnt) {
       int iwl;
-      if (sel_advance_iwl<KIND>(rec(k), a, base + k, &iwl)) {
-        int u = sel_ub(s_iwt, a.nwave, iwl, hint);
+      if (sel_advance_iwl<KIND>(rec(i), a, base + k, &iwl)) {
+        u = sel_ub(s_iwt, a.nwave, iwl, hint);
         hint = u;
         if (u > a.nwave + 1) {
-          sel_error(a.err, base + k, kSelErrSentinel);
+          sel_error(a.ctl, base + k, kSelErrSentinel);
           u = a.nwave + 1;
         }
-        ubs[i] = u;
-        run = u > run ? u : run;
       }
     }
-  }
-  int agg;
-  const int pre = block_scan_excl<kSelThreads>(run, s_warp, &agg, true);
-  const int nu_in = tile_nu > pre ? tile_nu : pre;  // NU before this thread's records
-
-  // the filter at each record's NU, operands gathered a group at a time; a
-  // selected record's LINEDATA replaces it in its slot
-  int nu = nu_in;
-  unsigned sel = 0, keep = 0, fixbits = 0;
-  int mycount = 0;
+    const int up = __shfl_up_sync(FULL, u, 1);
+    if (!__all_sync(FULL, lane == 0 || u >= up)) {  // (records in order: UB is its own running maximum)
 #pragma unroll
-  for (int g0 = 0; g0 < kSelItems; g0 += kSelGroup) {
-    SelOps ops[kSelGroup];
-    int nug[kSelGroup];
-#pragma unroll
-    for (int j = 0; j < kSelGroup; ++j) {
-      const int i = g0 + j, k = t * kSelItems + i;
-      nu = ubs[i] > nu ? ubs[i] : nu;
-      nug[j] = nu;
-      if (k < cnt) sel_gather<KIND>(rec(k), a, nu, s_molcor, ops[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < kSelGroup; ++j) {
-      const int i = g0 + j, k = t * kSelItems + i;
-      if (k < cnt) {
-        unsigned fx;
-        double c, y;
-        int4 o;
-        const int d = sel_decide<KIND>(rec(k), a, base + k, nug[j], ops[j], &o, &fx, &c, &y);
-        if (d) {
-          *reinterpret_cast<int4*>(&s_slot[sel_slot(k)]) = o;
-          sel |= 1u << i;
-          if (d == 2) keep |= 1u << i;
-          fixbits |= fx << (2 * i);
-          ++mycount;
-        }
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, u, o);
+        if (lane >= o) u = max(u, y);
       }
     }
+    nus[i] = max(u, run);
+    run = max(run, __shfl_sync(FULL, u, 31));
   }
-  int total;
-  const int opre = block_scan_excl<kSelThreads>(mycount, s_warp, &total, false);
-  if (t == 0) a.tile_count[tile] = total;
+  if (lane == 0) s_nu[wid] = run;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w)
+    if (w < wid) pre = max(pre, s_nu[w]);
 
-  // the tile's LINEDATA to its scratch place in file order; the host's cases
-  // (the original record comes from global memory: its slot holds LINEDATA)
-  int4* sc = a.scratch + base;
-  int q = opre;
-  nu = nu_in;
+  // the estimate at each record's NU
+  unsigned left = 0;
+  int n = 0;
 #pragma unroll
   for (int i = 0; i < kSelItems; ++i) {
-    nu = ubs[i] > nu ? ubs[i] : nu;
-    if (sel >> i & 1u) {
-      const int k = t * kSelItems + i;
-      sc[q] = *reinterpret_cast<const int4*>(&s_slot[sel_slot(k)]);
-      const unsigned fx = (fixbits >> (2 * i)) & 3u;
-      if ((keep >> i & 1u) || fx) sel_push_fixes<KIND>(a, g[k], base + k, base + q, nu, keep >> i & 1u, fx, s_molcor);
-      ++q;
-    }
+    nus[i] = max(nus[i], pre);
+    const bool keep = k0 + 32 * i < cnt && !sel_quick_reject<KIND>(rec(i), a, nus[i], s_molcor);
+    if (keep) left |= 1u << i;
+    n += __popc(__ballot_sync(FULL, keep));
   }
+  if (lane == 0) s_n[wid] = n;
+  __syncthreads();
+  int q = 0, nleft = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    q += w < wid ? s_n[w] : 0;
+    nleft += s_n[w];
+  }
+#pragma unroll
+  for (int i = 0; i < kSelItems; ++i) {
+    const unsigned b = __ballot_sync(FULL, left >> i & 1u);
+    if (left >> i & 1u) s_left[q + __popc(b & ((1u << lane) - 1u))] = (k0 + 32 * i) | nus[i] << 11;
+    q += __popc(b);
+  }
+  __syncthreads();
+
+  // the exact tests
+  int4* sc = a.scratch + base;
+  int done = 0, par = 0;
+  for (int s0 = 0; s0 < nleft; s0 += kSelThreads) {
+    int d = 0, k = 0, rnu = 0;
+    unsigned fx = 0;
+    int4 o;
+    if (s0 + t < nleft) {
+      const int e = s_left[s0 + t];
+      k = e & 2047;
+      rnu = e >> 11;
+      SelOps ops;
+      double c, y;
+      const R r = g[k];
+      sel_gather<KIND>(r, a, rnu, s_molcor, ops);
+      d = sel_decide<KIND>(r, a, base + k, rnu, ops, &o, &fx, &c, &y);
+    }
+    const unsigned b = __ballot_sync(FULL, d != 0);
+    if (lane == 0) s_cnt[par][wid] = __popc(b);
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const int c = s_cnt[par][w];
+      before += w < wid ? c : 0;
+      total += c;
+    }
+    if (d) {
+      const int pos = done + before + __popc(b & ((1u << lane) - 1u));
+      sc[pos] = o;
+      if (d == 2 || fx) sel_push_fixes<KIND>(a, g[k], base + k, base + pos, rnu, d == 2, fx, s_molcor);
+    }
+    done += total;
+    par ^= 1;
+  }
+  if (t == 0) a.tile_count[tile] = done;
 }
 
 // Pass C: every tile's LINEDATA from its scratch place to its offset (the
-// exclusive sum of the counts); positions at or past cap are not written
+// exclusive sum of the counts), positions at or past cap not written; the fix
+// list's scratch positions to output positions; what the host reads back
 __global__ void __launch_bounds__(256) k_sel_move(const int4* __restrict__ scratch, const int* __restrict__ count,
-                                                  const long long* __restrict__ off, int ntiles, int4* out,
-                                                  long long cap) {
+                                                  const long long* __restrict__ off,
+                                                  const long long* __restrict__ tile_nu, int ntiles, int4* out,
+                                                  long long cap, SelFix* fix, unsigned fixcap, SelCtl* ctl) {
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int c = count[tile];
     const long long o = off[tile];
@@ -664,14 +731,15 @@ __global__ void __launch_bounds__(256) k_sel_move(const int4* __restrict__ scrat
     for (int k = threadIdx.x; k < c; k += blockDim.x)
       if (o + k < cap) out[o + k] = src[k];
   }
-}
-
-// the fix list's scratch positions -> output positions
-__global__ void k_sel_fixpos(SelFix* fix, const unsigned* nfix, unsigned fixcap, const long long* __restrict__ off) {
-  const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= min(*nfix, fixcap)) return;
-  const long long p = fix[e].pos;
-  fix[e].pos = off[p / kSelTile] + p % kSelTile;
+  const unsigned nfix = min(ctl->nfix, fixcap);
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nfix; e += gridDim.x * blockDim.x) {
+    const long long p = fix[e].pos;
+    fix[e].pos = off[p / kSelTile] + p % kSelTile;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->nu = tile_nu[ntiles];
+    ctl->total = off[ntiles];
+  }
 }
 
 // drop the records at sorted positions rm [nrm] from in [n] into out

@@ -218,3 +218,27 @@ def test_driver_order_matches_oracle(sel, po):
         np.testing.assert_array_equal(got, np.concatenate(parts))
         assert st == state
         assert (counts[5] == 0) == (teff > 8000.0)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("scale", [1.0, 1e6, 1e300])
+def test_records_around_the_cut(po, gpu_ctx, tables, sel, kind, scale):
+    """Populations scaled so that half, most and all records pass (at 1e300 CENRATIO
+    overflows for some), and populations set so that each species' records lie
+    within a factor 1.1 of the cut: the FP32 estimate decides none of them wrongly."""
+    xn = np.minimum(sel["xn"] * scale, 1e300)
+    dev = linelists.SelectLines(gpu_ctx, 72, xn, sel["hckt"], sel["tc"], sel["iwt"], sel["wt"])
+    xmax = po.xnfdopmax(72, xn, sel["tc"])
+    for n, seed in ((2049, 5), (70_001, 6)):
+        recs = synthetic.selectlines_records(kind, n, sel["wt"], seed=seed + kind)
+        if scale == 1.0 and kind not in (5, 6):
+            # IELO of a record at the cut, give or take 5 %: E = ln(CENRATIO) / (HCKT) from a first pass at E = 0
+            rng = np.random.default_rng(seed)
+            e = np.clip(16384 + 1000 * np.log10(rng.uniform(0.5, 30.0, n) / sel["hckt"][-1]), 1, 32767).astype(np.int64)
+            recs[:, 1] = (recs[:, 1] & 0xFFFF) | (e.astype(np.int32) << 16)
+        st0 = start(sel)
+        want, err, bad, wst = oracle(po, sel, kind, recs, st0, xmax=xmax)
+        assert err == 0
+        st = dict(st0)
+        np.testing.assert_array_equal(dev.select(kind, recs, st), want)
+        assert st == wst
