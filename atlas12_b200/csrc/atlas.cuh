@@ -546,7 +546,9 @@ static __device__ __forceinline__ void linop_wings(const LinopArgs& a, int slot,
 #pragma unroll 1
   for (int s = 0;;) {
     if (kX) blue = blue && !(wb < wcon);  // the continuum edge
-    const double vr = (wr - wlvac) * w.rdop, vb = (wlvac - wb) * w.rdop;
+    // (a line less than 1 nm past the last wavelength is kept, with NU at that one: its
+    // V as the distance, so that the table index cannot be negative)
+    const double vr = fabs(wr - wlvac) * w.rdop, vb = (wlvac - wb) * w.rdop;
     // the next grid wavelengths, one step ahead
     if (s + 1 < nr) wr = ws[s + 1];
     if (s + 1 < nb) wb = ws[-2 - s];

@@ -62,3 +62,24 @@ def test_linop_walks(po, gpu_ctx, tables, h_tables, ross, nrhox, numnu, nlines, 
     assert n == used
     np.testing.assert_array_equal(got != 0, ref != 0)
     assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-300), initial=0.0) < tol
+
+
+@pytest.mark.parametrize("prec", [_lib.PREC_FP64, _lib.PREC_MIXED])
+@pytest.mark.parametrize("past", [0.004, 0.3, 0.9])
+def test_line_past_the_last_wavelength(gpu_ctx, tables, h_tables, ross, past, prec):
+    """A line less than 1 nm past the last wavelength adds there at the distance V, as
+    on a grid with one more wavelength beyond it (its profile table has no
+    negative side).  The same additions in both: equal to rounding."""
+    c = case(ross, 72, 60, 1, seed=1, strength=1e8)
+    iwl = int(round(np.log(c["ws"][-1] + past) / np.log(1.0 + 1.0 / 2000000.0)))
+    lines = c["lines"][:1].copy()
+    lines[0, 0] = iwl
+    A = atlas.Atlas(gpu_ctx, tables, *h_tables)
+    gpu_ctx.set_precision(prec)
+    try:
+        a, b = (A.linop1(lines, 72, c["xnfdop"], c["dopple"], c["xne"], c["txnxn"], c["hckt"], c["tabcont"], c["iw"],
+                         ws)[0] for ws in (c["ws"], np.append(c["ws"], c["ws"][-1] + 5.0)))
+    finally:
+        gpu_ctx.set_precision(_lib.PREC_MIXED)
+    assert np.all(np.isfinite(a)) and np.count_nonzero(a[-1]) > 30 and a.min() >= 0.0
+    np.testing.assert_allclose(a[-1], b[-2], rtol=1e-9)
