@@ -28,6 +28,14 @@ int ensure_tablog(atlasgpu_ctx* ctx, double** out) {
   return 0;
 }
 
+void linop_launch(atlasgpu_ctx* ctx, const LinopArgs& a) {
+  const bool f32 = ctx->precision == ATLASGPU_PREC_MIXED, split = linop_split(a.n, a.nrhox);
+  auto* const kern = split ? (f32 ? k_atlas_linop<true, true> : k_atlas_linop<false, true>)
+                           : (f32 ? k_atlas_linop<true, false> : k_atlas_linop<false, false>);
+  const int64_t warps = split ? a.n * ((a.nrhox + 31) / 32) : a.n;
+  kern<<<grid_for(ctx, warps * 32, 256, 16), 256, 0, ctx->stream>>>(a);
+}
+
 }  // namespace atlasgpu
 
 namespace {
@@ -286,8 +294,7 @@ int atlasgpu_atlas_linop(atlasgpu_ctx* ctx, const int32_t* linedata, int64_t n, 
     a.work = work_counters(ctx, 1);
     {
       Timer tm(ctx, "atlas_linop");
-      if (ctx->precision == ATLASGPU_PREC_MIXED) k_atlas_linop<true><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
-      else k_atlas_linop<false><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
+      linop_launch(ctx, a);
       CKL(ctx);
       k_fix_finalize<<<grid_for(ctx, (int64_t)numnu * nrhox, 256, 8), 256, 0, s>>>(d_fix, d_fu, numnu, nrhox, kw,
                                                                                      d_xl);

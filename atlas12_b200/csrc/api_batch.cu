@@ -100,12 +100,12 @@ __global__ void k_batch_kapp(BatchDev d) {
 // entries, measured 5 % slower on the bench's 32-slot batch: 2.39 against
 // 2.27 ms per model-iteration.)
 // kDry: the counting pass of a timed iteration (the same walks, no adds)
-template <bool F32, bool kDry = false>
+template <bool F32, bool kDry = false, bool kSplit = false>
 __global__ void __launch_bounds__(256, kLinopMinBlocks) k_batch_linop(const __grid_constant__ LinopArgs a,
                                                                       const BatchCtl* ctl) {
   const int b = blockIdx.y;
   if (!running(ctl, b)) return;
-  linop_body<F32, kDry>(a, b);
+  linop_body<F32, kDry, false, kSplit>(a, b);
 }
 
 // the split RT pass (k_rt_pre / k_rt_solve / k_rt_post bodies) per running slot
@@ -251,10 +251,10 @@ int enqueue_batch(atlasgpu_ctx* ctx, atlasgpu_batch* B, bool timed) {
     la.work = work_counters(ctx, 1);
     {
       Timer tm(ctx, "batch_linop");
-      if (ctx->precision == ATLASGPU_PREC_MIXED)
-        k_batch_linop<true><<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
-      else
-        k_batch_linop<false><<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
+      const bool f32 = ctx->precision == ATLASGPU_PREC_MIXED, split = linop_split(B->nlines * nb, B->nrhox);
+      auto* const kern = split ? (f32 ? k_batch_linop<true, false, true> : k_batch_linop<false, false, true>)
+                               : (f32 ? k_batch_linop<true> : k_batch_linop<false>);
+      kern<<<dim3(B->grid_linop, nb), 256, 0, s>>>(la, B->d.ctl);
       CKL(ctx);
     }
     work_collect(ctx, la.work, {"batch_linop_points"});

@@ -193,6 +193,9 @@ int ensure_tablog(atlasgpu_ctx* ctx, double** out);
 int stehle_upload(atlasgpu_ctx* ctx, const atlasgpu_stehle_series* stehle, const char* prefix, const char* who,
                   StehleDev** out);
 
+struct LinopArgs;
+void linop_launch(atlasgpu_ctx* ctx, const LinopArgs& a);  // k_atlas_linop over a.n lines
+
 struct AtlasLine;
 int atlas_prep_lines(atlasgpu_ctx* ctx, const int32_t* d_ld, const int32_t* h_ld, int64_t n,
                      const double* d_tablog, const double* d_ws, const double* h_ws, int numnu,

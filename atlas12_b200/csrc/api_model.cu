@@ -149,10 +149,7 @@ int enqueue_begin(atlasgpu_ctx* ctx, atlasgpu_model* m, bool timed) {
     la.fscale = m->fscale;
     {
       Timer tm(ctx, "atlas_linop");
-      if (ctx->precision == ATLASGPU_PREC_MIXED)
-        k_atlas_linop<true><<<grid_for(ctx, m->nlines * 32, 256, 16), 256, 0, s>>>(la);
-      else
-        k_atlas_linop<false><<<grid_for(ctx, m->nlines * 32, 256, 16), 256, 0, s>>>(la);
+      linop_launch(ctx, la);
       CKL(ctx);
       k_fix_finalize<<<grid_for(ctx, (int64_t)m->numnu * m->nrhox, 256, 8), 256, 0, s>>>(
           m->xfix, m->funscale, m->numnu, m->nrhox, m->kw, m->xl);

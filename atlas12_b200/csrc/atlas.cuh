@@ -418,6 +418,16 @@ struct LinopArgs {
   size_t s_spec = 0, s_kw = 0, s_tab = 0, s_xl = 0;  // [nspec][kw], [kw], TABCONT, [numnu][kw]
 };
 
+// A line is one warp's, its rounds of 32 depths one after the other, and a round
+// of a strong line is 100 to 200 steps of some 700 ns: with few lines per
+// resident warp, the kernel takes as long as its longest lines.  Up to
+// kLinopSplit lines (over all slots) the rounds go to warps of their own (3,000
+// lines 178 -> 96 us, 20,000 332 -> 171, 100,000 637 -> 473); beyond, where every
+// warp has dozens of lines, the gating per round costs more than the balance
+// gains (8 slots of 50,000 lines 0.97 -> 1.24 ms, 500,000 lines 1.95 -> 2.10).
+constexpr int64_t kLinopSplit = 131072;
+inline bool linop_split(int64_t lines, int nrhox) { return nrhox > 32 && lines <= kLinopSplit; }
+
 // LINOP1's profile value at one wing point, V = (distance in nm) * RDOP with
 // RDOP = 1 / (DOPPLE * WLVAC) taken once per (line, depth): tabulated H(v, a)
 // for ADAMP <= 0.2 and v <= 10, the Lorentz wing 1/sqrt(pi) a / v^2 beyond,
@@ -605,11 +615,11 @@ static __device__ __forceinline__ void linop_wings(const LinopArgs& a, int slot,
 
 // The walks of one stored line by one warp (lanes over depths): the fine depth
 // gates and the red and blue wing walks of LINOP1 (:18236-18370); ifj: bit k
-// set where the coarse depth 8(k+1) passed.  walked / points count the walked
+// set where the coarse depth 8(k+1) passed; kSplit: only round's 32 depths.  walked / points count the walked
 // (line, depth) pairs and the wing points this lane added.
-template <bool F32, bool kDry, bool kX>
-static __device__ __forceinline__ void linop_line(const LinopArgs& a, int slot, int64_t il, unsigned ifj, int lane,
-                                                  unsigned& walked, unsigned& points, unsigned& atoms) {
+template <bool F32, bool kDry, bool kX, bool kSplit>
+static __device__ __forceinline__ void linop_line(const LinopArgs& a, int slot, int64_t il, unsigned ifj, int round,
+                                                  int lane, unsigned& walked, unsigned& points, unsigned& atoms) {
   const AtlasLine L = a.lines[il];
   const double cx = kX ? a.lcontx[il] : 0.0;
   const size_t os = (size_t)slot * a.s_spec + (size_t)(L.nelion - 1) * a.kw, ok = (size_t)slot * a.s_kw;
@@ -617,7 +627,8 @@ static __device__ __forceinline__ void linop_line(const LinopArgs& a, int slot, 
   const double* dpn = a.dopple + os;
   const double* tcv = a.tabcont + (size_t)slot * a.s_tab + (size_t)(L.nucont - 1) * a.kw;
   const double* hckt = a.hckt + ok;
-  for (int J0 = 1; J0 <= a.nrhox; J0 += 32) {
+  const int last = kSplit ? min(a.nrhox, 32 * round + 32) : a.nrhox;
+  for (int J0 = kSplit ? 32 * round + 1 : 1; J0 <= last; J0 += 32) {
     // a round of 32 depths can walk only where its coarse blocks, or the
     // block just above its first, passed: skip it before any load if none did
     {
@@ -694,7 +705,7 @@ __device__ __forceinline__ void linop_counts(const LinopArgs& a, int lane, unsig
 
 // kDry: the counting pass (walks, counts the wing points and the atomics the
 // adds would issue, adds nothing)
-template <bool F32, bool kDry = false, bool kX = false>
+template <bool F32, bool kDry = false, bool kX = false, bool kSplit = false>
 static __device__ __forceinline__ void linop_body(const LinopArgs& a, int slot) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -705,8 +716,14 @@ static __device__ __forceinline__ void linop_body(const LinopArgs& a, int slot) 
   // line g of the round at depth 8(k+1)); bit k of a line = IFJ at depth 8(k+1)
   const int ng = min(a.nrhox >> 3, 32), per = 32 / ng;
   const int lg = lane / ng, J = 8 * (lane - lg * ng + 1);
-  for (int64_t il0 = w0 * kLinopChunk; il0 < a.n; il0 += nw * kLinopChunk) {
-    const int64_t il1 = il0 + kLinopChunk < a.n ? il0 + kLinopChunk : a.n;
+  // items: chunks of lines, or (kSplit) single lines' rounds of 32 depths
+  constexpr int chunk = kSplit ? 1 : kLinopChunk;
+  const int rounds = (a.nrhox + 31) / 32;
+  const int64_t n = kSplit ? a.n * rounds : a.n;
+  for (int64_t it = w0 * chunk; it < n; it += nw * chunk) {
+    const int64_t il0 = kSplit ? it / rounds : it;
+    const int round = kSplit ? (int)(it - il0 * rounds) : 0;
+    const int64_t il1 = il0 + chunk < a.n ? il0 + chunk : a.n;
     for (int64_t ib = il0; ib < il1; ib += per) {
       bool pass = false;
       if (lg < per && ib + lg < il1) {
@@ -725,18 +742,22 @@ static __device__ __forceinline__ void linop_body(const LinopArgs& a, int slot) 
       for (int g = 0; g < per; ++g) {
         const unsigned ifj = (gates >> (g * ng)) & (0xffffffffu >> (32 - ng));
         if (ifj == 0) continue;
-        if (lane == 0 && a.used) atomicAdd(a.used, 1ull);
-        linop_line<F32, kDry, kX>(a, slot, ib + g, ifj, lane, walked, points, atoms);
+        if (lane == 0 && a.used && round == 0) atomicAdd(a.used, 1ull);
+        linop_line<F32, kDry, kX, kSplit>(a, slot, ib + g, ifj, round, lane, walked, points, atoms);
       }
     }
   }
   linop_counts(a, lane, walked, points, atoms);
 }
 
+template <bool F32, bool kSplit>
+static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_atlas_linop(const __grid_constant__ LinopArgs a) {
+  linop_body<F32, false, false, kSplit>(a, 0);
+}
 template <bool F32>
-static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_atlas_linop(const __grid_constant__ LinopArgs a) { linop_body<F32>(a, 0); }
-template <bool F32>
-static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_xlinop_walk(const __grid_constant__ LinopArgs a) { linop_body<F32, false, true>(a, 0); }
+static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_xlinop_walk(const __grid_constant__ LinopArgs a) {
+  linop_body<F32, false, true>(a, 0);
+}
 
 // XLINES(J, NU) from the fixed-point words, which are cleared for the next
 // accumulation (grid-stride over NU, threads over depths J < nrhox)

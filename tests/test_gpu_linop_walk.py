@@ -83,3 +83,26 @@ def test_line_past_the_last_wavelength(gpu_ctx, tables, h_tables, ross, past, pr
         gpu_ctx.set_precision(_lib.PREC_MIXED)
     assert np.all(np.isfinite(a)) and np.count_nonzero(a[-1]) > 30 and a.min() >= 0.0
     np.testing.assert_allclose(a[-1], b[-2], rtol=1e-9)
+
+
+@pytest.mark.parametrize("prec,tol", [(_lib.PREC_FP64, 1e-9), (_lib.PREC_MIXED, 1e-6)])
+@pytest.mark.parametrize("nrhox,nlines", [(72, 131072), (40, 131073)])
+def test_both_sides_of_the_split(po, gpu_ctx, tables, h_tables, ross, nrhox, nlines, prec, tol):
+    """The most lines whose rounds of 32 depths go to warps of their own, and one more.
+    (Lines past the last wavelength, whose table index is negative in the oracle, moved inside.)"""
+    c = case(ross, nrhox, 400, nlines, seed=nrhox)
+    lines = c["lines"].copy()
+    lines[:, 0] = np.minimum(lines[:, 0], int(np.log(c["ws"][-1]) / np.log(1.0 + 1.0 / 2000000.0)) - 1)
+    atm = dict(xnfdop=c["xnfdop"], dopple=c["dopple"], xne=c["xne"], txnxn=c["txnxn"], hckt=c["hckt"])
+    ref, used = po.atlas_linop1(*h_tables, po.build_tablog(), lines, atm, c["tabcont"], c["iw"], c["ws"])
+    assert np.all(np.isfinite(ref))
+    A = atlas.Atlas(gpu_ctx, tables, *h_tables)
+    gpu_ctx.set_precision(prec)
+    try:
+        got, n = A.linop1(lines, nrhox, c["xnfdop"], c["dopple"], c["xne"], c["txnxn"], c["hckt"], c["tabcont"],
+                          c["iw"], c["ws"])
+    finally:
+        gpu_ctx.set_precision(_lib.PREC_MIXED)
+    assert n == used
+    np.testing.assert_array_equal(got != 0, ref != 0)
+    assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-300), initial=0.0) < tol
