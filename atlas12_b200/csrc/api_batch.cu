@@ -6,7 +6,7 @@
 // `nslots` atmospheres that share one frequency grid, one line list and the
 // Voigt tables; each slot has its own parameters, structure, populations,
 // opacities and ROSSTAB history.  One captured CUDA graph runs one iteration
-// of every RUNNING slot (seven launches for the whole batch, model index in
+// of every RUNNING slot (eleven launches for the whole batch, model index in
 // the grid's y or x dimension).  A slot's own status word, written by the
 // finish kernel, takes it out of the iteration when it converges, when
 // max |FLXERR| stops being finite, or at its iteration cap, so the graph can

@@ -382,7 +382,7 @@ static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restri
                                                          int* __restrict__ csr) {
   extern __shared__ __align__(8) unsigned char s_raw[];
   int64_t* s_pos = reinterpret_cast<int64_t*>(s_raw);  // [ntiles] where the block's next entry of a tile goes
-  int* s_cnt = reinterpret_cast<int*>(s_pos + ntiles);  // [ntiles] entries of this round
+  int* s_cnt = reinterpret_cast<int*>(s_pos + ntiles);  // [ntiles] entries of the block's current records
   const int jj = blockIdx.y;
   const unsigned nf = nfar[jj];
   const FarLine* fj = far + (size_t)jj * nlines;

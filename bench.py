@@ -90,9 +90,9 @@ def rt_partial_rows(numnu, nsm, slots, waves, warps_per_block=4):
 LINOP_TRAFFIC_PER_MODEL = 240e6
 # bytes of one prepared LINOP1 line record on the device (AtlasLine)
 LINE_RECORD_BYTES = 56
-# FP64 operations of one SYNTHE Weideman Voigt evaluation (31 complex Horner
-# steps of 8, plus the setup and the closing terms)
-WEIDEMAN_FLOP = 278
+# FP64 operations of one SYNTHE Weideman Voigt evaluation (31 steps of the real
+# recurrence, two multiply-adds each, plus the setup and the closing terms)
+WEIDEMAN_FLOP = 161
 
 
 def parse():
