@@ -432,7 +432,10 @@ static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restri
 //     Taylor series in v = (i - centre)/h (h = kSub/2) about the centre,
 //       x/(D + h v)^2 = sum_k (x/D^2) (k+1) (-h/D)^k v^k,  D = centre - c,
 //     |h v / D| < 1/4, and the lane adds the first kFarTerms coefficients
-//     (relative truncation below 1e-8);
+//     (relative truncation below 1e-8).  A group of 32 whose lines are all far
+//     enough away stops after 12 or 8: what is left out is below the rounding of
+//     each line's own sum, since which lines share a group depends on the order
+//     that the atomics gave the list;
 //   * otherwise, if any of its bins is in the line's far wing, the line is
 //     broadcast to the warp (shuffles) and every bin takes x * (1/n^2) itself,
 //     the lines in list order.  n is a whole number, so 1/n^2 comes from a
@@ -450,8 +453,9 @@ constexpr int kSub = 128;       // bins per sub-tile (one warp)
 constexpr int kSubs = kTile / kSub;
 constexpr int kFarSep = 256;    // minimum |centre - c| for an expansion
 constexpr int kFarLong = 4096;  // entries
-constexpr int kFarTerms = 16;   // Taylor terms; half of them where every line of a group is
-constexpr int kFarSep8 = 1024;  // this far away (|h v / D| < 1/16, truncation below 3e-9)
+constexpr int kFarTerms = 16;      // Taylor terms
+constexpr int kFarSep12 = 2048;    // 12 where every line of a group is this far away (|h v / D| < 1/32: 13/32^12 = 1e-17)
+constexpr int kFarSep8 = 16384;    // 8 from here on (|h v / D| < 1/256: 9/256^8 = 5e-19)
 constexpr int kFarInv = 65536;  // 1/n^2, n < kFarInv (512 KB)
 
 static __global__ void k_far_inverse(double* __restrict__ inv2) {
@@ -514,10 +518,11 @@ static __global__ void __launch_bounds__(32 * kFarWarps) k_farwing(const FarLine
       const double g = -0.5 * kSub * r, g2 = g * g, g4 = g2 * g2;
       // powers p*g^k in four independent chains (k mod 4)
       double p0 = x * r * r, p1 = p0 * g, p2 = p0 * g2, p3 = p1 * g2;
-      const bool all = __any_sync(FULL, distant && fabs(D) < (double)kFarSep8);
+      const bool t12 = __any_sync(FULL, distant && fabs(D) < (double)kFarSep8);
+      const bool t16 = __any_sync(FULL, distant && fabs(D) < (double)kFarSep12);
 #pragma unroll
       for (int k = 0; k < kFarTerms; k += 4) {
-        if (k == 8 && !all) break;
+        if ((k == 8 && !t12) || (k == 12 && !t16)) break;
         b[k] = fma((double)(k + 1), p0, b[k]);
         b[k + 1] = fma((double)(k + 2), p1, b[k + 1]);
         b[k + 2] = fma((double)(k + 3), p2, b[k + 2]);
