@@ -288,7 +288,7 @@ static __global__ void __launch_bounds__(32 * kCoreWarps, 4) k_core(const __grid
         f.n10 = n10;
         f.m = maxstep;
         f.pad = jj;
-        f.x = xw;
+        f.x = fmin(xw, 1.0e300);  // overflows REAL(4) at every n <= MAXPROF as infinity does, but 0 x is 0 (k_farwing)
         Q.far[nbuf + __popc(pm & lt)] = f;
         // bins n10 < |i - nb| <= maxstep inside the grid
         const int r0 = max(nb + n10 + 1, 1), r1 = min(nb + maxstep, a.length);
@@ -553,7 +553,7 @@ static __global__ void __launch_bounds__(32 * kFarWarps) k_farwing(const FarLine
         if ((unsigned)(d - n1) < sp) v[k] = d < kFarInv ? inv2[d] : 1.0 / ((double)d * (double)d);
       }
 #pragma unroll
-      for (int k = 0; k < kPer; ++k) sum[k] = fma(x, v[k], sum[k]);
+      for (int k = 0; k < kPer; ++k) sum[k] = fma(x, v[k], sum[k]);  // x is finite
     }
     f = fn;
   }

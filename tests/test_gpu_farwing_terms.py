@@ -50,3 +50,20 @@ def test_wing_of_distant_lines_to_rounding(gpu_ctx, tables, lines, prec):
     op = op[:, BINS - 1]
     assert np.all(op > 0)
     assert max(spread(o) for o in op) <= 2e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lines", [1, 5000])
+def test_infinite_wing_stays_inside_its_reach(gpu_ctx, tables, lines):
+    """Lines of infinite strength: infinite up to their core's end, and nothing past
+    MAXPROF bins, also where that lies within a sub-tile."""
+    maxprof, far, core = 700, CENTRE + np.array([701, 740, 760, 5000]), CENTRE + np.array([0, 1, 49, 50])
+    rec = S.make_lte_lines(np.full(lines, CENTRE), np.full(lines, np.inf), np.ones(lines, int), np.zeros(lines),
+                           np.full(lines, 1e-7), np.zeros(lines), np.zeros(lines))
+    one = np.ones(1)
+    op = S.Synthe(gpu_ctx, tables).line_opacity(rec, dict(length=LENGTH), 500000.0,
+                                                np.full((1, LENGTH), 1e-14, np.float32), np.ones((1, 1)),
+                                                np.full((1, 1), 1e-5), one, one, one, maxprof=maxprof)[0]
+    assert np.all(op[far - 1] == 0.0)
+    assert np.all(np.isinf(op[core - 1]))
+    assert np.all(np.isinf(op[2 * CENTRE - core - 1]))
