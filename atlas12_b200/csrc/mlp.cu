@@ -375,7 +375,6 @@ int atlasgpu_mlp_create(atlasgpu_ctx* ctx, int nin, int nh1, int nh2, int nout, 
     delete p;
     return fail(ctx, ATLASGPU_ENOMEM, "mlp_create");
   }
-  CK(cudaMemset(p->ticket, 0, sizeof(unsigned)));
   // Glorot-uniform weights, zero biases
   std::vector<float> h(p->nparam, 0.f);
   uint64_t s = seed;
@@ -389,9 +388,18 @@ int atlasgpu_mlp_create(atlasgpu_ctx* ctx, int nin, int nh1, int nh2, int nout, 
   fill(o.w1, nh1, nin);
   fill(o.w2, nh2, nh1);
   fill(o.w3, nout, nh2);
-  CK(cudaMemcpy(p->w, h.data(), sizeof(float) * p->nparam, cudaMemcpyHostToDevice));
-  CK(cudaMemset(p->m, 0, sizeof(float) * p->nparam));
-  CK(cudaMemset(p->v, 0, sizeof(float) * p->nparam));
+  // on the context's stream, as all that reads them (a non-blocking stream does not wait for the default one)
+  cudaStream_t st = ctx->stream;
+  const size_t bytes = sizeof(float) * p->nparam;
+  cudaError_t e = cudaMemcpyAsync(p->w, h.data(), bytes, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->m, 0, bytes, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->v, 0, bytes, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->ticket, 0, sizeof(unsigned), st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    atlasgpu_mlp_destroy(ctx, p);
+    return fail(ctx, ATLASGPU_ECUDA, "mlp_create: %s", cudaGetErrorString(e));
+  }
   *out = p;
   return 0;
 }
