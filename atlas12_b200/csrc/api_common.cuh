@@ -28,6 +28,7 @@ struct atlasgpu_ctx {
   std::unique_ptr<atlasgpu::HostCopier> copier;  // made at the first large result
   atlasgpu::JoshOps* ops = nullptr;  // device
   bool ops_set = false;
+  bool far_inverse = false;  // the 1/n^2 table ("lo_inv2") has been filled
   bool kapp_set = false;     // atlasgpu_atlas_set_kapp_tables done
   bool kapp_h2_set = false;  // atlasgpu_atlas_set_kapp_h2_tables done
   bool atlas_stehle = false;  // atlasgpu_atlas_set_stehle_tables loaded tables

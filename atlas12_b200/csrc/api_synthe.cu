@@ -306,9 +306,8 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
       (r = bufT(ctx, "lo_base", nj, &base)))
     return r;
   double* inv2;
-  const bool fresh = ctx->bufs.find("lo_inv2") == ctx->bufs.end();
   if ((r = bufT(ctx, "lo_inv2", kFarInv, &inv2))) return r;
-  if (fresh) {
+  if (!ctx->far_inverse) {
     k_far_inverse<<<kFarInv / 256, 256, 0, ctx->stream>>>(inv2);
     CKL(ctx);
   }
@@ -340,6 +339,7 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
     CKL(ctx);
     CK(cudaMemcpyAsync(htot.data(), tot, nb * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    ctx->far_inverse = true;  // only now: a launch that was refused or captured has filled nothing
     int64_t run = 0;
     for (int k = 0; k < nb; ++k) {
       hbase[k] = run;
