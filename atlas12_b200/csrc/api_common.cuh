@@ -29,6 +29,7 @@ struct atlasgpu_ctx {
   atlasgpu::JoshOps* ops = nullptr;  // device
   bool ops_set = false;
   bool far_inverse = false;  // the 1/n^2 table ("lo_inv2") has been filled
+  cudaEvent_t spec_done = nullptr;  // the last spectrum's use of "spec_rec"
   bool kapp_set = false;     // atlasgpu_atlas_set_kapp_tables done
   bool kapp_h2_set = false;  // atlasgpu_atlas_set_kapp_h2_tables done
   bool atlas_stehle = false;  // atlasgpu_atlas_set_stehle_tables loaded tables

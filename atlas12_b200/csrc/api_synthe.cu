@@ -67,6 +67,7 @@ int atlasgpu_destroy(atlasgpu_ctx* ctx) {
   ctx->copier.reset();
   for (auto& kv : ctx->bufs) cudaFree(kv.second.first);
   if (ctx->ops) cudaFree(ctx->ops);
+  if (ctx->spec_done) cudaEventDestroy(ctx->spec_done);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return ATLASGPU_OK;
@@ -426,10 +427,8 @@ int atlasgpu_synthe_line_opacity(atlasgpu_ctx* ctx, const atlasgpu_lte_line* lin
 }
 
 // ---------------------------------------------------------------- spectrum
-static int spectrum_launch(atlasgpu_ctx* ctx, SpecArgs a) {
-  const int chunk = std::min(a.length, kSpecChunk);
-  int r;
-  if ((r = bufT(ctx, "spec_rec", scatter_rec_doubles((size_t)2 * chunk, kSpecStride), &a.rec))) return r;
+// the staged wavelength loop over a.rec, which holds chunk wavelengths' records
+static int spectrum_rounds(atlasgpu_ctx* ctx, SpecArgs a, int chunk) {
   CK(cudaFuncSetAttribute(k_spec_pre, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spec_smem_bytes()));
   CK(cudaFuncSetAttribute(k_spec_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes()));
   Timer tm(ctx, "josh_spectrum");
@@ -447,6 +446,31 @@ static int spectrum_launch(atlasgpu_ctx* ctx, SpecArgs a) {
     CKL(ctx);
   }
   return 0;
+}
+
+// The records are scratch of one call.  Calls share the context's buffer, each
+// behind the one before also where the stream was changed in between.  A call
+// that is being captured has its own, allocated and freed by the graph: the
+// context's may be replaced by a larger one, or be in use, when the graph runs.
+static int spectrum_launch(atlasgpu_ctx* ctx, SpecArgs a) {
+  const int chunk = std::min(a.length, kSpecChunk);
+  const size_t doubles = scatter_rec_doubles((size_t)2 * chunk, kSpecStride);
+  cudaStream_t s = ctx->stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(s, &cap));
+  int r;
+  if (cap != cudaStreamCaptureStatusNone) {
+    CK(cudaMallocAsync((void**)&a.rec, doubles * sizeof(double), s));
+    r = spectrum_rounds(ctx, a, chunk);
+    CK(cudaFreeAsync(a.rec, s));
+    return r;
+  }
+  if ((r = bufT(ctx, "spec_rec", doubles, &a.rec))) return r;
+  if (ctx->spec_done) CK(cudaStreamWaitEvent(s, ctx->spec_done, 0));
+  else CK(cudaEventCreateWithFlags(&ctx->spec_done, cudaEventDisableTiming));
+  r = spectrum_rounds(ctx, a, chunk);
+  CK(cudaEventRecord(ctx->spec_done, s));
+  return r;
 }
 
 int atlasgpu_synthe_spectrum_dev(atlasgpu_ctx* ctx, const double* d_wledge, int nedge,

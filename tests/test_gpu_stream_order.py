@@ -78,3 +78,103 @@ def test_line_opacity_after_a_call_that_was_captured(tables):
     ctx.close()
     rt.cudaStreamDestroy(stream)
     np.testing.assert_allclose(got, want, rtol=1e-6)
+
+
+class Spectrum:
+    """synthe_spectrum_dev on device inputs of one case, with outputs of their own."""
+
+    def __init__(self, width, seed):
+        from atlas12_b200 import surrogate, synthetic
+        from atlas12_b200 import synthe as S
+        c = synthetic.synthe_case(nlines=1, wlbeg=400.0, wlend=400.0 + width, seed=seed, nrhox=48,
+                                  ross=surrogate.RossTable(nt=48, np_=48, nwave=300))
+        self.grid = S.synthe_grid(c["wlbeg"], c["wlend"], c["resolu"])
+        rng = np.random.default_rng(seed)
+        op = 10.0 ** rng.uniform(-6.0, 1.0, (48, self.grid["length"]))
+        self.v = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (
+            c["wledge"], c["contabs"], c["contscat"], c["atm"]["rhox"], c["atm"]["hkt"], op.astype(np.float32))]
+        self.out = [torch.zeros(self.grid["length"], dtype=torch.float64, device="cuda") for _ in range(2)]
+        torch.cuda.synchronize()
+
+    def call(self, ctx):
+        from atlas12_b200._lib import ptr
+        we, ca, cs, rx, hk, op = self.v
+        g = self.grid
+        ctx.call("atlasgpu_synthe_spectrum_dev", ptr(we), we.numel(), ptr(ca), ptr(cs), ca.shape[1], 48, ptr(rx), ptr(hk),
+                 g["wbegin"], g["ratio"], g["length"], ptr(op), *[ptr(o) for o in self.out])
+
+    def result(self):
+        r = np.stack([o.cpu().numpy() for o in self.out])
+        for o in self.out:
+            o.zero_()
+        torch.cuda.synchronize()
+        return r
+
+    def plain(self, tables):
+        ctx = spectrum_context(tables)
+        self.call(ctx)
+        ctx.close()
+        return self.result()
+
+
+def spectrum_context(tables):
+    from atlas12_b200 import _lib
+    ctx = _lib.Context(0)
+    ctx.set_operators(tables["xtau8"], tables["coefj"], tables["coefh"], tables["ch_j"], tables["ck_j"])
+    return ctx
+
+
+@pytest.mark.parametrize("before", [False, True])
+def test_spectrum_captured(tables, before):
+    """spectrum_dev launches kernels only, so it can be captured, also as a context's first
+    call, and the graph goes on giving the same bits after longer calls of the context."""
+    from cuda.bindings import runtime as rt
+    a, b = Spectrum(1.0, 1), Spectrum(30.0, 2)  # one round, and two of 32,768 wavelengths
+    want_a, want_b = a.plain(tables), b.plain(tables)
+    assert np.all(want_a > 0.0) and np.all(want_b > 0.0)
+    _, stream = rt.cudaStreamCreateWithFlags(rt.cudaStreamNonBlocking)
+    ctx = spectrum_context(tables)
+    ctx.synchronize()
+    ctx.set_stream(int(stream))
+    if before:
+        a.call(ctx)
+        ctx.synchronize()
+        assert np.array_equal(a.result(), want_a)
+    err, = rt.cudaStreamBeginCapture(stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeGlobal)
+    assert err == rt.cudaError_t.cudaSuccess
+    a.call(ctx)
+    err, graph = rt.cudaStreamEndCapture(stream)
+    assert err == rt.cudaError_t.cudaSuccess
+    err, run = rt.cudaGraphInstantiate(graph, 0)
+    assert err == rt.cudaError_t.cudaSuccess
+    for _ in range(3):
+        b.call(ctx)
+        assert rt.cudaGraphLaunch(run, stream)[0] == rt.cudaError_t.cudaSuccess
+        b.call(ctx)
+        ctx.synchronize()
+        assert np.array_equal(a.result(), want_a)
+        assert np.array_equal(b.result(), want_b)
+    rt.cudaGraphExecDestroy(run)
+    rt.cudaGraphDestroy(graph)
+    ctx.close()
+    rt.cudaStreamDestroy(stream)
+
+
+def test_spectra_of_one_context_on_two_streams(tables):
+    """The stream changed between calls that nothing waits for: each has its own result."""
+    from cuda.bindings import runtime as rt
+    a, b = Spectrum(12.0, 3), Spectrum(25.0, 4)
+    want_a, want_b = a.plain(tables), b.plain(tables)
+    streams = [rt.cudaStreamCreateWithFlags(rt.cudaStreamNonBlocking)[1] for _ in range(2)]
+    ctx = spectrum_context(tables)
+    ctx.synchronize()
+    for _ in range(5):
+        for x, s in ((a, 0), (b, 1), (a, 0), (b, 1)):
+            ctx.set_stream(int(streams[s]))
+            x.call(ctx)
+        torch.cuda.synchronize()
+        assert np.array_equal(a.result(), want_a)
+        assert np.array_equal(b.result(), want_b)
+    ctx.close()
+    for s in streams:
+        rt.cudaStreamDestroy(s)
