@@ -25,7 +25,7 @@ struct atlasgpu_ctx {
   std::map<std::string, double> kwork;  // counted work units of timed launches
   // named device buffers, grow-only
   std::map<std::string, std::pair<void*, size_t>> bufs;
-  std::unique_ptr<atlasgpu::HostCopier> copier;  // made at the first large result
+  std::shared_ptr<atlasgpu::HostCopier> copier;  // the process's, taken at the first large result
   atlasgpu::JoshOps* ops = nullptr;  // device
   bool ops_set = false;
   bool far_inverse = false;  // the 1/n^2 table ("lo_inv2") has been filled
@@ -165,8 +165,8 @@ inline int grid_for(atlasgpu_ctx* ctx, int64_t work, int threads, int per_sm = 8
   return (int)g;
 }
 
-// results to the host on the context's stream, complete on return: large
-// pageable arrays by the context's copier
+// results to the host on the context's stream (the caller synchronises it): large
+// pageable arrays by the copier, which are complete on return
 int host_out(atlasgpu_ctx* ctx, std::initializer_list<CopySeg> segs);
 
 // (eight independent sums of 0 x: a compare and a branch per element ran at a

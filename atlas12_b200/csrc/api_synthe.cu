@@ -683,12 +683,7 @@ int host_out(atlasgpu_ctx* ctx, std::initializer_list<CopySeg> segs) try {
         bytes += q.bytes;
       }
     }
-  if (bytes >= kStagedMin) {
-    if (!ctx->copier) ctx->copier.reset(new HostCopier(ctx->device));
-    if (!ctx->copier->ready()) large.clear();
-  } else {
-    large.clear();
-  }
+  if (bytes < kStagedMin) large.clear();
   auto staged = [&](const CopySeg& q) {
     for (const CopySeg& l : large)
       if (l.host == q.host && l.dev == q.dev) return true;
@@ -698,7 +693,12 @@ int host_out(atlasgpu_ctx* ctx, std::initializer_list<CopySeg> segs) try {
     if (q.bytes == 0 || staged(q)) continue;
     CK(cudaMemcpyAsync(q.host, q.dev, q.bytes, cudaMemcpyDeviceToHost, s));
   }
-  if (!large.empty()) CK(ctx->copier->out(s, large));
+  if (large.empty()) return 0;
+  if (!ctx->copier) ctx->copier = HostCopier::of(ctx->device);
+  cudaError_t e = cudaSuccess;
+  if (!ctx->copier->out(s, large, bytes, &e))
+    for (const CopySeg& q : large) CK(cudaMemcpyAsync(q.host, q.dev, q.bytes, cudaMemcpyDeviceToHost, s));
+  CK(e);
   return 0;
 } catch (const std::exception& e) {
   return fail(ctx, ATLASGPU_ENOMEM, "host copy: %s", e.what());

@@ -6,15 +6,19 @@
 // faults of its first touch, which take most of the time (52 MB: 11.7 ms into
 // fresh pages, 3.2 ms into touched ones; the link needs 1.0).  Here up to
 // kWorkers threads touch the pages (MADV_POPULATE_WRITE: contents stay) while the
-// kernels still run, then move chunks from the ring to the array, the copies
-// staying on the caller's stream in order: 52 MB fresh 2.8 ms, and the page
-// touching overlaps the kernels.  Below kStagedMin a plain copy is as quick;
-// arrays the caller has pinned are copied directly.  (The other way, chunks
-// written by several threads read back over the link at half the rate of the
-// driver's own staging: inputs are copied plainly.)
+// kernels still run, sleep until the first chunk is there, then move chunks from
+// the ring to the array, the copies staying on the caller's stream in order: 52 MB
+// fresh 2.8 ms, and the page touching overlaps the kernels.  Below kStagedMin a
+// plain copy is as quick; arrays the caller has pinned are copied directly.  (The
+// other way, chunks written by several threads read back over the link at half the
+// rate of the driver's own staging: inputs are copied plainly.)
 //
-// The ring (6 MB) and the threads belong to a context, are made at its first
-// large result and go with it.
+// The ring (6 MB) and the threads are the process's, one set per device, shared
+// by its contexts and gone with the last of them that used it.  One call uses
+// them at a time; another one meanwhile copies plainly.  They take 3 to 10 ms to
+// make (nearly all of it the pinning), which is what they save on some 30 MB: so
+// the first kPlainFirst bytes are copied plainly, and a program that has one window
+// to copy pays nothing for them.
 #pragma once
 #include <cuda_runtime.h>
 #include <sys/mman.h>
@@ -23,7 +27,10 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstdint>
+#include <algorithm>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -36,8 +43,9 @@ struct CopySeg {
   size_t bytes;
 };
 
-constexpr size_t kStagedMin = 8 << 20;   // bytes of a call's large arrays from which the threads are used: making
-                                         // them costs some 10 ms once, below this they save under 1 ms a call
+constexpr size_t kStagedMin = 8 << 20;    // bytes of a call's large arrays from which the threads are used (below:
+                                          // under 1 ms a call)
+constexpr size_t kPlainFirst = 32 << 20;  // bytes of such calls copied plainly before the ring and the threads are made
 constexpr size_t kStagedSeg = 256 << 10;  // smaller arrays of the same call are copied plainly
 
 class HostCopier {
@@ -60,10 +68,33 @@ class HostCopier {
     if (pin_) cudaFreeHost(pin_);
   }
 
-  // false: no ring to be had, the caller copies plainly
-  bool ready() {
-    if (pin_) return pid_ == getpid();
+  // the process's copier for a device
+  static std::shared_ptr<HostCopier> of(int device) {
+    static std::mutex m;
+    static std::map<int, std::weak_ptr<HostCopier>> all;
+    std::lock_guard<std::mutex> l(m);
+    std::shared_ptr<HostCopier> c = all[device].lock();
+    if (!c) all[device] = c = std::make_shared<HostCopier>(device);
+    return c;
+  }
+
+  // Device to host, complete on return, the outcome in *e; false: nothing done,
+  // the caller copies plainly (another call is using the ring, or there is none).
+  bool out(cudaStream_t s, const std::vector<CopySeg>& segs, size_t bytes, cudaError_t* e) {
+    std::unique_lock<std::mutex> use(use_, std::try_to_lock);
+    if (!use || pid_ != getpid() || !ready(bytes)) return false;
+    *e = run(s, segs);
+    return true;
+  }
+
+ private:
+  bool ready(size_t bytes) {
+    if (pin_) return true;
     if (failed_) return false;
+    if (plain_ < kPlainFirst) {
+      plain_ += bytes;
+      return false;
+    }
     failed_ = true;
     for (; nev_ < kSlots; ++nev_)
       if (cudaEventCreateWithFlags(&ev_[nev_], cudaEventDisableTiming) != cudaSuccess) {
@@ -86,24 +117,32 @@ class HostCopier {
     return true;
   }
 
-  // device to host, complete on return
-  cudaError_t out(cudaStream_t s, const std::vector<CopySeg>& segs) {
+  cudaError_t issue(cudaStream_t s, int k) {
+    const int sl = k % kSlots;
+    const Chunk& c = chunks_[k];
+    cudaError_t e = cudaMemcpyAsync(pin_ + (size_t)sl * kChunk, c.dev, c.bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaEventRecord(ev_[sl], s);
+    return e;
+  }
+
+  cudaError_t run(cudaStream_t s, const std::vector<CopySeg>& segs) {
     cut(segs);
-    open();
-    const int n = (int)chunks_.size();
+    const int n = (int)chunks_.size(), first = std::min(n, kSlots);
     cudaError_t e = cudaSuccess;
-    for (int k = 0; k < n && e == cudaSuccess && !abort_; ++k) {
-      const int sl = k % kSlots;
-      if (k < kSlots) e = cudaEventSynchronize(ev_[sl]);  // an earlier call's copy out of the slot
-      else
-        while (done_[sl].load(std::memory_order_acquire) != k - kSlots && !abort_)
-          if (!take_out()) std::this_thread::yield();
-      const Chunk& c = chunks_[k];
-      if (e == cudaSuccess && !abort_)
-        e = cudaMemcpyAsync(pin_ + (size_t)sl * kChunk, c.dev, c.bytes, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess && !abort_) e = cudaEventRecord(ev_[sl], s);
-      if (e == cudaSuccess && !abort_) issued_.store(k + 1, std::memory_order_release);
-      if (k + 1 == std::min(n, kSlots)) touch_pages();
+    for (int k = 0; k < first && e == cudaSuccess; ++k) {
+      e = cudaEventSynchronize(ev_[k]);  // a copy into the slot that an earlier call gave up on
+      if (e == cudaSuccess) e = issue(s, k);
+    }
+    if (e != cudaSuccess) return e;
+    open(first);
+    touch_pages();
+    e = cudaEventSynchronize(ev_[0]);  // the kernels: one thread waits for them, as in a plain copy
+    if (e == cudaSuccess) copying();
+    for (int k = kSlots; k < n && e == cudaSuccess && !abort_; ++k) {
+      while (done_[k % kSlots].load(std::memory_order_acquire) != k - kSlots && !abort_)
+        if (!take_out()) std::this_thread::yield();
+      if (!abort_) e = issue(s, k);
+      if (!abort_ && e == cudaSuccess) issued_.store(k + 1, std::memory_order_release);
     }
     if (e != cudaSuccess) abort_ = true;
     while (!abort_ && take_out()) {
@@ -112,7 +151,6 @@ class HostCopier {
     return e != cudaSuccess ? e : err_;
   }
 
- private:
   static constexpr size_t kChunk = 512 << 10;
   static constexpr size_t kTouch = 2 << 20;
   static constexpr int kSlots = 12, kWorkers = 7;
@@ -132,16 +170,26 @@ class HostCopier {
     }
   }
 
-  void open() {
+  void open(int issued) {
     for (auto& d : done_) d.store(-1, std::memory_order_relaxed);
-    issued_ = ticket_ = touched_ = 0;
+    ticket_ = touched_ = 0;
+    issued_ = issued;
     abort_ = false;
     err_ = cudaSuccess;
     {
       std::lock_guard<std::mutex> l(m_);
       job_ = true;
+      copying_ = false;
       want_ = (int)std::min(threads_.size(), chunks_.size() / 2);
       ++gen_;
+    }
+    if (want_) cv_.notify_all();
+  }
+  // the first chunk is there
+  void copying() {
+    {
+      std::lock_guard<std::mutex> l(m_);
+      copying_ = true;
     }
     if (want_) cv_.notify_all();
   }
@@ -149,6 +197,7 @@ class HostCopier {
   void close() {
     std::unique_lock<std::mutex> l(m_);
     job_ = false;
+    if (!copying_) cv_.notify_all();
     idle_.wait(l, [this] { return running_ == 0; });
   }
 
@@ -165,6 +214,9 @@ class HostCopier {
       l.unlock();
       const int n = (int)chunks_.size();
       touch_pages();
+      l.lock();
+      cv_.wait(l, [this] { return copying_ || !job_; });
+      l.unlock();
       for (int k; !abort_ && (k = ticket_.fetch_add(1)) < n;) {
         while (issued_.load(std::memory_order_acquire) <= k && !abort_) std::this_thread::yield();
         if (!abort_) copy_out(k);
@@ -210,6 +262,8 @@ class HostCopier {
 
   int device_;
   pid_t pid_;
+  std::mutex use_;      // held by the call that uses the rest
+  size_t plain_ = 0;    // bytes copied plainly before there was a ring
   char* pin_ = nullptr;
   bool failed_ = false;
   int nev_ = 0;
@@ -219,7 +273,7 @@ class HostCopier {
   std::condition_variable cv_, idle_;
   uint64_t gen_ = 0;
   bool quit_ = false;
-  bool job_ = false;
+  bool job_ = false, copying_ = false;
   int want_ = 0, running_ = 0;
   std::vector<Chunk> chunks_, touch_;
   std::atomic<int> done_[kSlots];
