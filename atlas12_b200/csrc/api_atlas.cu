@@ -28,12 +28,23 @@ int ensure_tablog(atlasgpu_ctx* ctx, double** out) {
   return 0;
 }
 
-void linop_launch(atlasgpu_ctx* ctx, const LinopArgs& a) {
-  const bool f32 = ctx->precision == ATLASGPU_PREC_MIXED, split = linop_split(a.n, a.nrhox);
-  auto* const kern = split ? (f32 ? k_atlas_linop<true, true> : k_atlas_linop<false, true>)
-                           : (f32 ? k_atlas_linop<true, false> : k_atlas_linop<false, false>);
+static void walk_launch(atlasgpu_ctx* ctx, const LinopArgs& a, bool split, void (*kern)(LinopArgs)) {
   const int64_t warps = split ? a.n * ((a.nrhox + 31) / 32) : a.n;
   kern<<<grid_for(ctx, warps * 32, 256, 16), 256, 0, ctx->stream>>>(a);
+}
+
+void linop_launch(atlasgpu_ctx* ctx, const LinopArgs& a) {
+  const bool f32 = ctx->precision == ATLASGPU_PREC_MIXED, split = linop_split(a.n, a.nrhox);
+  walk_launch(ctx, a, split,
+              split ? (f32 ? k_atlas_linop<true, true> : k_atlas_linop<false, true>)
+                    : (f32 ? k_atlas_linop<true, false> : k_atlas_linop<false, false>));
+}
+
+static void xlinop_launch(atlasgpu_ctx* ctx, const LinopArgs& a) {
+  const bool f32 = ctx->precision == ATLASGPU_PREC_MIXED, split = linop_split(a.n, a.nrhox);
+  walk_launch(ctx, a, split,
+              split ? (f32 ? k_xlinop_walk<true, true> : k_xlinop_walk<false, true>)
+                    : (f32 ? k_xlinop_walk<true, false> : k_xlinop_walk<false, false>));
 }
 
 }  // namespace atlasgpu
@@ -387,8 +398,7 @@ int atlasgpu_atlas_xlinop(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* recs, int
                 (const double*)ctx->bufs["tab_h2"].first, (const float4*)ctx->bufs["tab_hf"].first, d_xl, nullptr,
                 nullptr, 1, 0, 2000, 0.5642, d_lc, d_em};
     Timer tm(ctx, "atlas_xlinop");
-    if (ctx->precision == ATLASGPU_PREC_MIXED) k_xlinop_walk<true><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
-    else k_xlinop_walk<false><<<grid_for(ctx, n * 32, 256, 16), 256, 0, s>>>(a);
+    xlinop_launch(ctx, a);
     CKL(ctx);
     if (pops) {
       double *d_xp, *d_rho;

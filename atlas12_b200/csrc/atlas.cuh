@@ -529,14 +529,26 @@ static __device__ __noinline__ void linop_finish_warp(const LinopArgs& a, const 
 // larger loop costs in instruction fetch what it saves), the table test peeled
 // into a loop of its own (1.51 ms), 48 or 80 registers (1.32, 1.32 ms).
 // XLINOP's wings reach 2000 points: when at most kLinopFew lanes are left after
-// kLinopLanePts steps, the warp finishes them one at a time, lanes over points.
-// (LINOP1 with that from step 16 on: 2.12 ms with at most 4 lanes left, 2.31 with
-// 8, against 1.72 without at the time; its adds do not coalesce.)
+// kLinopLanePts steps, the warp finishes them one at a time, lanes over points:
+// 2 x 62 steps a lane for the 2000 that all of them take together, so sixteen
+// lanes break even.  With the hand-over only at four lanes and 128 steps, and the
+// rounds of 32 depths one after the other in a warp whatever the number of
+// records, XLINOP was slower than the hand-over of everything after 16 points
+// that it replaced wherever 5 to 16 lanes walked far (mixed precision, 9000 K,
+// 1,000 records on 4,000 points of 300-600 nm: 2.80 -> 4.08 ms).  Kernel time
+// relative to that first form, over 54 forms a precision (300, 1,000 and 30,000
+// records, 4000 to 9000 K, three grids), FP64 / mixed, mean and (worst): at four
+// lanes 0.74 / 0.88 (1.14 / 1.44), at twelve 0.55 / 0.62 (0.80 / 1.04), rounds to
+// warps of their own and four lanes 0.29 / 0.32 (0.63 / 0.67), twelve 0.25 / 0.27
+// (0.41 / 0.51), sixteen 0.25 / 0.27 (0.39 / 0.51); from step 16, 32 or 64 on
+// makes 2 % of difference.
+// (LINOP1 with a hand-over from step 16 on: 2.12 ms with at most 4 lanes left, 2.31
+// with 8, against 1.72 without at the time; its adds do not coalesce.)
 // A warp takes kLinopChunk consecutive lines at a time, so the warps of a
 // CTA work on neighbouring lines (the lines are in wavelength order) and
 // share the WAVESET window and the XLINES lines they touch in cache.
-constexpr int kLinopLanePts = 128;
-constexpr int kLinopFew = 4;
+constexpr int kLinopLanePts = 32;
+constexpr int kLinopFew = 16;
 constexpr int kLinopChunk = 4;
 constexpr int kLinopMinBlocks = 4;
 
@@ -754,9 +766,9 @@ template <bool F32, bool kSplit>
 static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_atlas_linop(const __grid_constant__ LinopArgs a) {
   linop_body<F32, false, false, kSplit>(a, 0);
 }
-template <bool F32>
+template <bool F32, bool kSplit>
 static __global__ void __launch_bounds__(256, kLinopMinBlocks) k_xlinop_walk(const __grid_constant__ LinopArgs a) {
-  linop_body<F32, false, true>(a, 0);
+  linop_body<F32, false, true, kSplit>(a, 0);
 }
 
 // XLINES(J, NU) from the fixed-point words, which are cleared for the next
