@@ -846,16 +846,17 @@ int atlasgpu_synthe_nlte_opacity(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* re
   CK(cudaMemcpyAsync(d_cx, contx, 26 * 17 * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(cudaMemsetAsync(d_acc, 0, nm * sizeof(double), s));
   if (n > 0) {
-    double* d_wave;
-    NlteRest* d_rest;
-    int* d_nrest;
+    const bool shortw = length <= kNlteShort;
+    double* d_wave = nullptr;
+    NlteRest* d_rest = nullptr;
+    int* d_nrest = nullptr;
     const int64_t restcap = std::min<int64_t>(2 * n * nrhox, kNlteRestMax);
-    if ((r = bufT(ctx, "sn_wave", (size_t)2 * length, &d_wave)) || (r = bufT(ctx, "sn_rest", (size_t)restcap, &d_rest)) ||
-        (r = bufT(ctx, "sn_nrest", 2, &d_nrest)))
+    if ((!shortw || hyd) && (r = bufT(ctx, "sn_wave", (size_t)2 * length, &d_wave))) return r;
+    if (!shortw && ((r = bufT(ctx, "sn_rest", (size_t)restcap, &d_rest)) || (r = bufT(ctx, "sn_nrest", 2, &d_nrest))))
       return r;
-    CK(cudaMemsetAsync(d_nrest, 0, 2 * sizeof(int), s));
     NlteArgs a{d_rec, n, length, nrhox, nspec, wbegin, ratio, wlend, 1.0 + velshift_kms / 299792.458, d_wave,
-               d_wave + length, d_cont, d_xd, d_dp, d_xne, d_tx, d_hc, d_em, d_cx, d_acc, d_rest, d_nrest, (int)restcap};
+               d_wave ? d_wave + length : nullptr, d_cont, d_xd, d_dp, d_xne, d_tx, d_hc, d_em, d_cx, d_acc, d_rest, d_nrest,
+               (int)restcap, n * nrhox <= 2ll * kNlteResident * ctx->nsm ? kNlteSoloFew : kNlteSolo};
     if (xnfpel) {
       double* d_xp;
       if ((r = bufT(ctx, "sn_xp", nd, &d_xp))) return r;
@@ -888,12 +889,20 @@ int atlasgpu_synthe_nlte_opacity(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* re
       }
     }
     Timer tm(ctx, "synthe_nlte");
-    k_grid_wave<<<(length + 255) / 256, 256, 0, s>>>(wbegin, ratio, length, d_wave, d_wave + length);
-    CKL(ctx);
-    k_synthe_nlte<<<grid_for(ctx, n * nrhox * 32, 256, 16), 256, 0, s>>>(a);
-    CKL(ctx);
-    k_synthe_nlte_rest<<<grid_for(ctx, restcap * 32 * kNlteWarps, 32 * kNlteWarps, 4), 32 * kNlteWarps, 0, s>>>(a);
-    CKL(ctx);
+    const int solo = grid_for(ctx, n * nrhox * 32, 256, 16);
+    if (d_wave) {
+      k_grid_wave<<<(length + 255) / 256, 256, 0, s>>>(wbegin, ratio, length, d_wave, d_wave + length, d_nrest);
+      CKL(ctx);
+    }
+    if (shortw) {
+      k_synthe_nlte<true><<<solo, 256, 0, s>>>(a);
+      CKL(ctx);
+    } else {
+      k_synthe_nlte<false><<<solo, 256, 0, s>>>(a);
+      CKL(ctx);
+      k_synthe_nlte_rest<<<grid_for(ctx, restcap * 32 * kNlteWarps, 32 * kNlteWarps, 4), 32 * kNlteWarps, 0, s>>>(a);
+      CKL(ctx);
+    }
     if (hyd && (r = synthe_hydrogen_launch(ctx, recs, n, length, nrhox, wbegin, ratio, wlend, a.dopratio, continuum,
                                            xnfdop, d_wave, d_cont, d_xd, d_dp, nspec, xne, d_xne, hckt, d_hc, hyd,
                                            d_acc)))

@@ -751,16 +751,25 @@ static __global__ void k_spec_flux(SpecArgs a) {
 //
 // Most wings end within a few steps of 32 points, a Shore line's or an edge's
 // run over the window (15,000 points for 12 nm at 390 nm), and those few chains
-// of 470 latency-bound steps were the kernel.  So a warp walks a wing for
-// kNlteSolo steps and then lists what is left; a block per listed wing walks on,
-// 256 points a step (k_synthe_nlte_rest).  With the wavelengths from a table
-// (a power per point before) and one division a Shore point for five: 300
-// records, 72 depths, 12 nm: 818 -> 290 us.
+// of 470 latency-bound steps were the kernel.  So a warp walks a wing for some
+// steps and then lists what is left; a block per listed wing walks on, 256 points
+// a step (k_synthe_nlte_rest).  With the wavelengths from a table (a power per
+// point before) and one division a Shore point for five: 300 records, 72 depths,
+// 12 nm: 818 -> 290 us.
+// A block takes 256 lanes for what is often a part of that, and the set-up again,
+// so listing only pays for a chip that is not full or a chain that is long: after
+// 8 steps where a resident warp has two (record, depth) pairs at most (30 records,
+// 72 depths, 4 nm at 400 nm: 152 us with one warp a wing and powers, 120 after 64
+// steps, 58 after 8), after 64 steps otherwise (3,000 records, 1 nm at 900 nm: 497,
+// 382, 655; 300 records, 12 nm: 577, 272, 258), never in a window of up to
+// kNlteShort points (1,000 records, half of them Shore, 1 nm at 900 nm: 243, 183,
+// 372).
 struct NlteRest {
   int64_t pair;  // record * nrhox + depth
   int pos, red;  // next grid point (1-based) and direction
 };
-constexpr int kNlteSolo = 8;                // steps of a warp before a wing is listed
+constexpr int kNlteSoloFew = 8, kNlteSolo = 64;  // steps of a warp before a wing is listed
+constexpr int kNlteResident = 24;                // warps an SM holds
 constexpr int kNlteWarps = 8;               // warps per listed wing
 constexpr int64_t kNlteRestMax = 1 << 18;   // a full list: the warp walks its wing to the end
 struct NlteArgs {
@@ -775,8 +784,8 @@ struct NlteArgs {
   const double* contx;              // CONTX(26,17) column-major
   double* acc;                      // [nrhox][length]
   NlteRest* rest;                   // [restcap]
-  int* nrest;                       // items listed, items taken
-  int restcap;
+  int* nrest;                       // items listed, items taken (2 words)
+  int restcap, solo;                // wings the list holds, steps before a wing is listed
   const double* xnfpel = nullptr;   // [nrhox][nspec] XNFPEL = populations / RHO; null: Shore lines skipped
   // merged-continuum edges (TYPE >= 4): per record its ordinal m (-1: none)
   // and per (m, depth) the grid indices NBUFF1, NBUFF2, NBUFF3 and a flag
@@ -785,9 +794,11 @@ struct NlteArgs {
   const int4* mbins = nullptr;
 };
 
+// (and the unit-19 list's counters, if there is one, zeroed)
 static __global__ void k_grid_wave(double wbegin, double ratio, int length, double* __restrict__ wave,
-                                   double* __restrict__ freq) {
+                                   double* __restrict__ freq, int* __restrict__ nrest) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (nrest && i < 2) nrest[i] = 0;
   if (i >= length) return;
   const double w = wbegin * powi(ratio, i);
   wave[i] = w;
@@ -877,8 +888,9 @@ __device__ __forceinline__ bool nlte_setup(const NlteArgs& a, int64_t p, NlteWal
 // walks one wing from point pos on, 32 (kBlock: 32 kNlteWarps) points a step;
 // returns where it stands after maxsteps steps, 0 when the wing has ended
 template <bool kBlock>
-__device__ __forceinline__ int nlte_walk(const NlteArgs& a, const NlteWalk& w, int j, bool red, int pos, int maxsteps,
-                                         int t, BlockVote<kNlteWarps>* vote, int& par) {
+__device__ __forceinline__ int nlte_walk(const NlteArgs& a, const double* waves, const double* freqs,
+                                         const NlteWalk& w, int j, bool red, int pos, int maxsteps, int t,
+                                         BlockVote<kNlteWarps>* vote, int& par) {
   constexpr int W = kBlock ? 32 * kNlteWarps : 32;
   const float* cont = a.cont + (size_t)j * a.length;
   double* acc = a.acc + (size_t)j * a.length;
@@ -890,7 +902,7 @@ __device__ __forceinline__ int nlte_walk(const NlteArgs& a, const NlteWalk& w, i
     double kappa = 0.0;
     if (use) {
       if (w.kind == 0) {
-        const double wave = a.wave[ib - 1];
+        const double wave = waves[ib - 1];
         use = wave >= w.wcon;
         if (use) {
           kappa = w.k0 * voigt_weideman(fabs(wave - w.wl) * w.rdopwl, w.adamp);
@@ -898,7 +910,7 @@ __device__ __forceinline__ int nlte_walk(const NlteArgs& a, const NlteWalk& w, i
           stop = kappa < (double)cont[ib - 1] * kLineCutoff;
         }
       } else if (w.kind == 1) {
-        const double eps = w.gr2 * (a.freq[ib - 1] - w.frelin);
+        const double eps = w.gr2 * (freqs[ib - 1] - w.frelin);
         kappa = w.k0 * (w.gs * eps + w.gw) / (eps * eps + 1.0);
         stop = kappa < (double)cont[ib - 1] * kLineCutoff;
       } else {
@@ -918,7 +930,24 @@ __device__ __forceinline__ int nlte_walk(const NlteArgs& a, const NlteWalk& w, i
   return 0;
 }
 
+// kShort: a window of at most kNlteShort points.  A warp walks its wings to their
+// ends, nothing is listed, and the wavelengths (the same ones) are formed by every
+// block in shared memory: one launch in place of three (50 points, 5 records, 16
+// depths, the call: 94 us with three launches and a memset, 84 with one).
+constexpr int kNlteShort = 1024;
+static_assert(kNlteShort <= 32 * kNlteSolo, "a wing of a short window is never listed");
+template <bool kShort>
 static __global__ void __launch_bounds__(256) k_synthe_nlte(const __grid_constant__ NlteArgs a) {
+  __shared__ double s_wave[kShort ? kNlteShort : 1], s_freq[kShort ? kNlteShort : 1];
+  if (kShort) {
+    for (int i = threadIdx.x; i < a.length; i += blockDim.x) {
+      const double w = a.wbegin * powi(a.ratio, i);
+      s_wave[i] = w;
+      s_freq[i] = kClightNms / w;
+    }
+    __syncthreads();
+  }
+  const double *waves = kShort ? s_wave : a.wave, *freqs = kShort ? s_freq : a.freq;
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -933,15 +962,15 @@ static __global__ void __launch_bounds__(256) k_synthe_nlte(const __grid_constan
       const bool red = dir == 0;
       int pos = red ? w.red : w.blue;
       if (pos < 1) continue;
-      pos = nlte_walk<false>(a, w, j, red, pos, kNlteSolo, lane, nullptr, par);
-      if (pos < 1) continue;
+      pos = nlte_walk<false>(a, waves, freqs, w, j, red, pos, kShort ? kNlteSolo : a.solo, lane, nullptr, par);
+      if (kShort || pos < 1) continue;
       int slot = 0;
       if (lane == 0) slot = atomicAdd(a.nrest, 1);
       slot = __shfl_sync(0xffffffffu, slot, 0);
       if (slot < a.restcap) {
         if (lane == 0) a.rest[slot] = NlteRest{p, pos, red};
       } else {
-        nlte_walk<false>(a, w, j, red, pos, 0x7fffffff, lane, nullptr, par);
+        nlte_walk<false>(a, waves, freqs, w, j, red, pos, 0x7fffffff, lane, nullptr, par);
       }
     }
   }
@@ -978,7 +1007,8 @@ static __global__ void __launch_bounds__(32 * kNlteWarps, 3) k_synthe_nlte_rest(
     if (s_i >= n) break;
     const NlteWalk w = walk;
     const NlteRest q = item;
-    nlte_walk<true>(a, w, (int)(q.pair % a.nrhox), q.red != 0, q.pos, 0x7fffffff, threadIdx.x, &vote, par);
+    nlte_walk<true>(a, a.wave, a.freq, w, (int)(q.pair % a.nrhox), q.red != 0, q.pos, 0x7fffffff, threadIdx.x, &vote,
+                    par);
     __syncthreads();
   }
 }
