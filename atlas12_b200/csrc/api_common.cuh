@@ -32,6 +32,7 @@ struct atlasgpu_ctx {
   cudaEvent_t spec_done = nullptr;  // the last spectrum's use of "spec_rec"
   bool kapp_set = false;     // atlasgpu_atlas_set_kapp_tables done
   bool kapp_h2_set = false;  // atlasgpu_atlas_set_kapp_h2_tables done
+  bool synthe_stehle = false;  // atlasgpu_synthe_set_hydrogen_tables loaded Stehle tables
   bool atlas_stehle = false;  // atlasgpu_atlas_set_stehle_tables loaded tables
   int nsm = 148;
   size_t smem_optin = 0;

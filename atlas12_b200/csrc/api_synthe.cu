@@ -656,8 +656,11 @@ static int synthe_hydrogen_launch(atlasgpu_ctx* ctx, const atlasgpu_nlte_line* r
            d_hv, d_hv + nrhox, d_hv + 2 * nrhox, d_hv + 3 * nrhox, d_hv + 4 * nrhox,
            (const atlasgpu_hydrogen_tables*)ctx->bufs["sh_tab"].first,
            (const StehleDev*)ctx->bufs["sh_stehle"].first, d_acc};
-  const int blocks = grid_for(ctx, nh * nrhox * kShThreads, kShThreads, 32);
-  k_synthe_hydrogen<<<blocks, kShThreads, 0, s>>>(a);
+  const int64_t np = nh * nrhox;
+  if (!ctx->synthe_stehle && length <= kShShort && 2ll * ctx->nsm * length <= kShWave * np)
+    k_synthe_hydrogen<1><<<grid_for(ctx, np * 32, 32, 256), 32, 0, s>>>(a);
+  else
+    k_synthe_hydrogen<kShWarps><<<grid_for(ctx, np * kShThreads, kShThreads, 32), kShThreads, 0, s>>>(a);
   CKL(ctx);
   CK(cudaStreamSynchronize(s));  // the host vectors go out of scope
   return 0;
@@ -781,6 +784,8 @@ int atlasgpu_synthe_set_hydrogen_tables(atlasgpu_ctx* ctx, const atlasgpu_hydrog
   if ((r = bufT(ctx, "sh_tab", 1, &d_tab))) return r;
   CK(cudaMemcpyAsync(d_tab, tables, sizeof *tables, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  ctx->synthe_stehle = false;
+  for (int q = 0; stehle && q < 4; ++q) ctx->synthe_stehle |= stehle[q].n_dens > 0;
   return 0;
 }
 

@@ -487,12 +487,23 @@ __device__ inline double sh_prof_stehle(const atlasgpu_hydrogen_tables& h, const
   return result;
 }
 
-static __global__ void __launch_bounds__(kShThreads, 2) k_synthe_hydrogen(const __grid_constant__ ShArgs a) {
+// kW: warps per block.  The convolution takes the eight of kShWarps.  Analytic
+// profiles take blocks of one warp in a window of up to kShShort points that has at
+// most kShWave points per wave of blocks of eight: a few steps of points leave most
+// of such a block's lanes without one, and the set-up by one of its threads keeps
+// the others waiting.  (92 records, 72 depths, 22 waves, 50 points: 316 us with
+// eight warps, 200 with one; 500 points 325, 254; 1,000 points 340, 300; 4,000
+// points 438, 582.  10 records, 2.4 waves, 50 points 104, 89; 256 points 101, 111;
+// 1,000 points 111, 174.)
+constexpr int kShShort = 1024, kShWave = 64;
+template <int kW>
+static __global__ void __launch_bounds__(32 * kW, 16 / kW) k_synthe_hydrogen(const __grid_constant__ ShArgs a) {
   __shared__ ShConv cv;
   __shared__ ShLine L;
   __shared__ ShDepth d;
   __shared__ ShKp kp;
-  __shared__ BlockVote<kShWarps> vote;
+  __shared__ BlockVote<kW> vote;
+  constexpr int kT = 32 * kW;
   const int tid = threadIdx.x;
   const atlasgpu_hydrogen_tables& h = *a.tab;
   const double CUTOFF = 1.0e-3;
@@ -511,10 +522,10 @@ static __global__ void __launch_bounds__(kShThreads, 2) k_synthe_hydrogen(const 
     const float dopph_h = dopph;
     if (r.deut) dopph = __fdiv_rn(dopph, 1.4142f);
     const double hwdop = (double)dopph;
-    const bool st = sh_use_stehle(a.stehle, r.n, r.m, a.xne[j]);
+    const bool st = kW == kShWarps && sh_use_stehle(a.stehle, r.n, r.m, a.xne[j]);
     __syncthreads();  // the previous pair's walk has read these
     if (tid == 0) sh_line(h, r.n, r.m, L);
-    if (tid == 32) sh_depth(a.xne[j], a.t[j], a.xnfph1[j], a.xnfph2[j], a.xnfhe1[j], a.xnfh2[j], d);
+    if (tid == (kW > 1 ? 32 : 0)) sh_depth(a.xne[j], a.t[j], a.xnfph1[j], a.xnfph2[j], a.xnfhe1[j], a.xnfh2[j], d);
     __syncthreads();
     if (st) {
       const float dconv = (pr.flags & 2) ? __fdiv_rn(dopph_h, 1.4142f) : dopph_h;
@@ -562,7 +573,7 @@ static __global__ void __launch_bounds__(kShThreads, 2) k_synthe_hydrogen(const 
     }
     bool exited = false;
     if (red) {
-      for (int b0 = red0; b0 <= length; b0 += kShThreads) {
+      for (int b0 = red0; b0 <= length; b0 += kT) {
         const int ib = b0 + tid;
         const bool in = ib <= length;
         const double wave = in ? a.wave[ib - 1] : 0.0;
@@ -572,7 +583,7 @@ static __global__ void __launch_bounds__(kShThreads, 2) k_synthe_hydrogen(const 
         int fo, fb;
         block_vote(vote, par, over, ok && kappa < (double)cont[ib - 1] * CUTOFF, tid, fo, fb);
         if (ok && tid < fo && tid <= fb) atomicAdd(acc + ib - 1, kappa);
-        if (min(fo, fb) < kShThreads) {
+        if (min(fo, fb) < kT) {
           exited = true;
           break;
         }
@@ -594,7 +605,7 @@ static __global__ void __launch_bounds__(kShThreads, 2) k_synthe_hydrogen(const 
     // blue wing (:3499-3508, :3531-3541, :3592-3605): add, then stop below the
     // continuum cutoff; higher members also stop (not added) blueward of WCON
     const int ib0 = min(length + 1, r.nbuff), maxblue = ib0 - 1;
-    for (int s0 = 1; s0 <= maxblue; s0 += kShThreads) {
+    for (int s0 = 1; s0 <= maxblue; s0 += kT) {
       const int s = s0 + tid, ib = ib0 - s;
       const bool valid = s <= maxblue;
       const double wave = valid ? a.wave[ib - 1] : 0.0;
@@ -603,7 +614,7 @@ static __global__ void __launch_bounds__(kShThreads, 2) k_synthe_hydrogen(const 
       int fe, fb;
       block_vote(vote, par, edge, valid && !edge && kappa < (double)cont[ib - 1] * CUTOFF, tid, fe, fb);
       if (valid && !edge && tid < fe && tid <= fb) atomicAdd(acc + ib - 1, kappa);
-      if (min(fe, fb) < kShThreads) break;
+      if (min(fe, fb) < kT) break;
     }
   }
 }

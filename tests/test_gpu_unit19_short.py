@@ -67,3 +67,28 @@ def test_listed_wings(po, gpu_ctx, tables, n, length, nrhox, lo, hi):
     assert np.all(ref > 0)
     err = np.abs(got.astype(np.float64) - ref) / (ref + cont.astype(np.float64))
     assert err.max() <= 1e-6, err.max()
+
+
+@pytest.mark.parametrize("length", [1, 31, 32, 33, 300, 1024, 1025])
+def test_hydrogen_by_warps(po, gpu_ctx, tables, length):
+    """Analytic hydrogen profiles of 19 waves of blocks, one warp a pair (up to 1,024 points) and
+    one block a pair, at both ends of the window and outside it."""
+    g = dict(po.synthe_grid(400.0, 410.0, 500000.0), length=length)
+    wav = g["wbegin"] * g["ratio"] ** np.arange(length)
+    recs = synthetic.hydrogen_records(100.0, 3000.0, g["wbegin"], g["ratio"])
+    recs = recs[(recs["nblo"] == 2) | (recs["nblo"] == 3)]
+    recs["nbuff"] = np.random.default_rng(length).integers(-2, length + 4, recs.size)
+    recs["wlvac"] = g["wbegin"] * g["ratio"] ** (recs["nbuff"] - 1.0)
+    h = synthetic.hydrogen_atmosphere()
+    nr = h["t"].size
+    assert recs.size * nr * 64 >= 2 * 148 * 1024
+    cont = np.full((nr, length), 1e-3, np.float32)
+    ref = po.synthe_hydrogen_opacity(recs, length, g["wbegin"], g["ratio"], wav[-1], 0.0, cont, h,
+                                     po.HTab.from_tables(tables, "s_"), None)
+    assert np.count_nonzero(ref) > 0.3 * ref.size
+    syn = S.Synthe(gpu_ctx, tables)
+    syn.set_hydrogen_tables(tables, None)
+    got = syn.nlte_opacity(recs, g, wav[-1], cont, h["xnfdop"], h["dopple"], h["xne"], h["txnxn"], h["hckt"],
+                           np.zeros((17, 26)), np.zeros((nr, length), np.float32), hydrogen=h)
+    err = np.abs(got.astype(np.float64) - ref) / (ref + cont.astype(np.float64))
+    assert err.max() <= 1e-6, err.max()
