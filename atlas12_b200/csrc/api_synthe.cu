@@ -360,7 +360,8 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
     {
       Timer tm(ctx, "synthe_farwing", true);
       dim3 g(ntiles * kSubs, nb);
-      if (run < (int64_t)kFarLong * ntiles * nb)
+      const int64_t most = *std::max_element(htot.begin(), htot.begin() + nb);
+      if (far_four_warps((double)run, (double)most / ntiles, ntiles, nb, ctx->nsm))
         k_farwing<4><<<g, 128, 0, ctx->stream>>>(far, nn, off, base, csr, ntiles, length, j0, inv2, acc, d_opac, work);
       else
         k_farwing<1><<<g, 32, 0, ctx->stream>>>(far, nn, off, base, csr, ntiles, length, j0, inv2, acc, d_opac, work);

@@ -422,10 +422,14 @@ static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restri
 // of each warp the bins lane + 32k; its warps walk the CSR list of the kTile-bin
 // tile the sub-tile belongs to in turn, 32 lines at a time (one line record per
 // lane, the next group's records already in flight), and classify each line
-// against the sub-tile.  Four warps where the lists are short (fewer than
-// kFarLong entries on average), so that small grids fill the GPU (0.5 nm, 500
-// lines: 45 against 22 us); one where they are long and the sums of four warps
-// only cost (1M lines: 8.2 against 8.8 ms).
+// against the sub-tile.  Four warps where they shorten the longest lists (few
+// sub-tiles, or much longer lists in the deepest layers), one where the sub-tiles
+// fill the GPU by themselves and the sums of four only cost: far_four_warps.
+// Measured one against four: 576 sub-tiles (0.5 nm), 500 lines 45, 22 us; 4,032 (5
+// nm), 10,000 lines 166, 115; 3,072 (20 nm, 16 depths), 100,000 lines 140, 157;
+// 13,824 (20 nm), 1M lines 9.7, 10.3 ms; 338,688 (700 nm), 1,000 lines 0.49, 1.63
+// ms.  (With four wherever a list had fewer than 4,096 entries, up to 10,000 lines
+// over 100 to 700 nm took up to 3.2 times what one warp a sub-tile takes.)
 //   * distant: the whole sub-tile lies inside one far wing of the line
 //     (n10 < |i - c| <= m for every bin i) and the sub-tile centre is at
 //     least kFarSep bins from c.  The line's terms x/(i - c)^2 are then the
@@ -452,7 +456,7 @@ static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restri
 constexpr int kSub = 128;       // bins per sub-tile (one warp)
 constexpr int kSubs = kTile / kSub;
 constexpr int kFarSep = 256;    // minimum |centre - c| for an expansion
-constexpr int kFarLong = 4096;  // entries
+constexpr int kFarResident = 24;  // warps an SM holds
 constexpr int kFarTerms = 16;      // Taylor terms
 constexpr int kFarSep12 = 2048;    // 12 where every line of a group is this far away (|h v / D| < 1/32: 13/32^12 = 1e-17)
 constexpr int kFarSep8 = 16384;    // 8 from here on (|h v / D| < 1/256: 9/256^8 = 5e-19)
@@ -461,6 +465,19 @@ constexpr int kFarInv = 65536;  // 1/n^2, n < kFarInv (512 KB)
 static __global__ void k_far_inverse(double* __restrict__ inv2) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n < kFarInv) inv2[n] = n ? 1.0 / ((double)n * (double)n) : 0.0;
+}
+
+// Whether four warps a sub-tile are quicker than one, in list entries that a warp
+// works through (17 a us, whether few warps run or all that fit): with one the
+// longest lists (maxlist: a tile's average at the depth with the most) or an even
+// share of all entries, whichever is more; with four a quarter of the longest or
+// the share, a fifth more for the sums, and 3 us for every round of blocks.  The
+// line lies within 10 % of the quicker one on 150 forms (0.2 to 100 nm, 1 to 1M
+// lines, 16, 40 and 72 depths).
+inline bool far_four_warps(double entries, double maxlist, int ntiles, int nb, int nsm) {
+  const double blocks = (double)ntiles * kSubs * nb, share = entries * kSubs / ((double)kFarResident * nsm);
+  const double one = share > maxlist ? share : maxlist, part = share > 0.25 * maxlist ? share : 0.25 * maxlist;
+  return 1.2 * part + 8.7 * blocks / nsm < one;  // 51 entries for 5.9 blocks on every SM
 }
 
 template <int kFarWarps>
@@ -492,6 +509,14 @@ static __global__ void __launch_bounds__(32 * kFarWarps) k_farwing(const FarLine
   const int64_t* o = off + (size_t)jj * (ntiles + 1);
   const int* list = csr + base[jj] + o[t];
   const int ne = (int)(o[t + 1] - o[t]);
+  if (ne == 0) {  // the core alone
+    for (int i = lo + threadIdx.x; i <= hi; i += 32 * kFarWarps) {
+      double& v = acc[(size_t)j * length + i - 1];
+      opac[(size_t)j * length + i - 1] = (float)v;
+      v = 0.0;
+    }
+    return;
+  }
   const FarLine* fj = far + (size_t)jj * nlines;
   const FarLine none{0, 0x7fffffff, 0, 0, 0.0};  // no bin of any sub-tile in its far wing
   // two-stage prefetch: the record of the next group, the index of the one after
