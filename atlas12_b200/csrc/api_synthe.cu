@@ -329,12 +329,13 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
       k_core<<<grid_for(ctx, groups, 32 * kCoreWarps, 4), 32 * kCoreWarps, 0, ctx->stream>>>(a);
       CKL(ctx);
     }
-    // list kernels: blocks of kFarBlock far-wing records, at most about four waves over the depths
-    const dim3 gfar((unsigned)std::max<int64_t>(1, std::min<int64_t>((nn + kFarBlock - 1) / kFarBlock,
+    // list kernels: blocks of chunk far-wing records, at most about four waves over the depths
+    const int chunk = far_chunk(nn, nb, ntiles, ctx->nsm);
+    const dim3 gfar((unsigned)std::max<int64_t>(1, std::min<int64_t>((nn + chunk - 1) / chunk,
                                                                      ctx->nsm * 32 / std::max(1, nb) + 1)), nb);
-    const bool fsm = ntiles < kFarTilesMax;
+    const bool fsm = ntiles < kFarTilesMax && chunk == kFarBlock;
     k_far_count<<<gfar, 256, fsm ? (ntiles + 1) * sizeof(int) : 0, ctx->stream>>>(far, nfar, nn, length, ntiles,
-                                                                                  tdiff);
+                                                                                  chunk, tdiff);
     CKL(ctx);
     k_far_scan<<<nb, 32, 0, ctx->stream>>>(tdiff, ntiles, off, fillptr, tot);
     CKL(ctx);
@@ -354,7 +355,7 @@ int atlasgpu_synthe_line_opacity_dev(atlasgpu_ctx* ctx, const atlasgpu_lte_line*
       const size_t fsmem = fsm ? ntiles * (sizeof(int64_t) + sizeof(int)) : 0;
       CK(cudaFuncSetAttribute(k_far_fill, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(kFarTilesMax * (sizeof(int64_t) + sizeof(int)))));
-      k_far_fill<<<gfar, 256, fsmem, ctx->stream>>>(far, nfar, nn, length, base, fillptr, ntiles, csr);
+      k_far_fill<<<gfar, 256, fsmem, ctx->stream>>>(far, nfar, nn, length, base, fillptr, ntiles, chunk, csr);
       CKL(ctx);
     }
     {

@@ -336,35 +336,62 @@ static __global__ void k_far_scan(int* __restrict__ tdiff, int ntiles, int64_t* 
   total[jj] = run;
 }
 
-// The far-wing lists' counts and entries.  A block takes kFarBlock consecutive
+// The far-wing lists' counts and entries.  A block takes chunk consecutive
 // far-wing records of one depth (blockIdx.y) at a time and keeps the tile
-// counters in shared memory (nsm of them; grids with more tiles use the global
+// counters in shared memory (grids with more than kFarTilesMax tiles use the global
 // ones): a line touches every tile within its wing, and all lines of a depth
 // touching the same few global counters bounded the fill (4.3 ms for 1M lines x
-// 72 depths against 0.45 for count and fill).
-constexpr int kFarBlock = 1024;
+// 72 depths against 0.45 for count and fill).  chunk is kFarBlock; where that makes
+// fewer blocks than the GPU has room for and the global counters are not crowded,
+// kFarFew, with global counters and a warp filling a record's tiles in place of a
+// thread (fill of 1,000 lines over 700 nm, 72 depths, 588 tiles: 62 us with blocks of
+// 1,024, 25 with 32; over 8,818 tiles, 4 depths 622, 29; over one tile, 72 depths 10,
+// 14, and of 2,000 lines 10, 20).
+constexpr int kFarBlock = 1024, kFarFew = 32;
+inline int far_chunk(int64_t n, int nb, int ntiles, int nsm) {
+  return n * nb <= (ntiles < 512 ? 512ll : 2048ll) * nsm ? kFarFew : kFarBlock;
+}
 constexpr int kFarTilesMax = 8192;
 
 __device__ __forceinline__ int2 far_tiles(const FarLine& f, int length) {
   return make_int2((max(f.c - f.m, 1) - 1) / kTile, (min(f.c + f.m, length) - 1) / kTile);
 }
 
+// op(tile, record) for every tile of the records s0 .. s1 - 1, by the whole block: a
+// thread a record, or (few) a warp
+template <class Op>
+__device__ __forceinline__ void far_each_tile(const FarLine* __restrict__ fj, unsigned s0, unsigned s1, int length,
+                                              bool few, Op&& op) {
+  if (few) {
+    for (unsigned s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x >> 5) {
+      const int2 t = far_tiles(fj[s], length);
+      for (int q = t.x + (threadIdx.x & 31); q <= t.y; q += 32) op(q, s);
+    }
+  } else {
+    for (unsigned s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
+      const int2 t = far_tiles(fj[s], length);
+      for (int q = t.x; q <= t.y; ++q) op(q, s);
+    }
+  }
+}
+
 // tile counts of every depth as differences (tdiff zeroed before)
 static __global__ void __launch_bounds__(256) k_far_count(const FarLine* __restrict__ far,
                                                           const unsigned* __restrict__ nfar, int64_t nlines,
-                                                          int length, int ntiles, int* __restrict__ tdiff) {
+                                                          int length, int ntiles, int chunk,
+                                                          int* __restrict__ tdiff) {
   extern __shared__ int s_cnt[];
   const int jj = blockIdx.y;
   const unsigned nf = nfar[jj];
   int* td = tdiff + (size_t)jj * (ntiles + 1);
-  if (blockIdx.x * kFarBlock >= nf) return;
-  const bool sm = ntiles < kFarTilesMax;
+  if (blockIdx.x * chunk >= nf) return;
+  const bool sm = ntiles < kFarTilesMax && chunk == kFarBlock;
   int* cnt = sm ? s_cnt : td;
   if (sm)
     for (int t = threadIdx.x; t <= ntiles; t += blockDim.x) s_cnt[t] = 0;
   __syncthreads();
-  for (unsigned s0 = blockIdx.x * kFarBlock; s0 < nf; s0 += gridDim.x * kFarBlock)
-    for (unsigned s = s0 + threadIdx.x; s < min(s0 + kFarBlock, nf); s += blockDim.x) {
+  for (unsigned s0 = blockIdx.x * chunk; s0 < nf; s0 += gridDim.x * chunk)
+    for (unsigned s = s0 + threadIdx.x; s < min(s0 + chunk, nf); s += blockDim.x) {
       const int2 t = far_tiles(far[(size_t)jj * nlines + s], length);
       atomicAdd(cnt + t.x, 1);
       atomicAdd(cnt + t.y + 1, -1);
@@ -378,7 +405,7 @@ static __global__ void __launch_bounds__(256) k_far_count(const FarLine* __restr
 static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restrict__ far,
                                                          const unsigned* __restrict__ nfar, int64_t nlines,
                                                          int length, const int64_t* __restrict__ base,
-                                                         int64_t* __restrict__ fillptr, int ntiles,
+                                                         int64_t* __restrict__ fillptr, int ntiles, int chunk,
                                                          int* __restrict__ csr) {
   extern __shared__ __align__(8) unsigned char s_raw[];
   int64_t* s_pos = reinterpret_cast<int64_t*>(s_raw);  // [ntiles] where the block's next entry of a tile goes
@@ -387,16 +414,13 @@ static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restri
   const unsigned nf = nfar[jj];
   const FarLine* fj = far + (size_t)jj * nlines;
   unsigned long long* fp = reinterpret_cast<unsigned long long*>(fillptr) + (size_t)jj * ntiles;
-  const bool sm = ntiles < kFarTilesMax;
-  for (unsigned s0 = blockIdx.x * kFarBlock; s0 < nf; s0 += gridDim.x * kFarBlock) {
-    const unsigned s1 = min(s0 + kFarBlock, nf);
+  const bool few = chunk < kFarBlock, sm = ntiles < kFarTilesMax && !few;
+  for (unsigned s0 = blockIdx.x * chunk; s0 < nf; s0 += gridDim.x * chunk) {
+    const unsigned s1 = min(s0 + chunk, nf);
     if (sm) {
       for (int t = threadIdx.x; t < ntiles; t += blockDim.x) s_cnt[t] = 0;
       __syncthreads();
-      for (unsigned s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
-        const int2 t = far_tiles(fj[s], length);
-        for (int q = t.x; q <= t.y; ++q) atomicAdd(s_cnt + q, 1);
-      }
+      far_each_tile(fj, s0, s1, length, few, [&](int q, unsigned) { atomicAdd(s_cnt + q, 1); });
       __syncthreads();
       for (int t = threadIdx.x; t < ntiles; t += blockDim.x)
         if (s_cnt[t]) {
@@ -405,13 +429,10 @@ static __global__ void __launch_bounds__(256) k_far_fill(const FarLine* __restri
         }
       __syncthreads();
     }
-    for (unsigned s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
-      const int2 t = far_tiles(fj[s], length);
-      for (int q = t.x; q <= t.y; ++q) {
-        const int64_t pos = sm ? s_pos[q] + atomicAdd(s_cnt + q, 1) : base[jj] + (int64_t)atomicAdd(fp + q, 1ull);
-        csr[pos] = (int)s;
-      }
-    }
+    far_each_tile(fj, s0, s1, length, few, [&](int q, unsigned s) {
+      const int64_t pos = sm ? s_pos[q] + atomicAdd(s_cnt + q, 1) : base[jj] + (int64_t)atomicAdd(fp + q, 1ull);
+      csr[pos] = (int)s;
+    });
     __syncthreads();
   }
 }
