@@ -1069,7 +1069,7 @@ constexpr int kRtSplitWarps = 4;      // warps per CTA of the pre and post stage
 struct RtPreWS {
   double abtot[kKwMax], alpha[kKwMax], snubar[kKwMax], taunu[kKwMax], rd[kKwMax], r2[kKwMax];
   double xsbar[kNx], xalpha[kNx], xs[kNx];
-  int lidx[2];
+  int last;
 };
 // The post stage's workspace: one warp's vectors carved from shared memory
 // at a stride of kv >= NRHOX doubles (rt_post_kv), its 51-point vectors, the

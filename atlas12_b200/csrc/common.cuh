@@ -24,7 +24,6 @@ constexpr double kBnuPrefac = 2.0 * kHplanck / (kClight * kClight) * 1.0e45;
 
 constexpr int kNx = ATLASGPU_NXTAU;  // JOSH's 51-point tau grid
 constexpr int kKwMax = 100;          // depth capacity (SYNTHE kw = 99, ATLAS kw = 80)
-constexpr int kLd = 52;              // leading dimension of the 51x51 SMEM matrix
 
 // JOSH operator set in device memory (atlas12_modules.f90:18409-18451, 18792-18860)
 struct JoshOps {

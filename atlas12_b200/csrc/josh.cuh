@@ -76,7 +76,7 @@ struct JoshWS {
   double t1[kKwMax];              // scratch (INTEG's terms)
   double red[8];                  // group reductions (multi-warp groups)
   double piv[kNx];                // pivots of the elimination without interchanges
-  int lidx[kKwMax + 4];           // MAP1 bracket indices
+  int last;                       // MAP1 bracket of the last grid point
   unsigned pk[4][3];              // pivot key exchange between a group's warps
 };
 
@@ -86,8 +86,6 @@ struct JoshWSFull {
   double knu1;
   int maxj;
 };
-
-__device__ __forceinline__ void wsync() { __syncwarp(0xffffffffu); }
 
 // ---------------------------------------------------------------- interpolation
 // PARCOE, INTEG, DERIV and MAP1 in Newton form.  On the interval
@@ -279,7 +277,7 @@ __device__ __noinline__ int g_map1_on(G g, const double* xo, const double* fo, i
 }
 template <class G>
 __device__ __forceinline__ int g_map1(G& g, const double* xo, const double* fo, int nold, const double* xn,
-                                      double* fn, int nnew, int* /*lidx*/) {
+                                      double* fn, int nnew) {
   return g_map1_on(g, xo, fo, nold, xn, fn, nnew);
 }
 
@@ -563,11 +561,11 @@ __device__ inline int g_josh_prepare(G& g, const JoshGrid& J, int nr, WS& ws, bo
     ws.xalpha[l] = xa;
     ws.xsbar[l] = xb;
     amax = fmax(amax, xa);
-    if (l == kNx - 1) ws.lidx[0] = last;
+    if (l == kNx - 1) ws.last = last;
   }
   amax = g.max(amax);
   g.sync();
-  const int L = ws.lidx[0];
+  const int L = ws.last;
   solve = amax > 0.0;
   if (!solve) {
     for (int l = g.r; l < kNx; l += G::N) ws.xs[l] = ws.xsbar[l];

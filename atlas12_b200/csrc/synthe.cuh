@@ -661,7 +661,7 @@ struct SpecWS {
   double xsbar[kNx], xalpha[kNx], xs[kNx];
   double snu[kKwMax], hnu[kKwMax], jmins[kKwMax], bnu[kKwMax];  // the unmapped surfaces' sweeps
   double *xw, *jnu, knu1;                                      // not used with IFSURF = 1
-  int lidx[2], maxj;
+  int last, maxj;
 };
 constexpr int kSpecWarps = 4;
 constexpr int kSpecChunk = 32768;  // wavelengths per round: two 104-double records each, 54 MB (they stay in L2)

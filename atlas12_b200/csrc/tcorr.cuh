@@ -579,9 +579,9 @@ __device__ inline double b_atlas_finish(ModelState* gms, double* gacc, int kw, i
       taustd[j] = exp10(-6.875 + (double)j * 0.125);
     }
     w.sync();
-    g_map1(w, s.tauros, s.t, n, taustd, tnew1, n, jw.lidx);
-    g_map1(w, s.tauros, s.prad, n, taustd, prdnew, n, jw.lidx);
-    g_map1(w, s.tauros, tplus, n, taustd, tnew2, n, jw.lidx);
+    g_map1(w, s.tauros, s.t, n, taustd, tnew1, n);
+    g_map1(w, s.tauros, s.prad, n, taustd, prdnew, n);
+    g_map1(w, s.tauros, tplus, n, taustd, tnew2, n);
     if (L == 0) {
       s_scal[0] = R.zerot;
       s_scal[1] = R.slopet;
@@ -612,7 +612,7 @@ __device__ inline double b_atlas_finish(ModelState* gms, double* gacc, int kw, i
     const int L = tid;
     for (int j = L; j < n; j += 32) ppp[j] = (pt2[j] - pt1[j]) / pt1[j];
     w.sync();
-    g_map1(w, taustd, ppp, n, s.tauros, rrr, n, jw.lidx);
+    g_map1(w, taustd, ppp, n, s.tauros, rrr, n);
     for (int j = L; j < n; j += 32) s.t[j] = s.t[j] + s.t1[j];
     w.sync();
     if (L == 0) {
@@ -631,7 +631,7 @@ __device__ inline double b_atlas_finish(ModelState* gms, double* gacc, int kw, i
     double* src[8] = {s.rhox, s.t, s.p, s.xne, s.abross, s.prad, s.vturb, s.pturb};
     const double ab_surf = s.abross[0];
     for (int q = 0; q < 8; ++q) {
-      g_map1(w, s.tauros, src[q], n, taustd, rmp, n, jw.lidx);
+      g_map1(w, s.tauros, src[q], n, taustd, rmp, n);
       for (int j = L; j < n; j += 32) {
         double v = rmp[j];
         if (q == 4 && s.tauros[0] > taustd[j] && v < 0.0) v = ab_surf;
