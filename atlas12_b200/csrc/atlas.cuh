@@ -5,11 +5,14 @@
 //                 iteration-invariant half of LINOP1, atlas12_modules.f90:18176-18235)
 //  k_atlas_linop  per line: coarse/fine depth gating and the <= 100-point red
 //                 and blue wing walks of LINOP1 (:18236-18370) with the
-//                 tabulated / full Kurucz Voigt, into XLINES (FP64 atomics)
-//  k_atlas_rt     per frequency (one warp): Planck terms, opacities, JOSH,
-//                 negative floor and the TCORR/RADIAP/ROSS mode-2 sums of
-//                 RUN_RT_PASS (:3905-3949), accumulated per warp in frequency
-//                 order (deterministic)
+//                 tabulated / full Kurucz Voigt, into exact fixed-point sums
+//                 (k_fix_finalize turns them into XLINES); k_xlinop_walk: the
+//                 same walk for XLINOP's records, FP64 atomics into XLINES
+//  k_rt_pre, _series, _solve, _post  the frequency loop of RUN_RT_PASS
+//                 (:3905-3949) in stages: Planck terms, opacities, JOSH, negative
+//                 floor and the TCORR/RADIAP/ROSS mode-2 sums, accumulated per
+//                 warp in frequency order (deterministic); k_atlas_rt: the same
+//                 in one launch, for callers that may not allocate
 //  k_atlas_reduce per depth: fixed-order sum of the per-warp partials
 #pragma once
 #include "common.cuh"

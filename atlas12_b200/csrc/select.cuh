@@ -1,7 +1,7 @@
 // select.cuh -- SELECTLINES (atlas12_modules.f90:19171-19781) on the device:
 // the filter that turns the line databases into the LINEDATA records LINOP1
-// walks.  HBM-bound streaming passes over tiles of 2048 records, with no
-// CTA waiting on another:
+// walks.  Streaming passes over tiles of 2048 records, with no CTA waiting on
+// another (the reading of pass A is bound by HBM, the filter by latency):
 //
 //  * the NU advance (DO WHILE (IWL >= IWAVETAB(NU)) ...) is a running
 //    maximum: after a record, NU = max(NU at entry, UB(max IWL so far)) with

@@ -664,7 +664,7 @@ struct SpecWS {
   int last, maxj;
 };
 constexpr int kSpecWarps = 4;
-constexpr int kSpecChunk = 32768;  // wavelengths per round: two 104-double records each, 54 MB (they stay in L2)
+constexpr int kSpecChunk = 32768;  // wavelengths per round: two 154-double records each, 81 MB (of 126 MB of L2)
 // record: XALPHA, XSBAR, then XS (its first word becomes H(1)), the solve flag
 constexpr int kSpecXs = 2 * kNx, kSpecSolve = 3 * kNx, kSpecStride = 3 * kNx + 1;
 inline size_t spec_smem_bytes() { return sizeof(JoshGrid) + kSpecWarps * sizeof(SpecWS); }

@@ -66,14 +66,14 @@ FLOPS_PER_NU = int(2 / 3 * 51 ** 3 + 8 * 51 ** 2 + 2 * 51 + 110 * 72)
 # (a 51x51 matrix-vector product and the update)
 FLOPS_PER_SOLVE = int(2 / 3 * 51 ** 3 + 4 * 51 ** 2)
 FLOPS_PER_SERIES_STEP = 2 * 51 ** 2 + 3 * 51
-# DRAM bytes per model of the three batched RT launches that do not depend on
-# the launch shape (ncu, 4-slot capture of this workload: 337 MB per model
-# less the 138 MB of partial-sum rows it wrote, one per frequency at 4 slots):
+# DRAM bytes per model of the four batched RT launches that do not depend on
+# the launch shape (ncu, 4-slot capture of a workload of this size: 267 MB per
+# model less the 69 MB of partial-sum rows it wrote, one per two frequencies):
 # ACONT, SIGMAC and XLINES read by the prepare and finish stages, the
 # per-frequency records written and read back.  The finish stage's
 # partial-sum rows (one 577-double row per finish warp) are added for the
 # tuned shape (rt_partial_rows).
-RT_TRAFFIC_FIXED_PER_MODEL = 199e6
+RT_TRAFFIC_FIXED_PER_MODEL = 198e6
 
 
 def rt_partial_rows(numnu, nsm, slots, waves, warps_per_block=4):
@@ -85,9 +85,9 @@ def rt_partial_rows(numnu, nsm, slots, waves, warps_per_block=4):
     n = -(-numnu // per)
     return -(-n // warps_per_block) * warps_per_block
 # DRAM bytes per model of one batched LINOP1 launch (ncu, 4-slot capture of
-# this workload: 959 MB): the prepared line records and the fixed-point XLINES
+# a workload of this size: 375 MB): the prepared line records and the fixed-point XLINES
 # words, whose write-backs dominate once several models' words exceed L2
-LINOP_TRAFFIC_PER_MODEL = 240e6
+LINOP_TRAFFIC_PER_MODEL = 94e6
 # bytes of one prepared LINOP1 line record on the device (AtlasLine)
 LINE_RECORD_BYTES = 56
 # FP64 operations of one SYNTHE Weideman Voigt evaluation (31 steps of the real
@@ -418,7 +418,7 @@ def run_ours(args):
             "unit": "TFLOP/s", "frac": ach / fp64_peak if fp64_peak > 0 else None,
             "executed_tflops": executed / (kms["rt"] * 1e-3) / 1e12,
             "traffic": rt_traffic * CFG["slots"],
-            "traffic_scaling": f"ncu capture of the three launches of a 4-slot batch (337 MB per model, 138 MB of "
+            "traffic_scaling": f"ncu capture of the four launches of a 4-slot batch (267 MB per model, 69 MB of "
                                f"them partial-sum rows); the rows rescaled to this shape's {rows} per model "
                                f"({rows * (8 * CFG['nrhox'] + 1) * 8 / 1e6:.0f} MB), times slots",
             "peak_source": "measured DFMA loop on this GPU (atlasgpu_fp64_peak_tflops); MEASURED_PEAKS.json has no FP64 figure",
