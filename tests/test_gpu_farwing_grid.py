@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("length,lines,nrhox,maxprof", [
     (1000, 1, 72, 1000000), (1000, 2000, 3, 1000000),    # one tile: one warp, four warps
-    (5000, 3000, 16, 1000000), (60000, 3000, 16, 1000000),  # the same lines on more tiles
+    (5000, 600, 16, 1000000), (60000, 600, 16, 1000000),    # the same lines on more tiles
     (200000, 12, 16, 700), (200000, 1, 72, 1000000),     # most sub-tiles without a wing
     (8191 * 1024, 10, 1, 1000000), (8191 * 1024 + 1, 10, 1, 1000000),
     (8192 * 1024, 310000, 1, 200), (8190 * 1024, 310000, 1, 200)])  # blocks of 1,024 records there
