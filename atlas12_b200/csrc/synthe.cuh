@@ -493,8 +493,8 @@ static __global__ void k_far_inverse(double* __restrict__ inv2) {
 // longest lists (maxlist: a tile's average at the depth with the most) or an even
 // share of all entries, whichever is more; with four a quarter of the longest or
 // the share, a fifth more for the sums, and 3 us for every round of blocks.  The
-// line lies within 10 % of the quicker one on 150 forms (0.2 to 100 nm, 1 to 1M
-// lines, 16, 40 and 72 depths).
+// choice is within 10 % or 5 us of the quicker one on 150 forms (0.2 to 100 nm, 1 to
+// 1M lines, 16, 40 and 72 depths).
 inline bool far_four_warps(double entries, double maxlist, int ntiles, int nb, int nsm) {
   const double blocks = (double)ntiles * kSubs * nb, share = entries * kSubs / ((double)kFarResident * nsm);
   const double one = share > maxlist ? share : maxlist, part = share > 0.25 * maxlist ? share : 0.25 * maxlist;
